@@ -500,6 +500,15 @@ int pe_fluid_probe_fp64_rate(int32_t device, double* gops);
  * token work per phase. 2 <= phases <= 4096. */
 int pe_fluid_probe_phase_overhead(int32_t device, uint32_t phases, double* node_us, double* barrier_us);
 
+/* Compares the step's block forms of division and square root (no reference
+ * counterpart) with the IEEE operations on n operand pairs from the host:
+ * out[0] counts pairs whose num / den differs in value, out[1] those whose
+ * sqrt(den) differs, out[2] those whose num / sqrt(den) differs (a zero's sign
+ * and a NaN's payload are not compared), out[3] those that took the block form
+ * of the quotient. Operands outside the block forms' range take the IEEE
+ * operation, as in the passes. */
+int pe_fluid_probe_exact_math(int32_t device, uint64_t n, const double* num, const double* den, uint64_t out[4]);
+
 /* Library version string. */
 const char* pe_fluid_version(void);
 

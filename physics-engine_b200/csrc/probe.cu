@@ -9,11 +9,15 @@
 // of a replayed CUDA graph (the batched step's form) and as a grid-wide
 // barrier inside one cooperative persistent kernel (the alternative). The
 // barrier is this file's own, with a bounded wait that raises an error flag.
+//
+// Exact math: the passes' block forms of division and square root against the
+// IEEE operations on operands from the host.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "../../include/pe_fluid_wcsph.h"
+#include "exact_math.cuh"
 
 namespace {
 
@@ -31,6 +35,25 @@ __global__ void k_fp64_issue(double* out, uint32_t iters, double m, double c) {
 #pragma unroll
     for (int k = 0; k < kChains; ++k) s += a[k];
     if (s == 12345.678) out[0] = s;  // keeps the chains live
+}
+
+__device__ __forceinline__ bool same_value(double a, double b) { return a == b || (a != a && b != b); }
+
+__global__ void k_exact_math(uint64_t n, const double* __restrict__ num, const double* __restrict__ den,
+                             unsigned long long* out) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double a = num[i], d = den[i];
+    const bool block = pe::moderate_or_zero(a) && pe::moderate(d) && pe::divisor_ok(d);
+    const double q = block ? pe::quot_rn(a, d, pe::recip_rn(d)) : a / d;
+    double s = sqrt(d), y = 0.0;
+    if (pe::moderate(d)) y = pe::sqrt_rn(d, &s);
+    const bool root = pe::moderate_or_zero(a) && pe::moderate(d) && pe::divisor_ok(s);
+    const double qs = root ? pe::quot_rn(a, s, pe::recip_refine(s, y)) : a / s;
+    if (!same_value(q, a / d)) atomicAdd(out, 1ull);
+    if (!same_value(s, sqrt(d))) atomicAdd(out + 1, 1ull);
+    if (!same_value(qs, a / sqrt(d))) atomicAdd(out + 2, 1ull);
+    if (block) atomicAdd(out + 3, 1ull);
 }
 
 constexpr uint32_t kPhaseThreads = 256;
@@ -189,6 +212,33 @@ extern "C" int pe_fluid_probe_fp64_rate(int32_t device, double* gops) {
     if (b) cudaEventDestroy(b);
     if (st) cudaStreamDestroy(st);
     if (out) cudaFree(out);
+    cudaGetLastError();
+    return rc;
+}
+
+extern "C" int pe_fluid_probe_exact_math(int32_t device, uint64_t n, const double* num, const double* den,
+                                         uint64_t out[4]) {
+    if (!num || !den || !out) return PE_ERR_NULL;
+    if (n == 0 || n > (1ull << 28)) return PE_ERR_BOUNDS;
+    if (device >= 0 && cudaSetDevice(device) != cudaSuccess) return PE_ERR_DEVICE;
+    double *a = nullptr, *b = nullptr;
+    unsigned long long* c = nullptr;
+    int rc = PE_ERR_DEVICE;
+    if (cudaMalloc(&a, n * sizeof(double)) == cudaSuccess && cudaMalloc(&b, n * sizeof(double)) == cudaSuccess &&
+        cudaMalloc(&c, 4 * sizeof(*c)) == cudaSuccess &&
+        cudaMemcpy(a, num, n * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
+        cudaMemcpy(b, den, n * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
+        cudaMemset(c, 0, 4 * sizeof(*c)) == cudaSuccess) {
+        k_exact_math<<<(uint32_t)((n + 255u) / 256u), 256>>>(n, a, b, c);
+        unsigned long long h[4];
+        if (cudaGetLastError() == cudaSuccess && cudaMemcpy(h, c, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess) {
+            for (int k = 0; k < 4; ++k) out[k] = h[k];
+            rc = PE_OK;
+        }
+    }
+    if (a) cudaFree(a);
+    if (b) cudaFree(b);
+    if (c) cudaFree(c);
     cudaGetLastError();
     return rc;
 }

@@ -75,8 +75,7 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_density(uint32_t n, StepCon
         [&](uint32_t t, uint32_t e, const double4& xj) {
         const uint32_t j = e & kEntrySlotMask;
         const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double wij = kw<CUBIC>(r, k);
+        const double wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, k);
         if (keep_w) {
             if (t & 1u) {
                 *reinterpret_cast<double2*>(wrow + (t & 2u)) = make_double2(wprev, wij);
@@ -161,18 +160,10 @@ __global__ void k_pressure(uint32_t n, StepConst k, Tanks tk, StateBufs s) {
 // Pressure + Monaghan viscosity force of fluid pair (k, j), seen from k:
 // rx = x_j - x_k (wcsph.rs:219), pi_ij(x_k, x_j, v_k, v_j, rho_k, rho_j).
 template <bool CUBIC, bool BETA0>
-__device__ __forceinline__ void fluid_pair(const StepConst& kc, double nac, double4 xk, double4 vk,
-                                           double4 xj, double4 vj, double& ax, double& ay,
-                                           double& az) {
+__device__ __forceinline__ void fluid_pair(const StepConst& kc, bool fast, double nac, const double4& xk, const double4& vk,
+                                           const double4& xj, const double4& vj, double (&f)[3]) {
     const double rx = xj.x - xk.x, ry = xj.y - xk.y, rz = xj.z - xk.z;
     const double r2 = rx * rx + ry * ry + rz * rz;
-    const double r = sqrt(r2);
-    if (r < 1e-30) return;
-    const double dwdr = kdwdr<CUBIC>(r, kc);
-    const double sc = -dwdr / r;
-    const double gx = rx * sc, gy = ry * sc, gz = rz * sc;
-    const double press = xk.w + xj.w;  // p_k/rho_k^2 + p_j/rho_j^2
-    const double mp = -kc.mass * press;
     // viscosity.rs:51-73 with r_ij = x_k - x_j, v_ij = v_k - v_j. Evaluated for
     // every pair and selected, so that approaching and receding pairs do not
     // split the warp; a receding pair's value is discarded (pi = 0 exactly).
@@ -181,36 +172,54 @@ __device__ __forceinline__ void fluid_pair(const StepConst& kc, double nac, doub
     // up to the sign of a zero, which only ever selects pi = 0.
     const double wx = vk.x - vj.x, wy = vk.y - vj.y, wz = vk.z - vj.z;
     const double vr = -(wx * rx + wy * ry + wz * rz);
-    const double mu = kc.h * vr / (r2 + kc.eps_h2);
     const double rho_bar = 0.5 * (vk.w + vj.w);
-    // With beta = 0 the beta mu^2 term is a signed zero, which leaves the
-    // nonzero nac * mu of an approaching pair (mu < 0) unchanged.
-    const double num = BETA0 ? nac * mu : nac * mu + kc.visc_beta * mu * mu;
-    const double pic = num / rho_bar;
+    const double d2 = r2 + kc.eps_h2;
+    double sc, pic;
+    double r = 0.0, y = 0.0;
+    bool block = fast && moderate(r2) && moderate(rho_bar) && moderate_or_zero(vr);
+    if (block) {
+        y = sqrt_rn(r2, &r);
+        block = divisor_ok(r) && divisor_ok(d2) && divisor_ok(rho_bar);
+    }
+    if (block) {
+        const double dwdr = CUBIC ? dwdr_cubic_block(r, kc) : kern_dwdr(r, kc);
+        sc = quot_rn(-dwdr, r, recip_refine(r, y));
+        const double mu = quot_rn(kc.h * vr, d2, recip_rn(d2));
+        // With beta = 0 the beta mu^2 term is a signed zero, which leaves the
+        // nonzero nac * mu of an approaching pair (mu < 0) unchanged.
+        const double num = BETA0 ? nac * mu : nac * mu + kc.visc_beta * mu * mu;
+        pic = quot_rn(num, rho_bar, recip_rn(rho_bar));
+    } else {
+        r = sqrt(r2);
+        if (r < 1e-30) return;
+        sc = -kdwdr<CUBIC>(r, kc) / r;
+        const double mu = kc.h * vr / d2;
+        const double num = BETA0 ? nac * mu : nac * mu + kc.visc_beta * mu * mu;
+        pic = num / rho_bar;
+    }
+    const double gx = rx * sc, gy = ry * sc, gz = rz * sc;
+    const double press = xk.w + xj.w;  // p_k/rho_k^2 + p_j/rho_j^2
+    const double mp = -kc.mass * press;
     const double pi = vr >= 0.0 ? 0.0 : pic;
     const double mv = -kc.mass * pi;
-    ax += gx * mp + gx * mv;
-    ay += gy * mp + gy * mv;
-    az += gz * mp + gz * mv;
+    f[0] = gx * mp + gx * mv;
+    f[1] = gy * mp + gy * mv;
+    f[2] = gz * mp + gz * mv;
 }
 
 // Akinci boundary pressure of fluid k against boundary sample j (wcsph.rs:244-255).
 template <bool CUBIC>
-__device__ __forceinline__ void boundary_pair(const StepConst& kc, double4 xk, double4 xj,
-                                              bool oriented, const double4* nout, uint32_t j,
-                                              double& ax, double& ay, double& az) {
+__device__ __forceinline__ void boundary_pair(const StepConst& kc, const double4& xk, const double4& xj,
+                                              bool oriented, const double4* nout, uint32_t j, double (&f)[3]) {
     double rx = xj.x - xk.x, ry = xj.y - xk.y, rz = xj.z - xk.z;
-    double r2 = rx * rx + ry * ry + rz * rz;
-    double r = sqrt(r2);
-    if (r < 1e-30) return;
+    double sc;
+    if (!grad_scale<CUBIC>(rx * rx + ry * ry + rz * rz, kc, &sc)) return;
     if (oriented && !sees_fluid(kc, xj, nout[j], xk.x, xk.y, xk.z)) return;
-    double dwdr = kdwdr<CUBIC>(r, kc);
-    double sc = -dwdr / r;
     double gx = rx * sc, gy = ry * sc, gz = rz * sc;
     double m = -(kc.rho0 * xj.w) * xk.w;  // -(rho0 psi_j) * p_k/rho_k^2
-    ax += gx * m;
-    ay += gy * m;
-    az += gz * m;
+    f[0] = gx * m;
+    f[1] = gy * m;
+    f[2] = gz * m;
 }
 
 template <bool INTEGRATE, int DIM, bool CUBIC, bool BETA0>
@@ -224,6 +233,7 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_forces(uint32_t n, StepCons
     if (s.flags[k] & kFlagBoundary) return;
     const double c0 = tk.c[tk.slot_tank[k]];
     const double nac = -kc.visc_alpha * c0;  // (-alpha) * c_bar, viscosity.rs:72
+    const bool fast = kc.moderate && moderate_or_zero(nac);
     const double4 xk = s.pos[k];
     const double4 vk = s.vel[k];
     double ax = 0.0, ay = 0.0, az = 0.0;
@@ -237,7 +247,11 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_forces(uint32_t n, StepCons
     };
     // fluid i < k, ascending original index
     for_each_loaded(list_ref(l, k, kListLower), load, [&](uint32_t, const PosVel& d) {
-        fluid_pair<CUBIC, BETA0>(kc, nac, xk, vk, d.x, d.v, ax, ay, az);
+        double f[3] = {0.0, 0.0, 0.0};
+        fluid_pair<CUBIC, BETA0>(kc, fast, nac, xk, vk, d.x, d.v, f);
+        ax += f[0];
+        ay += f[1];
+        az += f[2];
     });
     // fluid j > k and boundary j, visiting order: the visit list without the
     // entries flagged lower (those came from the lower list, in index order).
@@ -277,11 +291,15 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_forces(uint32_t n, StepCons
                 e = s_keep[(u + 1) * bd + tid];
                 d = load(e);
             }
+            double f[3] = {0.0, 0.0, 0.0};
             if (ec & kEntryBoundary) {
-                boundary_pair<CUBIC>(kc, xk, dc.x, (ec & kEntryOriented) != 0u, s.nout, ec & kEntrySlotMask, ax, ay, az);
+                boundary_pair<CUBIC>(kc, xk, dc.x, (ec & kEntryOriented) != 0u, s.nout, ec & kEntrySlotMask, f);
             } else {
-                fluid_pair<CUBIC, BETA0>(kc, nac, xk, vk, dc.x, dc.v, ax, ay, az);
+                fluid_pair<CUBIC, BETA0>(kc, fast, nac, xk, vk, dc.x, dc.v, f);
             }
+            ax += f[0];
+            ay += f[1];
+            az += f[2];
         }
     }
     ax += kc.gx;
@@ -324,12 +342,9 @@ __global__ void __launch_bounds__(kThreads) k_boundary_force(uint32_t n, StepCon
     for_each_entry(list_ref(l, b, kListLower), [&](uint32_t i) {
         double4 xi = s.pos[i];
         double rx = xb.x - xi.x, ry = xb.y - xi.y, rz = xb.z - xi.z;
-        double r2 = rx * rx + ry * ry + rz * rz;
-        double r = sqrt(r2);
-        if (r < 1e-30) return;
+        double sc;
+        if (!grad_scale<CUBIC>(rx * rx + ry * ry + rz * rz, kc, &sc)) return;
         if (oriented && !sees_fluid(kc, xb, nb, xi.x, xi.y, xi.z)) return;
-        double dwdr = kdwdr<CUBIC>(r, kc);
-        double sc = -dwdr / r;
         double m = mpsi * xi.w;
         double ffx = (rx * sc) * m, ffy = (ry * sc) * m, ffz = (rz * sc) * m;
         fx += ffx * mneg;
@@ -360,11 +375,10 @@ __device__ __forceinline__ double3 xsph_dv(uint32_t i, const StepConst& kc, cons
         if (e & kEntryBoundary) return;
         const double4 xj = d.x;
         const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double wij = kw<CUBIC>(r, kc);
+        const double wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, kc);
         const double4 vj = d.v;
         const double rho_bar = 0.5 * (vi.w + vj.w);
-        const double f = kc.mass / rho_bar * wij;
+        const double f = mass_over(rho_bar, kc) * wij;
         dvx += (vj.x - vi.x) * f;
         dvy += (vj.y - vi.y) * f;
         dvz += (vj.z - vi.z) * f;
@@ -439,7 +453,7 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_xsph_w(uint32_t n, StepCons
         if (e & kEntryBoundary) return;
         const double4 vj = d.v;
         const double rho_bar = 0.5 * (vi.w + vj.w);
-        const double f = kc.mass / rho_bar * d.w;
+        const double f = mass_over(rho_bar, kc) * d.w;
         dvx += (vj.x - vi.x) * f;
         dvy += (vj.y - vi.y) * f;
         dvz += (vj.z - vi.z) * f;

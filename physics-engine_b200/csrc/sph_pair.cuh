@@ -3,6 +3,7 @@
 // --fmad=false like every f64 pass.
 #pragma once
 
+#include "exact_math.cuh"
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
 
@@ -108,6 +109,63 @@ __device__ __forceinline__ double kdwdr(double r, const StepConst& k) {
 // r inside the kernel's support (kernels.rs:32)
 __device__ __forceinline__ bool in_support(double r, const StepConst& k) {
     return k.kernel <= 1 ? div_h(r, k) < 2.0 : r < k.h;
+}
+
+// ---- the same in one block, for pairs whose operands are moderate
+// (exact_math.cuh) and constants for which StepConst::moderate holds ----
+__device__ __forceinline__ double div_h_block(double a, const StepConst& k) {
+    const double q0 = a * k.inv_h;
+    return fma(fma(-q0, k.h, a), k.inv_h, q0);
+}
+
+__device__ __forceinline__ double w_cubic_block(double r, const StepConst& k) {
+    const double q = div_h_block(r, k), t = 2.0 - q;
+    const double in = k.alpha * (1.0 - 1.5 * q * q + 0.75 * q * q * q);
+    const double out = k.alpha * 0.25 * t * t * t;
+    return q < 1.0 ? in : q < 2.0 ? out : 0.0;
+}
+
+__device__ __forceinline__ double dwdr_cubic_block(double r, const StepConst& k) {
+    const double q = div_h_block(r, k), t = 2.0 - q;
+    const double in = k.alpha * (-3.0 * q + 2.25 * q * q);
+    const double out = k.alpha * (-0.75 * t * t);
+    const double d = div_h_block(q < 1.0 ? in : out, k);
+    return q < 2.0 ? d : 0.0;
+}
+
+// W(|x|) with r2 = |x|^2
+template <bool CUBIC>
+__device__ __forceinline__ double w_of_r2(double r2, const StepConst& k) {
+    if (k.moderate && moderate(r2)) {
+        double r;
+        sqrt_rn(r2, &r);
+        return CUBIC ? w_cubic_block(r, k) : kern_w(r, k);
+    }
+    return kw<CUBIC>(sqrt(r2), k);
+}
+
+// m / rho_bar
+__device__ __forceinline__ double mass_over(double rho_bar, const StepConst& k) {
+    if (k.moderate && moderate(rho_bar) && divisor_ok(rho_bar)) return quot_rn(k.mass, rho_bar, recip_rn(rho_bar));
+    return k.mass / rho_bar;
+}
+
+// -dW/dr / r with r = sqrt(r2); returns false for coincident points (r < 1e-30)
+template <bool CUBIC>
+__device__ __forceinline__ bool grad_scale(double r2, const StepConst& k, double* sc) {
+    if (k.moderate && moderate(r2)) {
+        double r;
+        const double y = sqrt_rn(r2, &r);
+        if (divisor_ok(r)) {
+            const double n = CUBIC ? dwdr_cubic_block(r, k) : kern_dwdr(r, k);
+            *sc = quot_rn(-n, r, recip_refine(r, y));
+            return true;
+        }
+    }
+    const double r = sqrt(r2);
+    if (r < 1e-30) return false;
+    *sc = -kdwdr<CUBIC>(r, k) / r;
+    return true;
 }
 
 // particles.rs:126 boundary_sees_fluid

@@ -87,6 +87,7 @@ struct StepConst {
     double xsph_eps;
     double boundary_eps_h;     // 0.15 * h (particles.rs:132)
     int adapt_sound_speed;
+    int moderate;              // h, eps_h2 and visc_beta are in the range of the block forms (exact_math.cuh)
     float r2_filter;           // conservative single-precision (2h)^2 bound
     // List-build modes of the sibling solvers: visit lists keep every
     // boundary candidate whatever its distance; lower lists are built for

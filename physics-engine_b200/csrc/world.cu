@@ -540,6 +540,9 @@ void World::refresh_step_const() {
     k.xsph_eps = prm_.xsph_epsilon;
     k.boundary_eps_h = 0.15 * h_;  // particles.rs:132
     k.adapt_sound_speed = prm_.adapt_sound_speed;
+    const auto moderate = [](double a) { return a > 0x1p-60 && a < 0x1p60; };
+    k.moderate = moderate(h_) && moderate(mass_) && (k.eps_h2 == 0.0 || moderate(k.eps_h2)) &&
+                 (k.visc_beta == 0.0 || moderate(std::fabs(k.visc_beta)));
     double sup = support_;
     k.r2_filter = list_all_candidates_
                       ? std::numeric_limits<float>::infinity()
