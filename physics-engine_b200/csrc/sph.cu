@@ -48,8 +48,15 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
+// Bound by the L1's data path (76 % of its wavefronts with two 16-byte loads a
+// gathered position, one 4-byte load an entry and a 16-byte store every other
+// W), then by fixed latencies. Rows of four entries are read, and their W
+// stored, in one access each, and a position is one 32-byte load: 1410 ->
+// 1105 us at 1M (the FP64 issue alone would take ~0.5 ms). Held to 80
+// registers (six CTAs of 128 threads an SM) with the data one entry ahead;
+// two ahead takes 95 registers and 1125 us, 64 registers spill and take 1527.
 template <bool CUBIC>
-__global__ void __launch_bounds__(kMaxPassThreads) k_density(uint32_t n, StepConst k, StateBufs s,
+__global__ void __launch_bounds__(kMaxPassThreads, 3) k_density(uint32_t n, StepConst k, StateBufs s,
                                                       ListBufs l) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -60,37 +67,33 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_density(uint32_t n, StepCon
     const double4 xi = s.pos[i];
     double rho = k.rho_self;  // 0.0 + mass * W(0)
     const ListRef vr = list_ref(l, i, kListVisit);
-    // W of entry t kept at the entry's pool index for the XSPH pass, two
-    // entries per 16-byte store (a whole sector over a group's four entries);
-    // wrow walks the slot's rows of 16-byte groups
+    // W of entry t kept at the entry's pool index for the XSPH pass, a row of
+    // four in one 32-byte store; wrow walks the slot's rows
     bool keep_w = false;
     if (l.wpair) {
         keep_w = w_fits(l, vr);
         if (!keep_w) atomicOr(l.w_short, 1u);
     }
     double* wrow = keep_w ? l.wpair + (vr.p - l.pool) : nullptr;
-    double wprev = 0.0;
-    for_each_loaded2_t(
-        vr, [&](uint32_t, uint32_t e) { return s.pos[e & kEntrySlotMask]; },
-        [&](uint32_t t, uint32_t e, const double4& xj) {
-        const uint32_t j = e & kEntrySlotMask;
-        const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const double wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, k);
-        if (keep_w) {
-            if (t & 1u) {
-                *reinterpret_cast<double2*>(wrow + (t & 2u)) = make_double2(wprev, wij);
-                if (t & 2u) wrow += vr.step;
-            } else {
-                wprev = wij;
+    double w4[4] = {0.0, 0.0, 0.0, 0.0};
+    for_each_row<1>(
+        vr, [&](uint32_t e) { return gather4(s.pos + (e & kEntrySlotMask)); }, [](uint32_t) {},
+        [&](uint32_t q, uint32_t e, const double4& xj) {
+            const uint32_t j = e & kEntrySlotMask;
+            const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+            const double wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, k);
+            w4[q] = wij;
+            if ((e & kEntryOriented) && !sees_fluid(k, xj, s.nout[j], xi.x, xi.y, xi.z)) return;
+            // fluid: mass * W; boundary: (rho0 * psi_j) * W (wcsph.rs:143-148)
+            const double f = (e & kEntryBoundary) ? k.rho0 * xj.w : k.mass;
+            rho += f * wij;
+        },
+        [&](uint32_t) {
+            if (keep_w) {
+                store4(wrow, w4);
+                wrow += vr.step;
             }
-        }
-        if ((e & kEntryOriented) && !sees_fluid(k, xj, s.nout[j], xi.x, xi.y, xi.z)) return;
-        // fluid: mass * W; boundary: (rho0 * psi_j) * W (wcsph.rs:143-148)
-        const double f = (e & kEntryBoundary) ? k.rho0 * xj.w : k.mass;
-        rho += f * wij;
-    });
-    if (keep_w && (vr.n & 1u))  // the last entry's W, unpaired
-        *reinterpret_cast<double2*>(wrow + ((vr.n - 1u) & 2u)) = make_double2(wprev, 0.0);
+        });
     rho = fmax(rho, 1e-12);  // wcsph.rs:152 (f64::max)
     s.vel[i].w = rho;
     // keep the cached p / rho^2 consistent with the new rho (the reference
@@ -241,8 +244,8 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_forces(uint32_t n, StepCons
     auto load = [&](uint32_t e) {
         PosVel d;
         const uint32_t j = e & kEntrySlotMask;
-        d.x = s.pos[j];
-        d.v = (e & kEntryBoundary) ? make_double4(0.0, 0.0, 0.0, 0.0) : s.vel[j];
+        d.x = gather4(s.pos + j);
+        d.v = gather4(s.vel + j);
         return d;
     };
     // fluid i < k, ascending original index
@@ -366,8 +369,8 @@ __device__ __forceinline__ double3 xsph_dv(uint32_t i, const StepConst& kc, cons
         [&](uint32_t e) {
             PosVel d{};
             if (!(e & kEntryBoundary)) {
-                d.x = s.pos[e & kEntrySlotMask];
-                d.v = s.vel[e & kEntrySlotMask];
+                d.x = gather4(s.pos + (e & kEntrySlotMask));
+                d.v = gather4(s.vel + (e & kEntrySlotMask));
             }
             return d;
         },
@@ -407,13 +410,16 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_xsph(uint32_t n, StepConst 
 
 // k_xsph with each pair's W(r) read from the density pass of the same lists
 // and positions (the bits the pair would compute) instead of recomputed from
-// the neighbour's position: per fluid pair one 8-byte read of a stream in
-// place of a 32-byte gather, a square root and the kernel polynomial
-// (XSPH 2.04 -> 1.44 ms at 1M, density 1.16 -> 1.43 ms for the stores).
+// the neighbour's position: per fluid pair a quarter of one 32-byte read of a
+// stream in place of a 32-byte gather, a square root and the kernel
+// polynomial. Bound by the L1's data path like k_density; with rows of four
+// entries and weights read in one access each, 32-byte gathers and the block
+// form of m / rho_bar, 1412 -> 958 us at 1M (80 registers, one velocity ahead;
+// 87 without the register limit 1016 us, two ahead 1270 us).
 // When the density pass met a list beyond the buffer, it does nothing and
 // the k_xsph launch after it recomputes W for every particle (a separate
 // kernel, so that this one keeps its own, smaller register count).
-__global__ void __launch_bounds__(kMaxPassThreads) k_xsph_w(uint32_t n, StepConst kc, StateBufs s,
+__global__ void __launch_bounds__(kMaxPassThreads, 3) k_xsph_w(uint32_t n, StepConst kc, StateBufs s,
                                                      ListBufs l, double4* __restrict__ vel_out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -430,34 +436,28 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_xsph_w(uint32_t n, StepCons
     // are prefetched into L1 (within the slot's own rows): 1.44 -> 1.40 ms at 1M.
     constexpr uint32_t kPfRows = 4;
     const uint32_t nrows = (vr.n + 3u) >> 2;
-    struct VelW {
-        double4 v;
-        double w;
-    };
-    for_each_loaded2_t(
-        vr,
-        [&](uint32_t t, uint32_t e) {  // called for t = 0, 1, 2, ... in order
-            if ((t & 3u) == 0u && (t >> 2) + kPfRows < nrows) {
-                prefetch_l1(vr.p + (size_t)((t >> 2) + kPfRows) * vr.step);
+    const uint32_t* erow = vr.p;
+    double w4[4];
+    for_each_row<1>(
+        vr, [&](uint32_t e) { return gather4(s.vel + (e & kEntrySlotMask)); },
+        [&](uint32_t row) {
+            load4(wrow, w4);
+            if (row + kPfRows < nrows) {
+                prefetch_l1(erow + (size_t)kPfRows * vr.step);
                 prefetch_l1(wrow + (size_t)kPfRows * vr.step);
             }
-            VelW d{};
-            if (!(e & kEntryBoundary)) {
-                d.v = s.vel[e & kEntrySlotMask];
-                d.w = __ldg(wrow + (t & 3u));
-            }
-            if ((t & 3u) == 3u) wrow += vr.step;
-            return d;
+            erow += vr.step;
+            wrow += vr.step;
         },
-        [&](uint32_t, uint32_t e, const VelW& d) {
-        if (e & kEntryBoundary) return;
-        const double4 vj = d.v;
-        const double rho_bar = 0.5 * (vi.w + vj.w);
-        const double f = mass_over(rho_bar, kc) * d.w;
-        dvx += (vj.x - vi.x) * f;
-        dvy += (vj.y - vi.y) * f;
-        dvz += (vj.z - vi.z) * f;
-    });
+        [&](uint32_t q, uint32_t e, const double4& vj) {
+            if (e & kEntryBoundary) return;
+            const double rho_bar = 0.5 * (vi.w + vj.w);
+            const double f = mass_over(rho_bar, kc) * w4[q];
+            dvx += (vj.x - vi.x) * f;
+            dvy += (vj.y - vi.y) * f;
+            dvz += (vj.z - vi.z) * f;
+        },
+        [](uint32_t) {});
     vel_out[i] = make_double4(vi.x + dvx * kc.xsph_eps, vi.y + dvy * kc.xsph_eps,
                               vi.z + dvz * kc.xsph_eps, vi.w);
 }
