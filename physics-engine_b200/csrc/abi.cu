@@ -560,6 +560,14 @@ int pe_fluid_wcsph_autotune(PeWcsph* w, uint32_t out[4]) {
     });
 }
 
+int pe_fluid_wcsph_set_lanes(PeWcsph* w, uint32_t lanes) {
+    if (!w) return PE_ERR_NULL;
+    return guard([&] {
+        w->world->set_lanes(lanes);
+        return PE_OK;
+    });
+}
+
 int pe_fluid_wcsph_shapes(PeWcsph* w, uint32_t out[4]) {
     if (!w || !out) return PE_ERR_NULL;
     const pe::World::Shapes r = w->world->shapes();

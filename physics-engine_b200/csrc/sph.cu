@@ -21,10 +21,14 @@
 // over the visiting-order list, skipping entries flagged lower, therefore
 // yields the reference's bits. Pairs outside the support contribute +-0,
 // which leaves a sum that started at +0 unchanged, so the lists may omit them.
+#include <algorithm>
+#include <type_traits>
+
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
 #include "sph_pair.cuh"
 #include "list_iter.cuh"
+#include "lane_group.cuh"
 
 namespace pe {
 
@@ -462,6 +466,300 @@ __global__ void __launch_bounds__(kMaxPassThreads, 3) k_xsph_w(uint32_t n, StepC
                               vi.z + dvz * kc.xsph_eps, vi.w);
 }
 
+// ---------------------------------------------------------------------------
+// The same passes with G lanes on each slot (lane_group.cuh).
+// ---------------------------------------------------------------------------
+template <bool CUBIC, int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_density_g(uint32_t n, StepConst k, StateBufs s, ListBufs l) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) s.vel[i].w = k.rho0;  // wcsph.rs:127
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef vr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    bool keep_w = false;
+    if (fluid) {
+        vr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        if (l.wpair) {
+            keep_w = w_fits(l, vr);
+            if (!keep_w && g.sub == 0) atomicOr(l.w_short, 1u);
+        }
+    }
+    // W of entry t kept at the entry's pool index: the lanes of a row store 32
+    // contiguous bytes
+    OrderedSum<G, 1> rho(s_words + g.warp * OrderedSum<G, 1>::kDoubles, g, k.rho_self);  // 0.0 + mass * W(0)
+    group_for_each<G>(
+        vr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t* p) {
+            double term[1] = {0.0};
+            if (has) {
+                const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+                const double wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, k);
+                if (keep_w) l.wpair[p - l.pool] = wij;
+                if (!((e & kEntryOriented) && !sees_fluid(k, xj, s.nout[e & kEntrySlotMask], xi.x, xi.y, xi.z))) {
+                    // fluid: mass * W; boundary: (rho0 * psi_j) * W (wcsph.rs:143-148)
+                    const double f = (e & kEntryBoundary) ? k.rho0 * xj.w : k.mass;
+                    term[0] = f * wij;
+                }
+            }
+            rho.add(term);
+        });
+    if (fluid && g.sub == 0) {
+        const double r = fmax(rho.acc, 1e-12);  // wcsph.rs:152 (f64::max)
+        s.vel[i].w = r;
+        s.pos[i].w = s.p[i] / (r * r);  // see k_density
+    }
+}
+
+// Entries of one slot queued in shared memory for the force pass (per group;
+// the padding spreads the groups of a warp over the banks).
+template <int G>
+struct ForceQueue {
+    static constexpr uint32_t kFill = 4u * G;  // entries a fill step takes from a list
+    static constexpr uint32_t kCap = G == 32 ? 256u : 128u;
+    static constexpr uint32_t kPitch = kCap + (G == 4 ? 4u : G == 8 ? 8u : 0u);
+    static constexpr uint32_t kWarpBytes = LaneGroup<G>::kPerWarp * kPitch * sizeof(uint32_t);
+};
+
+constexpr uint32_t kForceGroupThreads = 128;
+
+template <int G>
+constexpr size_t forces_smem(uint32_t threads) {
+    return (size_t)(threads / 32u) * (OrderedSum<G, 3>::kDoubles * sizeof(double) + ForceQueue<G>::kWarpBytes);
+}
+
+__device__ __forceinline__ double comp(const double4* a, uint32_t i, uint32_t c) {
+    return reinterpret_cast<const double*>(a + i)[c];
+}
+
+// The force pass with G lanes a slot. Five CTAs of 128 threads an SM (96
+// registers; without the limit 110 registers, four CTAs and 2750 us at 1M
+// against 2510). One stream of pairs per group: the lower list, then the visit entries not
+// flagged lower, queued in order in shared memory and taken G at a time. A
+// slot's two parts add up to its visit list, so the groups of a warp run
+// equally long, where loops over the lower and the kept entries of 32 slots
+// leave a quarter of the lanes idle.
+template <bool CUBIC, bool BETA0, int G>
+__global__ void __launch_bounds__(kForceGroupThreads, 5) k_forces_g(uint32_t n, StepConst kc, Tanks tk, StateBufs s,
+                                                              ListBufs l, int integrate, double dt,
+                                                              double4* __restrict__ pos_next,
+                                                              double4* __restrict__ vel_next,
+                                                              const double4* __restrict__ st_a) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t k = g.slot;
+    const bool fluid = k < n && !(s.flags[k] & kFlagBoundary);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    using Q = ForceQueue<G>;
+    const uint32_t warps = blockDim.x >> 5;
+    uint32_t* const queue = reinterpret_cast<uint32_t*>(s_words + warps * OrderedSum<G, 3>::kDoubles) +
+                            (g.warp * LaneGroup<G>::kPerWarp + g.grp) * Q::kPitch;
+    ListRef vr{l.pool, 0u, 0u}, lr{l.pool, 0u, 0u};
+    double4 xk = make_double4(0.0, 0.0, 0.0, 0.0), vk = xk;
+    double nac = 0.0;
+    bool fast = false;
+    if (fluid) {
+        vr = list_ref(l, k, kListVisit);
+        lr = list_ref(l, k, kListLower);
+        xk = s.pos[k];
+        vk = s.vel[k];
+        nac = -kc.visc_alpha * tk.c[tk.slot_tank[k]];  // (-alpha) * c_bar, viscosity.rs:72
+        fast = kc.moderate && moderate_or_zero(nac);
+    }
+    OrderedSum<G, 3> acc(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    // fill step f takes rows f * G + sub of the lower list, then of the visit list
+    const uint32_t lower_steps = warp_rounds(lr.n, Q::kFill), steps = lower_steps + warp_rounds(vr.n, Q::kFill);
+    uint32_t step = 0, tail = 0;
+    bool last;
+    do {
+        for (; step < steps && !__any_sync(kFullWarp, tail + Q::kFill > Q::kCap); ++step) {
+            const bool low = step < lower_steps;
+            const ListRef& r = low ? lr : vr;
+            const uint32_t row = (low ? step : step - lower_steps) * G + g.sub;
+            const uint32_t left = 4u * row < r.n ? r.n - 4u * row : 0u;  // entries from this row on
+            uint4 e4 = make_uint4(0u, 0u, 0u, 0u);
+            if (left) e4 = __ldg(reinterpret_cast<const uint4*>(r.p + (size_t)row * r.step));
+            const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+            uint32_t keep = left >= 4u ? 15u : (1u << left) - 1u;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                if (!low && (e[q] & kEntryLower)) keep &= ~(1u << q);
+            const uint32_t c = __popc(keep);
+            uint32_t incl = c;  // over the group's lanes
+#pragma unroll
+            for (uint32_t o = 1; o < G; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(kFullWarp, incl, o, G);
+                if (g.sub >= o) incl += v;
+            }
+            uint32_t at = tail + incl - c;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                if (keep & (1u << q)) queue[at++] = e[q];
+            tail += __shfl_sync(kFullWarp, incl, G - 1, G);
+        }
+        __syncwarp();
+        last = step >= steps;
+        const uint32_t queued = last ? (tail + G - 1u) / G : tail / G;
+        const uint32_t end = last ? tail : queued * G;
+        const uint32_t rounds = __reduce_max_sync(kFullWarp, queued);
+        uint32_t q = g.sub;
+        auto entry = [&]() { return end ? queue[min(q, end - 1u)] : 0u; };  // a lane past the end repeats the last
+        auto load = [&](uint32_t e) {
+            const uint32_t j = e & kEntrySlotMask;
+            return PosVel{gather4(s.pos + j), gather4(s.vel + j)};
+        };
+        uint32_t e0 = entry();
+        bool h0 = q < end;
+        PosVel d0 = load(e0);
+        q += G;
+        uint32_t e1 = entry();
+        bool h1 = q < end;
+        for (uint32_t u = 0; u < rounds; ++u) {
+            const uint32_t e = e0;
+            const bool h = h0;
+            const PosVel d = d0;
+            e0 = e1;
+            h0 = h1;
+            d0 = load(e0);
+            q += G;
+            e1 = entry();
+            h1 = q < end;
+            double f[3] = {0.0, 0.0, 0.0};
+            if (h) {
+                if (e & kEntryBoundary) {
+                    boundary_pair<CUBIC>(kc, xk, d.x, (e & kEntryOriented) != 0u, s.nout, e & kEntrySlotMask, f);
+                } else {
+                    fluid_pair<CUBIC, BETA0>(kc, fast, nac, xk, vk, d.x, d.v, f);
+                }
+            }
+            acc.add(f);
+        }
+        if (!last) {  // fewer than G queued entries carry over
+            const uint32_t left = tail - queued * G;
+            const uint32_t c = g.sub < left ? queue[queued * G + g.sub] : 0u;
+            __syncwarp();
+            if (g.sub < left) queue[g.sub] = c;
+            tail = left;
+            __syncwarp();
+        }
+    } while (!last);
+    // Lane c < 4 finishes component c (w: the carried psi or p / rho^2, and rho).
+    if (!fluid || g.sub >= 4u) return;
+    double a = 0.0;
+    if (g.sub < 3u) {
+        a = acc.acc + (g.sub == 0 ? kc.gx : g.sub == 1 ? kc.gy : kc.gz);
+        if (st_a) a += comp(st_a, k, g.sub);  // wcsph.rs:273-277 a += surface-tension acceleration
+    }
+    reinterpret_cast<double*>(s.acc + k)[g.sub] = a;
+    if (integrate) {
+        // wcsph.rs:336-341 symplectic Euler
+        double v = comp(s.vel, k, g.sub), x = comp(s.pos, k, g.sub);
+        if (g.sub < 3u) {
+            v = v + a * dt;
+            x = x + v * dt;
+            if (kc.dim == 2 && g.sub == 2u) v = x = 0.0;
+        }
+        reinterpret_cast<double*>(pos_next + k)[g.sub] = x;
+        reinterpret_cast<double*>(vel_next + k)[g.sub] = v;
+    }
+}
+
+template <bool CUBIC, int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_boundary_force_g(uint32_t n, StepConst kc, StateBufs s,
+                                                                      ListBufs l) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t b = g.slot;
+    const bool bound = b < n && (s.flags[b] & kFlagBoundary);
+    if (!__any_sync(kFullWarp, bound)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xb = make_double4(0.0, 0.0, 0.0, 0.0), nb = xb;
+    bool oriented = false;
+    if (bound) {
+        lr = list_ref(l, b, kListLower);
+        xb = s.pos[b];
+        oriented = (s.flags[b] & kFlagOriented) != 0;
+        if (oriented) nb = s.nout[b];
+    }
+    const double mpsi = -(kc.rho0 * xb.w);
+    const double mneg = -kc.mass;
+    OrderedSum<G, 3> acc(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    group_for_each<G>(
+        lr, g, [&](uint32_t i, const uint32_t*) { return gather4(s.pos + i); },
+        [&](bool has, uint32_t, const double4& xi, const uint32_t*) {
+            double f[3] = {0.0, 0.0, 0.0};
+            const double rx = xb.x - xi.x, ry = xb.y - xi.y, rz = xb.z - xi.z;
+            double sc;
+            if (has && grad_scale<CUBIC>(rx * rx + ry * ry + rz * rz, kc, &sc) &&
+                !(oriented && !sees_fluid(kc, xb, nb, xi.x, xi.y, xi.z))) {
+                const double m = mpsi * xi.w;
+                f[0] = ((rx * sc) * m) * mneg;
+                f[1] = ((ry * sc) * m) * mneg;
+                f[2] = ((rz * sc) * m) * mneg;
+            }
+            acc.add(f);
+        });
+    if (bound && g.sub < 4u) reinterpret_cast<double*>(s.bf + b)[g.sub] = g.sub < 3u ? acc.acc : 0.0;
+}
+
+// USE_W: each pair's W(r) read from the density pass of the same lists and
+// positions (see k_xsph_w); otherwise recomputed. short_only as in k_xsph.
+template <bool CUBIC, bool USE_W, int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_xsph_g(uint32_t n, StepConst kc, StateBufs s, ListBufs l,
+                                                            double4* __restrict__ vel_out, bool short_only) {
+    extern __shared__ __align__(16) double s_words[];
+    if (USE_W ? __ldg(l.w_short) != 0u : short_only && !__ldg(l.w_short)) return;
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    double4 vi = make_double4(0.0, 0.0, 0.0, 0.0), xi = vi;
+    if (i < n && !fluid && g.sub == 0) vel_out[i] = s.vel[i];
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef vr{l.pool, 0u, 0u};
+    if (fluid) {
+        vr = list_ref(l, i, kListVisit);
+        vi = s.vel[i];
+        if (!USE_W) xi = s.pos[i];
+    }
+    struct VelW {
+        double4 v, x;
+        double w;
+    };
+    OrderedSum<G, 3> dv(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    group_for_each<G>(
+        vr, g,
+        [&](uint32_t e, const uint32_t* p) {
+            VelW d{};
+            d.v = gather4(s.vel + (e & kEntrySlotMask));
+            if (USE_W) d.w = __ldg(l.wpair + (p - l.pool));
+            else d.x = gather4(s.pos + (e & kEntrySlotMask));
+            return d;
+        },
+        [&](bool has, uint32_t e, const VelW& d, const uint32_t*) {
+            double f[3] = {0.0, 0.0, 0.0};
+            if (has && !(e & kEntryBoundary)) {
+                double wij = d.w;
+                if (!USE_W) {
+                    const double dx = d.x.x - xi.x, dy = d.x.y - xi.y, dz = d.x.z - xi.z;
+                    wij = w_of_r2<CUBIC>(dx * dx + dy * dy + dz * dz, kc);
+                }
+                const double rho_bar = 0.5 * (vi.w + d.v.w);
+                const double m = mass_over(rho_bar, kc) * wij;
+                f[0] = (d.v.x - vi.x) * m;
+                f[1] = (d.v.y - vi.y) * m;
+                f[2] = (d.v.z - vi.z) * m;
+            }
+            dv.add(f);
+        });
+    if (fluid && g.sub < 4u) {
+        const double v = comp(s.vel, i, g.sub);
+        reinterpret_cast<double*>(vel_out + i)[g.sub] = g.sub < 3u ? v + dv.acc * kc.xsph_eps : v;
+    }
+}
+
 __global__ void k_in_support(uint32_t n, StepConst kc, StateBufs s, ListBufs l, uint32_t* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -498,18 +796,86 @@ void allow_compact_smem_all() {
 
 // The force pass's compaction buffer exceeds the 48 KB a launch gets without
 // opting in once a CTA has more than 192 threads.
+template <int G>
+void allow_forces_smem() {
+    auto allow = [](auto* f) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)forces_smem<G>(kForceGroupThreads));
+    };
+    allow(k_forces_g<true, true, G>);
+    allow(k_forces_g<true, false, G>);
+    allow(k_forces_g<false, true, G>);
+    allow(k_forces_g<false, false, G>);
+}
+
 void forces_prepare() {
     allow_compact_smem_all<true, 3>();
     allow_compact_smem_all<false, 3>();
     allow_compact_smem_all<true, 2>();
     allow_compact_smem_all<false, 2>();
+    allow_forces_smem<4>();
+    allow_forces_smem<8>();
+    allow_forces_smem<16>();
+    allow_forces_smem<32>();
 }
 
-void launch_density(uint32_t n, uint32_t threads, const StepConst& k, const StateBufs& s,
+// Lanes per slot of each pass, from the slots that have work and the pairs
+// each has (~250 in 3-D, ~50 in 2-D). More lanes shorten a slot's serial chain;
+// fewer waste less on the exchange of terms once the slots alone fill the SMs.
+// us a pass, 1 / 4 / 8 / 16 / 32 lanes, dam-break tanks of side^3 fluid:
+//            13^3                  32^3                    64^3                     80^3
+//   density  83/31/19/15/14.5      98/72/59/63/75          331/389/386/442/548      579/732/736/858/1065
+//   forces   187/53/35/24/19       228/129/118/121/141     767/707/773/849/1033     1344/1319/1468/1642/1998
+//   XSPH     70/32/25/19/20        96/92/71/82/110         301/430/446/519/782      507/793/841/1003/1507
+//   boundary 46/23/15/12/11        51/28/20/17/21          64/46/44/58/95           74/63/67/97/165
+// and of side^2: 40,000 particles density 24/20/20/25/37, forces 41/31/33/40/64;
+// 160,000 density 49/52/60/82/135, forces 86/94/113/148/256.
+PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t boundary) {
+    struct Limits {
+        uint64_t l32, l16, l8, l4;  // the most slots each lane count is taken for
+    };
+    auto pick = [](uint64_t n, const Limits& m) -> uint32_t {
+        return n <= m.l32 ? 32u : n <= m.l16 ? 16u : n <= m.l8 ? 8u : n <= m.l4 ? 4u : 1u;
+    };
+    PassLanes r;
+    const bool d3 = dim == 3;
+    r.density = pick(fluid, d3 ? Limits{3000, 10000, 190000, 190000} : Limits{600, 10000, 40000, 100000});
+    r.forces = pick(fluid, d3 ? Limits{8000, 20000, 40000, 700000} : Limits{1000, 3000, 12000, 80000});
+    r.xsph = pick(fluid, d3 ? Limits{1500, 10000, 45000, 45000} : Limits{1000, 3000, 12000, 25000});
+    r.boundary = pick(boundary, d3 ? Limits{10000, 25000, 100000, 1000000} : Limits{10000, 10000, 100000, 1000000});
+    return r;
+}
+
+// Calls f(integral_constant<int, G>) for the lanes per slot.
+template <class F>
+static void with_lanes(uint32_t lanes, F&& f) {
+    switch (lanes) {
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 16: f(std::integral_constant<int, 16>{}); break;
+        default: f(std::integral_constant<int, 32>{}); break;
+    }
+}
+
+template <int G, int K>
+static size_t sum_smem(uint32_t threads) {
+    return (size_t)(threads / 32u) * OrderedSum<G, K>::kDoubles * sizeof(double);
+}
+
+void launch_density(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const StateBufs& s,
                     const ListBufs& l, cudaStream_t st) {
     if (!n) return;
-    if (k.kernel == 0) k_density<true><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l);
-    else k_density<false><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l);
+    if (lanes == 1) {
+        if (k.kernel == 0) k_density<true><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l);
+        else k_density<false><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l);
+        return;
+    }
+    with_lanes(lanes, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        const uint32_t b = blocks_for((uint64_t)n * G, threads);
+        const size_t sm = sum_smem<G, 1>(threads);
+        if (k.kernel == 0) k_density_g<true, G><<<b, threads, sm, st>>>(n, k, s, l);
+        else k_density_g<false, G><<<b, threads, sm, st>>>(n, k, s, l);
+    });
 }
 
 void launch_vmax(uint32_t n, const Tanks& tk, const StateBufs& s, cudaStream_t st) {
@@ -521,13 +887,32 @@ void launch_pressure(uint32_t n, const StepConst& k, const Tanks& tk, const Stat
     if (n) k_pressure<<<blocks_for(n, 256), 256, 0, st>>>(n, k, tk, s);
 }
 
-void launch_forces(uint32_t n, uint32_t threads, const StepConst& k, const Tanks& tk,
+void launch_forces(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const Tanks& tk,
                    const StateBufs& s, const ListBufs& l, bool integrate, double dt,
                    double4* pos_next, double4* vel_next, const double4* st_a, cudaStream_t st) {
     if (!n) return;
+    const bool cubic = k.kernel == 0;
+    const bool beta0 = k.visc_beta == 0.0;
+    if (lanes != 1) {
+        with_lanes(lanes, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            const uint32_t t = std::min(threads, kForceGroupThreads), b = blocks_for((uint64_t)n * G, t);
+            const size_t sm = forces_smem<G>(t);
+            auto go = [&](auto* f) {
+                f<<<b, t, sm, st>>>(n, k, tk, s, l, integrate ? 1 : 0, dt, pos_next, vel_next, st_a);
+            };
+            if (cubic) {
+                if (beta0) go(k_forces_g<true, true, G>);
+                else go(k_forces_g<true, false, G>);
+            } else {
+                if (beta0) go(k_forces_g<false, true, G>);
+                else go(k_forces_g<false, false, G>);
+            }
+        });
+        return;
+    }
     const uint32_t b = blocks_for(n, threads);
     const size_t sm = (size_t)kCompact * threads * sizeof(uint32_t);
-    const bool cubic = k.kernel == 0;
 #define PE_FORCES(I, D, C, B) \
     k_forces<I, D, C, B><<<b, threads, sm, st>>>(n, k, tk, s, l, dt, pos_next, vel_next, st_a)
 #define PE_FORCES_B(I, D, C)              \
@@ -535,7 +920,6 @@ void launch_forces(uint32_t n, uint32_t threads, const StepConst& k, const Tanks
         if (beta0) PE_FORCES(I, D, C, true); \
         else PE_FORCES(I, D, C, false);   \
     } while (0)
-    const bool beta0 = k.visc_beta == 0.0;
     if (k.dim == 3) {
         if (cubic) {
             if (integrate) PE_FORCES_B(true, 3, true);
@@ -557,20 +941,41 @@ void launch_forces(uint32_t n, uint32_t threads, const StepConst& k, const Tanks
 #undef PE_FORCES
 }
 
-void launch_boundary_force(uint32_t n, const StepConst& k, const StateBufs& s, const ListBufs& l,
+void launch_boundary_force(uint32_t n, uint32_t lanes, const StepConst& k, const StateBufs& s, const ListBufs& l,
                            cudaStream_t st) {
     if (!n) return;
-    if (k.kernel == 0) k_boundary_force<true><<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, k, s, l);
-    else k_boundary_force<false><<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, k, s, l);
+    if (lanes == 1) {
+        if (k.kernel == 0) k_boundary_force<true><<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, k, s, l);
+        else k_boundary_force<false><<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, k, s, l);
+        return;
+    }
+    with_lanes(lanes, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        const uint32_t b = blocks_for((uint64_t)n * G, kThreads);
+        const size_t sm = sum_smem<G, 3>(kThreads);
+        if (k.kernel == 0) k_boundary_force_g<true, G><<<b, kThreads, sm, st>>>(n, k, s, l);
+        else k_boundary_force_g<false, G><<<b, kThreads, sm, st>>>(n, k, s, l);
+    });
 }
 
-void launch_xsph(uint32_t n, uint32_t threads, const StepConst& k, const StateBufs& s,
+void launch_xsph(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const StateBufs& s,
                  const ListBufs& l, double4* vel_out, cudaStream_t st, bool use_w) {
     if (!n) return;
     const bool w = use_w && l.wpair;
-    if (w) k_xsph_w<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out);
-    if (k.kernel == 0) k_xsph<true><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out, w);
-    else k_xsph<false><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out, w);
+    if (lanes == 1) {
+        if (w) k_xsph_w<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out);
+        if (k.kernel == 0) k_xsph<true><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out, w);
+        else k_xsph<false><<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, l, vel_out, w);
+        return;
+    }
+    with_lanes(lanes, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        const uint32_t b = blocks_for((uint64_t)n * G, threads);
+        const size_t sm = sum_smem<G, 3>(threads);
+        if (w) k_xsph_g<true, true, G><<<b, threads, sm, st>>>(n, k, s, l, vel_out, false);
+        if (k.kernel == 0) k_xsph_g<true, false, G><<<b, threads, sm, st>>>(n, k, s, l, vel_out, w);
+        else k_xsph_g<false, false, G><<<b, threads, sm, st>>>(n, k, s, l, vel_out, w);
+    });
 }
 
 void launch_in_support_counts(uint32_t n, const StepConst& k, const StateBufs& s,

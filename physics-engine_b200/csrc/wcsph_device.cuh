@@ -194,6 +194,13 @@ struct PassShape {
     uint32_t density = 128, forces = 128, xsph = 128;
 };
 
+// Lanes of a warp that share one slot's list in each f64 pass (lane_group.cuh):
+// 1, 4, 8, 16 or 32.
+struct PassLanes {
+    uint32_t density = 1, forces = 1, boundary = 1, xsph = 1;
+};
+PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t boundary);
+
 // Single-precision form (sph_f32.cu).
 struct F32Const {
     int dim;
@@ -258,20 +265,20 @@ void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32
                   bool visit_only = false, uint32_t chunk = 64);
 
 // ----- SPH passes -----
-void launch_density(uint32_t n, uint32_t threads, const StepConst& k, const StateBufs& s,
+void launch_density(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const StateBufs& s,
                     const ListBufs& l, cudaStream_t st);
 void launch_vmax(uint32_t n, const Tanks& tk, const StateBufs& s, cudaStream_t st);
 void launch_pressure(uint32_t n, const StepConst& k, const Tanks& tk, const StateBufs& s,
                      cudaStream_t st);
 void forces_prepare();  // once per context, before the first launch_forces
-void launch_forces(uint32_t n, uint32_t threads, const StepConst& k, const Tanks& tk,
+void launch_forces(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const Tanks& tk,
                    const StateBufs& s, const ListBufs& l, bool integrate, double dt,
                    double4* pos_next, double4* vel_next, const double4* st_a, cudaStream_t st);
-void launch_boundary_force(uint32_t n, const StepConst& k, const StateBufs& s, const ListBufs& l,
+void launch_boundary_force(uint32_t n, uint32_t lanes, const StepConst& k, const StateBufs& s, const ListBufs& l,
                            cudaStream_t st);
 // use_w: l.wpair holds the W of these lists and positions (written by the
 // density pass since the lists were built)
-void launch_xsph(uint32_t n, uint32_t threads, const StepConst& k, const StateBufs& s,
+void launch_xsph(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const StateBufs& s,
                  const ListBufs& l, double4* vel_out, cudaStream_t st, bool use_w = false);
 
 // ----- exports / diagnostics -----

@@ -347,6 +347,9 @@ World::World(const WorldParams& prm, const WorldConfig& cfg, int dim, double res
         DeviceScalars hs{};
         check(cudaMemcpyAsync(sc_, &hs, sizeof(hs), cudaMemcpyHostToDevice, st_), "upload");
 
+        for (uint64_t i = 0; i < n_; ++i) n_fluid_ += kind[i] == 0;
+        set_lanes(0);
+
         // ---- launch geometry of the list build: a persistent grid ----
         int sms = 148;
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "attribute");
@@ -706,7 +709,7 @@ void World::run_density(bool visit_only) {
     if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
     prof_begin(kDensity);
     if (f32_) launch_density_f32((uint32_t)n_, shape_.density, kf_, cur_, fb_, lists_, st_);
-    else launch_density((uint32_t)n_, shape_.density, kc_, cur_, lists_, st_);
+    else launch_density((uint32_t)n_, shape_.density, lanes_.density, kc_, cur_, lists_, st_);
     prof_end();
     launches_ += 1;
     check(cudaGetLastError(), "density");
@@ -746,11 +749,11 @@ void World::run_forces(bool integrate, double dt) {
         const bool surf = prm_.surface_tension_sigma != 0.0;  // wcsph.rs:262
         if (surf) run_surface_tension();
         prof_begin(kForces);
-        launch_forces((uint32_t)n_, shape_.forces, kc_, tanks_, cur_, lists_, integrate, dt, pos_nx_,
+        launch_forces((uint32_t)n_, shape_.forces, lanes_.forces, kc_, tanks_, cur_, lists_, integrate, dt, pos_nx_,
                       vel_nx_, surf ? st_a_ : nullptr, st_);
         prof_end();
         prof_begin(kBoundaryForce);
-        launch_boundary_force((uint32_t)n_, kc_, cur_, lists_, st_);
+        launch_boundary_force((uint32_t)n_, lanes_.boundary, kc_, cur_, lists_, st_);
         prof_end();
         launches_ += 2;
     }
@@ -808,7 +811,7 @@ void World::run_xsph() {
         std::swap(fb_.vel, velf_alt_);
         return;
     }
-    launch_xsph((uint32_t)n_, shape_.xsph, kc_, cur_, lists_, vel_nx_, st_, w_valid_);
+    launch_xsph((uint32_t)n_, shape_.xsph, lanes_.xsph, kc_, cur_, lists_, vel_nx_, st_, w_valid_);
     prof_end();
     launches_ += w_valid_ ? 2 : 1;  // with weights: the weight-reading kernel and its fallback
     check(cudaGetLastError(), "xsph");
@@ -948,6 +951,14 @@ bool World::capture_graph(double dt) {
     return graph_exec_ != nullptr;
 }
 
+void World::set_lanes(uint32_t lanes) {
+    if (lanes == 0) lanes_ = pass_lanes(dim_, n_fluid_, n_ - n_fluid_);
+    else if (lanes == 1 || lanes == 4 || lanes == 8 || lanes == 16 || lanes == 32)
+        lanes_.density = lanes_.forces = lanes_.boundary = lanes_.xsph = lanes;
+    else throw std::invalid_argument("lanes per slot");
+    invalidate_graph();
+}
+
 void World::configure_lists() {
     uint32_t per_sm = nlist_prepare(dim_, ucap_, list_chunk_);
     check(cudaGetLastError(), "nlist prepare");
@@ -1014,16 +1025,16 @@ World::Shapes World::autotune() {
     if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
     pick(shape_.density, [&] {
         if (f32_) launch_density_f32(n, shape_.density, kf_, cur_, fb_, lists_, st_);
-        else launch_density(n, shape_.density, kc_, cur_, lists_, st_);
+        else launch_density(n, shape_.density, lanes_.density, kc_, cur_, lists_, st_);
     });
     w_valid_ = pair_weights();  // the density launches wrote W for these lists
     pick(shape_.forces, [&] {
         if (f32_) launch_forces_f32(n, shape_.forces, kf_, tanks_, cur_, fb_, lists_, 0.f, pos_nx_, vel_nx_, nullptr, st_);
-        else launch_forces(n, shape_.forces, kc_, tanks_, cur_, lists_, true, 0.0, pos_nx_, vel_nx_,
+        else launch_forces(n, shape_.forces, lanes_.forces, kc_, tanks_, cur_, lists_, true, 0.0, pos_nx_, vel_nx_,
                            prm_.surface_tension_sigma != 0.0 ? st_a_ : nullptr, st_);
     });
     if (!f32_ && prm_.xsph_epsilon != 0.0)
-        pick(shape_.xsph, [&] { launch_xsph(n, shape_.xsph, kc_, cur_, lists_, vel_nx_, st_, w_valid_); });
+        pick(shape_.xsph, [&] { launch_xsph(n, shape_.xsph, lanes_.xsph, kc_, cur_, lists_, vel_nx_, st_, w_valid_); });
     // list build: tile (centre particles per chunk) x CTAs per SM (multiples
     // of the resident count). The lists' entries and order do not depend on
     // either; a smaller chunk never asks for more of the pool (each chunk

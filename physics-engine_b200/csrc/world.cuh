@@ -135,6 +135,11 @@ class World {
     Shapes shapes() const;
     Shapes autotune();
 
+    // Lanes of a warp on each slot's list in the f64 passes: 0 picks them per
+    // pass from the particle counts (pass_lanes, the default); 1, 4, 8, 16 or
+    // 32 sets them all. No choice changes a bit.
+    void set_lanes(uint32_t lanes);
+
     // The density pass keeps each visit entry's W(r) for the XSPH pass of the
     // same lists and positions, in a buffer of twice the list pool's bytes
     // (the pool's bytes in the single-precision form) that is kept only while
@@ -227,6 +232,8 @@ class World {
     Tanks tanks_{};
     std::vector<TankDesc> tank_host_;
     PassShape shape_{};
+    PassLanes lanes_{};
+    uint64_t n_fluid_ = 0;
     uint32_t list_ctas_per_sm_ = 0;  // 0: four times the resident count
     uint32_t list_chunk_ = 32;       // centre particles per list-build chunk
     StepConst kc_{};

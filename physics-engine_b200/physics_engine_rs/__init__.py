@@ -223,6 +223,7 @@ def load_library():
         "pe_fluid_wcsph_capacity_info": (C.c_int, [vp, vp]),
         "pe_fluid_wcsph_diagnostics": (C.c_int, [vp, C.POINTER(_Diag)]),
         "pe_fluid_wcsph_fluid_center_of_mass": (C.c_int, [vp, C.POINTER(C.c_double)]),
+        "pe_fluid_wcsph_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_wcsph_list_chunk": (C.c_int, [vp, C.POINTER(C.c_uint32)]),
         "pe_fluid_wcsph_set_pair_weights": (C.c_int, [vp, C.c_int32]),
         "pe_fluid_wcsph_pair_weights": (C.c_int, [vp, C.POINTER(C.c_int32)]),
@@ -590,6 +591,12 @@ class WcsphWorld:
         _ok(_lib.pe_fluid_wcsph_list_chunk(self._w, C.byref(c)), "list_chunk")
         r["list_chunk"] = int(c.value)
         return r
+
+    def set_lanes(self, lanes: int = 0):
+        """Lanes of a warp on each particle's list in the f64 pair passes: 0
+        (the default) picks them per pass from the particle counts; 1, 4, 8,
+        16 or 32 sets them all. The results are identical."""
+        _ok(_lib.pe_fluid_wcsph_set_lanes(self._w, int(lanes)), "set_lanes")
 
     def set_pair_weights(self, on: bool = True):
         """Let the density pass keep each neighbour entry's W for the XSPH pass
