@@ -904,6 +904,31 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
     if (tid == 0 && max_union) atomicMax(&sc->max_union, max_union);
 }
 
+// Largest neighbour-cell union of the current grid (a thread per occupied cell;
+// the cells of a z column are adjacent in the dense order).
+template <int DIM>
+__global__ void k_union_max(Tanks tk, const uint32_t* __restrict__ occ, const uint32_t* __restrict__ cell_start,
+                            DeviceScalars* sc) {
+    const uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t u = 0;
+    if (it < sc->nocc) {
+        const uint32_t c = occ[it];
+        const TankDesc td = tk.desc[tk.cell_tank[c]];
+        const uint32_t lc = c - td.cell_base;
+        const int cz = (int)(lc % (uint32_t)td.nz);
+        const int cy = (int)((lc / (uint32_t)td.nz) % (uint32_t)td.ny);
+        const int cx = (int)(lc / ((uint32_t)td.nz * (uint32_t)td.ny));
+        const int z0 = max(cz - 1, 0), z1 = min(cz + 1, td.nz - 1);
+        for (int qx = max(cx - 1, 0); qx <= min(cx + 1, td.nx - 1); ++qx)
+            for (int qy = max(cy - 1, 0); qy <= min(cy + 1, td.ny - 1); ++qy) {
+                const uint32_t base = td.cell_base + ((uint32_t)qx * (uint32_t)td.ny + (uint32_t)qy) * (uint32_t)td.nz;
+                u += cell_start[base + (uint32_t)z1 + 1u] - cell_start[base + (uint32_t)z0];
+            }
+    }
+    u = warp_max(u);
+    if ((threadIdx.x & 31u) == 0 && u) atomicMax(&sc->max_union, u);
+}
+
 size_t both_smem_bytes(uint32_t ucap, uint32_t chunk) {
     const size_t sort = (size_t)ucap * sizeof(uint16_t) + 16 * kNlThreads * sizeof(uint16_t);
     const size_t mask = (size_t)(ucap / 32) * chunk * sizeof(uint32_t);
@@ -940,10 +965,14 @@ size_t nlist_smem_bytes(uint32_t ucap, uint32_t chunk) {
 namespace {
 template <int DIM, uint32_t C>
 uint32_t prepare_for(uint32_t ucap) {
+    // the attribute is the kernel's, not the world's: the largest stage's bytes,
+    // so that no world's setting falls below another's launch
     const int sv = (int)visit_smem_bytes(ucap, C), sb = (int)both_smem_bytes(ucap, C);
     int bv = 0, bb = 0;
-    cudaFuncSetAttribute(k_nlist_visit<DIM, false, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv);
-    cudaFuncSetAttribute(k_nlist_both<DIM, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+    cudaFuncSetAttribute(k_nlist_visit<DIM, false, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)visit_smem_bytes(kMaxUnionStage, C));
+    cudaFuncSetAttribute(k_nlist_both<DIM, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)both_smem_bytes(kMaxUnionStage, C));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bv, k_nlist_visit<DIM, false, C>, kNlThreads, sv);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_nlist_both<DIM, C>, kNlThreads, sb);
     const int b = bv > bb ? bv : bb;
@@ -967,6 +996,13 @@ uint32_t nlist_prepare(int dim, uint32_t ucap, uint32_t chunk) {
     chunk = valid_chunk(chunk);
     if (dim == 3) return chunk == 32u ? prepare_for<3, 32>(ucap) : prepare_for<3, 64>(ucap);
     return chunk == 32u ? prepare_for<2, 32>(ucap) : prepare_for<2, 64>(ucap);
+}
+
+void launch_union_max(const GridDesc& g, const Tanks& tk, uint32_t ncell_max, const uint32_t* occ,
+                      const uint32_t* cell_start, DeviceScalars* sc, cudaStream_t st) {
+    const uint32_t b = (ncell_max + 255u) / 256u;
+    if (g.dim == 3) k_union_max<3><<<b, 256, 0, st>>>(tk, occ, cell_start, sc);
+    else k_union_max<2><<<b, 256, 0, st>>>(tk, occ, cell_start, sc);
 }
 
 void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32_t ucap,

@@ -259,6 +259,10 @@ void launch_surface_tension(uint32_t n, const StepConst& k, const SurfConst& c, 
 // and returns how many of its CTAs fit on one SM.
 // chunk = centre particles per chunk of the list build (32 or 64).
 uint32_t nlist_prepare(int dim, uint32_t ucap, uint32_t chunk = 64);
+// raises sc->max_union to the largest union of the current grid (ncell_max >=
+// the occupied cells)
+void launch_union_max(const GridDesc& g, const Tanks& tk, uint32_t ncell_max, const uint32_t* occ,
+                      const uint32_t* cell_start, DeviceScalars* sc, cudaStream_t st);
 void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32_t ucap,
                   uint32_t nblocks, const uint32_t* occ, const uint32_t* cell_start,
                   const StateBufs& s, const ListBufs& l, DeviceScalars* sc, cudaStream_t st,

@@ -656,6 +656,20 @@ void World::ensure_lists(bool visit_only) {
         check(cudaMemsetAsync(lists_.ldesc, 0, sizeof(uint2) * lists_.nslots, st_), "memset");
         check(cudaMemsetAsync(lists_.ncand, 0, sizeof(uint32_t) * lists_.nslots, st_), "memset");
     } else {
+        // Positions the host has set get a stage with the margin the initial
+        // ones got. Polls grow it only every 16 steps, and until then the cells
+        // beyond it take the slow path: a 40^3 block created on the exact
+        // lattice and set to jittered positions outgrew its 2,048 entries
+        // between two polls, 24 ms a build against 0.2.
+        if (!lists_checked_) {
+            launch_union_max(g_, tanks_, std::min<uint32_t>(g_.ncell, (uint32_t)std::max<uint64_t>(n_, 1)), occ_,
+                             cell_start_, sc_, st_);
+            launches_ += 1;
+            uint32_t largest = 0;
+            check(cudaMemcpyAsync(&largest, &sc_->max_union, sizeof(largest), cudaMemcpyDeviceToHost, st_), "lists");
+            check(cudaStreamSynchronize(st_), "lists");
+            grow_stage(nlist_union_capacity(largest));
+        }
         // Every pass of this loop builds into the current pool, so the loop
         // always ends with lists built in the pool they describe.
         for (int attempt = 0;; ++attempt) {
@@ -1096,14 +1110,14 @@ uint32_t World::status() {
     }
     // Grow the shared-memory stage of the list build when the fluid has
     // packed more particles into a neighbourhood than it holds.
-    if (hs.max_union > ucap_) {
-        uint32_t want = nlist_union_capacity(hs.max_union);
-        if (want > ucap_) {
-            ucap_ = want;
-            configure_lists();
-        }
-    }
+    if (hs.max_union > ucap_) grow_stage(nlist_union_capacity(hs.max_union));
     return hs.status;
+}
+
+void World::grow_stage(uint32_t want) {
+    if (want <= ucap_) return;
+    ucap_ = want;
+    configure_lists();
 }
 
 void World::capacity_info(uint64_t* out) {

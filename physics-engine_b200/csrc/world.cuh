@@ -201,6 +201,7 @@ class World {
     void refresh_f32();
     void configure_lists();
     void alloc_lists(unsigned long long groups);
+    void grow_stage(uint32_t want);
     void invalidate_graph() { ++epoch_; }
     bool graph_capturable() const;
     bool capture_graph(double dt);
