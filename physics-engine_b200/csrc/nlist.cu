@@ -5,14 +5,12 @@
 // per fluid particle per step. The 27 (3-D) or 9 (2-D) neighbour cells of a
 // CTA's cell are visited in the reference's (dz, dy, dx) order; their
 // particles (each cell's run already in ascending original index) are staged
-// in shared memory as single-precision coordinates relative to the cell
-// corner, one array per coordinate, and every particle of the centre cell
-// filters the staged union with a conservative squared-distance bound
-// (`r2_filter` exceeds (2h)^2 by a relative 1e-4, far above the
-// single-precision error of the staged coordinates), four candidates per
-// 16-byte read on paired f32x2 arithmetic, so every pair with q = r/h < 2 is
-// kept. Extra borderline candidates are harmless: the f64 passes evaluate q
-// exactly and such pairs contribute an exact +-0.
+// in shared memory as half-precision features, and every particle of the
+// centre cell filters the staged union with a conservative squared-distance
+// bound that exceeds the support's by far more than the features' rounding
+// (see Features), so every pair with q = r/h < 2 is kept. Extra borderline
+// candidates are harmless: the f64 passes evaluate q exactly and such pairs
+// contribute an exact +-0.
 //
 // k_nlist_both writes, for fluid particles, the "visit" list (in-support
 // candidates, self excluded, in visiting order, each flagged boundary /
@@ -27,13 +25,30 @@
 // The kernels work on chunks of up to 32 (or 64) centre particles with eight
 // (or four) threads per particle; the fused kernel is compiled for three
 // resident CTAs per SM (80 registers), which the 32-centre tile's shared
-// memory allows. A first pass, each thread taking a quarter of the candidates
-// (union words, or sorted positions), keeps the in-support bit masks in shared
-// memory and counts; the chunk's longest lists size one block of the list
-// pool, reserved with one atomic add; a second pass writes the entries, each
-// thread a quarter of the particle's list (a quarter of the words would leave
-// most of the kept candidates, which lie in the middle words, to two threads).
+// memory allows. Each warp computes the in-support bit masks of 32 centres
+// over its share of the union words on the tensor cores (word_bytes); the
+// chunk's longest list sizes one block of the list pool, reserved with one
+// atomic add; then the entries are written, each thread an equal share of its
+// particle's list (a share of the words would leave most of the kept
+// candidates, which lie in the middle words, to two threads). While a thread
+// walks its kept candidates it sets the bits of the lower ones in a second
+// mask over the sorted positions, from which the lower list is written.
+//
+// k_nlist_visit stages f32 offsets and tests them in packed f32 arithmetic: its
+// lists feed the single-precision form, whose compensated sums notice a
+// candidate more (a zero added moves a tie), and PBF's grid, whose cells of
+// eight particles leave the tensor tile half empty (125 us a build of 64,000
+// particles against 153).
+//
+// k_nlist_both is bound by instruction issue and barriers (529M warp instructions for 262,144 fluid
+// particles, IPC 2.4, with scalar distance tests and a lower mask read through
+// every sorted position; 391M as it is). At 1M 3.51 -> 2.43 ms, by parts: the
+// visit entries 0.75, radix sort 0.41, lower entries 0.28, staging 0.17, masks
+// 0.14 ms, barriers and the rest 0.7.
+#include <algorithm>
 #include <climits>
+
+#include <cuda_fp16.h>
 
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
@@ -48,16 +63,19 @@ constexpr int kNlThreads = 256;
 // centre particle. kDefaultChunk is what an unknown value falls back to.
 constexpr uint32_t kDefaultChunk = 64;
 constexpr uint32_t kWarps = kNlThreads / 32;
-// Largest stage: the fused kernel's 38 dynamic bytes per staged entry (f32
-// position 16, slot 4, sort index 2, visit masks 8, lower masks or sort
-// scratch 8) plus its ~2.4 KB of static shared memory must fit the 227 KB a
-// CTA can opt in to on sm_100 (232,448 bytes).
+// Largest stage: the fused kernel's dynamic bytes per staged entry at the
+// 32-centre tile (features 16, slot 4, sort index 2, rank 2, masks 8) and
+// ~2.4 KB of static shared memory must fit the 227 KB a CTA can opt in to on
+// sm_100 (232,448 bytes). The 64-centre tile's masks take 16; a stage too large
+// for it takes the 32-centre one.
 constexpr uint32_t kMaxUnionStage = 5888;
-static_assert(38u * kMaxUnionStage + 4096u <= 232448u, "list stage exceeds the shared-memory limit");
+constexpr size_t kMaxDynamicBytes = 232448u - 4096u;
+static_assert(32u * kMaxUnionStage + kMaxUnionStage / 8u <= kMaxDynamicBytes,
+              "list stage exceeds the shared-memory limit");
 constexpr uint32_t kStageStep = 256;               // stage capacities are multiples of this
 
 // Staged word w of a union entry: original index (29 bits) | kind flags.
-constexpr uint32_t kStageBoundary = 1u << 31;  // the sign bit (word_mask reads it so)
+constexpr uint32_t kStageBoundary = 1u << 31;
 constexpr uint32_t kStageOriented = 1u << 30;
 constexpr uint32_t kStageOrigMask = (1u << 29) - 1u;
 
@@ -187,6 +205,8 @@ __device__ __forceinline__ bool keep_entry(const float4& q, const float4& me, fl
     return within(q, me, r2f) || (keep_boundary && (__float_as_uint(q.w) & kStageBoundary));
 }
 
+// ---- the visit kernel's stage and test ----
+
 // The staged union in shared memory as four float arrays (cell-local x, y, z
 // and the staged word orig | kind flags), so that the candidates of a word can
 // be read four at a time per coordinate.
@@ -201,7 +221,6 @@ struct Stage {
         z[u] = p.z;
         w[u] = p.w;
     }
-    __device__ __forceinline__ uint32_t word(uint32_t u) const { return __float_as_uint(w[u]); }
 };
 
 // Packed single-precision pairs (two f32 in one 64-bit register) and the
@@ -263,12 +282,111 @@ __device__ __forceinline__ uint32_t word_mask(const Stage& st, uint32_t base, co
     return m;
 }
 
+// ---- the fused kernel's stage and test ----
+
+// Features of a staged candidate: eight halves (x, y, z, nh, nl, 1, 1, 0) with
+// (x, y, z) its offset from the middle of the centre cell in units of the cell
+// (within +-1.5), rounded to half, and nh + nl the squared length of the
+// rounded offset. With a centre's row (-2x, -2y, -2z, 1, 1, ah, al, 0),
+// ah + al = its own squared length minus the bound, the product of the two is
+// |xi - xj|^2 - bound, exact but for the splits (2^-20) and the f32 sum: the
+// sign bit is the test, and one m16n8k8 tensor instruction makes 128 of them.
+//
+// The bound: an offset's rounding error is at most 2^-11 a component, so a
+// pair's distance is off by at most 2 sqrt(3) 2^-11 = 0.0017 cells, and a pair
+// within the support (one cell) has a rounded squared distance of at most
+// 1.0034. The filter keeps ~0.5 % more candidates than the support holds.
+constexpr float kBound2 = 1.0036f;
+
+struct Features {
+    __half2 xy, zn, m1, one;
+};
+static_assert(sizeof(Features) == 16, "one 16-byte store a candidate");
+
+template <int DIM>
+__device__ __forceinline__ Features features(double px, double py, double pz, const CellUnion& cu, float inv_cell) {
+    Features f;
+    f.xy = __floats2half2_rn((float)(px - cu.ox) * inv_cell - 0.5f, (float)(py - cu.oy) * inv_cell - 0.5f);
+    const __half z = DIM == 3 ? __float2half_rn((float)(pz - cu.oz) * inv_cell - 0.5f) : __float2half_rn(0.0f);
+    const float2 c = __half22float2(f.xy);
+    const float cz = __half2float(z), n = c.x * c.x + c.y * c.y + cz * cz;
+    const __half nh = __float2half_rn(n);
+    f.zn = __halves2half2(z, nh);
+    f.m1 = __halves2half2(__float2half_rn(n - __half2float(nh)), __float2half_rn(1.0f));
+    f.one = __halves2half2(__float2half_rn(1.0f), __float2half_rn(0.0f));
+    return f;
+}
+
+// Where candidate u's features are staged: within a word of 32, so that the
+// two columns a lane receives of each of the word's four products are the
+// candidates of one byte of the mask.
+__device__ __forceinline__ uint32_t feature_pos(uint32_t u) {
+    return (u & ~31u) | ((u & 6u) << 2) | ((u & 24u) >> 2) | (u & 1u);
+}
+
+// The pair `pair` of the row of the centre staged at pos.
+__device__ __forceinline__ uint32_t centre_pair(const Features* st, uint32_t pos, uint32_t pair) {
+    constexpr uint32_t kHalfOne = 0x3c00u;
+    if (pair < 2u) {
+        const __half2 v = __hmul2(pair ? st[pos].zn : st[pos].xy, __floats2half2_rn(-2.0f, -2.0f));
+        const uint32_t r = *reinterpret_cast<const uint32_t*>(&v);
+        return pair ? (r & 0xffffu) | kHalfOne << 16 : r;  // (-2x, -2y) or (-2z, 1)
+    }
+    const float a = (__high2float(st[pos].zn) + __low2float(st[pos].m1)) - kBound2;
+    const __half ah = __float2half_rn(a);
+    if (pair == 2u) return kHalfOne | (uint32_t)__half_as_ushort(ah) << 16;
+    return __half_as_ushort(__float2half_rn(a - __half2float(ah)));
+}
+
+__device__ __forceinline__ void mma_m16n8k8(float (&d)[4], const uint32_t (&a)[2], uint32_t b) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(b), "f"(0.0f));
+}
+
+// In-support masks of 32 centres over the union words [wb, we): bit u of the
+// word of centre c (masks[word * kChunk + c]) says that candidate 32 word + u
+// passes the filter. A lane owns byte (lane & 3) of the words of the centres
+// lane / 4 + 0, 8, 16, 24: it shifts the eight signs of a centre's products
+// into the byte and stores it, 52 instructions a word for the warp's 1,024
+// tests where packed f32 arithmetic and compares took over 200.
+// With at most 16 centres the second half of the tile is left out.
+template <uint32_t kChunk, bool HALF>
+__device__ __forceinline__ void word_masks(const Features* st, uint32_t* masks, const uint32_t (&a0)[2],
+                                           const uint32_t (&a1)[2], uint32_t wb, uint32_t we) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t* feat = reinterpret_cast<const uint32_t*>(st) + lane;
+    unsigned char* out = reinterpret_cast<unsigned char*>(masks + (lane >> 2)) + (lane & 3u);
+    for (uint32_t w = wb; w < we; ++w) {
+        float d0[4][4], d1[4][4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const uint32_t b = feat[w * 128u + n * 32u];
+            mma_m16n8k8(d0[n], a0, b);
+            if (!HALF) mma_m16n8k8(d1[n], a1, b);
+        }
+        uint32_t m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int n = 3; n >= 0; --n)
+#pragma unroll
+            for (int j = 1; j >= 0; --j) {
+                m[0] = __funnelshift_l(__float_as_uint(d0[n][j]), m[0], 1);
+                m[1] = __funnelshift_l(__float_as_uint(d0[n][2 + j]), m[1], 1);
+                if (!HALF) {
+                    m[2] = __funnelshift_l(__float_as_uint(d1[n][j]), m[2], 1);
+                    m[3] = __funnelshift_l(__float_as_uint(d1[n][2 + j]), m[3], 1);
+                }
+            }
+#pragma unroll
+        for (int r = 0; r < (HALF ? 2 : 4); ++r) out[(w * kChunk + 8u * r) * 4u] = (unsigned char)m[r];
+    }
+}
+
 __device__ __forceinline__ uint32_t rows_for(uint32_t n) { return (n + 3u) >> 2; }
 
-// Reserved block of one chunk: `rows_a + rows_b` rows of `stride` groups.
+// Reserved block of one chunk: `rows` rows of `stride` groups.
 struct ChunkBlock {
     unsigned long long base;  // group index of row 0, lane 0
-    uint32_t rows_a, rows_b;
     bool ok;
 };
 
@@ -303,32 +421,22 @@ struct MaskCursor {
     }
 };
 
-// Every thread passes its (a, b) list lengths; thread 0 reserves the block for
-// the chunk's longest ones and all threads return it.
-__device__ __forceinline__ ChunkBlock reserve_chunk(const ListBufs& l, DeviceScalars* sc, uint32_t stride,
-                                                    uint32_t na, uint32_t nb, uint32_t (*s_red)[2],
-                                                    ChunkBlock* s_blk, bool* s_overflow) {
-    const uint32_t a = warp_max(na), b = warp_max(nb);
-    if ((threadIdx.x & 31u) == 0) {
-        s_red[threadIdx.x >> 5][0] = a;
-        s_red[threadIdx.x >> 5][1] = b;
-    }
+// Every thread passes its list's length; thread 0 reserves the block for the
+// chunk's longest one and all threads return it.
+__device__ __forceinline__ ChunkBlock reserve_chunk(const ListBufs& l, DeviceScalars* sc, uint32_t stride, uint32_t n,
+                                                    uint32_t* s_red, ChunkBlock* s_blk, bool* s_overflow) {
+    n = __reduce_max_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31u) == 0) s_red[threadIdx.x >> 5] = n;
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t ma = 0, mb = 0;
+        uint32_t m = 0;
 #pragma unroll
-        for (uint32_t w = 0; w < kWarps; ++w) {
-            ma = max(ma, s_red[w][0]);
-            mb = max(mb, s_red[w][1]);
-        }
+        for (uint32_t w = 0; w < kWarps; ++w) m = max(m, s_red[w]);
         ChunkBlock blk;
-        blk.rows_a = rows_for(ma);
-        blk.rows_b = rows_for(mb);
-        const unsigned long long groups = (unsigned long long)(blk.rows_a + blk.rows_b) * stride;
+        const unsigned long long groups = (unsigned long long)rows_for(m) * stride;
         blk.base = groups ? atomicAdd(&sc->list_used, groups) : 0ull;
-        // counts, strides and row offsets are stored in 16 bits
-        const bool fits16 = ma < 65536u && mb < 65536u && stride < 65536u && blk.rows_a < 65536u;
-        blk.ok = fits16 && blk.base + groups <= l.pool_groups;
+        // counts and strides are stored in 16 bits
+        blk.ok = m < 65536u && stride < 65536u && blk.base + groups <= l.pool_groups;
         if (!blk.ok) *s_overflow = true;
         *s_blk = blk;
     }
@@ -348,7 +456,7 @@ constexpr int kRadixBits = 9;
 constexpr uint32_t kRadixDigits = 1u << kRadixBits;
 static_assert(kRadixDigits * kWarps == 16 * kNlThreads, "radix counters fill the scan's 16 per thread");
 
-__device__ __forceinline__ void radix_sort_by_orig(const float* s_w, uint16_t* s_sorted, uint16_t* s_tmp,
+__device__ __forceinline__ void radix_sort_by_orig(const uint32_t* s_w, uint16_t* s_sorted, uint16_t* s_tmp,
                                                    uint16_t* s_cnt, uint32_t nf, uint32_t omin, uint32_t omax) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t span = nf ? omax - omin : 0u;
@@ -358,13 +466,16 @@ __device__ __forceinline__ void radix_sort_by_orig(const float* s_w, uint16_t* s
     uint16_t *src = s_sorted, *dst = s_tmp;
     for (int pass = 0; pass < npass; ++pass) {
         const int shift = kRadixBits * pass;
-        for (uint32_t i = tid; i < kRadixDigits * kWarps; i += blockDim.x) s_cnt[i] = 0;
+        {
+            uint4* const cw = reinterpret_cast<uint4*>(s_cnt);  // 512 16-byte words
+            cw[tid] = cw[tid + kNlThreads] = make_uint4(0u, 0u, 0u, 0u);
+        }
         __syncthreads();
         for (uint32_t b = e0; b < e1; b += 32u) {
             const uint32_t e = b + lane;
             const bool valid = e < e1;
             uint32_t d = kRadixDigits;  // lanes past the segment: a digit of their own
-            if (valid) d = (((__float_as_uint(s_w[src[e]]) & kStageOrigMask) - omin) >> shift) & (kRadixDigits - 1u);
+            if (valid) d = (((s_w[src[e]] & kStageOrigMask) - omin) >> shift) & (kRadixDigits - 1u);
             const uint32_t peers = __match_any_sync(0xffffffffu, d);
             if (valid && lane == (uint32_t)(__ffs(peers) - 1)) s_cnt[d * kWarps + warp] += (uint16_t)__popc(peers);
             __syncwarp();
@@ -400,7 +511,7 @@ __device__ __forceinline__ void radix_sort_by_orig(const float* s_w, uint16_t* s
             uint16_t pu = 0;
             if (valid) {
                 pu = src[e];
-                d = (((__float_as_uint(s_w[pu]) & kStageOrigMask) - omin) >> shift) & (kRadixDigits - 1u);
+                d = (((s_w[pu] & kStageOrigMask) - omin) >> shift) & (kRadixDigits - 1u);
             }
             const uint32_t peers = __match_any_sync(0xffffffffu, d);
             uint32_t base = 0;
@@ -427,7 +538,7 @@ __device__ __forceinline__ void radix_sort_by_orig(const float* s_w, uint16_t* s
 template <int DIM, bool LOWER_FLAGS>
 __device__ __forceinline__ void visit_slow(const StepConst& k, float r2f, const CellUnion& cu, uint32_t U,
                                            const StateBufs& s, const ListBufs& l, DeviceScalars* sc,
-                                           const uint32_t* s_cstart, const uint32_t* s_off, uint32_t (*s_red)[2],
+                                           const uint32_t* s_cstart, const uint32_t* s_off, uint32_t* s_red,
                                            ChunkBlock* s_blk, bool* s_overflow) {
     constexpr int NC = DIM == 3 ? 27 : 9;
     const uint32_t tid = threadIdx.x;
@@ -459,7 +570,7 @@ __device__ __forceinline__ void visit_slow(const StepConst& k, float r2f, const 
                 }
             }
         }
-        const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, 0u, s_red, s_blk, s_overflow);
+        const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, s_red, s_blk, s_overflow);
         if (active) {
             const uint32_t gv = (uint32_t)blk.base + tid;
             l.desc[kslot] = blk.ok ? make_uint4(gv, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
@@ -492,7 +603,7 @@ __device__ __forceinline__ void visit_slow(const StepConst& k, float r2f, const 
 template <int DIM>
 __device__ __forceinline__ void lower_slow(const StepConst& k, float r2f, const CellUnion& cu, const StateBufs& s,
                                            const ListBufs& l, DeviceScalars* sc, const uint32_t* s_cstart,
-                                           const uint32_t* s_off, uint32_t (*s_red)[2], ChunkBlock* s_blk,
+                                           const uint32_t* s_off, uint32_t* s_red, ChunkBlock* s_blk,
                                            bool* s_overflow) {
     constexpr int NC = DIM == 3 ? 27 : 9;
     const uint32_t tid = threadIdx.x;
@@ -526,7 +637,7 @@ __device__ __forceinline__ void lower_slow(const StepConst& k, float r2f, const 
                 }
             }
         }
-        const ChunkBlock blk = reserve_chunk(l, sc, nc, nl, 0u, s_red, s_blk, s_overflow);
+        const ChunkBlock blk = reserve_chunk(l, sc, nc, nl, s_red, s_blk, s_overflow);
         if (active) {
             const uint32_t gl = (uint32_t)blk.base + tid;
             l.ldesc[kslot] = blk.ok ? make_uint2(gl, nl | (nc << 16)) : make_uint2(0u, 0u);
@@ -565,12 +676,46 @@ __device__ __forceinline__ void lower_slow(const StepConst& k, float r2f, const 
     }
 }
 
+// The threads of a CTA shared out over a chunk's nc centres for the writing of
+// their entries: way `way` of `ways` of centre `lane`, so that a cell's last,
+// shorter chunk costs its share. ways = 0 for a thread left over.
+struct Share {
+    uint32_t lane, way, ways;
+    __device__ __forceinline__ explicit Share(uint32_t nc) : ways(kNlThreads / nc) {
+        way = threadIdx.x / nc;
+        lane = threadIdx.x - way * nc;
+        if (way >= ways) way = ways = 0;
+    }
+    // this way's entries [first, last) of n
+    __device__ __forceinline__ uint32_t first(uint32_t n) const { return ways ? n * way / ways : 0u; }
+    __device__ __forceinline__ uint32_t last(uint32_t n) const { return ways ? n * (way + 1u) / ways : 0u; }
+};
+
+// Where entry t of a list is written, and the next one's place after it.
+struct EntryOut {
+    uint32_t* p;
+    uint32_t t, row;  // row: from a row's last entry to the next row's first
+    __device__ __forceinline__ EntryOut(uint32_t* list, uint32_t step, uint32_t t0)
+        : p(list + (size_t)(t0 >> 2) * step + (t0 & 3u)), t(t0), row(step - 3u) {}
+    __device__ __forceinline__ void put(uint32_t e) const { *p = e; }
+    __device__ __forceinline__ void next() {
+        p += (t & 3u) == 3u ? row : 1u;
+        ++t;
+    }
+};
+
+// CTAs a cell: its chunks are shared out over several (each stages the union
+// again) while the occupied cells leave most of the grid idle.
+__device__ __forceinline__ uint32_t cell_parts(uint32_t nocc) {
+    return min(max(gridDim.x / (8u * max(nocc, 1u)), 1u), 4u);
+}
+
 // ----------------------------------------------------------------- visit
 // Dynamic shared memory (ucap a multiple of kStageStep): float x, y, z, w[ucap] (Stage);
 // uint32 s_ent[ucap]; uint32 s_mask[(ucap / 32) * kChunk] (word w of chunk
 // lane c at s_mask[w * kChunk + c]).
-template <int DIM, bool LOWER_FLAGS, uint32_t kChunk>
-__global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk, StepConst k, uint32_t ucap,
+template <int DIM, uint32_t kChunk>
+__global__ void __launch_bounds__(kNlThreads, 4) k_nlist_visit(GridDesc g, Tanks tk, StepConst k, uint32_t ucap,
                                                             const uint32_t* __restrict__ occ,
                                                             const uint32_t* __restrict__ cell_start,
                                                             StateBufs s, ListBufs l,
@@ -584,7 +729,7 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk
     __shared__ uint32_t s_cstart[NC];
     __shared__ uint32_t s_off[NC + 1];
     __shared__ uint32_t s_cv[kWays][kChunk];
-    __shared__ uint32_t s_red[kWarps][2];
+    __shared__ uint32_t s_red[kWarps];
     __shared__ ChunkBlock s_blk;
     __shared__ bool s_overflow;
 
@@ -595,7 +740,9 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk
     uint32_t max_union = 0;
     if (tid == 0) s_overflow = false;
 
-    for (uint32_t it = blockIdx.x; it < nocc; it += gridDim.x) {
+    const uint32_t parts = cell_parts(nocc);
+    for (uint32_t item = blockIdx.x; item < nocc * parts; item += gridDim.x) {
+        const uint32_t it = item / parts, part = item - it * parts;
         const CellUnion cu = cell_union<DIM>(g, tk, occ[it], cell_start, s_cstart, s_off);
         const uint32_t U = cu.U;
         max_union = max(max_union, U);
@@ -611,18 +758,16 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk
             __syncthreads();
             const uint32_t W = (U + 31u) >> 5;
             const uint32_t wb = W * q / kWays, we = W * (q + 1) / kWays;
-            for (uint32_t c0 = 0; c0 < cu.ncenter; c0 += kChunk) {
+            for (uint32_t c0 = part * kChunk; c0 < cu.ncenter; c0 += parts * kChunk) {
                 const uint32_t nc = min(kChunk, cu.ncenter - c0);
                 const bool active = lane < nc;
                 const uint32_t myu = cu.center_off + c0 + lane;
                 bool fluidc = false;
-                uint32_t myo = 0;
                 // ---- pass 1: in-support masks of this quarter's words, counts
                 if (active) {
                     const float4 me = st.get(myu);
                     const uint32_t mw = __float_as_uint(me.w);
                     fluidc = !(mw & kStageBoundary);
-                    myo = mw & kStageOrigMask;
                     uint32_t cv = 0;
                     if (fluidc) {
                         for (uint32_t w = wb; w < we; ++w) {
@@ -643,36 +788,30 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk
 #pragma unroll
                     for (uint32_t r = 0; r < kWays; ++r) nv += s_cv[r][lane];
                 }
-                const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, 0u, s_red, &s_blk, &s_overflow);
+                const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, s_red, &s_blk, &s_overflow);
                 // ---- pass 2: descriptors and entries
-                if (active) {
+                if (active && q == 0) {
                     const uint32_t kslot = cu.cs + c0 + lane;
                     const uint32_t gv = (uint32_t)blk.base + lane;  // < pool_groups < 2^32 when ok
-                    if (q == 0) {
-                        l.desc[kslot] = blk.ok ? make_uint4(gv, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
-                        l.ncand[kslot] = fluidc ? U : 0u;
-                    }
-                    // entries split evenly over the centre's threads
-                    const uint32_t v0 = nv * q / kWays, v1 = nv * (q + 1u) / kWays;
-                    if (blk.ok && fluidc && v0 < v1) {
-                        const size_t step = 4u * nc;
-                        uint32_t* pv = l.pool + 4 * (size_t)gv;
-                        MaskCursor<kChunk> cur(s_mask, s_cv, lane, W, v0);
-                        for (uint32_t t = v0; t < v1; ++t) {
-                            const uint32_t u = cur.next();
-                            uint32_t e = s_ent[u];
-                            if (LOWER_FLAGS) {
-                                const uint32_t ow = st.word(u);
-                                e |= ow < myo ? kEntryLower : 0u;  // a boundary word has bit 31 set
-                            }
-                            pv[(t >> 2) * step + (t & 3u)] = e;
-                        }
+                    l.desc[kslot] = blk.ok ? make_uint4(gv, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
+                    l.ncand[kslot] = fluidc ? U : 0u;
+                }
+                if (blk.ok) {
+                    const Share sh(nc);
+                    uint32_t n = 0;
+#pragma unroll
+                    for (uint32_t r = 0; r < kWays; ++r) n += s_cv[r][sh.lane];
+                    const uint32_t v0 = sh.first(n), v1 = sh.last(n);
+                    if (v0 < v1) {
+                        EntryOut out(l.pool + 4 * (size_t)(blk.base + sh.lane), 4u * nc, v0);
+                        MaskCursor<kChunk> cur(s_mask, s_cv, sh.lane, W, v0);
+                        for (; out.t < v1; out.next()) out.put(s_ent[cur.next()]);
                     }
                 }
                 __syncthreads();  // masks and counts are reused by the next chunk
             }
-        } else {
-            visit_slow<DIM, LOWER_FLAGS>(k, r2f, cu, U, s, l, sc, s_cstart, s_off, s_red, &s_blk, &s_overflow);
+        } else if (part == 0) {
+            visit_slow<DIM, false>(k, r2f, cu, U, s, l, sc, s_cstart, s_off, s_red, &s_blk, &s_overflow);
         }
         __syncthreads();  // shared memory is reused by the next cell
     }
@@ -681,15 +820,63 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_visit(GridDesc g, Tanks tk
 }
 
 // ----------------------------------------------------------------- both
+// ----------------------------------------------------------------- both
+// Stages candidate u of a union: features, list entry and staged word.
+template <int DIM>
+__device__ __forceinline__ uint32_t stage_candidate(const StateBufs& s, const CellUnion& cu, float inv_cell,
+                                                    uint32_t slot, uint32_t u, Features* st, uint32_t* s_ent) {
+    const double4 p = s.pos[slot];
+    const uint8_t fl = s.flags[slot];
+    const uint32_t w = s.orig[slot] | ((fl & kFlagBoundary) ? kStageBoundary : 0u) |
+                       ((fl & kFlagOriented) ? kStageOriented : 0u);
+    st[feature_pos(u)] = features<DIM>(p.x, p.y, p.z, cu, inv_cell);
+    s_ent[u] = slot | entry_flags(w);
+    return w;
+}
+
+// In-support masks of the nc (1 to 32) centres from union position u0 over
+// the words [wb, we). Rows past nc repeat the last centre.
+template <uint32_t kChunk>
+__device__ __forceinline__ void centre_masks(const Features* st, uint32_t* masks, uint32_t u0, uint32_t nc,
+                                             uint32_t wb, uint32_t we) {
+    const uint32_t row = (threadIdx.x & 31u) >> 2, pair = threadIdx.x & 3u;
+    auto at = [&](uint32_t r) { return centre_pair(st, feature_pos(u0 + min(r, nc - 1u)), pair); };
+    const uint32_t a0[2] = {at(row), at(row + 8u)};
+    if (nc <= 16u) {
+        word_masks<kChunk, true>(st, masks, a0, a0, wb, we);
+    } else {
+        const uint32_t a1[2] = {at(row + 16u), at(row + 24u)};
+        word_masks<kChunk, false>(st, masks, a0, a1, wb, we);
+    }
+}
+
+// A fluid centre's share [wb, we) of the mask words m[w * kChunk] made whole:
+// candidates past the union and the centre itself (union position myu) out,
+// every candidate in (all) or every boundary candidate (keep_boundary).
+// Returns their count.
+template <uint32_t kChunk>
+__device__ __forceinline__ uint32_t finish_masks(uint32_t* m, const uint32_t* s_fluid, uint32_t U, uint32_t myu,
+                                                 uint32_t wb, uint32_t we, bool all, int keep_boundary) {
+    if (all || keep_boundary)
+        for (uint32_t w = wb; w < we; ++w) m[w * kChunk] = all ? 0xffffffffu : m[w * kChunk] | ~s_fluid[w];
+    const uint32_t tail = U >> 5, own = myu >> 5;
+    if ((U & 31u) && tail >= wb && tail < we) m[tail * kChunk] &= (1u << (U & 31u)) - 1u;
+    if (own >= wb && own < we) m[own * kChunk] &= ~(1u << (myu & 31u));
+    uint32_t n = 0;
+    for (uint32_t w = wb; w < we; ++w) n += __popc(m[w * kChunk]);
+    return n;
+}
+
 // One pass per occupied cell for both lists: the union is staged once, the
-// visit masks of a chunk's fluid centres are computed once, and a fluid
-// centre's lower list is read out of its own visit mask in ascending original
-// index (through the radix-sorted fluid positions); boundary centres test the
-// sorted fluid positions directly. One reservation per chunk holds both lists
-// (visit rows first). Dynamic shared memory: float x, y, z, w[ucap] (Stage); uint32
-// s_ent[ucap] (slot | flags); uint32 s_vmask[(ucap / 32) * kChunk]; uint16
-// s_sorted[ucap]; then a region used first by the radix sort and then by the
-// lower masks over sorted positions.
+// in-support masks of a chunk's centres are computed once, and a centre's lower
+// list comes out of its own mask: each kept candidate below the centre's rank
+// sets its bit in a mask over the radix-sorted fluid positions. Visit rows and
+// lower rows are reserved one after the other. Dynamic shared memory:
+// Features[ucap]; uint32 s_ent[ucap] (slot | flags); uint32
+// s_vmask[(ucap / 32) * kChunk], which holds the staged words until the sort is
+// done; uint32 s_fluid[ucap / 32]; uint16 s_sorted[ucap]; uint16 s_rank[ucap],
+// until then the sort's scratch; then the sort's counters, whose place the
+// lower masks take. At 2,304 entries 74 KB, so three CTAs fit an SM.
 template <int DIM, uint32_t kChunk>
 __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks tk, StepConst k, uint32_t ucap,
                                                            const uint32_t* __restrict__ occ,
@@ -698,29 +885,37 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
     constexpr int NC = DIM == 3 ? 27 : 9;
     constexpr uint32_t kWays = kNlThreads / kChunk;
     extern __shared__ __align__(16) unsigned char smem[];
-    Stage st(reinterpret_cast<float*>(smem), ucap);
-    uint32_t* s_ent = reinterpret_cast<uint32_t*>(smem) + 4 * (size_t)ucap;
+    Features* st = reinterpret_cast<Features*>(smem);
+    uint32_t* s_ent = reinterpret_cast<uint32_t*>(st + ucap);
     uint32_t* s_vmask = s_ent + ucap;
-    uint16_t* s_sorted = reinterpret_cast<uint16_t*>(s_vmask + (ucap / 32) * kChunk);
-    uint32_t* s_lmask = reinterpret_cast<uint32_t*>(s_sorted + ucap);
-    uint16_t* s_tmp = reinterpret_cast<uint16_t*>(s_lmask);
-    uint16_t* s_cnt = s_tmp + ucap;
+    uint32_t* s_fluid = s_vmask + (ucap / 32) * kChunk;
+    uint16_t* s_sorted = reinterpret_cast<uint16_t*>(s_fluid + ucap / 32);
+    uint16_t* s_rank = s_sorted + ucap;
+    uint32_t* s_lmask = reinterpret_cast<uint32_t*>(s_rank + ucap);
+    uint32_t* s_w = s_vmask;
+    uint16_t* s_tmp = s_rank;
+    uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_lmask);
     __shared__ uint32_t s_cstart[NC];
     __shared__ uint32_t s_off[NC + 1];
     __shared__ uint32_t s_nf, s_omin, s_omax;
     __shared__ uint32_t s_cv[kWays][kChunk], s_cl[kWays][kChunk];
-    __shared__ uint32_t s_red[kWarps][2];
+    __shared__ uint32_t s_red[kWarps];
     __shared__ ChunkBlock s_blk;
     __shared__ bool s_overflow;
 
+    constexpr uint32_t kNoRank = 0xffffu;  // of a boundary candidate (a stage holds fewer)
     const float r2f = k.r2_filter;
+    const bool all = isinf(r2f);
+    const float inv_cell = (float)g.inv_cell;
     const uint32_t nocc = sc->nocc;
     const uint32_t tid = threadIdx.x;
-    const uint32_t lane = tid % kChunk, q = tid / kChunk;
+    const uint32_t lane = tid % kChunk, q = tid / kChunk, cb = lane & ~31u;
     uint32_t max_union = 0;
     if (tid == 0) s_overflow = false;
 
-    for (uint32_t it = blockIdx.x; it < nocc; it += gridDim.x) {
+    const uint32_t parts = cell_parts(nocc);
+    for (uint32_t item = blockIdx.x; item < nocc * parts; item += gridDim.x) {
+        const uint32_t it = item / parts, part = item - it * parts;
         if (tid == 0) {
             s_nf = 0;
             s_omin = 0xffffffffu;
@@ -737,21 +932,21 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
                 const uint32_t u = u0 + tid;
                 bool fluid = false;
                 if (u < U) {
-                    const uint32_t slot = slot_of_union<NC>(s_off, s_cstart, u);
-                    uint8_t fl;
-                    uint32_t o;
-                    const float4 p = stage_entry<DIM>(s, slot, cu, &fl, &o);
-                    st.put(u, p);
-                    s_ent[u] = slot | entry_flags(__float_as_uint(p.w));
-                    fluid = !(fl & kFlagBoundary);
+                    const uint32_t w = stage_candidate<DIM>(s, cu, inv_cell, slot_of_union<NC>(s_off, s_cstart, u), u,
+                                                            st, s_ent);
+                    s_w[u] = w;
+                    fluid = !(w & kStageBoundary);
                     if (fluid) {
-                        tmin = min(tmin, o);
-                        tmax = max(tmax, o);
+                        tmin = min(tmin, w & kStageOrigMask);
+                        tmax = max(tmax, w & kStageOrigMask);
                     }
                 }
                 const uint32_t fm = __ballot_sync(0xffffffffu, fluid);
                 uint32_t base = 0;
-                if ((tid & 31u) == 0 && fm) base = atomicAdd(&s_nf, (uint32_t)__popc(fm));
+                if ((tid & 31u) == 0) {
+                    if (fm) base = atomicAdd(&s_nf, (uint32_t)__popc(fm));
+                    if (u < U) s_fluid[u >> 5] = fm;
+                }
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (fluid) s_sorted[base + __popc(fm & ((1u << (tid & 31u)) - 1u))] = (uint16_t)u;
             }
@@ -763,138 +958,118 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
             }
             __syncthreads();
             const uint32_t nf = s_nf;
-            radix_sort_by_orig(st.w, s_sorted, s_tmp, s_cnt, nf, s_omin, s_omax);
-            // sorted positions past nf up to the next multiple of 32 read as
-            // union position 0: the lower-mask pass reads whole words (their
-            // bits past a centre's prefix are cleared)
-            for (uint32_t i = nf + tid; i < ((nf + 31u) & ~31u); i += blockDim.x) s_sorted[i] = 0;
+            radix_sort_by_orig(s_w, s_sorted, s_tmp, s_cnt, nf, s_omin, s_omax);
+            for (uint32_t u = 2u * tid; u < U; u += 2u * blockDim.x)
+                *reinterpret_cast<uint32_t*>(s_rank + u) = kNoRank | kNoRank << 16;
+            __syncthreads();
+            for (uint32_t i = tid; i < nf; i += blockDim.x) s_rank[s_sorted[i]] = (uint16_t)i;
             __syncthreads();
             const uint32_t W = (U + 31u) >> 5;
             const uint32_t wb = W * q / kWays, we = W * (q + 1) / kWays;
-            for (uint32_t c0 = 0; c0 < cu.ncenter; c0 += kChunk) {
+            for (uint32_t c0 = part * kChunk; c0 < cu.ncenter; c0 += parts * kChunk) {
                 const uint32_t nc = min(kChunk, cu.ncenter - c0);
                 const bool active = lane < nc;
                 const uint32_t myu = cu.center_off + c0 + lane;
+                // ---- pass 1: in-support masks of this share of the union words
+                // (no fluid in reach: no list to build)
+                if (cb < nc && !all && nf)
+                    centre_masks<kChunk>(st, s_vmask + cb, cu.center_off + c0 + cb, min(nc - cb, 32u), wb, we);
+                __syncwarp();
+                // R: the centre's lower list holds the kept fluid candidates of
+                // rank below R (all of them for a boundary centre)
                 bool fluidc = false;
-                uint32_t myo = 0, R = 0;
-                float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
-                // ---- pass 1a: visit masks of this quarter's union words (fluid centres)
+                uint32_t R = 0, cv = 0;
                 if (active) {
-                    me = st.get(myu);
-                    const uint32_t mw = __float_as_uint(me.w);
-                    fluidc = !(mw & kStageBoundary);
-                    myo = mw & kStageOrigMask;
-                    uint32_t cv = 0;
+                    const uint32_t rank = s_rank[myu];
+                    fluidc = rank != kNoRank;
+                    R = fluidc ? rank : nf;
                     if (fluidc) {
+                        cv = finish_masks<kChunk>(s_vmask + lane, s_fluid, U, myu, wb, we, all, k.keep_boundary);
+                    } else if (nf) {  // a boundary centre: the fluid candidates in reach, or all of them
                         for (uint32_t w = wb; w < we; ++w) {
-                            uint32_t m = k.keep_boundary ? word_mask<true>(st, w << 5, me, r2f)
-                                                         : word_mask<false>(st, w << 5, me, r2f);
-                            if (w == W - 1u && (U & 31u)) m &= (1u << (U & 31u)) - 1u;
-                            if (w == (myu >> 5)) m &= ~(1u << (myu & 31u));
+                            uint32_t m = s_fluid[w];
+                            if (!all && !k.keep_boundary) m &= s_vmask[w * kChunk + lane];
                             s_vmask[w * kChunk + lane] = m;
                             cv += __popc(m);
                         }
                     }
                     s_cv[q][lane] = cv;
-                    // R = sorted fluid positions below this particle's index
-                    // (all of them for a boundary particle)
-                    if (!fluidc) {
-                        R = nf;
-                    } else if (!k.lower_boundary_only) {
-                        uint32_t lo = 0, hi = nf;
-                        while (lo < hi) {
-                            const uint32_t mid = (lo + hi) >> 1;
-                            const uint32_t o = st.word(s_sorted[mid]) & kStageOrigMask;
-                            if (o < myo) lo = mid + 1;
-                            else hi = mid;
+                }
+                // this share of the lower mask's words, cleared
+                const bool lowers = !(fluidc && k.lower_boundary_only);
+                const uint32_t WR = lowers ? (R + 31u) >> 5 : 0u;
+                const uint32_t lb = WR * q / kWays, le = WR * (q + 1) / kWays;
+                if (active)
+                    for (uint32_t w = lb; w < le; ++w) s_lmask[w * kChunk + lane] = 0u;
+                __syncthreads();
+                // ---- the visit list: length, block, entries; lower bits
+                uint32_t nv = 0;
+                if (active && fluidc) {
+#pragma unroll
+                    for (uint32_t r = 0; r < kWays; ++r) nv += s_cv[r][lane];
+                }
+                const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, s_red, &s_blk, &s_overflow);
+                const uint32_t kslot = cu.cs + c0 + lane;
+                if (active && q == 0) {
+                    const uint32_t gv = (uint32_t)blk.base + lane;  // < pool_groups < 2^32 when ok
+                    l.desc[kslot] = blk.ok ? make_uint4(gv, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
+                    l.ncand[kslot] = fluidc ? U : 0u;
+                }
+                // Entries are split evenly over the threads (split by words, a
+                // few would hold most of the kept candidates).
+                const Share sh(nc);
+                {
+                    uint32_t n = 0;  // kept candidates
+#pragma unroll
+                    for (uint32_t r = 0; r < kWays; ++r) n += s_cv[r][sh.lane];
+                    const uint32_t v0 = sh.first(n), v1 = sh.last(n);
+                    if (v0 < v1) {
+                        const uint32_t rank = s_rank[cu.center_off + c0 + sh.lane];
+                        const bool fl = rank != kNoRank, put = blk.ok && fl;
+                        const uint32_t below = fl ? rank : nf, lower_below = fl && k.lower_boundary_only ? 0u : below;
+                        EntryOut out(l.pool + 4 * (size_t)(blk.base + sh.lane), 4u * nc, v0);
+                        uint32_t* const lm = s_lmask + sh.lane;
+                        MaskCursor<kChunk> cur(s_vmask, s_cv, sh.lane, W, v0);
+                        for (; out.t < v1; out.next()) {
+                            const uint32_t u = cur.next();
+                            const uint32_t r = s_rank[u];
+                            if (put) out.put(s_ent[u] | (r < below ? kEntryLower : 0u));
+                            if (r < lower_below) atomicOr(lm + (r >> 5) * kChunk, 1u << (r & 31u));
                         }
-                        R = lo;
                     }
                 }
-                __syncthreads();  // every quarter's visit words are in place
-                // ---- pass 1b: lower masks of this quarter's sorted words
-                const uint32_t WR = (R + 31u) >> 5;
-                const uint32_t lb = WR * q / kWays, le = WR * (q + 1) / kWays;
+                __syncthreads();  // every share's lower bits are in place
+                // ---- the lower list
                 if (active) {
-                    const float r2c = (!fluidc && k.keep_boundary) ? __int_as_float(0x7f800000) : r2f;
                     uint32_t cl = 0;
-                    for (uint32_t w = lb; w < le; ++w) {
-                        uint32_t m = 0;
-                        if (fluidc) {
-                            const uint4* sw = reinterpret_cast<const uint4*>(s_sorted + (w << 5));
-#pragma unroll
-                            for (int v = 0; v < 4; ++v) {
-                                const uint4 x = sw[v];
-                                const uint32_t pr[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                                for (int h = 0; h < 8; ++h) {
-                                    const uint32_t u = (pr[h >> 1] >> ((h & 1) * 16)) & 0xffffu;
-                                    m |= ((s_vmask[(u >> 5) * kChunk + lane] >> (u & 31u)) & 1u) << (v * 8 + h);
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int bit = 0; bit < 32; ++bit) {
-                                const uint32_t i = (w << 5) + bit;
-                                m |= within(st.get(s_sorted[i]), me, r2c) ? (1u << bit) : 0u;
-                            }
-                        }
-                        if (w == WR - 1u && (R & 31u)) m &= (1u << (R & 31u)) - 1u;
-                        s_lmask[w * kChunk + lane] = m;
-                        cl += __popc(m);
-                    }
+                    for (uint32_t w = lb; w < le; ++w) cl += __popc(s_lmask[w * kChunk + lane]);
                     s_cl[q][lane] = cl;
                 }
                 __syncthreads();
-                // ---- list lengths and the chunk's block
-                uint32_t nv = 0, nl = 0;
+                uint32_t nl = 0;
                 if (active) {
 #pragma unroll
-                    for (uint32_t r = 0; r < kWays; ++r) {
-                        nv += s_cv[r][lane];
-                        nl += s_cl[r][lane];
-                    }
+                    for (uint32_t r = 0; r < kWays; ++r) nl += s_cl[r][lane];
                 }
-                const ChunkBlock blk = reserve_chunk(l, sc, nc, nv, nl, s_red, &s_blk, &s_overflow);
-                // ---- pass 2: descriptors and entries
-                if (active) {
-                    const uint32_t kslot = cu.cs + c0 + lane;
-                    const uint32_t gv = (uint32_t)blk.base + lane;  // < pool_groups < 2^32 when ok
-                    const uint32_t gl = (uint32_t)(blk.base + (unsigned long long)blk.rows_a * nc) + lane;
-                    if (q == 0) {
-                        l.desc[kslot] = blk.ok ? make_uint4(gv, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
-                        l.ncand[kslot] = fluidc ? U : 0u;
-                        l.ldesc[kslot] = blk.ok ? make_uint2(gl, nl | (nc << 16)) : make_uint2(0u, 0u);
-                    }
-                    if (blk.ok) {
-                        const size_t step = 4u * nc;
-                        // Entries are split evenly over the centre's threads
-                        // (split by words, the middle ways would hold most of
-                        // the kept candidates).
-                        const uint32_t v0 = nv * q / kWays, v1 = nv * (q + 1u) / kWays;
-                        if (fluidc && v0 < v1) {
-                            uint32_t* pv = l.pool + 4 * (size_t)gv;
-                            MaskCursor<kChunk> cur(s_vmask, s_cv, lane, W, v0);
-                            for (uint32_t t = v0; t < v1; ++t) {
-                                const uint32_t u = cur.next();
-                                uint32_t e = s_ent[u];
-                                const uint32_t ow = st.word(u);
-                                e |= ow < myo ? kEntryLower : 0u;  // a boundary word has bit 31 set
-                                pv[(t >> 2) * step + (t & 3u)] = e;
-                            }
-                        }
-                        const uint32_t l0 = nl * q / kWays, l1 = nl * (q + 1u) / kWays;
-                        if (l0 < l1) {
-                            uint32_t* pl = l.pool + 4 * (size_t)gl;
-                            MaskCursor<kChunk> cur(s_lmask, s_cl, lane, WR, l0);
-                            for (uint32_t t = l0; t < l1; ++t)
-                                pl[(t >> 2) * step + (t & 3u)] = s_ent[s_sorted[cur.next()]] & kEntrySlotMask;
-                        }
+                const ChunkBlock lblk = reserve_chunk(l, sc, nc, nl, s_red, &s_blk, &s_overflow);
+                const bool ok = blk.ok && lblk.ok;
+                if (active && q == 0)
+                    l.ldesc[kslot] = ok ? make_uint2((uint32_t)lblk.base + lane, nl | (nc << 16)) : make_uint2(0u, 0u);
+                if (ok) {
+                    uint32_t n = 0;
+#pragma unroll
+                    for (uint32_t r = 0; r < kWays; ++r) n += s_cl[r][sh.lane];
+                    const uint32_t l0 = sh.first(n), l1 = sh.last(n);
+                    if (l0 < l1) {
+                        const uint32_t rank = s_rank[cu.center_off + c0 + sh.lane];
+                        EntryOut out(l.pool + 4 * (size_t)(lblk.base + sh.lane), 4u * nc, l0);
+                        MaskCursor<kChunk> cur(s_lmask, s_cl, sh.lane, ((rank != kNoRank ? rank : nf) + 31u) >> 5, l0);
+                        for (; out.t < l1; out.next()) out.put(s_ent[s_sorted[cur.next()]] & kEntrySlotMask);
                     }
                 }
                 __syncthreads();  // masks and counts are reused by the next chunk
             }
-        } else {
+        } else if (part == 0) {
             visit_slow<DIM, true>(k, r2f, cu, U, s, l, sc, s_cstart, s_off, s_red, &s_blk, &s_overflow);
             lower_slow<DIM>(k, r2f, cu, s, l, sc, s_cstart, s_off, s_red, &s_blk, &s_overflow);
         }
@@ -930,16 +1105,20 @@ __global__ void k_union_max(Tanks tk, const uint32_t* __restrict__ occ, const ui
 }
 
 size_t both_smem_bytes(uint32_t ucap, uint32_t chunk) {
-    const size_t sort = (size_t)ucap * sizeof(uint16_t) + 16 * kNlThreads * sizeof(uint16_t);
-    const size_t mask = (size_t)(ucap / 32) * chunk * sizeof(uint32_t);
-    return (size_t)ucap * (sizeof(float4) + sizeof(uint32_t) + sizeof(uint16_t)) + mask + (sort > mask ? sort : mask);
+    const size_t cnt = 16 * kNlThreads * sizeof(uint16_t), mask = (size_t)(ucap / 32) * chunk * sizeof(uint32_t);
+    return (size_t)ucap * (sizeof(Features) + sizeof(uint32_t) + 2 * sizeof(uint16_t)) + mask +
+           (ucap / 32) * sizeof(uint32_t) + (cnt > mask ? cnt : mask);
 }
 
 size_t visit_smem_bytes(uint32_t ucap, uint32_t chunk) {
     return (size_t)ucap * (sizeof(float4) + sizeof(uint32_t)) + (size_t)(ucap / 32) * chunk * sizeof(uint32_t);
 }
 
-uint32_t valid_chunk(uint32_t chunk) { return chunk == 32u ? 32u : kDefaultChunk; }
+// the tile a stage of ucap entries is built with
+uint32_t valid_chunk(uint32_t ucap, uint32_t chunk) {
+    if (chunk != 32u) chunk = kDefaultChunk;
+    return both_smem_bytes(ucap, chunk) > kMaxDynamicBytes ? 32u : chunk;
+}
 
 }  // namespace
 
@@ -957,7 +1136,7 @@ uint32_t nlist_union_capacity(uint32_t max_union) {
 }
 
 size_t nlist_smem_bytes(uint32_t ucap, uint32_t chunk) {
-    chunk = valid_chunk(chunk);
+    chunk = valid_chunk(ucap, chunk);
     const size_t a = visit_smem_bytes(ucap, chunk), b = both_smem_bytes(ucap, chunk);
     return a > b ? a : b;
 }
@@ -969,11 +1148,11 @@ uint32_t prepare_for(uint32_t ucap) {
     // so that no world's setting falls below another's launch
     const int sv = (int)visit_smem_bytes(ucap, C), sb = (int)both_smem_bytes(ucap, C);
     int bv = 0, bb = 0;
-    cudaFuncSetAttribute(k_nlist_visit<DIM, false, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)visit_smem_bytes(kMaxUnionStage, C));
+    cudaFuncSetAttribute(k_nlist_visit<DIM, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)std::min(visit_smem_bytes(kMaxUnionStage, C), kMaxDynamicBytes));
     cudaFuncSetAttribute(k_nlist_both<DIM, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)both_smem_bytes(kMaxUnionStage, C));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bv, k_nlist_visit<DIM, false, C>, kNlThreads, sv);
+                         (int)std::min(both_smem_bytes(kMaxUnionStage, C), kMaxDynamicBytes));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bv, k_nlist_visit<DIM, C>, kNlThreads, sv);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, k_nlist_both<DIM, C>, kNlThreads, sb);
     const int b = bv > bb ? bv : bb;
     return b > 0 ? (uint32_t)b : 1u;
@@ -984,7 +1163,7 @@ void launch_for(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32_t
                 const uint32_t* occ, const uint32_t* cell_start, const StateBufs& s, const ListBufs& l,
                 DeviceScalars* sc, cudaStream_t st, bool visit_only) {
     if (visit_only)
-        k_nlist_visit<DIM, false, C><<<nblocks, kNlThreads, visit_smem_bytes(ucap, C), st>>>(
+        k_nlist_visit<DIM, C><<<nblocks, kNlThreads, visit_smem_bytes(ucap, C), st>>>(
             g, tk, k, ucap, occ, cell_start, s, l, sc);
     else
         k_nlist_both<DIM, C><<<nblocks, kNlThreads, both_smem_bytes(ucap, C), st>>>(g, tk, k, ucap, occ,
@@ -993,7 +1172,7 @@ void launch_for(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32_t
 }  // namespace
 
 uint32_t nlist_prepare(int dim, uint32_t ucap, uint32_t chunk) {
-    chunk = valid_chunk(chunk);
+    chunk = valid_chunk(ucap, chunk);
     if (dim == 3) return chunk == 32u ? prepare_for<3, 32>(ucap) : prepare_for<3, 64>(ucap);
     return chunk == 32u ? prepare_for<2, 32>(ucap) : prepare_for<2, 64>(ucap);
 }
@@ -1009,7 +1188,7 @@ void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32
                   uint32_t nblocks, const uint32_t* occ, const uint32_t* cell_start,
                   const StateBufs& s, const ListBufs& l, DeviceScalars* sc, cudaStream_t st,
                   bool visit_only, uint32_t chunk) {
-    chunk = valid_chunk(chunk);
+    chunk = valid_chunk(ucap, chunk);
     if (g.dim == 3) {
         if (chunk == 32u) launch_for<3, 32>(g, tk, k, ucap, nblocks, occ, cell_start, s, l, sc, st, visit_only);
         else launch_for<3, 64>(g, tk, k, ucap, nblocks, occ, cell_start, s, l, sc, st, visit_only);
