@@ -275,6 +275,10 @@ int pe_fluid_dfsph_suggest_dt(PeDfsph* w, double* out);
 int pe_fluid_dfsph_rebuild_neighbours(PeDfsph* w);
 int pe_fluid_dfsph_compute_density(PeDfsph* w);
 int pe_fluid_dfsph_compute_alpha(PeDfsph* w);
+/* Lanes of a warp that share each particle's list in the pair passes (no
+ * reference counterpart): 0 (the default) picks them from the fluid count; 1, 8
+ * or 32 sets them, other values return PE_ERR_ARG. No choice changes a bit. */
+int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes);
 int pe_fluid_dfsph_len(const PeDfsph* w, uint64_t* out_len);
 int pe_fluid_dfsph_get_time(const PeDfsph* w, double* t);
 int pe_fluid_dfsph_get_last_dt(const PeDfsph* w, double* out);

@@ -32,8 +32,10 @@
 #include <algorithm>
 #include <cmath>
 #include <limits>
+#include <type_traits>
 
 #include "dfsph.cuh"
+#include "lane_group.cuh"
 #include "list_iter.cuh"
 
 namespace pe {
@@ -60,10 +62,16 @@ __device__ __forceinline__ bool sees(const DfsphConst& k, const double4& xb, con
 // A candidate beyond the kernel's support adds an exact +-0 to the gradient
 // and kernel sums (W and grad W vanish there); those sums skip it. The margin
 // on far2 keeps the test conservative under rounding.
-__device__ __forceinline__ bool far_pair(const DfsphConst& k, const double4& xi, const double4& xj) {
-    const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    return dx * dx + dy * dy + dz * dz > k.far2;
-}
+struct Offset {
+    double x, y, z, r2;
+    __device__ __forceinline__ Offset(const double4& xi, const double4& xj)
+        : x(xj.x - xi.x), y(xj.y - xi.y), z(xj.z - xi.z), r2(x * x + y * y + z * z) {}
+    __device__ __forceinline__ bool far(const DfsphConst& k) const { return r2 > k.far2; }
+};
+
+struct TwoStates {
+    double4 x, v;
+};
 
 // dfsph.rs:309-323 neighbour_mass_for
 __device__ __forceinline__ double nmass(const DfsphConst& k, const StateBufs& s, uint32_t e, const double4& xj,
@@ -98,33 +106,56 @@ __global__ void k_df_begin(uint32_t n, DfsphConst k, double dt, StateBufs s) {
     s.acc[i] = a;
 }
 
+// The pair passes run G lanes a slot (lane_group.cuh, df_lanes): a group's lanes
+// compute the terms of G consecutive entries, added in entry order, a skipped
+// entry as +0. Every lane of a warp stays to the end of each walk.
+
 // dfsph.rs:382-416 XSPH on v* (fluid neighbours)
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_xsph(uint32_t n, DfsphConst k, StateBufs s, ListBufs l,
                                                        double4* __restrict__ dv) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (is_boundary(s, i)) {
-        dv[i] = make_double4(0.0, 0.0, 0.0, 0.0);
-        return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !is_boundary(s, i);
+    if (i < n && !fluid && g.sub == 0) dv[i] = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0), vi = xi;
+    double rho_i = 0.0;
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        vi = s.acc[i];
+        rho_i = s.vel[i].w;
     }
-    const double4 xi = s.pos[i], vi = s.acc[i];
-    const double rho_i = s.vel[i].w;
-    double cx = 0.0, cy = 0.0, cz = 0.0;
-    for_each_entry(list_ref(l, i, kListVisit), [&](uint32_t e) {
-        if (e & kEntryBoundary) return;
-        const uint32_t j = e & kEntrySlotMask;
-        const double4 xj = s.pos[j];
-        if (far_pair(k, xi, xj)) return;
-        const double4 vj = s.acc[j];
-        const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const double wij = kfn_w(k.kf, sqrt(dx * dx + dy * dy + dz * dz));
-        const double rho_bar = 0.5 * (rho_i + s.vel[j].w);
-        const double f = k.mass / fmax(rho_bar, 1e-12) * wij;
-        cx = cx + (vj.x - vi.x) * f;
-        cy = cy + (vj.y - vi.y) * f;
-        cz = cz + (vj.z - vi.z) * f;
-    });
-    dv[i] = make_double4(cx * k.xsph_eps, cy * k.xsph_eps, cz * k.xsph_eps, 0.0);
+    struct Neighbour {
+        double4 x, v;
+        double rho;
+    };
+    OrderedSum<G, 3> c(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
+            const uint32_t j = e & kEntrySlotMask;
+            return Neighbour{gather4(s.pos + j), gather4(s.acc + j), s.vel[j].w};
+        },
+        [&](bool has, uint32_t e, const Neighbour& d, const uint32_t*) {
+            double t[3] = {0.0, 0.0, 0.0};
+            const Offset o(xi, d.x);
+            if (has && !(e & kEntryBoundary) && !o.far(k)) {
+                const double wij = kfn_w_r2(k.kf, o.r2);
+                const double rho_bar = 0.5 * (rho_i + d.rho);
+                const double f = quot_any(k.mass, fmax(rho_bar, 1e-12)) * wij;
+                t[0] = (d.v.x - vi.x) * f;
+                t[1] = (d.v.y - vi.y) * f;
+                t[2] = (d.v.z - vi.z) * f;
+            }
+            c.add(t);
+        });
+    double r[3];
+    c.totals(r);
+    if (fluid && g.sub == 0) dv[i] = make_double4(r[0] * k.xsph_eps, r[1] * k.xsph_eps, r[2] * k.xsph_eps, 0.0);
 }
 
 __global__ void k_df_xsph_apply(uint32_t n, StateBufs s, const double4* __restrict__ dv) {
@@ -155,44 +186,66 @@ __global__ void k_df_warm_zero(uint32_t n, int which, StateBufs s) {
     else s.acc[i].w = 0.0;
 }
 
-// dfsph.rs:326-351 density_derivative with v*
+// dfsph.rs:326-351 density_derivative of slot i with v* (every lane of the
+// group gets it; fluid: the group has a slot to do)
+template <int G>
 __device__ __forceinline__ double density_rate(const DfsphConst& k, const StateBufs& s, const ListBufs& l,
-                                               uint32_t i) {
-    const double4 xi = s.pos[i], vi = s.acc[i];
-    double drho = 0.0;
-    for_each_loaded(
-        list_ref(l, i, kListVisit), [&](uint32_t e) { return s.pos[e & kEntrySlotMask]; },
-        [&](uint32_t e, const double4& xj) {
-            if (far_pair(k, xi, xj)) return;
-            const double mj = nmass(k, s, e, xj, xi);
-            if (mj == 0.0) return;
+                                               const LaneGroup<G>& g, bool fluid, double* words) {
+    const uint32_t i = g.slot;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0), vi = xi;
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        vi = s.acc[i];
+    }
+    OrderedSum<G, 1> drho(words, g, 0.0);
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
             const uint32_t j = e & kEntrySlotMask;
-            double gx, gy, gz;
-            kfn_grad(k.kf, xj.x - xi.x, xj.y - xi.y, xj.z - xi.z, &gx, &gy, &gz);
-            const double4 vj = (e & kEntryBoundary) ? s.vel[j] : s.acc[j];
-            const double wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
-            drho += mj * (wx * gx + wy * gy + wz * gz);
+            return TwoStates{gather4(s.pos + j), gather4(((e & kEntryBoundary) ? s.vel : s.acc) + j)};
+        },
+        [&](bool has, uint32_t e, const TwoStates& d, const uint32_t*) {
+            double t[1] = {0.0};
+            const Offset o(xi, d.x);
+            if (has && !o.far(k)) {
+                const double mj = nmass(k, s, e, d.x, xi);
+                if (mj != 0.0) {
+                    const double sc = kfn_grad_scale(k.kf, o.r2);
+                    const double gx = o.x * sc, gy = o.y * sc, gz = o.z * sc;
+                    const double wx = vi.x - d.v.x, wy = vi.y - d.v.y, wz = vi.z - d.v.z;
+                    t[0] = mj * (wx * gx + wy * gy + wz * gz);
+                }
+            }
+            drho.add(t);
         });
-    return drho;
+    double r[1];
+    drho.totals(r);
+    return r[0];
 }
 
 // One error pass of a solver (dfsph.rs:552-569 density, 604-616 divergence):
 // kappa, the warm-start accumulation, the pressure diagnostic and the error
 // term of each particle in original order.
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_error(uint32_t n, DfsphConst k, int divergence, double dt,
                                                         double dt2, StateBufs s, ListBufs l,
                                                         const double* __restrict__ alpha, double* __restrict__ kappa,
                                                         double* __restrict__ kr, double* __restrict__ err_orig) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t o = s.orig[i];
-    if (is_boundary(s, i)) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !is_boundary(s, i);
+    if (i < n && !fluid && g.sub == 0) {
         kappa[i] = 0.0;
         kr[i] = 0.0 / k.rho0;  // dfsph.rs:462-469: kj = 0, rho_j = rho0
-        err_orig[o] = 0.0;
-        return;
+        err_orig[s.orig[i]] = 0.0;
     }
-    const double drho = density_rate(k, s, l, i);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    const double drho = density_rate<G>(k, s, l, g, fluid, s_words + g.warp * OrderedSum<G, 1>::kDoubles);
+    if (!fluid || g.sub != 0) return;
+    const uint32_t o = s.orig[i];
     double kap, e;
     if (!divergence) {
         const double rho_star = s.vel[i].w + dt * drho;
@@ -253,38 +306,65 @@ __global__ void k_df_serial_sum(uint32_t n, const double* __restrict__ v, double
 
 // dfsph.rs:422-530, fluid side: dv from kappa, the cap, the reaction total and
 // weight sum, v* += dv.
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, DfsphConst k, double dt,
                                                                  double inv_dt, StateBufs s, ListBufs l,
                                                                  const double* __restrict__ kr,
                                                                  double4* __restrict__ react) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (is_boundary(s, i)) return;
-    const double4 xi = s.pos[i];
-    const double kri = kr[i];  // ki / rho_i
-    double dx = 0.0, dy = 0.0, dz = 0.0, bx = 0.0, by = 0.0, bz = 0.0;
-    const ListRef lr = list_ref(l, i, kListVisit);
-    for_each_loaded(
-        lr, [&](uint32_t e) { return s.pos[e & kEntrySlotMask]; },
-        [&](uint32_t e, const double4& xj) {
-            if (far_pair(k, xi, xj)) return;
-            const double mj = nmass(k, s, e, xj, xi);
-            if (mj == 0.0) return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !is_boundary(s, i);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    double kri = 0.0;  // ki / rho_i
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        kri = kr[i];
+    }
+    // the sums over all neighbours, and over the boundary ones (exchanged only
+    // in rounds that have one)
+    double* const words = s_words + g.warp * 2u * OrderedSum<G, 3>::kDoubles;
+    OrderedSum<G, 3> all(words, g, 0.0), bnd(words + OrderedSum<G, 3>::kDoubles, g, 0.0);
+    struct Neighbour {
+        double4 x;
+        double kr;
+    };
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
             const uint32_t j = e & kEntrySlotMask;
-            double gx, gy, gz;
-            kfn_grad(k.kf, xj.x - xi.x, xj.y - xi.y, xj.z - xi.z, &gx, &gy, &gz);
-            const bool bnd = e & kEntryBoundary;
-            const double coeff = mj * (kri + kr[j]);  // mj (ki / rho_i + kj / rho_j)
-            const double tx = gx * coeff, ty = gy * coeff, tz = gz * coeff;
-            dx = dx + tx;
-            dy = dy + ty;
-            dz = dz + tz;
-            if (bnd) {
-                bx = bx + tx;
-                by = by + ty;
-                bz = bz + tz;
+            return Neighbour{gather4(s.pos + j), __ldg(kr + j)};
+        },
+        [&](bool has, uint32_t e, const Neighbour& d, const uint32_t*) {
+            double t[3] = {0.0, 0.0, 0.0}, tb[3] = {0.0, 0.0, 0.0};
+            bool b = false;
+            const Offset o(xi, d.x);
+            if (has && !o.far(k)) {
+                const double mj = nmass(k, s, e, d.x, xi);
+                if (mj != 0.0) {
+                    const double sc = kfn_grad_scale(k.kf, o.r2);
+                    const double coeff = mj * (kri + d.kr);  // mj (ki / rho_i + kj / rho_j)
+                    t[0] = (o.x * sc) * coeff;
+                    t[1] = (o.y * sc) * coeff;
+                    t[2] = (o.z * sc) * coeff;
+                    b = e & kEntryBoundary;
+                    if (b) {
+                        tb[0] = t[0];
+                        tb[1] = t[1];
+                        tb[2] = t[2];
+                    }
+                }
             }
+            all.add(t);
+            if (__any_sync(kFullWarp, b)) bnd.add(tb);
         });
+    double ra[3], rb[3];
+    all.totals(ra);
+    bnd.totals(rb);
+    double dx = ra[0], dy = ra[1], dz = ra[2], bx = rb[0], by = rb[1], bz = rb[2];
     dx = dx * (-dt);
     dy = dy * (-dt);
     dz = dz * (-dt);
@@ -305,23 +385,32 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, Df
     by = by * scale;
     bz = bz * scale;
     double4 rec = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (bx * bx + by * by + bz * bz > 0.0) {
-        double wsum = 0.0;
-        for_each_entry(lr, [&](uint32_t e) {
-            if (!(e & kEntryBoundary)) return;
-            const uint32_t j = e & kEntrySlotMask;
-            const double4 xj = s.pos[j];
-            const bool oriented = e & kEntryOriented;
-            if (!sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi)) return;
-            const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
-            const double r = sqrt(rx * rx + ry * ry + rz * rz);
-            wsum += fmin(1.0 / fmax(r, 1e-9), 1e6);
-        });
-        if (wsum > 0.0) {
+    const bool reacts = fluid && bx * bx + by * by + bz * bz > 0.0;
+    if (__any_sync(kFullWarp, reacts)) {
+        if (!reacts) lr.n = 0u;
+        OrderedSum<G, 1> wsum(words, g, 0.0);
+        __syncwarp();  // the words change hands
+        group_for_each<G>(
+            lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+            [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
+                double t[1] = {0.0};
+                const bool b = has && (e & kEntryBoundary);
+                if (b) {
+                    const bool oriented = e & kEntryOriented;
+                    const uint32_t j = e & kEntrySlotMask;
+                    if (sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi))
+                        t[0] = fmin(quot_any(1.0, fmax(sqrt(Offset(xi, xj).r2), 1e-9)), 1e6);
+                }
+                if (__any_sync(kFullWarp, b)) wsum.add(t);
+            });
+        double r[1];
+        wsum.totals(r);
+        if (reacts && r[0] > 0.0) {
             const double m = -k.mass * inv_dt;
-            rec = make_double4(bx * m, by * m, bz * m, wsum);
+            rec = make_double4(bx * m, by * m, bz * m, r[0]);
         }
     }
+    if (!fluid || g.sub != 0) return;
     react[i] = rec;
     double4 a = s.acc[i];
     a.x = a.x + dx;
@@ -332,29 +421,48 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, Df
 
 // dfsph.rs:508-517, boundary side: the reaction shares of the fluid
 // candidates, in ascending original index.
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_pressure_boundary(uint32_t n, DfsphConst k, StateBufs s,
                                                                     ListBufs l, const double4* __restrict__ react) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n || !is_boundary(s, j)) return;
-    const double4 xj = s.pos[j];
-    const bool oriented = s.flags[j] & kFlagOriented;
-    const double4 nj = oriented ? s.nout[j] : make_double4(0, 0, 0, 0);
-    double4 f = s.bf[j];
-    for_each_entry(list_ref(l, j, kListLower), [&](uint32_t e) {
-        const uint32_t i = e & kEntrySlotMask;
-        const double4 rec = react[i];
-        if (!(rec.w > 0.0)) return;
-        const double4 xi = s.pos[i];
-        if (!sees(k, xj, nj, oriented, xi)) return;
-        const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
-        const double r = sqrt(rx * rx + ry * ry + rz * rz);
-        const double wt = fmin(1.0 / fmax(r, 1e-9), 1e6);
-        const double sh = wt / rec.w;
-        f.x = f.x + rec.x * sh;
-        f.y = f.y + rec.y * sh;
-        f.z = f.z + rec.z * sh;
-    });
-    s.bf[j] = f;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t j = g.slot;
+    const bool bound = j < n && is_boundary(s, j);
+    if (!__any_sync(kFullWarp, bound)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xj = make_double4(0.0, 0.0, 0.0, 0.0), nj = xj, f = xj;
+    bool oriented = false;
+    if (bound) {
+        lr = list_ref(l, j, kListLower);
+        xj = s.pos[j];
+        f = s.bf[j];
+        oriented = s.flags[j] & kFlagOriented;
+        if (oriented) nj = s.nout[j];
+    }
+    const double start[3] = {f.x, f.y, f.z};
+    OrderedSum<G, 3> sum(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, start);
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
+            const uint32_t i = e & kEntrySlotMask;
+            return TwoStates{gather4(s.pos + i), gather4(react + i)};
+        },
+        [&](bool has, uint32_t, const TwoStates& d, const uint32_t*) {
+            const double4 &xi = d.x, &rec = d.v;
+            double t[3] = {0.0, 0.0, 0.0};
+            const bool adds = has && rec.w > 0.0 && sees(k, xj, nj, oriented, xi);
+            if (adds) {
+                const double wt = fmin(quot_any(1.0, fmax(sqrt(Offset(xi, xj).r2), 1e-9)), 1e6);
+                const double sh = quot_any(wt, rec.w);
+                t[0] = rec.x * sh;
+                t[1] = rec.y * sh;
+                t[2] = rec.z * sh;
+            }
+            if (__any_sync(kFullWarp, adds)) sum.add(t);
+        });
+    double r[3];
+    sum.totals(r);
+    if (bound && g.sub == 0) s.bf[j] = make_double4(r[0], r[1], r[2], f.w);
 }
 
 // dfsph.rs:742-748 x += v* dt (fluid; 2-D: z = 0)
@@ -395,70 +503,94 @@ __global__ void k_df_free_slip(uint32_t n, DfsphConst k, StateBufs s) {
 }
 
 // dfsph.rs:214-244 density with the oriented-boundary filter
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_density(uint32_t n, DfsphConst k, StateBufs s, ListBufs l) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (is_boundary(s, i)) {
-        s.vel[i].w = k.rho0;
-        return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !is_boundary(s, i);
+    if (i < n && !fluid && g.sub == 0) s.vel[i].w = k.rho0;
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
     }
-    const double4 xi = s.pos[i];
-    double rho = k.rho_self;
-    for_each_loaded(
-        list_ref(l, i, kListVisit), [&](uint32_t e) { return s.pos[e & kEntrySlotMask]; },
-        [&](uint32_t e, const double4& xj) {
-            if (far_pair(k, xi, xj)) return;
-            const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            const double wij = kfn_w(k.kf, sqrt(dx * dx + dy * dy + dz * dz));
-            if (!(e & kEntryBoundary)) {
-                rho += k.mass * wij;
-            } else {
-                const uint32_t j = e & kEntrySlotMask;
-                const bool oriented = e & kEntryOriented;
-                if (sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi))
-                    rho += k.rho0 * xj.w * wij;
+    OrderedSum<G, 1> rho(s_words + g.warp * OrderedSum<G, 1>::kDoubles, g, k.rho_self);
+    group_for_each<G>(
+        lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
+            double t[1] = {0.0};
+            const Offset o(xi, xj);
+            if (has && !o.far(k)) {
+                const double wij = kfn_w_r2(k.kf, o.r2);
+                if (!(e & kEntryBoundary)) {
+                    t[0] = k.mass * wij;
+                } else {
+                    const uint32_t j = e & kEntrySlotMask;
+                    const bool oriented = e & kEntryOriented;
+                    if (sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi))
+                        t[0] = k.rho0 * xj.w * wij;
+                }
             }
+            rho.add(t);
         });
-    s.vel[i].w = fmax(rho, 1e-12);
+    double r[1];
+    rho.totals(r);
+    if (fluid && g.sub == 0) s.vel[i].w = fmax(r[0], 1e-12);
 }
 
 // dfsph.rs:252-307 alpha = rho / max(|sum m grad W|^2 + sum |m grad W|^2, floor)
+template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_alpha(uint32_t n, DfsphConst k, StateBufs s, ListBufs l,
                                                         double* __restrict__ alpha) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (is_boundary(s, i)) {
-        alpha[i] = 0.0;
-        return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !is_boundary(s, i);
+    if (i < n && !fluid && g.sub == 0) alpha[i] = 0.0;
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
     }
-    const double4 xi = s.pos[i];
-    double sx = 0.0, sy = 0.0, sz = 0.0, sq = 0.0;
+    OrderedSum<G, 4> sum(s_words + g.warp * OrderedSum<G, 4>::kDoubles, g, 0.0);  // m grad W, |m grad W|^2
     uint32_t nb_all = 0, nb_kept = 0;
-    for_each_loaded(
-        list_ref(l, i, kListVisit), [&](uint32_t e) { return s.pos[e & kEntrySlotMask]; },
-        [&](uint32_t e, const double4& xj) {
-            const double mj = nmass(k, s, e, xj, xi);
-            if (e & kEntryBoundary) {
-                ++nb_all;
-                if (mj == 0.0) return;
-                ++nb_kept;
+    group_for_each<G>(
+        lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
+            if (has) {
+                const double mj = nmass(k, s, e, xj, xi);
+                const bool bnd = e & kEntryBoundary;
+                nb_all += bnd ? 1u : 0u;
+                nb_kept += bnd && mj != 0.0 ? 1u : 0u;
+                const Offset o(xi, xj);
+                if (!(bnd && mj == 0.0) && !o.far(k)) {
+                    const double sc = kfn_grad_scale(k.kf, o.r2);
+                    t[0] = (o.x * sc) * mj;
+                    t[1] = (o.y * sc) * mj;
+                    t[2] = (o.z * sc) * mj;
+                    t[3] = t[0] * t[0] + t[1] * t[1] + t[2] * t[2];
+                }
             }
-            if (far_pair(k, xi, xj)) return;
-            double gx, gy, gz;
-            kfn_grad(k.kf, xj.x - xi.x, xj.y - xi.y, xj.z - xi.z, &gx, &gy, &gz);
-            const double ax = gx * mj, ay = gy * mj, az = gz * mj;
-            sx = sx + ax;
-            sy = sy + ay;
-            sz = sz + az;
-            sq += ax * ax + ay * ay + az * az;
+            sum.add(t);
         });
+    nb_all = g.sum(nb_all);
+    nb_kept = g.sum(nb_kept);
+    double r[4];
+    sum.totals(r);
+    if (!fluid || g.sub != 0) return;
     // every fluid candidate but i itself, and the boundary ones of non-zero mass
     const uint32_t nn = (l.ncand[i] - 1u - nb_all) + nb_kept;
     if (nn < 2) {
         alpha[i] = 0.0;
         return;
     }
-    const double denom = fmax(sx * sx + sy * sy + sz * sz + sq, k.denom_floor);
+    const double denom = fmax(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3], k.denom_floor);
     alpha[i] = s.vel[i].w / denom;
 }
 
@@ -481,6 +613,24 @@ __global__ void k_df_export_orig(uint32_t n, const uint32_t* __restrict__ orig, 
     out[orig[i]] = src[i];
 }
 
+// Calls f(integral_constant<int, G>) for the lanes a slot of the pair passes.
+template <class F>
+void with_df_lanes(uint32_t lanes, F&& f) {
+    if (lanes == 1) f(std::integral_constant<int, 1>{});
+    else if (lanes == 8) f(std::integral_constant<int, 8>{});
+    else f(std::integral_constant<int, 32>{});
+}
+
+template <int G, int K>
+size_t df_smem(uint32_t sums = 1) {
+    return (size_t)sums * (kDfThreads / 32u) * OrderedSum<G, K>::kDoubles * sizeof(double);
+}
+
+template <int G>
+uint32_t df_blocks(uint32_t n) {
+    return blocks_for((uint64_t)n * G, kDfThreads);
+}
+
 }  // namespace
 
 DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim, double rest_density, double mass,
@@ -498,6 +648,7 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
             vs[3 * i + 2] = 0.0;
         }
     for (uint64_t i = 0; i < n; ++i) n_fluid_ += kind[i] == 0;
+    set_lanes(0);
     WorldParams wp{};
     wp.kernel = 0;
     wp.eos_rest_density = rest_density;
@@ -532,13 +683,25 @@ DfsphSolver::~DfsphSolver() {
     if (sum_host_) cudaFreeHost(sum_host_);
 }
 
+// ms for two steps with 1 / 8 / 32 lanes (16^3 fluid particles 15.0 / 4.2 / 2.7,
+// 36^3 24.1 / 13.0 / 14.1, 64^3 50.9 / 52.1 / 65.9, 90^3 102 / 130 / 172): many
+// lanes while the slots do not fill the chip, one where they do.
+void DfsphSolver::set_lanes(uint32_t lanes) {
+    if (lanes == 0) lanes = n_fluid_ <= 30000 ? 32u : n_fluid_ <= 230000 ? 8u : 1u;
+    if (lanes != 1 && lanes != 8 && lanes != 32) throw std::invalid_argument("lanes per slot");
+    df_lanes_ = lanes;
+}
+
 void DfsphSolver::rebuild_neighbours() { rebuild(); }
 
 void DfsphSolver::compute_density() {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     if (!n) return;
-    k_df_density<<<blocks_for(n, kDfThreads), kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_);
+    with_df_lanes(df_lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_df_density<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, 1>(), w.st_>>>(n, kc_, w.cur_, w.lists_);
+    });
     w.launches_ += 1;
 }
 
@@ -546,7 +709,11 @@ void DfsphSolver::compute_alpha() {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     if (!n) return;
-    k_df_alpha<<<blocks_for(n, kDfThreads), kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_, alpha_);
+    with_df_lanes(df_lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_df_alpha<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, (G < 4 ? 1 : 4)>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
+                                                                                            alpha_);
+    });
     w.launches_ += 1;
 }
 
@@ -646,31 +813,33 @@ void DfsphSolver::rebuild() {
 }
 
 void DfsphSolver::density_and_alpha() {
-    World& w = *w_;
-    const uint32_t n = (uint32_t)w.n_;
-    if (!n) return;
-    const uint32_t nb = blocks_for(n, kDfThreads);
-    k_df_density<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_);
-    k_df_alpha<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_, alpha_);
-    w.launches_ += 2;
+    compute_density();
+    compute_alpha();
 }
 
 void DfsphSolver::pressure_update(double dt, bool /*divergence*/) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
-    const uint32_t nb = blocks_for(n, kDfThreads);
     const double inv_dt = 1.0 / std::fmax(dt, 1e-12);
-    k_df_pressure_fluid<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, dt, inv_dt, w.cur_, w.lists_, kr_, react_);
-    k_df_pressure_boundary<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_, react_);
+    with_df_lanes(df_lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        constexpr int K = G < 3 ? 1 : 3;
+        k_df_pressure_fluid<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(2), w.st_>>>(n, kc_, dt, inv_dt, w.cur_,
+                                                                                         w.lists_, kr_, react_);
+        k_df_pressure_boundary<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
+                                                                                           react_);
+    });
     w.launches_ += 2;
 }
 
 double DfsphSolver::solve_error(double dt, bool divergence) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
-    const uint32_t nb = blocks_for(n, kDfThreads);
-    k_df_error<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, divergence ? 1 : 0, dt, dt * dt, w.cur_, w.lists_, alpha_,
-                                             kappa_, kr_, err_orig_);
+    with_df_lanes(df_lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_df_error<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, 1>(), w.st_>>>(
+            n, kc_, divergence ? 1 : 0, dt, dt * dt, w.cur_, w.lists_, alpha_, kappa_, kr_, err_orig_);
+    });
     k_df_partial_sums<<<kSumBlocks, kSumThreads, 0, w.st_>>>(n, err_orig_, part_);
     k_df_final_sum<<<1, kSumThreads, 0, w.st_>>>(part_, sum_);
     w.launches_ += 3;
@@ -765,7 +934,11 @@ void DfsphSolver::step(double dt_in) {
     k_df_begin<<<nb, kDfThreads, 0, st>>>(n, kc_, dt, w.cur_);
     w.launches_ += 1;
     if (prm_.xsph_epsilon != 0.0) {
-        k_df_xsph<<<nb, kDfThreads, 0, st>>>(n, kc_, w.cur_, w.lists_, dv_);
+        with_df_lanes(df_lanes_, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            k_df_xsph<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, (G < 3 ? 1 : 3)>(), st>>>(n, kc_, w.cur_, w.lists_,
+                                                                                            dv_);
+        });
         k_df_xsph_apply<<<nb, kDfThreads, 0, st>>>(n, w.cur_, dv_);
         w.launches_ += 2;
     }

@@ -57,6 +57,9 @@ class DfsphSolver {
     World& world() { return *w_; }
     const DfsphParams& params() const { return prm_; }
     void set_params(const DfsphParams& p);
+    // lanes of a warp on each slot's list in the pair passes: 1, 8 or 32, or 0
+    // to pick by the fluid count (the default); no choice changes a bit
+    void set_lanes(uint32_t lanes);
     double last_dt() const { return last_dt_; }
     // iterations of the last step's density and divergence solvers
     uint64_t last_density_iters() const { return it_density_; }
@@ -87,6 +90,7 @@ class DfsphSolver {
     DfsphParams prm_;
     DfsphConst kc_{};
     uint64_t n_fluid_ = 0;
+    uint32_t df_lanes_ = 1;  // lanes a slot of the pair passes: 1, 8 or 32
     double last_dt_ = 0.0;
     bool a_adv_set_ = false;  // the non-pressure accelerations (gravity) have been computed
     uint64_t it_density_ = 0, it_divergence_ = 0;

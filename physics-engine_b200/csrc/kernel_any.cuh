@@ -9,6 +9,7 @@
 
 #include <cmath>
 
+#include "exact_math.cuh"
 #include "pe_math.cuh"
 
 namespace pe {
@@ -19,6 +20,7 @@ struct KernelFn {
     int kind;
     double h, inv_h;  // inv_h = RN(1 / h)
     double alpha;     // the kind's normalisation for (h, dim)
+    int moderate;     // h is in the range of the block forms (exact_math.cuh)
 };
 
 // kernels.rs:32 support_radius
@@ -36,7 +38,7 @@ inline double kernel_alpha(int kind, double h, int dim) {
 }
 
 inline KernelFn make_kernel_fn(int kind, double h, int dim) {
-    return KernelFn{kind, h, 1.0 / h, kernel_alpha(kind, h, dim)};
+    return KernelFn{kind, h, 1.0 / h, kernel_alpha(kind, h, dim), h > 0x1p-60 && h < 0x1p60};
 }
 
 // RN(a / h): on the device by one multiply and a Markstein correction, on the
@@ -137,5 +139,54 @@ PE_HD void kfn_grad(const KernelFn& k, double rx, double ry, double rz, double* 
     *gy = ry * s;
     *gz = rz * s;
 }
+
+#if defined(__CUDACC__)
+// ---- W and grad W from r^2, the same bits, as one block where r^2 is moderate ----
+__device__ __forceinline__ double kdiv_h_block(double a, const KernelFn& k) {
+    const double q0 = a * k.inv_h;
+    return fma(fma(-q0, k.h, a), k.inv_h, q0);
+}
+
+// W(sqrt(r2))
+__device__ __forceinline__ double kfn_w_r2(const KernelFn& k, double r2) {
+    if (!(k.moderate && moderate(r2))) return kfn_w(k, sqrt(r2));
+    double r;
+    sqrt_rn(r2, &r);
+    if (k.kind != kCubic) return kfn_w(k, r);
+    const double q = kdiv_h_block(r, k), t = 2.0 - q;
+    const double in = k.alpha * (1.0 - 1.5 * q * q + 0.75 * q * q * q);
+    const double out = k.alpha * 0.25 * t * t * t;
+    return q < 1.0 ? in : q < 2.0 ? out : 0.0;
+}
+
+// grad W = (rx, ry, rz) s, s = -(dW/dr) / r at r = sqrt(r2); 0 for coincident points
+__device__ __forceinline__ double kfn_grad_scale(const KernelFn& k, double r2) {
+    if (k.moderate && moderate(r2)) {
+        double r;
+        const double y = sqrt_rn(r2, &r);
+        if (divisor_ok(r)) {
+            double n;
+            if (k.kind == kCubic) {
+                const double q = kdiv_h_block(r, k), t = 2.0 - q;
+                const double in = k.alpha * (-3.0 * q + 2.25 * q * q);
+                const double out = k.alpha * (-0.75 * t * t);
+                n = q < 2.0 ? kdiv_h_block(q < 1.0 ? in : out, k) : 0.0;
+            } else {
+                n = kfn_dwdr(k, r);
+            }
+            return quot_rn(-n, r, recip_refine(r, y));
+        }
+    }
+    if (k.h <= 0.0) return 0.0;
+    const double r = sqrt(r2);
+    return r < 1e-30 ? 0.0 : -kfn_dwdr(k, r) / r;
+}
+
+// a / d (a of moderate size or 0 takes the block form with a moderate d)
+__device__ __forceinline__ double quot_any(double a, double d) {
+    if (moderate_or_zero(a) && moderate(d) && divisor_ok(d)) return quot_rn(a, d, recip_rn(d));
+    return a / d;
+}
+#endif
 
 }  // namespace pe

@@ -33,11 +33,18 @@ struct LaneGroup {
     __device__ __forceinline__ uint32_t bits(uint32_t ballot) const {
         return G == 32 ? ballot : (ballot >> (grp * G)) & ((1u << (G % 32)) - 1u);
     }
+    // sum over the group's lanes, on each of them
+    __device__ __forceinline__ uint32_t sum(uint32_t v) const {
+#pragma unroll
+        for (uint32_t o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullWarp, v, o);
+        return v;
+    }
 };
 
-// K ordered sums per group; lane k < K of the group holds sum k.
+// K ordered sums per group (K <= G); lane k < K of the group holds sum k.
 template <int G, int K>
 struct OrderedSum {
+    static_assert(K <= G, "a lane a sum");
     // Terms t and t + 1 of a component form one 16-byte word; the words of one
     // pair index (a plane) are adjacent over groups and components, and planes
     // are padded so that a half warp's stores fall into different banks.
@@ -53,6 +60,12 @@ struct OrderedSum {
         : acc(start),
           put(warp_words + (g.sub >> 1) * kPlane + 2u * (g.grp * K) + (g.sub & 1u)),
           get(warp_words + 2u * (g.grp * K + min(g.sub, (uint32_t)K - 1u))), flip(0u), adds(g.sub < (uint32_t)K) {}
+    __device__ __forceinline__ OrderedSum(double* warp_words, const LaneGroup<G>& g, const double (&start)[K])
+        : OrderedSum(warp_words, g, 0.0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (g.sub == (uint32_t)k) acc = start[k];
+    }
     // Adds this round's G terms to each sum in lane order. Every lane of the
     // warp calls it.
     __device__ __forceinline__ void add(const double (&t)[K]) {
@@ -71,6 +84,34 @@ struct OrderedSum {
         }
         flip = kBuf - flip;
     }
+    // Every sum, on each lane of the group. Every lane of the warp calls it.
+    __device__ __forceinline__ void totals(double (&r)[K]) const {
+#pragma unroll
+        for (int k = 0; k < K; ++k) r[k] = __shfl_sync(kFullWarp, acc, k, G);
+    }
+};
+
+// One lane a slot: the sums are its own.
+template <int K>
+struct OrderedSum<1, K> {
+    static constexpr uint32_t kDoubles = 0u;
+    double acc[K];
+    __device__ __forceinline__ OrderedSum(double*, const LaneGroup<1>&, double start) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] = start;
+    }
+    __device__ __forceinline__ OrderedSum(double*, const LaneGroup<1>&, const double (&start)[K]) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] = start[k];
+    }
+    __device__ __forceinline__ void add(const double (&t)[K]) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[k] += t[k];
+    }
+    __device__ __forceinline__ void totals(double (&r)[K]) const {
+#pragma unroll
+        for (int k = 0; k < K; ++k) r[k] = acc[k];
+    }
 };
 
 __device__ __forceinline__ uint32_t warp_rounds(uint32_t n, uint32_t lanes) {
@@ -84,11 +125,11 @@ __device__ __forceinline__ uint32_t warp_rounds(uint32_t n, uint32_t lanes) {
 template <int G>
 struct GroupWalk {
     const uint32_t* p;
-    uint32_t step;  // between rounds (u32 units)
+    uint32_t step;  // between rounds (u32 units; one lane: from a row's end to the next row)
     uint32_t t, n;
     __device__ __forceinline__ GroupWalk(const ListRef& r, uint32_t sub)
-        : p(r.p + (sub < r.n ? (size_t)(sub >> 2) * r.step + (sub & 3u) : 0u)), step((G / 4) * r.step), t(sub),
-          n(r.n) {}
+        : p(r.p + (sub < r.n ? (size_t)(sub >> 2) * r.step + (sub & 3u) : 0u)),
+          step(G == 1 ? r.step - 3u : (G / 4) * r.step), t(sub), n(r.n) {}
     __device__ __forceinline__ bool has() const { return t < n; }
     __device__ __forceinline__ uint32_t peek() const {
         const uint32_t e = __ldg(p);
@@ -96,7 +137,7 @@ struct GroupWalk {
     }
     __device__ __forceinline__ void advance() {
         t += G;
-        if (t < n) p += step;
+        if (t < n) p += G > 1 || (t & 3u) == 0u ? step : 1u;  // one lane: along the row, then to the next
     }
 };
 

@@ -389,6 +389,14 @@ int pe_fluid_dfsph_step_adaptive(PeDfsph* w, double* dt_out) {
     });
 }
 
+int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes) {
+    if (!w) return PE_ERR_NULL;
+    return guard([&] {
+        w->s->set_lanes(lanes);
+        return PE_OK;
+    });
+}
+
 int pe_fluid_dfsph_suggest_dt(PeDfsph* w, double* out) {
     if (!w || !out) return PE_ERR_NULL;
     return guard([&] {

@@ -261,6 +261,7 @@ def load_library():
         "pe_fluid_dfsph_suggest_dt": (C.c_int, [vp, D3]),
         "pe_fluid_dfsph_rebuild_neighbours": (C.c_int, [vp]),
         "pe_fluid_dfsph_compute_density": (C.c_int, [vp]),
+        "pe_fluid_dfsph_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_dfsph_compute_alpha": (C.c_int, [vp]),
         "pe_fluid_dfsph_len": (C.c_int, [vp, C.POINTER(u64)]),
         "pe_fluid_dfsph_get_time": (C.c_int, [vp, D3]),
@@ -1094,6 +1095,11 @@ class DfsphWorld:
 
     def compute_alpha(self):
         _ok(_lib.pe_fluid_dfsph_compute_alpha(self._w), "dfsph_compute_alpha")
+
+    def set_lanes(self, lanes: int = 0):
+        """Lanes of a warp on each particle's list: 0 (the default) picks them
+        from the fluid count; 1, 8 or 32 sets them. The results are identical."""
+        _ok(_lib.pe_fluid_dfsph_set_lanes(self._w, int(lanes)), "dfsph_set_lanes")
 
     @property
     def t(self) -> float:

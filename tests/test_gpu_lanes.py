@@ -96,3 +96,38 @@ def test_unknown_lane_counts_are_refused():
         with pytest.raises(pe.PeError):
             w.set_lanes(lanes)
     w.close()
+
+
+@pytest.mark.parametrize("dim,kernel", [(3, 0), (3, 1), (2, 0)])
+def test_dfsph_lane_counts_bit_exact(dim, kernel):
+    """The divergence-free solver's pair passes with 1, 8 and 32 lanes: plates of oriented samples, warm start,
+    boundary reactions, lists whose lengths are no multiple of any lane count."""
+    dx = 0.05
+    mass = pe.mass_calibrated_to_rest(1000.0, dx, 2 * dx, dim)
+    ps, os_ = pe.Particles(dim, 1000.0, mass, 2 * dx), O.Scene(dim, 1000.0, mass, 2 * dx)
+    for s in (ps, os_):
+        s.fill_box((0.1, 0.1, 0.1 if dim == 3 else 0.0), 7, 6, 5 if dim == 3 else 1, dx)
+        s.jitter_fluid(9, 0.05 * dx)
+        s.fill_box_boundary((0.0, 0.0, 0.0), (0.6, 0.5, 0.5 if dim == 3 else 0.0), dx, 1)
+        for j in range(5):
+            wall = ((0.05, 0.1 + dx * j, 0.1 if dim == 3 else 0.0), 1e-4, (1.0 if j % 2 else -1.0, 0.0, 0.0))
+            s.push_boundary_oriented(*wall) if isinstance(s, pe.Particles) else s.push_boundary(*wall)
+    ps.recomputed_akinci_psi()
+    os_.recompute_psi()
+    p = pe.DfsphParams(kernel=kernel, adaptive_dt=False, particle_diameter=dx, max_density_iters=5,
+                       max_divergence_iters=5)
+    q = O.dfsph_default_params()
+    q.kernel, q.adaptive_dt, q.particle_diameter, q.max_density_iters, q.max_divergence_iters = kernel, 0, dx, 5, 5
+    o = O.DfsphWorld(os_, q)
+    o.run(1.0 / 240.0, 4)
+    for lanes in (0, 1, 8, 32):
+        w = pe.DfsphWorld(ps, p)
+        w.set_lanes(lanes)
+        w.compute_density()
+        w.compute_alpha()
+        w.run(1.0 / 240.0, 4)
+        for a, b, what in ((w.positions(), o.x(), "x"), (w.velocities(), o.v(), "v"), (w.densities(), o.rho(), "rho"),
+                           (w.boundary_forces(), o.boundary_force(), "boundary force"), (w.alphas(), o.alpha(), "alpha")):
+            assert_bits_equal(a, b, f"{lanes} lanes {what}")
+        assert w.last_iterations() == o.iterations()
+        w.close()
