@@ -56,7 +56,6 @@ struct EdgeHopArgs {
 bool edge_hop_prepare();
 void launch_edge_hop(const EdgeHopArgs& a, int sms, cudaStream_t st);
 
-size_t gemm_smem_bytes();
 bool gemm_prepare();
 void launch_gemm(const GemmArgs& g, int splits, cudaStream_t st);
 void launch_gemm_reduce(int M, int N, int ldc, int splits, const float* part, const float* bias, int relu,

@@ -90,32 +90,166 @@ __global__ void k_loss(int n, const float* __restrict__ Y, const float* __restri
 }
 
 // dZ (fp32 [R x N]) masked in place by mask > 0; bf16 copies dZ [R8 x N] and
-// dZ^T [N x R8] (zero-padded rows / columns); column sums into gbias
-__global__ void k_grad_prep(int R, int R8, int N, float* __restrict__ dZ, const __nv_bfloat16* __restrict__ mask,
-                            __nv_bfloat16* __restrict__ g16, __nv_bfloat16* __restrict__ gT,
-                            float* __restrict__ gbias) {
+// dZ^T [N x R8] (zero-padded rows / columns); column sums into gbias. A block
+// takes `tiles` tiles of 32 rows, so that a column's sum costs one atomic a
+// block: one a tile and row group put 306,000 edges' sums on 128 addresses
+// 9,556 x 8 times over (802 us of a pass that moves 470 MB). Unmasked, dZ stays
+// as it is and is not written back.
+__global__ void k_grad_prep(int R, int R8, int N, int tiles, float* __restrict__ dZ,
+                            const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ g16,
+                            __nv_bfloat16* __restrict__ gT, float* __restrict__ gbias) {
     __shared__ float tile[32][33];
-    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    __shared__ float sums[8][32];
+    const int c0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     float csum = 0.f;
-    for (int k = ty; k < 32; k += 8) {
-        const int r = r0 + k, c = c0 + tx;
-        float v = 0.f;
-        if (r < R && c < N) {
-            v = dZ[(size_t)r * N + c];
-            if (mask && !(__bfloat162float(mask[(size_t)r * N + c]) > 0.f)) v = 0.f;
-            dZ[(size_t)r * N + c] = v;
+    for (int t = 0; t < tiles; ++t) {
+        const int r0 = (blockIdx.x * tiles + t) * 32;
+        if (r0 >= R8) break;
+        for (int k = ty; k < 32; k += 8) {
+            const int r = r0 + k, c = c0 + tx;
+            float v = 0.f;
+            if (r < R && c < N) {
+                v = dZ[(size_t)r * N + c];
+                if (mask) {
+                    if (!(__bfloat162float(mask[(size_t)r * N + c]) > 0.f)) v = 0.f;
+                    dZ[(size_t)r * N + c] = v;
+                }
+            }
+            if (r < R8 && c < N) g16[(size_t)r * N + c] = __float2bfloat16_rn(v);
+            tile[k][tx] = v;
+            csum += v;
         }
-        if (r < R8 && c < N) g16[(size_t)r * N + c] = __float2bfloat16_rn(v);
-        tile[k][tx] = v;
-        csum += v;
+        __syncthreads();
+        for (int k = ty; k < 32; k += 8) {
+            const int c = c0 + k, r = r0 + tx;
+            if (c < N && r < R8) gT[(size_t)c * R8 + r] = __float2bfloat16_rn(tile[tx][k]);
+        }
+        __syncthreads();
     }
+    if (!gbias) return;
+    sums[ty][tx] = csum;
     __syncthreads();
-    for (int k = ty; k < 32; k += 8) {
-        const int c = c0 + k, r = r0 + tx;
-        if (c < N && r < R8) gT[(size_t)c * R8 + r] = __float2bfloat16_rn(tile[tx][k]);
+    if (ty == 0 && c0 + tx < N) {
+        float v = sums[0][tx];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += sums[k][tx];
+        if (v != 0.f) atomicAdd(&gbias[c0 + tx], v);
     }
-    if (gbias && c0 + tx < N && csum != 0.f) atomicAdd(&gbias[c0 + tx], csum);
+}
+
+// k_grad_prep for 128 columns, and with idx (rows gathered: dZ's row r is in's
+// row idx[r]; nothing is written back): a warp reads whole 512-byte rows, and
+// the transposed copy leaves through shared memory in 16-byte pieces. 64 rows a
+// tile. Bound by HBM: 306,000 rows move 400 to 550 MB in 101 us (202 us with
+// k_grad_prep, 802 before its sums were a block's, and 142 more for the gathered
+// copy it needed).
+constexpr int kPrepRows = 64;
+__global__ void __launch_bounds__(256) k_grad_prep128(int R, int R8, int tiles, float* __restrict__ dZ,
+                                                      const int* __restrict__ idx,
+                                                      const __nv_bfloat16* __restrict__ mask,
+                                                      __nv_bfloat16* __restrict__ g16, __nv_bfloat16* __restrict__ gT,
+                                                      float* __restrict__ gbias) {
+    // element (c, r) of the transposed tile; 16-byte piece p of column c at p ^ ((c / 4) & 7)
+    __shared__ __align__(16) __nv_bfloat16 tile[kWidth][kPrepRows];
+    __shared__ float4 sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = lane * 4;
+    float4 csum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = 0; t < tiles; ++t) {
+        const int r0 = (blockIdx.x * tiles + t) * kPrepRows;
+        if (r0 >= R8) break;
+#pragma unroll
+        for (int k = 0; k < kPrepRows / 8; ++k) {
+            const int lr = k * 8 + warp, r = r0 + lr;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < R) {
+                const size_t at = (size_t)r * kWidth + c0;
+                v = *reinterpret_cast<const float4*>(idx ? dZ + (size_t)idx[r] * kWidth + c0 : dZ + at);
+                if (mask) {
+                    const uint2 mb = *reinterpret_cast<const uint2*>(mask + at);
+                    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mb.x));
+                    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mb.y));
+                    if (!(a.x > 0.f)) v.x = 0.f;
+                    if (!(a.y > 0.f)) v.y = 0.f;
+                    if (!(b.x > 0.f)) v.z = 0.f;
+                    if (!(b.y > 0.f)) v.w = 0.f;
+                    *reinterpret_cast<float4*>(dZ + at) = v;
+                }
+            }
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            if (r < R8)
+                *reinterpret_cast<uint2*>(g16 + (size_t)r * kWidth + c0) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            const int at = (((lr >> 3) ^ (lane & 7)) << 3) | (lr & 7);
+            tile[c0][at] = lo.x;
+            tile[c0 + 1][at] = lo.y;
+            tile[c0 + 2][at] = hi.x;
+            tile[c0 + 3][at] = hi.y;
+            csum.x += v.x;
+            csum.y += v.y;
+            csum.z += v.z;
+            csum.w += v.w;
+        }
+        __syncthreads();
+        // eight lanes a column: its 64 rows are 128 contiguous bytes
+        for (int c = threadIdx.x >> 3; c < kWidth; c += 32) {
+            const int p = threadIdx.x & 7, r = r0 + p * 8;
+            if (r < R8)
+                *reinterpret_cast<uint4*>(gT + (size_t)c * R8 + r) =
+                    *reinterpret_cast<const uint4*>(&tile[c][(p ^ ((c >> 2) & 7)) << 3]);
+        }
+        __syncthreads();
+    }
+    if (!gbias) return;
+    sums[warp][lane] = csum;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            const float4 v = sums[k][lane];
+            csum.x += v.x;
+            csum.y += v.y;
+            csum.z += v.z;
+            csum.w += v.w;
+        }
+        atomicAdd(&gbias[c0], csum.x);
+        atomicAdd(&gbias[c0 + 1], csum.y);
+        atomicAdd(&gbias[c0 + 2], csum.z);
+        atomicAdd(&gbias[c0 + 3], csum.w);
+    }
+}
+
+// k_transpose for K a multiple of 16: a tile of 64 rows x 16 columns a warp,
+// 16-byte reads and writes through shared memory (306,000 x 128: 24 us, 76 with
+// 2-byte accesses; 157 MB at the copy rate take 24).
+__global__ void __launch_bounds__(256) k_transpose16(int R, int R8, int K, const __nv_bfloat16* __restrict__ X,
+                                                     __nv_bfloat16* __restrict__ XT) {
+    __shared__ __align__(16) __nv_bfloat16 tile[8][16][kPrepRows];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * kPrepRows, c0 = (blockIdx.y * 8 + warp) * 16;
+    if (c0 >= K) return;  // a whole warp; warps do not meet below
+    __nv_bfloat16(*t)[kPrepRows] = tile[warp];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {  // 16 rows a pass, two 16-byte halves a row
+        const int lr = k * 16 + (lane >> 1), h = lane & 1, r = r0 + lr;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (r < R) v = *reinterpret_cast<const uint4*>(X + (size_t)r * K + c0 + h * 8);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = h * 8 + j;
+            const uint16_t b = (uint16_t)(w[j >> 1] >> ((j & 1) * 16));
+            *reinterpret_cast<uint16_t*>(&t[c][(((lr >> 3) ^ (c & 7)) << 3) | (lr & 7)]) = b;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {  // eight lanes a column, four columns a pass
+        const int c = k * 4 + (lane >> 3), p = lane & 7, r = r0 + p * 8;
+        if (r < R8)
+            *reinterpret_cast<uint4*>(XT + (size_t)(c0 + c) * R8 + r) =
+                *reinterpret_cast<const uint4*>(&t[c][(p ^ (c & 7)) << 3]);
+    }
 }
 
 // X (bf16 [R x K]) -> X^T (bf16 [K x R8]), zero columns R..R8
@@ -149,13 +283,6 @@ __global__ void k_split_dxn(int n, const float* __restrict__ dH, const float* __
     const size_t node = i / kWidth, c = i % kWidth;
     dHp[i] = dH[i] + dXN[node * 2 * kWidth + c];
     da[i] = scale * dXN[node * 2 * kWidth + kWidth + c];
-}
-
-__global__ void k_gather_rows(int E, const int* __restrict__ idx, const float* __restrict__ in,
-                              float* __restrict__ out) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)E * kWidth) return;
-    out[i] = in[(size_t)idx[i / kWidth] * kWidth + i % kWidth];
 }
 
 __global__ void k_scatter_add(int E, const int* __restrict__ idx, const float* __restrict__ in,
@@ -534,14 +661,28 @@ void Surrogate::get_outputs(float* y) {
 }
 
 void Surrogate::linear_bwd(Linear& L, const __nv_bfloat16* X, int R, float* dZ, const __nv_bfloat16* mask,
-                           float* dX) {
+                           float* dX, const int* rows) {
     if (R <= 0) return;
     const int R8 = round8(R);
     dim3 tb(32, 8);
-    dim3 gz(blocks(R8, 32), blocks(L.Np, 32));
-    k_grad_prep<<<gz, tb, 0, st_>>>(R, R8, L.Np, dZ, mask, gb16_, gbT_, L.has_bias ? L.gb : nullptr);
-    dim3 gx(blocks(R8, 32), blocks(L.K, 32));
-    k_transpose<<<gx, tb, 0, st_>>>(R, R8, L.K, X, xT_);
+    // eight resident blocks an SM, up to 32 tiles each
+    float* const gb = L.has_bias ? L.gb : nullptr;
+    if (L.Np == kWidth) {
+        const int row_tiles = (int)blocks(R8, kPrepRows);
+        const int tiles = std::max(1, std::min(32, row_tiles / (8 * sms_)));
+        k_grad_prep128<<<blocks(row_tiles, tiles), 256, 0, st_>>>(R, R8, tiles, dZ, rows, mask, gb16_, gbT_, gb);
+    } else {
+        const int row_tiles = (int)blocks(R8, 32), col_tiles = (int)blocks(L.Np, 32);
+        const int tiles = std::max(1, std::min(32, row_tiles * col_tiles / (8 * sms_)));
+        dim3 gz(blocks(row_tiles, tiles), col_tiles);
+        k_grad_prep<<<gz, tb, 0, st_>>>(R, R8, L.Np, tiles, dZ, mask, gb16_, gbT_, gb);
+    }
+    if (L.K % 16 == 0) {
+        k_transpose16<<<dim3(blocks(R8, kPrepRows), blocks(L.K, 128)), 256, 0, st_>>>(R, R8, L.K, X, xT_);
+    } else {
+        dim3 gx(blocks(R8, 32), blocks(L.K, 32));
+        k_transpose<<<gx, tb, 0, st_>>>(R, R8, L.K, X, xT_);
+    }
     // dW^T [Np x K] = dZ^T [Np x R] * X [R x K]
     const int splits = std::max(1, std::min(64, R8 / 8192));
     gemm(gbT_, R8, xT_, R8, L.Np, L.K, R8, L.gWt, nullptr, L.K, nullptr, false, splits);
@@ -588,8 +729,7 @@ float Surrogate::train_step(float lr) {
         k_split_dxn<<<blocks(nW, 256), 256, 0, st_>>>(n, dH_, dXN_, kAggScale, dHp_, A_);
         if (E > 0) {
             const size_t eW = (size_t)E * kWidth;
-            k_gather_rows<<<blocks(eW, 256), 256, 0, st_>>>(E, g_.dst, A_, M_);
-            linear_bwd(layers_[base + 4], eh2_[l], E, M_, nullptr, dE2_);
+            linear_bwd(layers_[base + 4], eh2_[l], E, A_, nullptr, dE2_, g_.dst);  // the messages' rows of A_
             linear_bwd(layers_[base + 3], eh1_[l], E, dE2_, eh2_[l], dE_);
             linear_bwd(layers_[base + 2], g_.xe, E, dE_, eh1_[l], nullptr);  // masks dE_ to dZ1
             k_segsum<<<blocks((size_t)n * 32, 256), 256, 0, st_>>>(n, g_.row, dE_, 1.f, dP_);

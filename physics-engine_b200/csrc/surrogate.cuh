@@ -116,8 +116,10 @@ class Surrogate {
     void linear_fwd(const Linear& L, const __nv_bfloat16* X, int R, float* Yf, __nv_bfloat16* Yb, bool relu);
     void mlp_fwd(int first, const __nv_bfloat16* X, int R, __nv_bfloat16* A1, __nv_bfloat16* A2, float* Yf);
     // backward of one Linear: dZ fp32 [R x Np] (masked by mask > 0 if mask) ->
-    // grads; dX fp32 [R x K] if dX
-    void linear_bwd(Linear& L, const __nv_bfloat16* X, int R, float* dZ, const __nv_bfloat16* mask, float* dX);
+    // grads; dX fp32 [R x K] if dX. With rows (128 outputs, no mask) dZ's row r
+    // is row rows[r] of the array given.
+    void linear_bwd(Linear& L, const __nv_bfloat16* X, int R, float* dZ, const __nv_bfloat16* mask, float* dX,
+                    const int* rows = nullptr);
     void mlp_bwd(int first, const __nv_bfloat16* X, int R, const __nv_bfloat16* A1, const __nv_bfloat16* A2,
                  float* dY, float* dX);
     void adam(Linear& L, float lr);
