@@ -349,10 +349,11 @@ int pe_fluid_wcsph_get_sound_speeds(PeWcsph* w, double* out, uint32_t n_tanks);
  * out (may be NULL) = {density, forces, xsph block sizes, list CTAs per SM}. */
 int pe_fluid_wcsph_autotune(PeWcsph* w, uint32_t out[4]);
 int pe_fluid_wcsph_shapes(PeWcsph* w, uint32_t out[4]);
-/* Lanes of a warp that share each particle's neighbour list in the f64 step's
- * pair passes (no reference counterpart): 0 (the default) picks them per pass
- * from the particle counts; 1, 4, 8, 16 or 32 sets them all, other values
- * return PE_ERR_ARG. No choice changes a bit of the results. */
+/* Lanes of a warp that share each particle's neighbour list in the step's pair
+ * passes (no reference counterpart): 0 (the default) picks them per pass from
+ * the particle counts; 1, 4, 8, 16 or 32 (single precision: 1, 8 or 32) sets
+ * them all, other values return PE_ERR_ARG. No choice changes a bit of the
+ * results. */
 int pe_fluid_wcsph_set_lanes(PeWcsph* w, uint32_t lanes);
 
 /* The list build's tile in use: centre particles per chunk (32 or 64). */

@@ -11,6 +11,9 @@
 // re-expressed against the new cell after each sort). This form does not
 // reproduce the reference's bits; `bench.py --form f32` reports its error
 // against the f64 path.
+#include <type_traits>
+
+#include "lane_group.cuh"
 #include "list_iter.cuh"
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
@@ -26,6 +29,13 @@ struct Kahan {
     float s = 0.f, c = 0.f;
     __device__ __forceinline__ void add(float x) {
         const float y = x - c;
+        const float t = s + y;
+        c = (t - s) - y;
+        s = t;
+    }
+    // add(a b), the product fused with the compensation
+    __device__ __forceinline__ void add_product(float a, float b) {
+        const float y = fmaf(a, b, -c);
         const float t = s + y;
         c = (t - s) - y;
         s = t;
@@ -104,34 +114,31 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_density_f32(uint32_t n, F32
         if (!keep_w) atomicOr(l.w_short, 1u);
     }
     float* wrow = keep_w ? l.wpair32 + (vr.p - l.pool) : nullptr;
-    float w0 = 0.f, w1 = 0.f, w2 = 0.f;
-    for_each_loaded_t(
+    float w4[4] = {0.f, 0.f, 0.f, 0.f};
+    for_each_row<2>(
         vr,
-        [&](uint32_t, uint32_t e) {
+        [&](uint32_t e) {
             Nb32 b;
             b.p = f.pos[e & kEntrySlotMask];
             b.km = f.kmod[e & kEntrySlotMask];
             return b;
         },
-        [&](uint32_t t, uint32_t e, const Nb32& b) {
+        [](uint32_t) {},
+        [&](uint32_t q, uint32_t e, const Nb32& b) {
             const float4 pj = b.p;
             const float3 d = rel(ci, pi, b.km, pj, k.cell);
             const float r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
             const float w = w_f32(r, k);
-            if (keep_w) {
-                switch (t & 3u) {
-                    case 0: w0 = w; break;
-                    case 1: w1 = w; break;
-                    case 2: w2 = w; break;
-                    default:
-                        *reinterpret_cast<float4*>(wrow) = make_float4(w0, w1, w2, w);
-                        wrow += vr.step;
-                }
-            }
+            w4[q] = w;
             if ((e & kEntryOriented) && !sees_fluid_f32(k, s.nout[e & kEntrySlotMask], d)) return;
             rho.add(((e & kEntryBoundary) ? k.rho0 * pj.w : k.mass) * w);
+        },
+        [&](uint32_t) {
+            if (keep_w) {
+                *reinterpret_cast<float4*>(wrow) = make_float4(w4[0], w4[1], w4[2], w4[3]);
+                wrow += vr.step;
+            }
         });
-    if (keep_w && (vr.n & 3u)) *reinterpret_cast<float4*>(wrow) = make_float4(w0, w1, w2, 0.f);
     const float r = fmaxf(rho.s, 1e-12f);
     f.vel[i].w = r;
     s.vel[i].w = (double)r;
@@ -193,6 +200,65 @@ __global__ void k_pressure_f32(uint32_t n, F32Const k, Tanks tk, StateBufs s, F3
     const float p = b * (pw - 1.f);
     s.p[i] = (double)p;
     f.pos[i].w = p / (rho * rho);
+}
+
+// One pair of the force pass seen from fluid i: d = x_j - x_i and the factor of
+// d (fluid neighbour) or of d grad (boundary sample) in the acceleration.
+struct PairF32 {
+    float grad, scale;
+    bool counts;
+};
+
+__device__ __forceinline__ PairF32 force_pair_f32(const F32Const& k, const StateBufs& s, float nac, uint32_t ci,
+                                                  const float4& pi, const float4& vi, uint32_t e, const Nb32& b,
+                                                  float3* d_out) {
+    PairF32 t{0.f, 0.f, false};
+    const float4 pj = b.p;
+    const float3 d = rel(ci, pi, b.km, pj, k.cell);  // x_j - x_i
+    *d_out = d;
+    const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+    if (r2 < 1e-30f) return t;
+    const float inv_r = rsqrtf(r2);
+    const float r = r2 * inv_r;
+    t.grad = -dwdr_over_r_f32(r, inv_r, k);  // grad_i W = d * grad
+    if (e & kEntryBoundary) {
+        if ((e & kEntryOriented) && !sees_fluid_f32(k, s.nout[e & kEntrySlotMask], d)) return t;
+        t.scale = -(k.rho0 * pj.w) * pi.w;
+        t.counts = true;
+        return t;
+    }
+    const float4 vj = b.v;
+    const float press = pi.w + pj.w;
+    const float vr = (vi.x - vj.x) * -d.x + (vi.y - vj.y) * -d.y + (vi.z - vj.z) * -d.z;
+    float pic = 0.f;
+    if (vr < 0.f) {
+        const float mu = k.h * vr / (r2 + k.eps_h2);
+        pic = (nac * mu + k.visc_beta * mu * mu) * (2.f / (vi.w + vj.w));
+    }
+    t.scale = t.grad * -k.mass * (press + pic);
+    t.counts = true;
+    return t;
+}
+
+// Kick and drift of fluid slot i (symplectic Euler in cell-local single
+// precision) from its pair sums.
+template <int DIM>
+__device__ __forceinline__ void integrate_f32(const F32Const& k, const StateBufs& s, uint32_t i, const float4& pi,
+                                              const float4& vi, float ax, float ay, float az, float dt,
+                                              double4* __restrict__ pos_next, double4* __restrict__ vel_next) {
+    const int4 ki = s.key[i];
+    const float a_x = ax + k.gx, a_y = ay + k.gy, a_z = az + k.gz;
+    s.acc[i] = make_double4(a_x, a_y, a_z, 0.0);
+    float vx = vi.x + a_x * dt, vy = vi.y + a_y * dt, vz = vi.z + a_z * dt;
+    float lx = pi.x + vx * dt, ly = pi.y + vy * dt, lz = pi.z + vz * dt;
+    if (DIM == 2) {
+        lz = 0.f;
+        vz = 0.f;
+    }
+    // f64 position for the grid: key * cell + local, one f64 rounding
+    pos_next[i] = make_double4((double)ki.x * k.cell_d + (double)lx, (double)ki.y * k.cell_d + (double)ly,
+                               DIM == 2 ? 0.0 : (double)ki.z * k.cell_d + (double)lz, s.pos[i].w);
+    vel_next[i] = make_double4(vx, vy, vz, vi.w);
 }
 
 template <int DIM>
@@ -327,31 +393,251 @@ __global__ void __launch_bounds__(kMaxPassThreads) k_xsph_f32_w(uint32_t n, F32C
     Kahan dx, dy, dz;
     const ListRef vr = list_ref(l, i, kListVisit);
     const float* wrow = l.wpair32 + (vr.p - l.pool);
-    struct VelW {
-        float4 v;
-        float w;
-    };
-    auto load = [&](uint32_t t, uint32_t e) {  // t = 0, 1, 2, ... in order
-        VelW b{};
-        if (!(e & kEntryBoundary)) {
-            b.v = f.vel[e & kEntrySlotMask];
-            b.w = __ldg(wrow + (t & 3u));
-        }
-        if ((t & 3u) == 3u) wrow += vr.step;
-        return b;
-    };
-    for_each_loaded_t(vr, load, [&](uint32_t, uint32_t e, const VelW& b) {
-        if (e & kEntryBoundary) return;
-        const float4 vj = b.v;
-        const float g = k.mass * 2.f / (vi.w + vj.w) * b.w;
-        dx.add((vj.x - vi.x) * g);
-        dy.add((vj.y - vi.y) * g);
-        dz.add((vj.z - vi.z) * g);
-    });
+    float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    for_each_row<1>(
+        vr, [&](uint32_t e) { return f.vel[e & kEntrySlotMask]; },
+        [&](uint32_t) {
+            w4 = __ldg(reinterpret_cast<const float4*>(wrow));
+            wrow += vr.step;
+        },
+        [&](uint32_t q, uint32_t e, const float4& vj) {
+            if (e & kEntryBoundary) return;
+            const float w = q == 0 ? w4.x : q == 1 ? w4.y : q == 2 ? w4.z : w4.w;
+            const float g = k.mass * 2.f / (vi.w + vj.w) * w;
+            dx.add((vj.x - vi.x) * g);
+            dy.add((vj.y - vi.y) * g);
+            dz.add((vj.z - vi.z) * g);
+        },
+        [](uint32_t) {});
     const float4 vn = make_float4(vi.x + dx.s * k.xsph_eps, vi.y + dy.s * k.xsph_eps,
                                   vi.z + dz.s * k.xsph_eps, vi.w);
     vel_out[i] = vn;
     s.vel[i] = make_double4(vn.x, vn.y, vn.z, vn.w);
+}
+
+// ---------------------------------------------------------------------------
+// The passes with G lanes a slot (lane_group.cuh), while the slots do not fill
+// the chip. A compensated sum is no sum of rounded terms: the product that makes
+// a term is fused with the subtraction of the compensation, and a skipped entry
+// is not an added zero (a zero added can move a tie). So the lanes exchange the
+// two factors of each term and which entries count, and the sums come out bit
+// for bit as one thread's.
+// ---------------------------------------------------------------------------
+template <int G, int K>
+struct OrderedKahan {
+    static constexpr uint32_t kPitch = G + 4u;  // floats between a group's components
+    static constexpr uint32_t kBuf = (32u / G) * (K + 1) * kPitch;
+    static constexpr uint32_t kFloats = 2u * kBuf;  // per warp
+    Kahan sum;
+    float *put, *get_a, *get_b;
+    uint32_t flip;
+    bool adds;
+    __device__ __forceinline__ OrderedKahan(float* warp_words, const LaneGroup<G>& g, float start) : flip(0u) {
+        float* const base = warp_words + g.grp * (K + 1) * kPitch;
+        sum.s = start;
+        put = base + g.sub;
+        get_a = base + min(g.sub, (uint32_t)K - 1u) * kPitch;
+        get_b = base + K * kPitch;
+        adds = g.sub < (uint32_t)K;
+    }
+    // Adds a[k] b of this round's entries with `counts` to sum k, in lane order.
+    __device__ __forceinline__ void add(const LaneGroup<G>& g, const float (&a)[K], float b, bool counts) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) put[flip + k * kPitch] = a[k];
+        put[flip + K * kPitch] = b;
+        const uint32_t m = g.bits(__ballot_sync(kFullWarp, counts));
+        __syncwarp();
+        if (adds) {
+#pragma unroll
+            for (int j = 0; j < G / 4; ++j) {
+                const float4 va = *reinterpret_cast<const float4*>(get_a + flip + 4 * j);
+                const float4 vb = *reinterpret_cast<const float4*>(get_b + flip + 4 * j);
+                const float x[4] = {va.x, va.y, va.z, va.w}, y[4] = {vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (m & (1u << (4 * j + q))) sum.add_product(x[q], y[q]);
+            }
+        }
+        flip = kBuf - flip;
+    }
+    // Sum k, on each lane of the group. Every lane of the warp calls it.
+    __device__ __forceinline__ float total(int k) const { return __shfl_sync(kFullWarp, sum.s, k, G); }
+};
+
+template <int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_density_f32_g(uint32_t n, F32Const k, StateBufs s, F32Bufs f,
+                                                                   ListBufs l) {
+    extern __shared__ __align__(16) float s_floats[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) f.vel[i].w = k.rho0;
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef vr{l.pool, 0u, 0u};
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t ci = 0;
+    bool keep_w = false;
+    if (fluid) {
+        vr = list_ref(l, i, kListVisit);
+        pi = f.pos[i];
+        ci = f.kmod[i];
+        if (l.wpair32) {
+            keep_w = w_fits(l, vr);
+            if (!keep_w && g.sub == 0) atomicOr(l.w_short, 1u);
+        }
+    }
+    OrderedKahan<G, 1> rho(s_floats + g.warp * OrderedKahan<G, 1>::kFloats, g, k.rho_self);
+    group_for_each<G>(
+        vr, g,
+        [&](uint32_t e, const uint32_t*) {
+            Nb32 b;
+            b.p = f.pos[e & kEntrySlotMask];
+            b.km = f.kmod[e & kEntrySlotMask];
+            return b;
+        },
+        [&](bool has, uint32_t e, const Nb32& b, const uint32_t* p) {
+            const float3 d = rel(ci, pi, b.km, b.p, k.cell);
+            const float r = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+            const float w = w_f32(r, k);
+            if (has && keep_w) l.wpair32[p - l.pool] = w;
+            const bool counts =
+                has && !((e & kEntryOriented) && !sees_fluid_f32(k, s.nout[e & kEntrySlotMask], d));
+            const float m[1] = {(e & kEntryBoundary) ? k.rho0 * b.p.w : k.mass};
+            rho.add(g, m, w, counts);
+        });
+    if (fluid && g.sub == 0) {
+        const float r = fmaxf(rho.sum.s, 1e-12f);
+        f.vel[i].w = r;
+        s.vel[i].w = (double)r;
+    }
+}
+
+template <int DIM, int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_forces_f32_g(uint32_t n, F32Const k, Tanks tk, StateBufs s,
+                                                                  F32Bufs f, ListBufs l, float dt,
+                                                                  double4* __restrict__ pos_next,
+                                                                  double4* __restrict__ vel_next,
+                                                                  float* __restrict__ bf) {
+    extern __shared__ __align__(16) float s_floats[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef vr{l.pool, 0u, 0u};
+    float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = make_float4(0.f, 0.f, 0.f, 1.f);
+    uint32_t ci = 0;
+    float nac = 0.f;
+    if (fluid) {
+        vr = list_ref(l, i, kListVisit);
+        pi = f.pos[i];
+        vi = f.vel[i];
+        ci = f.kmod[i];
+        const float c0 = (float)tk.c[tk.slot_tank[i]];
+        nac = -k.visc_alpha * c0;
+    }
+    OrderedKahan<G, 3> acc(s_floats + g.warp * OrderedKahan<G, 3>::kFloats, g, 0.f);
+    group_for_each<G>(
+        vr, g,
+        [&](uint32_t e, const uint32_t*) {
+            Nb32 b;
+            b.p = f.pos[e & kEntrySlotMask];
+            b.km = f.kmod[e & kEntrySlotMask];
+            b.v = f.vel[e & kEntrySlotMask];
+            return b;
+        },
+        [&](bool has, uint32_t e, const Nb32& b, const uint32_t*) {
+            float a[3] = {0.f, 0.f, 0.f}, m = 0.f;
+            bool counts = false;
+            if (has) {
+                float3 d;
+                const PairF32 t = force_pair_f32(k, s, nac, ci, pi, vi, e, b, &d);
+                counts = t.counts;
+                if (counts) {
+                    a[0] = d.x;
+                    a[1] = d.y;
+                    a[2] = d.z;
+                    m = t.scale;
+                    if (e & kEntryBoundary) {  // the rounded force is the term
+                        a[0] = d.x * t.grad * m;
+                        a[1] = d.y * t.grad * m;
+                        a[2] = d.z * t.grad * m;
+                        m = 1.f;
+                        if (bf) {
+                            const size_t j = 4 * (size_t)(e & kEntrySlotMask);
+                            atomicAdd(&bf[j], a[0] * -k.mass);
+                            atomicAdd(&bf[j + 1], a[1] * -k.mass);
+                            atomicAdd(&bf[j + 2], a[2] * -k.mass);
+                        }
+                    }
+                }
+            }
+            acc.add(g, a, m, counts);
+        });
+    const float ax = acc.total(0), ay = acc.total(1), az = acc.total(2);
+    if (fluid && g.sub == 0)
+        integrate_f32<DIM>(k, s, i, pi, vi, ax, ay, az, dt, pos_next, vel_next);
+}
+
+// USE_W: each pair's W read from the density pass (k_xsph_f32_w), otherwise
+// recomputed (k_xsph_f32, short_only as there).
+template <bool USE_W, int G>
+__global__ void __launch_bounds__(kMaxPassThreads) k_xsph_f32_g(uint32_t n, F32Const k, StateBufs s, F32Bufs f,
+                                                                ListBufs l, float4* __restrict__ vel_out,
+                                                                bool short_only) {
+    extern __shared__ __align__(16) float s_floats[];
+    if (USE_W ? __ldg(l.w_short) != 0u : short_only && !__ldg(l.w_short)) return;
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) vel_out[i] = f.vel[i];
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef vr{l.pool, 0u, 0u};
+    float4 vi = make_float4(0.f, 0.f, 0.f, 1.f), pi = vi;
+    uint32_t ci = 0;
+    if (fluid) {
+        vr = list_ref(l, i, kListVisit);
+        vi = f.vel[i];
+        if (!USE_W) {
+            pi = f.pos[i];
+            ci = f.kmod[i];
+        }
+    }
+    struct VelW {
+        float4 v, p;
+        uint32_t km;
+        float w;
+    };
+    OrderedKahan<G, 3> dv(s_floats + g.warp * OrderedKahan<G, 3>::kFloats, g, 0.f);
+    group_for_each<G>(
+        vr, g,
+        [&](uint32_t e, const uint32_t* p) {
+            VelW b{};
+            const uint32_t j = e & kEntrySlotMask;
+            b.v = f.vel[j];
+            if (USE_W) {
+                b.w = __ldg(l.wpair32 + (p - l.pool));
+            } else {
+                b.p = f.pos[j];
+                b.km = f.kmod[j];
+            }
+            return b;
+        },
+        [&](bool has, uint32_t e, const VelW& b, const uint32_t*) {
+            float w = b.w;
+            if (!USE_W) {
+                const float3 d = rel(ci, pi, b.km, b.p, k.cell);
+                w = w_f32(sqrtf(d.x * d.x + d.y * d.y + d.z * d.z), k);
+            }
+            const float m = k.mass * 2.f / (vi.w + b.v.w) * w;
+            const float a[3] = {b.v.x - vi.x, b.v.y - vi.y, b.v.z - vi.z};
+            dv.add(g, a, m, has && !(e & kEntryBoundary));
+        });
+    const float dx = dv.total(0), dy = dv.total(1), dz = dv.total(2);
+    if (fluid && g.sub == 0) {
+        const float4 vn = make_float4(vi.x + dx * k.xsph_eps, vi.y + dy * k.xsph_eps, vi.z + dz * k.xsph_eps, vi.w);
+        vel_out[i] = vn;
+        s.vel[i] = make_double4(vn.x, vn.y, vn.z, vn.w);
+    }
 }
 
 // Cell-local single-precision state from the (sorted) f64 state.
@@ -376,14 +662,58 @@ __global__ void k_bf_to_f64(uint32_t n, const float* __restrict__ bf, StateBufs 
 
 }  // namespace
 
+// Lanes of a particle's list in the three pair passes. One lane a particle
+// streams its rows best once the particles alone fill the chip; below that the
+// walk of one list is the pass's length, and 8 lanes (32 for the smallest
+// scenes) shorten it. Cubes of the dam break, us a pass, 1 / 8 / 32 lanes:
+//   particles   density          forces           XSPH
+//         216   56 / 21 / 13     101 / 31 / 20    51 / 21 / 16
+//       2,197   62 / 22 / 18     112 / 32 / 27    61 / 22 / 20
+//       6,859   64 / 28 / 30     112 / 40 / 40    64 / 26 / 31
+//      32,768   73 / 62 / 100    132 / 83 / 119   74 / 56 / 94
+//      68,921   91 / 110 / 198   171 / 144 / 228  100 / 98 / 181
+//     125,000   134 / 186 / 351  250 / 242 / 401  111 / 161 / 320
+//   2-D   900   17 / 10 / 9      33 / 18 / 14     18 / 12 / 13
+//       6,400   18 / 11 / 13     34 / 18 / 22     21 / 13 / 17
+//      40,000   19 / 20 / 39     38 / 31 / 53     23 / 22 / 43
+// (Four lanes were slower than one or eight at every size.)
+PassLanes pass_lanes_f32(int dim, uint64_t fluid) {
+    const uint64_t few = dim == 2 ? 2048 : 4096;
+    const auto rule = [&](uint64_t eight) { return fluid <= few ? 32u : fluid <= eight ? 8u : 1u; };
+    PassLanes r;
+    r.density = rule(dim == 2 ? 32768 : 49152);
+    r.forces = rule(98304);
+    r.xsph = rule(dim == 2 ? 40960 : 65536);
+    return r;
+}
+
+template <class F>
+static void with_f32_lanes(uint32_t lanes, F&& f) {
+    if (lanes == 8) f(std::integral_constant<int, 8>{});
+    else f(std::integral_constant<int, 32>{});
+}
+
+template <int G, int K>
+static size_t kahan_smem(uint32_t threads) {
+    return (size_t)(threads / 32u) * OrderedKahan<G, K>::kFloats * sizeof(float);
+}
+
 void launch_f32_from_f64(uint32_t n, double cell, const StateBufs& s, const F32Bufs& f,
                          cudaStream_t st) {
     if (n) k_f32_from_f64<<<blocks_for(n, 256), 256, 0, st>>>(n, cell, s, f);
 }
 
-void launch_density_f32(uint32_t n, uint32_t threads, const F32Const& k, const StateBufs& s,
+void launch_density_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const StateBufs& s,
                         const F32Bufs& f, const ListBufs& l, cudaStream_t st) {
-    if (n) k_density_f32<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, f, l);
+    if (!n) return;
+    if (lanes == 1) {
+        k_density_f32<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, f, l);
+        return;
+    }
+    with_f32_lanes(lanes, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_density_f32_g<G><<<blocks_for((uint64_t)n * G, threads), threads, kahan_smem<G, 1>(threads), st>>>(n, k, s, f, l);
+    });
 }
 
 void launch_pressure_f32(uint32_t n, const F32Const& k, const Tanks& tk, const StateBufs& s,
@@ -393,24 +723,42 @@ void launch_pressure_f32(uint32_t n, const F32Const& k, const Tanks& tk, const S
     k_pressure_f32<<<blocks_for(n, 256), 256, 0, st>>>(n, k, tk, s, f);
 }
 
-void launch_forces_f32(uint32_t n, uint32_t threads, const F32Const& k, const Tanks& tk,
+void launch_forces_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const Tanks& tk,
                        const StateBufs& s, const F32Bufs& f, const ListBufs& l, float dt,
                        double4* pos_next, double4* vel_next, float* bf, cudaStream_t st) {
     if (!n) return;
     if (bf) cudaMemsetAsync(bf, 0, sizeof(float) * 4 * (size_t)n, st);
     const uint32_t b = blocks_for(n, threads);
-    if (k.dim == 3)
+    if (lanes != 1) {
+        with_f32_lanes(lanes, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            const uint32_t bg = blocks_for((uint64_t)n * G, threads);
+            const size_t sm = kahan_smem<G, 3>(threads);
+            if (k.dim == 3) k_forces_f32_g<3, G><<<bg, threads, sm, st>>>(n, k, tk, s, f, l, dt, pos_next, vel_next, bf);
+            else k_forces_f32_g<2, G><<<bg, threads, sm, st>>>(n, k, tk, s, f, l, dt, pos_next, vel_next, bf);
+        });
+    } else if (k.dim == 3)
         k_forces_f32<3><<<b, threads, 0, st>>>(n, k, tk, s, f, l, dt, pos_next, vel_next, bf);
     else
         k_forces_f32<2><<<b, threads, 0, st>>>(n, k, tk, s, f, l, dt, pos_next, vel_next, bf);
     if (bf) k_bf_to_f64<<<blocks_for(n, 256), 256, 0, st>>>(n, bf, s);
 }
 
-void launch_xsph_f32(uint32_t n, uint32_t threads, const F32Const& k, const StateBufs& s,
+void launch_xsph_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const StateBufs& s,
                      const F32Bufs& f, const ListBufs& l, float4* vel_out, cudaStream_t st,
                      bool use_w) {
     if (!n) return;
     const bool w = use_w && l.wpair32;
+    if (lanes != 1) {
+        with_f32_lanes(lanes, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            const uint32_t b = blocks_for((uint64_t)n * G, threads);
+            const size_t sm = kahan_smem<G, 3>(threads);
+            if (w) k_xsph_f32_g<true, G><<<b, threads, sm, st>>>(n, k, s, f, l, vel_out, false);
+            k_xsph_f32_g<false, G><<<b, threads, sm, st>>>(n, k, s, f, l, vel_out, w);
+        });
+        return;
+    }
     if (w) k_xsph_f32_w<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, f, l, vel_out);
     k_xsph_f32<<<blocks_for(n, threads), threads, 0, st>>>(n, k, s, f, l, vel_out, w);
 }

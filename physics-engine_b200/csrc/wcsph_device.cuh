@@ -201,7 +201,8 @@ struct PassLanes {
 };
 PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t boundary);
 
-// Single-precision form (sph_f32.cu).
+// Single-precision form (sph_f32.cu): 1, 8 or 32 lanes.
+PassLanes pass_lanes_f32(int dim, uint64_t fluid);
 struct F32Const {
     int dim;
     float h, inv_h, alpha, mass, rho0, rho_self, cell;
@@ -223,14 +224,14 @@ struct F32Bufs {
 
 void launch_f32_from_f64(uint32_t n, double cell, const StateBufs& s, const F32Bufs& f,
                          cudaStream_t st);
-void launch_density_f32(uint32_t n, uint32_t threads, const F32Const& k, const StateBufs& s,
+void launch_density_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const StateBufs& s,
                         const F32Bufs& f, const ListBufs& l, cudaStream_t st);
 void launch_pressure_f32(uint32_t n, const F32Const& k, const Tanks& tk, const StateBufs& s,
                          const F32Bufs& f, cudaStream_t st);
-void launch_forces_f32(uint32_t n, uint32_t threads, const F32Const& k, const Tanks& tk,
+void launch_forces_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const Tanks& tk,
                        const StateBufs& s, const F32Bufs& f, const ListBufs& l, float dt,
                        double4* pos_next, double4* vel_next, float* bf, cudaStream_t st);
-void launch_xsph_f32(uint32_t n, uint32_t threads, const F32Const& k, const StateBufs& s,
+void launch_xsph_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Const& k, const StateBufs& s,
                      const F32Bufs& f, const ListBufs& l, float4* vel_out, cudaStream_t st,
                      bool use_w = false);
 

@@ -722,7 +722,7 @@ void World::run_density(bool visit_only) {
     ensure_lists(visit_only);
     if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
     prof_begin(kDensity);
-    if (f32_) launch_density_f32((uint32_t)n_, shape_.density, kf_, cur_, fb_, lists_, st_);
+    if (f32_) launch_density_f32((uint32_t)n_, shape_.density, lanes_.density, kf_, cur_, fb_, lists_, st_);
     else launch_density((uint32_t)n_, shape_.density, lanes_.density, kc_, cur_, lists_, st_);
     prof_end();
     launches_ += 1;
@@ -755,7 +755,7 @@ void World::run_forces(bool integrate, double dt) {
         // the single-precision form always integrates into the next buffers;
         // without a kick/drift request the step is taken with dt = 0
         prof_begin(kForces);
-        launch_forces_f32((uint32_t)n_, shape_.forces, kf_, tanks_, cur_, fb_, lists_,
+        launch_forces_f32((uint32_t)n_, shape_.forces, lanes_.forces, kf_, tanks_, cur_, fb_, lists_,
                           integrate ? (float)dt : 0.f, pos_nx_, vel_nx_, bf32_, st_);
         prof_end();
         launches_ += 2;
@@ -818,7 +818,7 @@ void World::run_xsph() {
     ensure_lists();
     prof_begin(kXsph);
     if (f32_) {
-        launch_xsph_f32((uint32_t)n_, shape_.xsph, kf_, cur_, fb_, lists_, velf_alt_, st_, w_valid_);
+        launch_xsph_f32((uint32_t)n_, shape_.xsph, lanes_.xsph, kf_, cur_, fb_, lists_, velf_alt_, st_, w_valid_);
         prof_end();
         launches_ += w_valid_ ? 2 : 1;  // with weights: the weight-reading kernel and its fallback
         check(cudaGetLastError(), "xsph");
@@ -966,8 +966,8 @@ bool World::capture_graph(double dt) {
 }
 
 void World::set_lanes(uint32_t lanes) {
-    if (lanes == 0) lanes_ = pass_lanes(dim_, n_fluid_, n_ - n_fluid_);
-    else if (lanes == 1 || lanes == 4 || lanes == 8 || lanes == 16 || lanes == 32)
+    if (lanes == 0) lanes_ = f32_ ? pass_lanes_f32(dim_, n_fluid_) : pass_lanes(dim_, n_fluid_, n_ - n_fluid_);
+    else if (lanes == 1 || lanes == 8 || lanes == 32 || (!f32_ && (lanes == 4 || lanes == 16)))
         lanes_.density = lanes_.forces = lanes_.boundary = lanes_.xsph = lanes;
     else throw std::invalid_argument("lanes per slot");
     invalidate_graph();
@@ -1038,12 +1038,12 @@ World::Shapes World::autotune() {
     };
     if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
     pick(shape_.density, [&] {
-        if (f32_) launch_density_f32(n, shape_.density, kf_, cur_, fb_, lists_, st_);
+        if (f32_) launch_density_f32(n, shape_.density, lanes_.density, kf_, cur_, fb_, lists_, st_);
         else launch_density(n, shape_.density, lanes_.density, kc_, cur_, lists_, st_);
     });
     w_valid_ = pair_weights();  // the density launches wrote W for these lists
     pick(shape_.forces, [&] {
-        if (f32_) launch_forces_f32(n, shape_.forces, kf_, tanks_, cur_, fb_, lists_, 0.f, pos_nx_, vel_nx_, nullptr, st_);
+        if (f32_) launch_forces_f32(n, shape_.forces, lanes_.forces, kf_, tanks_, cur_, fb_, lists_, 0.f, pos_nx_, vel_nx_, nullptr, st_);
         else launch_forces(n, shape_.forces, lanes_.forces, kc_, tanks_, cur_, lists_, true, 0.0, pos_nx_, vel_nx_,
                            prm_.surface_tension_sigma != 0.0 ? st_a_ : nullptr, st_);
     });

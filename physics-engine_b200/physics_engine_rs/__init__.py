@@ -594,9 +594,9 @@ class WcsphWorld:
         return r
 
     def set_lanes(self, lanes: int = 0):
-        """Lanes of a warp on each particle's list in the f64 pair passes: 0
-        (the default) picks them per pass from the particle counts; 1, 4, 8,
-        16 or 32 sets them all. The results are identical."""
+        """Lanes of a warp on each particle's list in the pair passes: 0 (the
+        default) picks them per pass from the particle counts; 1, 4, 8, 16 or
+        32 (single precision: 1, 8 or 32) sets them all. The results are identical."""
         _ok(_lib.pe_fluid_wcsph_set_lanes(self._w, int(lanes)), "set_lanes")
 
     def set_pair_weights(self, on: bool = True):

@@ -1,4 +1,5 @@
-"""Every lane count of the f64 pair passes reproduces the oracle bit for bit:
+"""Every lane count of the pair passes reproduces the oracle bit for bit (single
+precision: the one-lane form):
 lists of 0 to 17 entries (shorter than, equal to and just beyond a round of
 any lane count, with rows of one to four entries), lists longer than the force
 pass's queue, oriented and plain boundary samples, both viscosity terms, the
@@ -86,6 +87,28 @@ def test_lane_counts_bit_exact(scene):
             if scene == "dense" and lanes == 1:
                 assert int(w.neighbour_counts()[1].max()) > 512
             w.close()
+
+
+@pytest.mark.parametrize("scene", list(SCENES)[:3] + ["planar"])
+def test_single_precision_lane_counts_agree(scene):
+    """The compensated sums of the single-precision form come out the same bits for 1, 8 and 32 lanes."""
+    build, dim, _, beta, steps = SCENES[scene]
+    ps = pe.Particles(dim, 1000.0, pe.mass_from_spacing(1000.0, DX, dim), 2 * DX)
+    build(ps)
+    prm = dam_break_params_pe(False)
+    prm.visc_beta, prm.precision = beta, pe.PRECISION_F32
+    for weights in (True, False):
+        want = None
+        for lanes in (1, 8, 32, 0):
+            w = pe.WcsphWorld(ps, prm)
+            w.set_lanes(lanes)
+            w.set_pair_weights(weights)
+            w.run(1e-5, steps)
+            got = [w.positions(), w.velocities(), w.densities(), w.accelerations()]
+            w.close()
+            want = want or got
+            for a, b, what in zip(got, want, ("x", "v", "rho", "a")):
+                assert_bits_equal(a, b, f"{scene}, {lanes} lanes, weights {weights} {what}")
 
 
 def test_unknown_lane_counts_are_refused():
