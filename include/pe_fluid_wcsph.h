@@ -227,6 +227,10 @@ int pe_fluid_pbf_set_velocities(PePbf* w, const double* in, uint64_t n);
 /* pbf.rs:440-455 mean |rho/rho0 - 1|, pbf.rs:458 v_max. */
 int pe_fluid_pbf_mean_density_error(PePbf* w, double* out);
 int pe_fluid_pbf_v_max(PePbf* w, double* out);
+/* Lanes of a warp that share each particle's list in the constraint passes (no
+ * reference counterpart): 0 (the default) picks them from the fluid count; 1 or
+ * 8 sets them, other values return PE_ERR_ARG. No choice changes a bit. */
+int pe_fluid_pbf_set_lanes(PePbf* w, uint32_t lanes);
 int pe_fluid_pbf_status(PePbf* w, uint32_t* status);
 int pe_fluid_pbf_kernel_launches(PePbf* w, uint64_t* out, int32_t reset);
 /* The CUDA stream (cudaStream_t) all of the world's work is issued on. */

@@ -36,9 +36,7 @@
 //
 // k_nlist_visit stages f32 offsets and tests them in packed f32 arithmetic: its
 // lists feed the single-precision form, whose compensated sums notice a
-// candidate more (a zero added moves a tie), and PBF's grid, whose cells of
-// eight particles leave the tensor tile half empty (125 us a build of 64,000
-// particles against 153).
+// candidate more (a zero added moves a tie). k_nlist_near makes PBF's.
 //
 // k_nlist_both is bound by instruction issue and barriers (529M warp instructions for 262,144 fluid
 // particles, IPC 2.4, with scalar distance tests and a lower mask read through
@@ -47,9 +45,12 @@
 // 0.14 ms, barriers and the rest 0.7.
 #include <algorithm>
 #include <climits>
+#include <cmath>
+#include <limits>
 
 #include <cuda_fp16.h>
 
+#include "list_iter.cuh"
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
 
@@ -819,7 +820,247 @@ __global__ void __launch_bounds__(kNlThreads, 4) k_nlist_visit(GridDesc g, Tanks
     if (tid == 0 && max_union) atomicMax(&sc->max_union, max_union);
 }
 
-// ----------------------------------------------------------------- both
+// ----------------------------------------------------------------- near
+// Visit lists of the fluid slots' candidates within the support radius of their
+// present positions, the candidates taken from the cells of the last grid: what
+// PBF's constraint iterations need, whose predictions move between two grids.
+// A warp a cell, for cells of a few particles (PBF's support is one cell, ~8 of
+// them, ~216 candidates): the CTA a cell of the kernels above leaves three
+// quarters of its threads idle there. Positions are staged as f32 offsets from
+// the cell; as they may be any number of cells away from it, the test's margin
+// follows the largest staged offset (a candidate more adds +-0 to PBF's sums).
+// 64,000 fluid particles and 43,000 samples: 51 us, bound by its own chain of
+// loads and instruction issue (24M warp instructions, 30% of the ALU); lists of
+// every candidate took 126 us once a step, but then each of the twelve passes
+// over them 86 to 122 us instead of 28 to 32.
+constexpr uint32_t kNearWarps = 4;    // warps a CTA
+constexpr uint32_t kNearTile = 320;   // candidates staged at once
+constexpr uint32_t kNearWords = kNearTile / 32u;
+
+struct NearStage {
+    float4 at[kNearTile];               // offset from the cell's corner, list entry
+    uint32_t mask[32][kNearWords + 1];  // word w of centre c; the odd pitch spreads the words of 32 centres
+    uint32_t head[kNearWords];          // union positions of the tile where a non-empty cell begins
+    uint32_t shift[32];                 // non-empty cell k of the union: its slots minus its union positions
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(32 * kNearWarps, 8) k_nlist_near(GridDesc g, Tanks tk, float support,
+                                                                  const uint32_t* __restrict__ occ,
+                                                                  const uint32_t* __restrict__ cell_start,
+                                                                  StateBufs s, ListBufs l, DeviceScalars* sc) {
+    constexpr int NC = DIM == 3 ? 27 : 9;
+    constexpr int CENTER = DIM == 3 ? 13 : 4;
+    constexpr uint32_t kAll = 0xffffffffu;
+    __shared__ NearStage s_stage[kNearWarps];
+    NearStage& sm = s_stage[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nocc = sc->nocc, warps = gridDim.x * kNearWarps;
+    const uint32_t parts = min(max(warps / max(nocc, 1u), 1u), 8u);  // warps a cell while there are more than cells
+    uint32_t max_union = 0;
+    bool overflow = false;
+
+    for (uint32_t item = blockIdx.x * kNearWarps + (threadIdx.x >> 5); item < nocc * parts; item += warps) {
+        const uint32_t it = parts == 1u ? item : item / parts, part = item - it * parts;
+        const uint32_t c = occ[it];
+        const TankDesc td = tk.desc[tk.cell_tank[c]];
+        const uint32_t lc = c - td.cell_base;
+        // ---- lane r: range of neighbour cell r, in visiting order
+        const int cz = (int)(lc % (uint32_t)td.nz), cxy = (int)(lc / (uint32_t)td.nz);
+        const int cx = (int)((uint32_t)cxy / (uint32_t)td.ny), cy = cxy - cx * td.ny;
+        uint32_t st = 0, cnt = 0;
+        if (lane < (uint32_t)NC) {
+            const int qz = cz + (DIM == 3 ? (int)lane / 9 - 1 : 0);
+            const int qy = cy + (DIM == 3 ? ((int)lane / 3) % 3 - 1 : (int)lane / 3 - 1);
+            const int qx = cx + (int)lane % 3 - 1;
+            if (qx >= 0 && qy >= 0 && qz >= 0 && qx < td.nx && qy < td.ny && qz < td.nz) {
+                const uint32_t nc = td.cell_base + ((uint32_t)qx * (uint32_t)td.ny + (uint32_t)qy) * (uint32_t)td.nz +
+                                    (uint32_t)qz;
+                st = cell_start[nc];
+                cnt = cell_start[nc + 1] - st;
+            }
+        }
+        uint32_t off = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(kAll, off, o);
+            if ((int)lane >= o) off += x;
+        }
+        const uint32_t U = __shfl_sync(kAll, off, 31);
+        off -= cnt;
+        const uint32_t cs = __shfl_sync(kAll, st, CENTER), coff = __shfl_sync(kAll, off, CENTER);
+        const uint32_t ncenter = __shfl_sync(kAll, cnt, CENTER);
+        max_union = max(max_union, U);
+        const uint32_t tiles = (U + kNearTile - 1u) / kNearTile;
+        const double ox = (double)(td.kx0 + cx) * g.cell_size, oy = (double)(td.ky0 + cy) * g.cell_size;
+        const double oz = DIM == 3 ? (double)(td.kz0 + cz) * g.cell_size : 0.0;
+        const uint32_t filled = __ballot_sync(kAll, cnt != 0u);
+        uint32_t staged = kAll;  // tile in the stage
+        float limit = 0.f;       // squared distance a candidate of it is kept within
+
+        auto offset = [&](const double4& p) {
+            return make_float4((float)(p.x - ox), (float)(p.y - oy), DIM == 3 ? (float)(p.z - oz) : 0.f, 0.f);
+        };
+        auto stage_tile = [&](uint32_t tile) {
+            if (staged == tile) return;
+            staged = tile;
+            const uint32_t t0 = tile * kNearTile, m = min(kNearTile, U - t0);
+            __syncwarp();
+            // Union position u lies in the non-empty cell whose beginning is the
+            // last at or below it; the tile's first position counts as one.
+            if (lane < kNearWords) sm.head[lane] = 0u;
+            __syncwarp();
+            if (cnt) {
+                sm.shift[__popc(filled & ((1u << lane) - 1u))] = st - off;
+                if (off > t0 && off - t0 < kNearTile) atomicOr(&sm.head[(off - t0) >> 5], 1u << ((off - t0) & 31u));
+            }
+            uint32_t cell = __popc(__ballot_sync(kAll, cnt && off <= t0)) - 1u;  // of the tile's first position
+            __syncwarp();
+            float far = 0.f;
+#pragma unroll 4
+            for (uint32_t w = 0; w < (m + 31u) >> 5; ++w) {
+                const uint32_t u = 32u * w + lane, h = sm.head[w];
+                const uint32_t k = cell + __popc(h & (kAll >> (31u - lane)));
+                cell += __popc(h);
+                const uint32_t slot = sm.shift[k] + min(t0 + u, U - 1u);
+                float4 p = offset(gather4(s.pos + slot));
+                const uint8_t fl = s.flags[slot];
+                far = fmaxf(far, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+                p.w = __uint_as_float(slot | ((fl & kFlagBoundary) ? kEntryBoundary : 0u) |
+                                      ((fl & kFlagOriented) ? kEntryOriented : 0u));
+                sm.at[u] = p;
+            }
+            // The centres' offsets count too, where another tile stages them.
+            for (uint32_t j = lane; tiles > 1u && j < ncenter; j += 32u) {
+                const float4 p = offset(gather4(s.pos + cs + j));
+                far = fmaxf(far, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
+            }
+            // An offset is rounded by at most far / 2^24, a difference of two by
+            // twice that and its own rounding (far / 2^23): 3.5 far / 2^23 in
+            // distance, and the squares and their sum by 2^-22 of themselves.
+            const float r = support + __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(far))) * 0x1p-21f;
+            limit = r * r * (1.f + 0x1p-20f);
+            __syncwarp();
+        };
+
+        // ---- the part's centres, 32 at a time
+        const uint32_t b0 = (uint32_t)((unsigned long long)ncenter * part / parts);
+        const uint32_t b1 = (uint32_t)((unsigned long long)ncenter * (part + 1u) / parts);
+        for (uint32_t c0 = b0; c0 < b1; c0 += 32u) {
+            const uint32_t nc = min(32u, b1 - c0), kslot = cs + c0 + min(lane, nc - 1u);
+            const bool fluid = lane < nc && !(s.flags[kslot] & kFlagBoundary);
+            const uint32_t fluids = __ballot_sync(kAll, fluid);
+            // masks of a tile's words, two centres at a time: their tests share a candidate's loads
+            auto tile_masks = [&](uint32_t tile) {
+                const uint32_t t0 = tile * kNearTile, m = min(kNearTile, U - t0), words = (m + 31u) >> 5;
+                stage_tile(tile);
+                for (uint32_t left = fluids; left; left &= left - 1u) {
+                    const uint32_t q0 = (uint32_t)__ffs(left) - 1u;
+                    left &= left - 1u;
+                    const uint32_t q1 = left ? (uint32_t)__ffs(left) - 1u : q0;
+                    if (!left) left = 1u;  // the last round
+                    const uint32_t self0 = coff + c0 + q0 - t0, self1 = coff + c0 + q1 - t0;
+                    const float4 a = tiles == 1u ? sm.at[self0] : offset(gather4(s.pos + cs + c0 + q0));
+                    const float4 b = tiles == 1u ? sm.at[self1] : offset(gather4(s.pos + cs + c0 + q1));
+                    uint32_t keep0 = 0, keep1 = 0;
+#pragma unroll 2
+                    for (uint32_t w = 0; w < words; ++w) {
+                        const float4 p = sm.at[32u * w + lane];
+                        const float ax = p.x - a.x, ay = p.y - a.y, az = p.z - a.z;
+                        const float bx = p.x - b.x, by = p.y - b.y, bz = p.z - b.z;
+                        // a position that is no number stays in, as in every pass
+                        const uint32_t ma = __ballot_sync(kAll, !(ax * ax + ay * ay + az * az > limit));
+                        const uint32_t mb = __ballot_sync(kAll, !(bx * bx + by * by + bz * bz > limit));
+                        if (lane == w) {
+                            keep0 = ma;
+                            keep1 = mb;
+                        }
+                    }
+                    if (lane < words) {  // candidates past the union and the centre itself out
+                        if (lane == words - 1u && (m & 31u)) {
+                            keep0 &= (1u << (m & 31u)) - 1u;
+                            keep1 &= (1u << (m & 31u)) - 1u;
+                        }
+                        if (lane == (self0 >> 5)) keep0 &= ~(1u << (self0 & 31u));
+                        if (lane == (self1 >> 5)) keep1 &= ~(1u << (self1 & 31u));
+                        sm.mask[q0][lane] = keep0;
+                        sm.mask[q1][lane] = keep1;
+                    }
+                }
+                __syncwarp();
+            };
+            // The lanes share out the centres' words: lane r * nc + q takes the
+            // r-th of `ways` shares of centre q's (a lane past them none).
+            const uint32_t ways = 32u / nc, q = lane % nc, r = lane / nc;
+            const bool mine = r < ways && ((fluids >> q) & 1u);
+            auto share = [&](uint32_t tile, uint32_t* wb, uint32_t* we) {
+                const uint32_t words = (min(kNearTile, U - tile * kNearTile) + 31u) >> 5;
+                *wb = mine ? words * r / ways : 0u;
+                *we = mine ? words * (r + 1u) / ways : 0u;
+                uint32_t n = 0;
+                for (uint32_t w = *wb; w < *we; ++w) n += __popc(sm.mask[q][w]);
+                return n;
+            };
+            // sum over centre q's lanes of v, and over its lanes before this one
+            auto centre_sum = [&](uint32_t v, uint32_t* before) {
+                uint32_t tot = 0, pre = 0;
+                for (uint32_t w = 0; w < ways; ++w) {
+                    const uint32_t x = __shfl_sync(kAll, v, w * nc + q);
+                    if (w < r) pre += x;
+                    tot += x;
+                }
+                *before = pre;
+                return tot;
+            };
+            uint32_t nv = 0, wb = 0, we = 0, before = 0, n = 0;  // the centre's entries, this lane's share of them
+            if (fluids) {
+                for (uint32_t tile = 0; tile < tiles; ++tile) {
+                    tile_masks(tile);
+                    n = share(tile, &wb, &we);
+                    nv += centre_sum(n, &before);
+                }
+            }
+            // ---- the chunk's block
+            const uint32_t longest = __reduce_max_sync(kAll, nv);
+            const unsigned long long groups = (unsigned long long)rows_for(longest) * nc;
+            unsigned long long base = 0;
+            if (lane == 0 && groups) base = atomicAdd(&sc->list_used, groups);
+            base = __shfl_sync(kAll, base, 0);
+            const bool ok = longest < 65536u && base + groups <= l.pool_groups;  // counts are stored in 16 bits
+            overflow |= !ok;
+            if (lane < nc) {
+                l.desc[kslot] = ok ? make_uint4((uint32_t)base + lane, nc, nv, 0u) : make_uint4(0u, 0u, 0u, 0u);
+                l.ncand[kslot] = fluid ? U : 0u;
+            }
+            if (!ok || !longest) continue;
+            // ---- the entries: a lane writes those of its words
+            uint32_t* const out = l.pool + 4 * (size_t)(base + q);
+            uint32_t done = 0;  // entries of the centre written from earlier tiles
+            for (uint32_t tile = 0; tile < tiles; ++tile) {
+                uint32_t all = nv;
+                if (tiles > 1u) {
+                    tile_masks(tile);
+                    n = share(tile, &wb, &we);
+                    all = centre_sum(n, &before);
+                }
+                if (n) {
+                    uint32_t t = done + before, w = wb, b = sm.mask[q][w];
+                    for (const uint32_t end = t + n; t < end; ++t) {
+                        while (!b) b = sm.mask[q][++w];
+                        out[(size_t)(t >> 2) * (4u * nc) + (t & 3u)] = __float_as_uint(sm.at[32u * w + (uint32_t)__ffs(b) - 1u].w);
+                        b &= b - 1u;
+                    }
+                }
+                done += all;
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    }
+    if (lane == 0 && overflow) atomicOr(&sc->status, kStatusListOverflow);
+    if (lane == 0 && max_union) atomicMax(&sc->max_union, max_union);
+}
+
 // ----------------------------------------------------------------- both
 // Stages candidate u of a union: features, list entry and staged word.
 template <int DIM>
@@ -1182,6 +1423,16 @@ void launch_union_max(const GridDesc& g, const Tanks& tk, uint32_t ncell_max, co
     const uint32_t b = (ncell_max + 255u) / 256u;
     if (g.dim == 3) k_union_max<3><<<b, 256, 0, st>>>(tk, occ, cell_start, sc);
     else k_union_max<2><<<b, 256, 0, st>>>(tk, occ, cell_start, sc);
+}
+
+void launch_nlist_near(const GridDesc& g, const Tanks& tk, double support, uint32_t ncell_max, uint32_t sms,
+                       const uint32_t* occ, const uint32_t* cell_start, const StateBufs& s, const ListBufs& l,
+                       DeviceScalars* sc, cudaStream_t st) {
+    // several CTAs a resident one: cells of boundary samples alone are done at once
+    const uint32_t b = std::min((ncell_max + kNearWarps - 1u) / kNearWarps * 8u, 40u * sms);
+    const float r = std::nextafter((float)support, std::numeric_limits<float>::infinity());
+    if (g.dim == 3) k_nlist_near<3><<<b, 32 * kNearWarps, 0, st>>>(g, tk, r, occ, cell_start, s, l, sc);
+    else k_nlist_near<2><<<b, 32 * kNearWarps, 0, st>>>(g, tk, r, occ, cell_start, s, l, sc);
 }
 
 void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32_t ucap,

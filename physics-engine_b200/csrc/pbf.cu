@@ -7,10 +7,16 @@
 // vel = (v, rho). Every pass is a gather over the slot's visit list in the
 // reference's visiting order, so each per-particle sum is the reference's
 // sequence of additions; candidates outside the support add +-0 and are left
-// out of the lists. Compiled with --fmad=false.
+// out of the lists, which are built anew for each iteration's predictions
+// (~33 of ~216 candidates are in support): an iteration of 64,000 particles
+// takes 51 us of lists, 28 of density and lambda and 32 of corrections, where
+// passes that dropped the far candidates themselves took 86, 100 and 122.
+// Compiled with --fmad=false.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
+#include "lane_group.cuh"
 #include "list_iter.cuh"
 #include "pbf.cuh"
 
@@ -19,17 +25,12 @@ namespace pe {
 namespace {
 
 constexpr uint32_t kPbfThreads = 128;
-constexpr size_t kKeepBytes = (size_t)kKeepChunk * kPbfThreads * sizeof(uint32_t);  // for_each_kept buffer
 
 inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
 
 struct D3 {
     double x, y, z;
 };
-
-__device__ __forceinline__ double4 load_pos(const StateBufs& s, uint32_t e) {
-    return s.pos[e & kEntrySlotMask];
-}
 
 // A candidate beyond both kernels' support contributes an exact +-0 to every
 // sum (W and grad W vanish there), which leaves the sums unchanged: it is
@@ -62,130 +63,168 @@ __global__ void k_pbf_predict(uint32_t n, PbfConst k, double dt, StateBufs s, do
     pred[i] = make_double4(px, py, pz, p.w);
 }
 
+// The passes of a constraint iteration run G lanes a slot (lane_group.cuh) over
+// lists that hold the entries in support at the present positions.
+
 // pbf.rs:159-187 density at the predicted positions into vel.w
+template <int G>
 __global__ void __launch_bounds__(kPbfThreads) k_pbf_density(uint32_t n, PbfConst k, StateBufs s, ListBufs l) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (s.flags[i] & kFlagBoundary) {
-        s.vel[i].w = k.rho0;
-        return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) s.vel[i].w = k.rho0;
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
     }
-    extern __shared__ uint32_t s_keep[];
-    const double4 xi = s.pos[i];
-    double rho = k.rho_self;
-    for_each_kept(
-        list_ref(l, i, kListVisit), s_keep, [&](uint32_t e) { return load_pos(s, e); },
-        [&](uint32_t, const double4& xj) { return !far_pair(k, xi, xj); },
-        [&](uint32_t e, const double4& xj) {
-            const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            const double r = sqrt(dx * dx + dy * dy + dz * dz);
-            const double wij = kfn_w(k.dk, r);
-            if (e & kEntryBoundary) rho += k.rho0 * xj.w * wij;
-            else rho += k.mass * wij;
+    OrderedSum<G, 1> rho(s_words + g.warp * OrderedSum<G, 1>::kDoubles, g, k.rho_self);
+    group_for_each<G>(
+        lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
+            double t[1] = {0.0};
+            if (has) {
+                const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+                const double wij = kfn_w_r2(k.dk, dx * dx + dy * dy + dz * dz);
+                t[0] = ((e & kEntryBoundary) ? k.rho0 * xj.w : k.mass) * wij;
+            }
+            rho.add(t);
         });
-    s.vel[i].w = fmax(rho, 1e-12);
+    double r[1];
+    rho.totals(r);
+    if (fluid && g.sub == 0) s.vel[i].w = fmax(r[0], 1e-12);
 }
 
-// pbf.rs:189-227 lambda_i = -C_i / (sum |grad C|^2 + eps)
+// pbf.rs:159-227 the same with lambda_i = -C_i / (sum |grad C|^2 + eps), which
+// reads no other particle's density: one walk of the list for both
+template <int G>
 __global__ void __launch_bounds__(kPbfThreads) k_pbf_lambda(uint32_t n, PbfConst k, StateBufs s, ListBufs l,
                                                            double* __restrict__ lambda,
                                                            double* __restrict__ lambda_orig) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (s.flags[i] & kFlagBoundary) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) {
+        s.vel[i].w = k.rho0;
         lambda[i] = 0.0;
         lambda_orig[s.orig[i]] = 0.0;
-        return;
     }
-    const double4 xi = s.pos[i];
-    const double ci = s.vel[i].w / k.rho0 - 1.0;
-    double sum_grad_sq = 0.0;
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    extern __shared__ uint32_t s_keep[];
-    for_each_kept(
-        list_ref(l, i, kListVisit), s_keep, [&](uint32_t e) { return load_pos(s, e); },
-        [&](uint32_t, const double4& xj) { return !far_pair(k, xi, xj); },
-        [&](uint32_t e, const double4& xj) {
-            double wx, wy, wz;
-            kfn_grad(k.gk, xj.x - xi.x, xj.y - xi.y, xj.z - xi.z, &wx, &wy, &wz);
-            const bool fluid = !(e & kEntryBoundary);
-            const double scale = fluid ? k.mass_over_rho0 : xj.w;
-            const double cx = wx * scale, cy = wy * scale, cz = wz * scale;
-            gx = gx + cx;
-            gy = gy + cy;
-            gz = gz + cz;
-            if (fluid) sum_grad_sq += cx * cx + cy * cy + cz * cz;
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+    }
+    const double start[5] = {0.0, 0.0, 0.0, 0.0, k.rho_self};
+    OrderedSum<G, 5> sum(s_words + g.warp * OrderedSum<G, 5>::kDoubles, g, start);  // grad C, fluid |grad C|^2, rho
+    group_for_each<G>(
+        lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
+            double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            if (has) {
+                const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const bool nf = !(e & kEntryBoundary);
+                t[4] = (nf ? k.mass : k.rho0 * xj.w) * kfn_w_r2(k.dk, r2);
+                const double gs = kfn_grad_scale(k.gk, r2);
+                const double scale = nf ? k.mass_over_rho0 : xj.w;
+                t[0] = dx * gs * scale;
+                t[1] = dy * gs * scale;
+                t[2] = dz * gs * scale;
+                t[3] = nf ? t[0] * t[0] + t[1] * t[1] + t[2] * t[2] : 0.0;
+            }
+            sum.add(t);
         });
-    sum_grad_sq += gx * gx + gy * gy + gz * gz;
-    const double li = -ci / (sum_grad_sq + k.eps_lambda);
-    lambda[i] = li;
-    lambda_orig[s.orig[i]] = li;
+    double r[5];
+    sum.totals(r);
+    if (fluid && g.sub == 0) {
+        const double rho = fmax(r[4], 1e-12);
+        s.vel[i].w = rho;
+        const double ci = rho / k.rho0 - 1.0;
+        const double sum_grad_sq = r[3] + (r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+        const double li = -ci / (sum_grad_sq + k.eps_lambda);
+        lambda[i] = li;
+        lambda_orig[s.orig[i]] = li;
+    }
 }
 
 // pbf.rs:229-235
 __device__ __forceinline__ double art_pressure(const PbfConst& k, double wij) {
     if (k.w_dq <= 1e-30 || k.art_k == 0.0) return 0.0;
-    const double ratio = fmin(wij / k.w_dq, 1.0);
+    const double ratio = fmin(quot_any(wij, k.w_dq), 1.0);
     const double pw = k.art_n_is_int ? pow_int_dd(ratio, k.art_n_int) : pow(ratio, k.art_n);
     return -k.art_k * pw;
 }
 
-// pbf.rs:237-286 position correction, clamped to 0.4 h
+// pbf.rs:237-286 position correction, clamped to 0.4 h, and pbf.rs:403-409
+// pred += dp (fluid; 2-D: z = 0) into pos_next
+template <int G>
 __global__ void __launch_bounds__(kPbfThreads) k_pbf_delta_p(uint32_t n, PbfConst k, StateBufs s, ListBufs l,
                                                             const double* __restrict__ lambda,
-                                                            double4* __restrict__ dp) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (s.flags[i] & kFlagBoundary) {
-        dp[i] = make_double4(0.0, 0.0, 0.0, 0.0);
-        return;
+                                                            double4* __restrict__ pos_next) {
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) pos_next[i] = s.pos[i];
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    double li = 0.0;
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        li = lambda[i];
     }
-    const double4 xi = s.pos[i];
-    const double li = lambda[i];
-    double cx = 0.0, cy = 0.0, cz = 0.0;
-    extern __shared__ uint32_t s_keep[];
-    for_each_kept(
-        list_ref(l, i, kListVisit), s_keep, [&](uint32_t e) { return load_pos(s, e); },
-        [&](uint32_t, const double4& xj) { return !far_pair(k, xi, xj); },
-        [&](uint32_t e, const double4& xj) {
-            const double rx = xj.x - xi.x, ry = xj.y - xi.y, rz = xj.z - xi.z;
-            const double r = sqrt(rx * rx + ry * ry + rz * rz);
-            const double wij = kfn_w(k.dk, r);
-            double wx, wy, wz;
-            kfn_grad(k.gk, rx, ry, rz, &wx, &wy, &wz);
-            const double s_corr = art_pressure(k, wij);
-            double f;
-            if (e & kEntryBoundary) {
-                const double coeff = li + s_corr;
-                f = xj.w * coeff;
-            } else {
-                const double coeff = li + lambda[e & kEntrySlotMask] + s_corr;
-                f = k.mass_over_rho0 * coeff;
+    struct Neighbour {
+        double4 x;
+        double lambda;
+    };
+    OrderedSum<G, 3> corr(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
+            const uint32_t j = e & kEntrySlotMask;
+            return Neighbour{gather4(s.pos + j), __ldg(lambda + j)};
+        },
+        [&](bool has, uint32_t e, const Neighbour& b, const uint32_t*) {
+            double t[3] = {0.0, 0.0, 0.0};
+            if (has) {
+                const double rx = b.x.x - xi.x, ry = b.x.y - xi.y, rz = b.x.z - xi.z;
+                const double r2 = rx * rx + ry * ry + rz * rz;
+                const double gs = kfn_grad_scale(k.gk, r2);
+                const double s_corr = art_pressure(k, kfn_w_r2(k.dk, r2));
+                double f;
+                if (e & kEntryBoundary) {
+                    const double coeff = li + s_corr;
+                    f = b.x.w * coeff;
+                } else {
+                    const double coeff = li + b.lambda + s_corr;
+                    f = k.mass_over_rho0 * coeff;
+                }
+                t[0] = rx * gs * f;
+                t[1] = ry * gs * f;
+                t[2] = rz * gs * f;
             }
-            cx = cx + wx * f;
-            cy = cy + wy * f;
-            cz = cz + wz * f;
+            corr.add(t);
         });
-    const double mag = sqrt(cx * cx + cy * cy + cz * cz);
-    if (mag > k.max_corr && mag > 0.0) {
-        const double sc = k.max_corr / mag;
-        cx = cx * sc;
-        cy = cy * sc;
-        cz = cz * sc;
+    double c[3];
+    corr.totals(c);
+    if (fluid && g.sub == 0) {
+        const double mag = sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+        if (mag > k.max_corr && mag > 0.0) {
+            const double sc = k.max_corr / mag;
+            c[0] = c[0] * sc;
+            c[1] = c[1] * sc;
+            c[2] = c[2] * sc;
+        }
+        pos_next[i] = make_double4(xi.x + c[0], xi.y + c[1], k.dim == 2 ? 0.0 : xi.z + c[2], xi.w);
     }
-    dp[i] = make_double4(cx, cy, cz, 0.0);
-}
-
-// pbf.rs:403-409 pred += dp (fluid; 2-D: z = 0)
-__global__ void k_pbf_apply_dp(uint32_t n, int dim, StateBufs s, const double4* __restrict__ dp) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (s.flags[i] & kFlagBoundary)) return;
-    double4 p = s.pos[i];
-    const double4 d = dp[i];
-    p.x = p.x + d.x;
-    p.y = p.y + d.y;
-    p.z = dim == 2 ? 0.0 : p.z + d.z;
-    s.pos[i] = p;
 }
 
 // pbf.rs:413-421 v = (pred - x) * (1 / dt) when dt > 0; x = pred (pos already is)
@@ -202,32 +241,48 @@ __global__ void k_pbf_finalize(uint32_t n, double dt, StateBufs s) {
 }
 
 // pbf.rs:298-317 XSPH-style viscosity: dv_i = eps * sum_j (v_j - v_i) m / rho_bar W
+template <int G>
 __global__ void __launch_bounds__(kPbfThreads) k_pbf_viscosity(uint32_t n, PbfConst k, StateBufs s, ListBufs l,
                                                               double4* __restrict__ dv) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (s.flags[i] & kFlagBoundary) {
-        dv[i] = make_double4(0.0, 0.0, 0.0, 0.0);
-        return;
+    extern __shared__ __align__(16) double s_words[];
+    const LaneGroup<G> g;
+    const uint32_t i = g.slot;
+    const bool fluid = i < n && !(s.flags[i] & kFlagBoundary);
+    if (i < n && !fluid && g.sub == 0) dv[i] = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (!__any_sync(kFullWarp, fluid)) return;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0), vi = xi;
+    if (fluid) {
+        lr = list_ref(l, i, kListVisit);
+        xi = s.pos[i];
+        vi = s.vel[i];
     }
-    const double4 xi = s.pos[i], vi = s.vel[i];
-    double cx = 0.0, cy = 0.0, cz = 0.0;
-    for_each_entry(list_ref(l, i, kListVisit), [&](uint32_t e) {
-        if (e & kEntryBoundary) return;
-        const uint32_t j = e & kEntrySlotMask;
-        const double4 xj = s.pos[j];
-        if (far_pair(k, xi, xj)) return;
-        const double4 vj = s.vel[j];
-        const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double wij = kfn_w(k.dk, r);
-        const double rho_bar = 0.5 * (vi.w + vj.w);
-        const double f = k.mass / fmax(rho_bar, 1e-12) * wij;
-        cx = cx + (vj.x - vi.x) * f;
-        cy = cy + (vj.y - vi.y) * f;
-        cz = cz + (vj.z - vi.z) * f;
-    });
-    dv[i] = make_double4(cx * k.visc_eps, cy * k.visc_eps, cz * k.visc_eps, 0.0);
+    struct Neighbour {
+        double4 x, v;
+    };
+    OrderedSum<G, 3> sum(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, 0.0);
+    group_for_each<G>(
+        lr, g,
+        [&](uint32_t e, const uint32_t*) {
+            const uint32_t j = e & kEntrySlotMask;
+            return Neighbour{gather4(s.pos + j), gather4(s.vel + j)};
+        },
+        [&](bool has, uint32_t e, const Neighbour& b, const uint32_t*) {
+            double t[3] = {0.0, 0.0, 0.0};
+            if (has && !(e & kEntryBoundary)) {
+                const double dx = b.x.x - xi.x, dy = b.x.y - xi.y, dz = b.x.z - xi.z;
+                const double wij = kfn_w_r2(k.dk, dx * dx + dy * dy + dz * dz);
+                const double rho_bar = 0.5 * (vi.w + b.v.w);
+                const double f = quot_any(k.mass, fmax(rho_bar, 1e-12)) * wij;
+                t[0] = (b.v.x - vi.x) * f;
+                t[1] = (b.v.y - vi.y) * f;
+                t[2] = (b.v.z - vi.z) * f;
+            }
+            sum.add(t);
+        });
+    double c[3];
+    sum.totals(c);
+    if (fluid && g.sub == 0) dv[i] = make_double4(c[0] * k.visc_eps, c[1] * k.visc_eps, c[2] * k.visc_eps, 0.0);
 }
 
 // pbf.rs:318-320 v += dv for every particle
@@ -309,12 +364,31 @@ __global__ void __launch_bounds__(kPbfThreads) k_pbf_confine(uint32_t n, PbfCons
     }
 }
 
+// Calls f(integral_constant<int, G>) for the lanes a slot of the pair passes.
+template <class F>
+void with_lanes(uint32_t lanes, F&& f) {
+    if (lanes == 1) f(std::integral_constant<int, 1>{});
+    else f(std::integral_constant<int, 8>{});
+}
+
+template <int G, int K>
+size_t lane_smem() {
+    return (size_t)(kPbfThreads / 32u) * OrderedSum<G, K>::kDoubles * sizeof(double);
+}
+
+template <int G>
+uint32_t lane_blocks(uint32_t n) {
+    return blocks_for((uint64_t)n * G, kPbfThreads);
+}
+
 }  // namespace
 
 PbfSolver::PbfSolver(const PbfParams& prm, const WorldConfig& cfg, int dim, double rest_density, double mass,
                      double h, uint64_t n, const double* x, const double* v, const uint8_t* kind,
                      const double* psi, const double* n_out)
     : prm_(prm) {
+    for (uint64_t i = 0; i < n; ++i) n_fluid_ += kind[i] == 0;
+    set_lanes(0);
     WorldParams wp{};
     wp.kernel = 0;
     wp.eos_rest_density = rest_density;
@@ -432,14 +506,54 @@ void PbfSolver::refresh_const() {
     k.gz = prm_.gravity[2];
 }
 
-void PbfSolver::lists(bool all_candidates) {
+// Lists at the present positions. A new state's pool is first sized by its
+// candidates where the cells outlive the positions (reused): no later iteration's
+// lists can be longer.
+void PbfSolver::lists(bool reused) {
     World& w = *w_;
-    if (w.list_all_candidates_ != all_candidates) {
-        w.list_all_candidates_ = all_candidates;
+    if (!w.lists_checked_) {
+        w.list_all_candidates_ = reused;
         w.refresh_step_const();
         w.lists_valid_ = false;
+        w.ensure_lists(true);
+        w.list_all_candidates_ = false;
+        w.refresh_step_const();
     }
-    w.ensure_lists(true);
+    w.build_near_lists();
+}
+
+// ms for ten steps with 1 / 8 lanes: 6^3 fluid particles 3.7 / 2.4, 20^3 5.4 / 4.1,
+// 30^3 6.0 / 5.3, 40^3 7.4 / 7.5, 50^3 11.4 / 11.7, 70^3 25.4 / 29.2: a list of ~33
+// entries shared out while the slots do not fill the chip.
+void PbfSolver::set_lanes(uint32_t lanes) {
+    if (lanes == 0) lanes = n_fluid_ <= 48000 ? 8u : 1u;
+    if (lanes != 1 && lanes != 8) throw std::invalid_argument("lanes per slot");
+    lanes_ = lanes;
+}
+
+void PbfSolver::density() {
+    World& w = *w_;
+    const uint32_t n = (uint32_t)w.n_;
+    with_lanes(lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_pbf_density<G><<<lane_blocks<G>(n), kPbfThreads, lane_smem<G, 1>(), w.st_>>>(n, kc_, w.cur_, w.lists_);
+    });
+    w.launches_ += 1;
+}
+
+// pbf.rs:403-411 density, lambda and the position correction of one iteration
+void PbfSolver::constrain() {
+    World& w = *w_;
+    const uint32_t n = (uint32_t)w.n_;
+    with_lanes(lanes_, [&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        k_pbf_lambda<G><<<lane_blocks<G>(n), kPbfThreads, lane_smem<G, 5>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
+                                                                                     lambda_, lambda_orig_);
+        k_pbf_delta_p<G><<<lane_blocks<G>(n), kPbfThreads, lane_smem<G, 3>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
+                                                                                      lambda_, w.pos_nx_);
+    });
+    std::swap(w.cur_.pos, w.pos_nx_);
+    w.launches_ += 2;
 }
 
 void PbfSolver::step(double dt) {
@@ -455,23 +569,15 @@ void PbfSolver::step(double dt) {
     k_pbf_predict<<<nb, kPbfThreads, 0, st>>>(n, kc_, dt, w.cur_, w.pos_nx_);
     w.launches_ += 1;
     w.build_grid(w.pos_nx_, nullptr);
-    // pbf.rs:146-156: lists the constraint iterations reuse while the
-    // predictions move hold every candidate of the neighbour cells, as the
-    // reference's; lists used only at the positions they were built for keep
-    // the candidates in support (the others add +-0)
+    // pbf.rs:146-156: candidates of the neighbour cells, kept while the
+    // predictions move (reuse_neighbours). The others add +-0, so each
+    // iteration's lists hold the candidates then in support.
     const bool reused = prm_.reuse_neighbours && prm_.iterations > 1;
-    lists(reused);
     // pbf.rs:403-411: constraint iterations
     for (uint64_t it = 0; it < prm_.iterations; ++it) {
-        k_pbf_density<<<nb, kPbfThreads, kKeepBytes, st>>>(n, kc_, w.cur_, w.lists_);
-        k_pbf_lambda<<<nb, kPbfThreads, kKeepBytes, st>>>(n, kc_, w.cur_, w.lists_, lambda_, lambda_orig_);
-        k_pbf_delta_p<<<nb, kPbfThreads, kKeepBytes, st>>>(n, kc_, w.cur_, w.lists_, lambda_, dp_);
-        k_pbf_apply_dp<<<nb, kPbfThreads, 0, st>>>(n, w.dim_, w.cur_, dp_);
-        w.launches_ += 4;
-        if (!prm_.reuse_neighbours) {
-            w.build_grid(nullptr, nullptr);
-            lists(false);
-        }
+        if (it > 0 && !prm_.reuse_neighbours) w.build_grid(nullptr, nullptr);
+        lists(reused);
+        constrain();
     }
     // pbf.rs:413-426: velocities from the displacement, x = pred, grid and
     // lists on the final positions, density there
@@ -479,11 +585,14 @@ void PbfSolver::step(double dt) {
     w.launches_ += 1;
     w.build_grid(nullptr, nullptr);
     lists(false);
-    k_pbf_density<<<nb, kPbfThreads, kKeepBytes, st>>>(n, kc_, w.cur_, w.lists_);
-    w.launches_ += 1;
+    density();
     // pbf.rs:288-381: the grid on x equals the one just built
     if (prm_.viscosity_eps != 0.0) {
-        k_pbf_viscosity<<<nb, kPbfThreads, 0, st>>>(n, kc_, w.cur_, w.lists_, dp_);
+        with_lanes(lanes_, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            k_pbf_viscosity<G><<<lane_blocks<G>(n), kPbfThreads, lane_smem<G, 3>(), st>>>(n, kc_, w.cur_, w.lists_,
+                                                                                         dp_);
+        });
         k_pbf_add_dv<<<nb, kPbfThreads, 0, st>>>(n, w.cur_, dp_);
         w.launches_ += 2;
     }

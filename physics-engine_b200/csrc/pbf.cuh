@@ -54,15 +54,22 @@ class PbfSolver {
     // in original index order, as the reference); pbf.rs:458 v_max
     double mean_density_error();
     double v_max();
+    // lanes of a warp on each slot's list in the constraint passes: 1 or 8, or 0
+    // for the solver's choice. No choice changes a bit.
+    void set_lanes(uint32_t lanes);
     // lambda of the last constraint iteration, original order
     void get_lambda(double* out);
 
    private:
     void refresh_const();
-    void lists(bool all_candidates);
+    void lists(bool reused);
+    void density();
+    void constrain();
     std::unique_ptr<World> w_;
     PbfParams prm_;
     PbfConst kc_{};
+    uint64_t n_fluid_ = 0;
+    uint32_t lanes_ = 8;         // lanes a slot of the constraint passes
     double* lambda_ = nullptr;   // per slot
     double* lambda_orig_ = nullptr;  // the same values in original order
     double4* dp_ = nullptr;      // per slot: position correction / viscosity dv

@@ -279,6 +279,14 @@ int pe_fluid_pbf_v_max(PePbf* w, double* out) {
     });
 }
 
+int pe_fluid_pbf_set_lanes(PePbf* w, uint32_t lanes) {
+    if (!w) return PE_ERR_NULL;
+    return guard([&] {
+        w->s->set_lanes(lanes);
+        return PE_OK;
+    });
+}
+
 int pe_fluid_pbf_status(PePbf* w, uint32_t* status) {
     if (!w || !status) return PE_ERR_NULL;
     return guard([&] {

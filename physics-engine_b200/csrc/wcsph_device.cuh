@@ -268,6 +268,11 @@ void launch_nlist(const GridDesc& g, const Tanks& tk, const StepConst& k, uint32
                   uint32_t nblocks, const uint32_t* occ, const uint32_t* cell_start,
                   const StateBufs& s, const ListBufs& l, DeviceScalars* sc, cudaStream_t st,
                   bool visit_only = false, uint32_t chunk = 64);
+// Visit lists at the present positions from the cells of the last grid:
+// candidates within the support radius (ncell_max >= the occupied cells)
+void launch_nlist_near(const GridDesc& g, const Tanks& tk, double support, uint32_t ncell_max, uint32_t sms,
+                       const uint32_t* occ, const uint32_t* cell_start, const StateBufs& s, const ListBufs& l,
+                       DeviceScalars* sc, cudaStream_t st);
 
 // ----- SPH passes -----
 void launch_density(uint32_t n, uint32_t threads, uint32_t lanes, const StepConst& k, const StateBufs& s,

@@ -718,6 +718,19 @@ void World::ensure_lists(bool visit_only) {
     lists_full_ = grid_built_ && !build_visit_only;
 }
 
+void World::build_near_lists() {
+    check(cudaMemsetAsync(&sc_->list_used, 0, sizeof(unsigned long long), st_), "memset");
+    prof_begin(kLists);
+    launch_nlist_near(g_, tanks_, support_, std::min<uint32_t>(g_.ncell, (uint32_t)std::max<uint64_t>(n_, 1)), sms_, occ_,
+                      cell_start_, cur_, lists_, sc_, st_);
+    prof_end();
+    launches_ += 1;
+    check(cudaGetLastError(), "neighbour lists");
+    w_valid_ = false;
+    lists_valid_ = true;
+    lists_full_ = false;
+}
+
 void World::run_density(bool visit_only) {
     ensure_lists(visit_only);
     if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");

@@ -189,6 +189,9 @@ class World {
     void check(cudaError_t e, const char* what);
     void build_grid(const double4* pos_next, const double4* vel_next);
     void ensure_lists(bool visit_only = false);
+    // Visit lists of the candidates (cells of the last grid) within the
+    // support radius at the present positions. The pool must have been sized (lists_checked_).
+    void build_near_lists();
     void run_density(bool visit_only = false);
     void run_pressure();
     void run_forces(bool integrate, double dt);

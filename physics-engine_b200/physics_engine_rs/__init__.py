@@ -262,6 +262,7 @@ def load_library():
         "pe_fluid_dfsph_rebuild_neighbours": (C.c_int, [vp]),
         "pe_fluid_dfsph_compute_density": (C.c_int, [vp]),
         "pe_fluid_dfsph_set_lanes": (C.c_int, [vp, C.c_uint32]),
+        "pe_fluid_pbf_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_dfsph_compute_alpha": (C.c_int, [vp]),
         "pe_fluid_dfsph_len": (C.c_int, [vp, C.POINTER(u64)]),
         "pe_fluid_dfsph_get_time": (C.c_int, [vp, D3]),
@@ -946,6 +947,12 @@ class PbfWorld:
         d = C.c_double()
         _ok(_lib.pe_fluid_pbf_v_max(self._w, C.byref(d)), "pbf_v_max")
         return d.value
+
+    def set_lanes(self, lanes: int = 0):
+        """Lanes of a warp on each particle's list in the constraint passes: 0
+        (the default) picks them from the fluid count; 1 or 8 sets them. The
+        results are identical."""
+        _ok(_lib.pe_fluid_pbf_set_lanes(self._w, int(lanes)), "pbf_set_lanes")
 
     def status(self) -> int:
         s = C.c_uint32()
