@@ -617,8 +617,7 @@ void PbfSolver::run(double dt, uint64_t steps) {
 void PbfSolver::get_lambda(double* out) {
     World& w = *w_;
     if (!w.n_) return;
-    w.check(cudaMemcpyAsync(out, lambda_orig_, sizeof(double) * w.n_, cudaMemcpyDeviceToHost, w.st_), "lambda");
-    w.check(cudaStreamSynchronize(w.st_), "lambda");
+    w.check(w.io_.to_host(out, lambda_orig_, sizeof(double) * w.n_, w.device_, w.st_), "lambda");
 }
 
 double PbfSolver::mean_density_error() {

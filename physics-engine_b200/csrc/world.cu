@@ -1156,8 +1156,7 @@ void World::gather_orig_vec(const double4* src, double* out) {
     uint32_t n = (uint32_t)n_;
     if (!n) return;
     k_export_vec<<<blocks_for(n, 256), 256, 0, st_>>>(n, slot_of_orig_, src, xfer_);
-    check(cudaMemcpyAsync(out, xfer_, sizeof(double) * 3 * n_, cudaMemcpyDeviceToHost, st_), "export");
-    check(cudaStreamSynchronize(st_), "export");
+    check(io_.to_host(out, xfer_, sizeof(double) * 3 * n_, device_, st_), "export");
 }
 
 void World::get_vec(int which, double* out) {
@@ -1168,7 +1167,7 @@ void World::get_vec(int which, double* out) {
 bool World::set_vec(int which, const double* in) {
     uint32_t n = (uint32_t)n_;
     if (!n) return true;
-    check(cudaMemcpyAsync(xfer_, in, sizeof(double) * 3 * n_, cudaMemcpyHostToDevice, st_), "import");
+    check(io_.to_device(xfer_, in, sizeof(double) * 3 * n_, device_, st_), "import");
     // The input is checked for non-finite values on the device (a host scan of
     // the caller's buffer costs more than the copy); a rejected input leaves
     // the state untouched.
@@ -1204,14 +1203,13 @@ void World::get_scalar(int which, double* out) {
     if (!n) return;
     k_export_w<<<blocks_for(n, 256), 256, 0, st_>>>(n, slot_of_orig_, which == 0 ? cur_.vel : nullptr,
                                                     cur_.p, xfer_);
-    check(cudaMemcpyAsync(out, xfer_, sizeof(double) * n_, cudaMemcpyDeviceToHost, st_), "export");
-    check(cudaStreamSynchronize(st_), "export");
+    check(io_.to_host(out, xfer_, sizeof(double) * n_, device_, st_), "export");
 }
 
 void World::set_scalar(int which, const double* in) {
     uint32_t n = (uint32_t)n_;
     if (!n) return;
-    check(cudaMemcpyAsync(xfer_, in, sizeof(double) * n_, cudaMemcpyHostToDevice, st_), "import");
+    check(io_.to_device(xfer_, in, sizeof(double) * n_, device_, st_), "import");
     k_import_w<<<blocks_for(n, 256), 256, 0, st_>>>(n, slot_of_orig_, xfer_,
                                                     which == 0 ? cur_.vel : nullptr, cur_.p);
     k_refresh_pr2<<<blocks_for(n, 256), 256, 0, st_>>>(n, cur_.flags, cur_.p, cur_.pos, cur_.vel);

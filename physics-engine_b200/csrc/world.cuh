@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+#include "transfer.cuh"
 #include "wcsph_device.cuh"
 
 namespace pe {
@@ -229,6 +230,7 @@ class World {
     WorldConfig cfg_;
     double t_ = 0.0;
     int device_ = 0;
+    HostTransfer io_;
     cudaStream_t st_ = nullptr;
 
     GridDesc g_{};
