@@ -808,7 +808,7 @@ void DfsphSolver::refresh_const() {
 
 void DfsphSolver::rebuild() {
     World& w = *w_;
-    w.build_grid(nullptr, nullptr);
+    w.build_grid(nullptr, nullptr, true);
     w.ensure_lists(false);  // visit lists (fluid) and ascending fluid lists (boundary)
 }
 

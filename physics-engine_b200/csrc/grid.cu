@@ -9,6 +9,14 @@
 // within-cell order is ascending original index, exactly as the reference's
 // tie-break. The dense linearisation is ix-major, so ascending linear cell id
 // equals ascending CellKey (the derived Ord on {ix, iy, iz}).
+//
+// Four launches, no memset: small worlds wait on launches and on nothing else
+// (930 particles: with seven launches and two memsets a step took 116 us, now 92;
+// 16,000 in 2-D 146 and 127; 57,570 487 and 457).
+// The counting pass keeps each slot's rank in its cell, so that placing needs no
+// second round of atomics, and adds up the scan's tiles, so that the scan is one
+// pass; the scan clears the counts and the placing pass the tiles for the next
+// build; a slot's thread finds its place in its cell and moves the state there.
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
 
@@ -22,10 +30,13 @@ constexpr uint32_t kScanTile = kScanThreads * kScanItems;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
+// count and tiles are zero on entry. tiles[t] holds the particles (low word) and
+// occupied cells (high word) of the scan's tile t.
 __global__ void k_cell_ids(GridDesc g, Tanks tk, uint32_t n, const double4* __restrict__ pos_cur,
                            const double4* __restrict__ pos_next, const uint8_t* __restrict__ flags,
                            uint32_t* __restrict__ cellid, int4* __restrict__ key_tmp,
-                           uint32_t* __restrict__ count, DeviceScalars* sc) {
+                           uint32_t* __restrict__ count, uint32_t* __restrict__ rank,
+                           unsigned long long* __restrict__ tiles, DeviceScalars* sc) {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     bool active = s < n;
     uint32_t c = 0;
@@ -63,10 +74,19 @@ __global__ void k_cell_ids(GridDesc g, Tanks tk, uint32_t n, const double4* __re
         cellid[s] = c;
     }
     unsigned mask = __ballot_sync(0xffffffffu, active);
-    if (active) {
-        unsigned peers = __match_any_sync(mask, c);
-        if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(&count[c], (uint32_t)__popc(peers));
-    }
+    if (!active) return;
+    const unsigned peers = __match_any_sync(mask, c);
+    const int leader = __ffs(peers) - 1;
+    const bool leads = (int)lane_id() == leader;
+    uint32_t base = 0;
+    if (leads) base = atomicAdd(&count[c], (uint32_t)__popc(peers));
+    const unsigned opened = __ballot_sync(mask, leads && base == 0u);  // cells that were empty
+    base = __shfl_sync(mask, base, leader);
+    rank[s] = base + __popc(peers & ((1u << lane_id()) - 1u));
+    const uint32_t t = c / kScanTile;
+    const unsigned same = __match_any_sync(mask, t);
+    if ((int)lane_id() == __ffs(same) - 1)
+        atomicAdd(&tiles[t], (unsigned long long)__popc(same) | ((unsigned long long)__popc(same & opened) << 32));
 }
 
 // Block-wide exclusive scan of (a, b) pairs with warp shuffles.
@@ -104,42 +124,20 @@ __device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t* ea
     __syncthreads();
 }
 
-// Pass 1: per-tile totals of (particles, occupied cells).
-__global__ void k_scan_reduce(uint32_t ncell, const uint32_t* __restrict__ count,
-                              uint2* __restrict__ tile_sums) {
-    uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t a = 0, b = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i) {
-        uint32_t c = base + i;
-        uint32_t v = c < ncell ? count[c] : 0u;
-        a += v;
-        b += v != 0u;
+// cell_start (exclusive) and the list of occupied cells in linear order; each
+// tile adds up the ones before it. Clears count. clear_lists: a list build and
+// its density pass follow, their counters are cleared too.
+__global__ void k_scan(uint32_t ncell, uint32_t* __restrict__ count, const unsigned long long* __restrict__ tiles,
+                       uint32_t* __restrict__ cell_start, uint32_t* __restrict__ occ, DeviceScalars* sc,
+                       int clear_lists) {
+    uint32_t pa = 0, pb = 0;
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) {
+        const unsigned long long v = tiles[t];
+        pa += (uint32_t)v;
+        pb += (uint32_t)(v >> 32);
     }
-    uint32_t ea, eb, ta, tb;
-    block_scan2(a, b, &ea, &eb, &ta, &tb);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = make_uint2(ta, tb);
-}
-
-// Pass 2: exclusive scan of the tile totals (one block, any tile count).
-__global__ void k_scan_top(uint32_t ntiles, uint2* __restrict__ tile_sums, DeviceScalars* sc) {
-    uint32_t carry_a = 0, carry_b = 0;
-    for (uint32_t off = 0; off < ntiles; off += blockDim.x) {
-        uint32_t i = off + threadIdx.x;
-        uint2 v = i < ntiles ? tile_sums[i] : make_uint2(0u, 0u);
-        uint32_t ea, eb, ta, tb;
-        block_scan2(v.x, v.y, &ea, &eb, &ta, &tb);
-        if (i < ntiles) tile_sums[i] = make_uint2(carry_a + ea, carry_b + eb);
-        carry_a += ta;
-        carry_b += tb;
-    }
-    if (threadIdx.x == 0) sc->nocc = carry_b;
-}
-
-// Pass 3: cell_start (exclusive) and the list of occupied cells in linear order.
-__global__ void k_scan_down(uint32_t ncell, const uint32_t* __restrict__ count,
-                            const uint2* __restrict__ tile_sums, uint32_t* __restrict__ cell_start,
-                            uint32_t* __restrict__ occ) {
+    uint32_t ea, eb, before_a, before_b;
+    block_scan2(pa, pb, &ea, &eb, &before_a, &before_b);
     uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t a = 0, b = 0;
@@ -147,13 +145,13 @@ __global__ void k_scan_down(uint32_t ncell, const uint32_t* __restrict__ count,
     for (int i = 0; i < kScanItems; ++i) {
         uint32_t c = base + i;
         v[i] = c < ncell ? count[c] : 0u;
+        if (v[i]) count[c] = 0u;
         a += v[i];
         b += v[i] != 0u;
     }
-    uint32_t ea, eb, ta, tb;
+    uint32_t ta, tb;
     block_scan2(a, b, &ea, &eb, &ta, &tb);
-    uint2 off = tile_sums[blockIdx.x];
-    uint32_t ra = off.x + ea, rb = off.y + eb;
+    uint32_t ra = before_a + ea, rb = before_b + eb;
 #pragma unroll
     for (int i = 0; i < kScanItems; ++i) {
         uint32_t c = base + i;
@@ -164,70 +162,58 @@ __global__ void k_scan_down(uint32_t ncell, const uint32_t* __restrict__ count,
         }
     }
     // The thread that owns the last cell writes the end sentinel.
-    if (ncell > 0 && base <= ncell - 1 && ncell - 1 < base + kScanItems) cell_start[ncell] = ra;
-}
-
-__global__ void k_place(uint32_t n, const uint32_t* __restrict__ cellid,
-                        const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ fill,
-                        const uint32_t* __restrict__ orig, uint32_t* __restrict__ tmp_old,
-                        uint32_t* __restrict__ tmp_orig) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = s < n;
-    uint32_t c = active ? cellid[s] : 0u;
-    unsigned mask = __ballot_sync(0xffffffffu, active);
-    if (!active) return;
-    unsigned peers = __match_any_sync(mask, c);
-    int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if ((int)lane_id() == leader) base = atomicAdd(&fill[c], (uint32_t)__popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    uint32_t rank = __popc(peers & ((1u << lane_id()) - 1u));
-    uint32_t pos = cell_start[c] + base + rank;
-    tmp_old[pos] = s;
-    tmp_orig[pos] = orig[s];
-}
-
-// One warp per occupied cell: rank each entry by original index (unique), so
-// the cell's run ends up in ascending original index (grid.rs:86-87 tie-break).
-__global__ void k_cellsort(const uint32_t* __restrict__ occ, const DeviceScalars* sc,
-                           const uint32_t* __restrict__ cell_start,
-                           const uint32_t* __restrict__ tmp_old,
-                           const uint32_t* __restrict__ tmp_orig, uint32_t* __restrict__ perm) {
-    uint32_t nocc = sc->nocc;
-    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t lane = lane_id();
-    for (uint32_t i = warp; i < nocc; i += nwarps) {
-        uint32_t c = occ[i];
-        uint32_t start = cell_start[c];
-        uint32_t n = cell_start[c + 1] - start;
-        if (n <= 32u) {
-            uint32_t mine = lane < n ? tmp_orig[start + lane] : 0xffffffffu;
-            uint32_t rank = 0;
-            for (uint32_t f = 0; f < n; ++f) {
-                uint32_t o = __shfl_sync(0xffffffffu, mine, f);
-                rank += o < mine;
-            }
-            if (lane < n) perm[start + rank] = tmp_old[start + lane];
-        } else {
-            for (uint32_t e0 = 0; e0 < n; e0 += 32u) {
-                uint32_t e = e0 + lane;
-                uint32_t mine = e < n ? tmp_orig[start + e] : 0xffffffffu;
-                uint32_t rank = 0;
-                for (uint32_t f = 0; f < n; ++f) rank += tmp_orig[start + f] < mine;
-                if (e < n) perm[start + rank] = tmp_old[start + e];
-            }
+    if (ncell > 0 && base <= ncell - 1 && ncell - 1 < base + kScanItems) {
+        cell_start[ncell] = ra;
+        sc->nocc = rb;
+        if (clear_lists) {
+            sc->list_used = 0ull;
+            sc->w_short = 0u;
         }
     }
 }
 
-__global__ void k_gather(uint32_t n, const uint32_t* __restrict__ perm, StateBufs src,
-                         const double4* __restrict__ pos_next, const double4* __restrict__ vel_next,
-                         const int4* __restrict__ key_tmp, StateBufs dst,
-                         uint32_t* __restrict__ slot_of_orig) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+// Slots by cell, in any order within it. Clears tiles.
+__global__ void k_place(uint32_t n, const uint32_t* __restrict__ cellid, const uint32_t* __restrict__ rank,
+                        const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ orig,
+                        uint2* __restrict__ placed, unsigned long long* __restrict__ tiles, uint32_t ntiles) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = s; t < ntiles; t += gridDim.x * blockDim.x) tiles[t] = 0ull;
     if (s >= n) return;
-    uint32_t old = perm[s];
+    placed[cell_start[cellid[s]] + rank[s]] = make_uint2(orig[s], s);
+}
+
+// The place of the k-th placed slot: its cell's run is ordered by original index
+// (unique; grid.rs:86-87 tie-break).
+__device__ __forceinline__ uint32_t sorted_place(uint32_t k, const uint2* __restrict__ placed,
+                                                 const uint32_t* __restrict__ cellid,
+                                                 const uint32_t* __restrict__ cell_start, uint32_t* old) {
+    const uint2 me = placed[k];
+    const uint32_t c = cellid[me.y];
+    const uint32_t b = cell_start[c], e = cell_start[c + 1];
+    uint32_t at = b;
+#pragma unroll 4
+    for (uint32_t j = b; j < e; ++j) at += placed[j].x < me.x;
+    *old = me.y;
+    return at;
+}
+
+__global__ void k_order(uint32_t n, const uint2* __restrict__ placed, const uint32_t* __restrict__ cellid,
+                        const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ perm) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    uint32_t old;
+    const uint32_t s = sorted_place(k, placed, cellid, cell_start, &old);
+    perm[s] = old;
+}
+
+__global__ void k_move(uint32_t n, const uint2* __restrict__ placed, const uint32_t* __restrict__ cellid,
+                       const uint32_t* __restrict__ cell_start, StateBufs src, const double4* __restrict__ pos_next,
+                       const double4* __restrict__ vel_next, const int4* __restrict__ key_tmp, StateBufs dst,
+                       uint32_t* __restrict__ slot_of_orig) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    uint32_t old;
+    const uint32_t s = sorted_place(k, placed, cellid, cell_start, &old);
     uint8_t fl = src.flags[old];
     bool moved = !(fl & kFlagBoundary);
     dst.pos[s] = (moved && pos_next) ? pos_next[old] : src.pos[old];
@@ -264,48 +250,30 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 
 
 }  // namespace
 
-void launch_cell_ids(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur,
-                     const double4* pos_next, const uint8_t* flags, uint32_t* cellid, int4* key_tmp,
-                     uint32_t* count, DeviceScalars* sc, cudaStream_t st) {
-    if (n == 0) return;
-    k_cell_ids<<<blocks_for(n, 256), 256, 0, st>>>(g, tk, n, pos_cur, pos_next, flags, cellid, key_tmp,
-                                                  count, sc);
+size_t scan_tiles_bytes(uint32_t ncell) {
+    return sizeof(unsigned long long) * (size_t)((ncell + kScanTile - 1) / kScanTile + 1);
 }
 
-size_t scan_temp_bytes(uint32_t ncell) {
-    return sizeof(uint2) * (size_t)((ncell + kScanTile - 1) / kScanTile + 1);
+void launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur, const double4* pos_next,
+                      const uint8_t* flags, const uint32_t* orig, const GridBufs& b, DeviceScalars* sc,
+                      bool clear_lists, cudaStream_t st) {
+    const uint32_t ntiles = (g.ncell + kScanTile - 1) / kScanTile, nb = blocks_for(n, 256);
+    if (n)
+        k_cell_ids<<<nb, 256, 0, st>>>(g, tk, n, pos_cur, pos_next, flags, b.cellid, b.key_tmp, b.count, b.rank,
+                                       b.tiles, sc);
+    k_scan<<<ntiles, kScanThreads, 0, st>>>(g.ncell, b.count, b.tiles, b.cell_start, b.occ, sc, clear_lists ? 1 : 0);
+    if (n) k_place<<<nb, 256, 0, st>>>(n, b.cellid, b.rank, b.cell_start, orig, b.placed, b.tiles, ntiles);
 }
 
-void launch_scan_cells(uint32_t ncell, const uint32_t* count, uint32_t* cell_start, uint32_t* occ,
-                       DeviceScalars* sc, void* temp, cudaStream_t st) {
-    uint32_t ntiles = (ncell + kScanTile - 1) / kScanTile;
-    uint2* tiles = static_cast<uint2*>(temp);
-    k_scan_reduce<<<ntiles, kScanThreads, 0, st>>>(ncell, count, tiles);
-    k_scan_top<<<1, kScanThreads, 0, st>>>(ntiles, tiles, sc);
-    k_scan_down<<<ntiles, kScanThreads, 0, st>>>(ncell, count, tiles, cell_start, occ);
+void launch_order(uint32_t n, const GridBufs& b, uint32_t* perm, cudaStream_t st) {
+    if (n) k_order<<<blocks_for(n, 256), 256, 0, st>>>(n, b.placed, b.cellid, b.cell_start, perm);
 }
 
-void launch_place(uint32_t n, const uint32_t* cellid, const uint32_t* cell_start, uint32_t* fill,
-                  const uint32_t* orig, uint32_t* tmp_old, uint32_t* tmp_orig, cudaStream_t st) {
-    if (n == 0) return;
-    k_place<<<blocks_for(n, 256), 256, 0, st>>>(n, cellid, cell_start, fill, orig, tmp_old, tmp_orig);
-}
-
-void launch_cellsort(uint32_t ncell_max, const uint32_t* occ, const DeviceScalars* sc,
-                     const uint32_t* cell_start, const uint32_t* tmp_old, const uint32_t* tmp_orig,
-                     uint32_t* perm, cudaStream_t st) {
-    uint32_t warps = ncell_max < 148u * 64u ? ncell_max : 148u * 64u;
-    if (warps == 0) return;
-    k_cellsort<<<blocks_for((uint64_t)warps * 32u, 256), 256, 0, st>>>(occ, sc, cell_start, tmp_old,
-                                                                       tmp_orig, perm);
-}
-
-void launch_gather(uint32_t n, const uint32_t* perm, const StateBufs& src, const double4* pos_next,
-                   const double4* vel_next, const int4* key_tmp, const StateBufs& dst,
-                   uint32_t* slot_of_orig, double /*rho0*/, cudaStream_t st) {
-    if (n == 0) return;
-    k_gather<<<blocks_for(n, 256), 256, 0, st>>>(n, perm, src, pos_next, vel_next, key_tmp, dst,
-                                                slot_of_orig);
+void launch_move(uint32_t n, const GridBufs& b, const StateBufs& src, const double4* pos_next,
+                 const double4* vel_next, const StateBufs& dst, uint32_t* slot_of_orig, cudaStream_t st) {
+    if (n)
+        k_move<<<blocks_for(n, 256), 256, 0, st>>>(n, b.placed, b.cellid, b.cell_start, src, pos_next, vel_next,
+                                                  b.key_tmp, dst, slot_of_orig);
 }
 
 void launch_occupied_export(const GridDesc& g, const uint32_t* occ, const DeviceScalars* sc,

@@ -47,15 +47,13 @@ constexpr size_t kOffFlags = kOffPos + align256(kMaxN * 32);           // uint8[
 constexpr size_t kOffOrig = kOffFlags + align256(kMaxN);               // uint32[kMaxN]
 constexpr size_t kOffCellId = kOffOrig + align256(kMaxN * 4);          // uint32[kMaxN]
 constexpr size_t kOffKey = kOffCellId + align256(kMaxN * 4);           // int4[kMaxN]
-constexpr size_t kOffTmpOld = kOffKey + align256(kMaxN * 16);          // uint32[kMaxN]
-constexpr size_t kOffTmpOrig = kOffTmpOld + align256(kMaxN * 4);       // uint32[kMaxN]
-constexpr size_t kOffPerm = kOffTmpOrig + align256(kMaxN * 4);         // uint32[kMaxN]
+constexpr size_t kOffPlaced = kOffKey + align256(kMaxN * 16);          // uint2[kMaxN]
+constexpr size_t kOffPerm = kOffPlaced + align256(kMaxN * 8);          // uint32[kMaxN] (first the ranks)
 constexpr size_t kOffSPos = kOffPerm + align256(kMaxN * 4);            // double4[kMaxN] (sorted)
 constexpr size_t kOffSFlags = kOffSPos + align256(kMaxN * 32);         // uint8[kMaxN]
 constexpr size_t kOffSOrig = kOffSFlags + align256(kMaxN);             // uint32[kMaxN]
 constexpr size_t kOffCount = kOffSOrig + align256(kMaxN * 4);         // uint32[kMaxCells]
-constexpr size_t kOffFill = kOffCount + align256(kMaxCells * 4);       // uint32[kMaxCells]
-constexpr size_t kOffStart = kOffFill + align256(kMaxCells * 4);       // uint32[kMaxCells + 1]
+constexpr size_t kOffStart = kOffCount + align256(kMaxCells * 4);      // uint32[kMaxCells + 1]
 constexpr size_t kOffOcc = kOffStart + align256((kMaxCells + 1) * 4);  // uint32[kMaxCells]
 constexpr size_t kOffScan = kOffOcc + align256(kMaxCells * 4);         // scan tile sums
 constexpr size_t kScratchBytes = kOffScan + align256(8 * (kMaxCells / 4096 + 2));
@@ -242,26 +240,22 @@ extern "C" int pe_fluid_density_noalloc(int32_t dim, double rest_density, double
     k.r2_filter = std::nextafter((float)(sup * sup * (1.0 + 1e-4)), INFINITY);
 
     DeviceScalars* sc = reinterpret_cast<DeviceScalars*>(scratch + kOffHeader);
-    uint32_t* count = reinterpret_cast<uint32_t*>(scratch + kOffCount);
-    uint32_t* fill = reinterpret_cast<uint32_t*>(scratch + kOffFill);
-    uint32_t* start = reinterpret_cast<uint32_t*>(scratch + kOffStart);
-    uint32_t* occ = reinterpret_cast<uint32_t*>(scratch + kOffOcc);
-    uint32_t* cellid = reinterpret_cast<uint32_t*>(scratch + kOffCellId);
-    int4* key = reinterpret_cast<int4*>(scratch + kOffKey);
+    uint32_t* perm = reinterpret_cast<uint32_t*>(scratch + kOffPerm);
+    const GridBufs b{reinterpret_cast<uint32_t*>(scratch + kOffCellId),
+                     reinterpret_cast<int4*>(scratch + kOffKey),
+                     perm,
+                     reinterpret_cast<uint2*>(scratch + kOffPlaced),
+                     reinterpret_cast<uint32_t*>(scratch + kOffCount),
+                     reinterpret_cast<unsigned long long*>(scratch + kOffScan),
+                     reinterpret_cast<uint32_t*>(scratch + kOffStart),
+                     reinterpret_cast<uint32_t*>(scratch + kOffOcc)};
     // counters that must start at zero on every call
-    if (cudaMemsetAsync(count, 0, sizeof(uint32_t) * g.ncell, st) != cudaSuccess ||
-        cudaMemsetAsync(fill, 0, sizeof(uint32_t) * g.ncell, st) != cudaSuccess)
+    if (cudaMemsetAsync(b.count, 0, sizeof(uint32_t) * g.ncell, st) != cudaSuccess ||
+        cudaMemsetAsync(b.tiles, 0, scan_tiles_bytes(g.ncell), st) != cudaSuccess)
         return PE_ERR_DEVICE;
-    launch_cell_ids(g, Tanks{}, nn, reinterpret_cast<const double4*>(scratch + kOffPos), nullptr,
-                    scratch + kOffFlags, cellid, key, count, sc, st);
-    launch_scan_cells(g.ncell, count, start, occ, sc, scratch + kOffScan, st);
-    launch_place(nn, cellid, start, fill, reinterpret_cast<const uint32_t*>(scratch + kOffOrig),
-                 reinterpret_cast<uint32_t*>(scratch + kOffTmpOld),
-                 reinterpret_cast<uint32_t*>(scratch + kOffTmpOrig), st);
-    launch_cellsort(g.ncell < nn ? g.ncell : nn, occ, sc, start,
-                    reinterpret_cast<const uint32_t*>(scratch + kOffTmpOld),
-                    reinterpret_cast<const uint32_t*>(scratch + kOffTmpOrig),
-                    reinterpret_cast<uint32_t*>(scratch + kOffPerm), st);
+    launch_cell_sort(g, Tanks{}, nn, reinterpret_cast<const double4*>(scratch + kOffPos), nullptr,
+                     scratch + kOffFlags, reinterpret_cast<const uint32_t*>(scratch + kOffOrig), b, sc, false, st);
+    launch_order(nn, b, perm, st);
     k_na_gather<<<blocks_for(nn, 256), 256, 0, st>>>(nn, scratch);
     if (dim == 3)
         k_na_density<3><<<blocks_for(nn, 128), 128, 0, st>>>(nn, g, k, scratch, n_out, rho);

@@ -568,14 +568,14 @@ void PbfSolver::step(double dt) {
     // pbf.rs:387-401: predict, grid and lists on the predictions
     k_pbf_predict<<<nb, kPbfThreads, 0, st>>>(n, kc_, dt, w.cur_, w.pos_nx_);
     w.launches_ += 1;
-    w.build_grid(w.pos_nx_, nullptr);
+    w.build_grid(w.pos_nx_, nullptr, true);
     // pbf.rs:146-156: candidates of the neighbour cells, kept while the
     // predictions move (reuse_neighbours). The others add +-0, so each
     // iteration's lists hold the candidates then in support.
     const bool reused = prm_.reuse_neighbours && prm_.iterations > 1;
     // pbf.rs:403-411: constraint iterations
     for (uint64_t it = 0; it < prm_.iterations; ++it) {
-        if (it > 0 && !prm_.reuse_neighbours) w.build_grid(nullptr, nullptr);
+        if (it > 0 && !prm_.reuse_neighbours) w.build_grid(nullptr, nullptr, true);
         lists(reused);
         constrain();
     }
@@ -583,7 +583,7 @@ void PbfSolver::step(double dt) {
     // lists on the final positions, density there
     k_pbf_finalize<<<nb, kPbfThreads, 0, st>>>(n, dt, w.cur_);
     w.launches_ += 1;
-    w.build_grid(nullptr, nullptr);
+    w.build_grid(nullptr, nullptr, true);
     lists(false);
     density();
     // pbf.rs:288-381: the grid on x equals the one just built

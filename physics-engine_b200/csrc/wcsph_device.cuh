@@ -236,20 +236,28 @@ void launch_xsph_f32(uint32_t n, uint32_t threads, uint32_t lanes, const F32Cons
                      bool use_w = false);
 
 // ----- grid build -----
-void launch_cell_ids(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur,
-                     const double4* pos_next, const uint8_t* flags, uint32_t* cellid, int4* key_tmp,
-                     uint32_t* count, DeviceScalars* sc, cudaStream_t st);
-size_t scan_temp_bytes(uint32_t ncell);
-void launch_scan_cells(uint32_t ncell, const uint32_t* count, uint32_t* cell_start, uint32_t* occ,
-                       DeviceScalars* sc, void* temp, cudaStream_t st);
-void launch_place(uint32_t n, const uint32_t* cellid, const uint32_t* cell_start, uint32_t* fill,
-                  const uint32_t* orig, uint32_t* tmp_old, uint32_t* tmp_orig, cudaStream_t st);
-void launch_cellsort(uint32_t ncell_max, const uint32_t* occ, const DeviceScalars* sc,
-                     const uint32_t* cell_start, const uint32_t* tmp_old, const uint32_t* tmp_orig,
-                     uint32_t* perm, cudaStream_t st);
-void launch_gather(uint32_t n, const uint32_t* perm, const StateBufs& src, const double4* pos_next,
-                   const double4* vel_next, const int4* key_tmp, const StateBufs& dst,
-                   uint32_t* slot_of_orig, double rho0, cudaStream_t st);
+// Working memory of a grid build (n slots, ncell cells).
+struct GridBufs {
+    uint32_t* cellid;           // [n]
+    int4* key_tmp;              // [n]
+    uint32_t* rank;             // [n] arrival number of a slot in its cell
+    uint2* placed;              // [n] (original index, slot) by cell
+    uint32_t* count;            // [ncell], zero between builds
+    unsigned long long* tiles;  // scan_tiles_bytes(ncell), zero between builds
+    uint32_t* cell_start;       // [ncell + 1]
+    uint32_t* occ;              // [ncell]
+};
+size_t scan_tiles_bytes(uint32_t ncell);
+// Cell ranges, occupied cells and the slots of each cell (in any order).
+// clear_lists: clears sc->list_used and sc->w_short for the list build and
+// density pass that follow.
+void launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur, const double4* pos_next,
+                      const uint8_t* flags, const uint32_t* orig, const GridBufs& b, DeviceScalars* sc,
+                      bool clear_lists, cudaStream_t st);
+// Then either perm (new slot -> old slot) or the state moved to its new slots.
+void launch_order(uint32_t n, const GridBufs& b, uint32_t* perm, cudaStream_t st);
+void launch_move(uint32_t n, const GridBufs& b, const StateBufs& src, const double4* pos_next,
+                 const double4* vel_next, const StateBufs& dst, uint32_t* slot_of_orig, cudaStream_t st);
 
 // ----- neighbour lists -----
 uint32_t nlist_union_capacity(uint32_t max_union);

@@ -268,15 +268,15 @@ World::World(const WorldParams& prm, const WorldConfig& cfg, int dim, double res
         vel_nx_ = alloc<double4>(N);
         slot_of_orig_ = alloc<uint32_t>(N);
         cellid_ = alloc<uint32_t>(N);
-        tmp_old_ = alloc<uint32_t>(N);
-        tmp_orig_ = alloc<uint32_t>(N);
-        perm_ = alloc<uint32_t>(N);
+        rank_ = alloc<uint32_t>(N);
+        placed_ = alloc<uint2>(N);
         key_tmp_ = alloc<int4>(N);
         count_ = alloc<uint32_t>(g_.ncell);
-        fill_ = alloc<uint32_t>(g_.ncell);
         cell_start_ = alloc<uint32_t>((size_t)g_.ncell + 1);
         occ_ = alloc<uint32_t>(g_.ncell);
-        scan_tmp_ = alloc<unsigned char>(scan_temp_bytes(g_.ncell));
+        tiles_ = alloc<unsigned long long>(scan_tiles_bytes(g_.ncell) / sizeof(unsigned long long));
+        check(cudaMemsetAsync(count_, 0, sizeof(uint32_t) * g_.ncell, st_), "memset");
+        check(cudaMemsetAsync(tiles_, 0, scan_tiles_bytes(g_.ncell), st_), "memset");
         lists_.nslots = (uint32_t)N;
         // first guess of the list pool: max_neighbours entries per slot (the
         // first build measures the need and resizes)
@@ -625,18 +625,14 @@ void World::set_sound_speed(double c) {
 
 void World::synchronize() { check(cudaStreamSynchronize(st_), "synchronize"); }
 
-void World::build_grid(const double4* pos_next, const double4* vel_next) {
+void World::build_grid(const double4* pos_next, const double4* vel_next, bool lists_follow) {
     const uint32_t n = (uint32_t)n_;
+    const GridBufs b{cellid_, key_tmp_, rank_, placed_, count_, tiles_, cell_start_, occ_};
     prof_begin(kGrid);
-    check(cudaMemsetAsync(count_, 0, sizeof(uint32_t) * g_.ncell, st_), "memset");
-    check(cudaMemsetAsync(fill_, 0, sizeof(uint32_t) * g_.ncell, st_), "memset");
-    launch_cell_ids(g_, tanks_, n, cur_.pos, pos_next, cur_.flags, cellid_, key_tmp_, count_, sc_, st_);
-    launch_scan_cells(g_.ncell, count_, cell_start_, occ_, sc_, scan_tmp_, st_);
-    launch_place(n, cellid_, cell_start_, fill_, cur_.orig, tmp_old_, tmp_orig_, st_);
-    launch_cellsort(std::min<uint32_t>(g_.ncell, n ? n : 1), occ_, sc_, cell_start_, tmp_old_, tmp_orig_,
-                    perm_, st_);
-    launch_gather(n, perm_, cur_, pos_next, vel_next, key_tmp_, alt_, slot_of_orig_, rho0_, st_);
-    launches_ += 7;
+    launch_cell_sort(g_, tanks_, n, cur_.pos, pos_next, cur_.flags, cur_.orig, b, sc_, lists_follow, st_);
+    launch_move(n, b, cur_, pos_next, vel_next, alt_, slot_of_orig_, st_);
+    launches_ += 4;
+    list_used_cleared_ = w_short_cleared_ = lists_follow;
     prof_end();
     std::swap(cur_, alt_);
     grid_built_ = true;
@@ -673,7 +669,7 @@ void World::ensure_lists(bool visit_only) {
         // Every pass of this loop builds into the current pool, so the loop
         // always ends with lists built in the pool they describe.
         for (int attempt = 0;; ++attempt) {
-            check(cudaMemsetAsync(&sc_->list_used, 0, sizeof(unsigned long long), st_), "memset");
+            clear_list_used();
             prof_begin(kLists);
             launch_nlist(g_, tanks_, kc_, ucap_, nl_blocks_, occ_, cell_start_, cur_, lists_, sc_, st_,
                          build_visit_only, list_chunk_);
@@ -718,8 +714,15 @@ void World::ensure_lists(bool visit_only) {
     lists_full_ = grid_built_ && !build_visit_only;
 }
 
+// The counter of the list build about to be launched, unless the grid build has
+// cleared it.
+void World::clear_list_used() {
+    if (!list_used_cleared_) check(cudaMemsetAsync(&sc_->list_used, 0, sizeof(unsigned long long), st_), "memset");
+    list_used_cleared_ = false;
+}
+
 void World::build_near_lists() {
-    check(cudaMemsetAsync(&sc_->list_used, 0, sizeof(unsigned long long), st_), "memset");
+    clear_list_used();
     prof_begin(kLists);
     launch_nlist_near(g_, tanks_, support_, std::min<uint32_t>(g_.ncell, (uint32_t)std::max<uint64_t>(n_, 1)), sms_, occ_,
                       cell_start_, cur_, lists_, sc_, st_);
@@ -733,7 +736,9 @@ void World::build_near_lists() {
 
 void World::run_density(bool visit_only) {
     ensure_lists(visit_only);
-    if (pair_weights()) check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
+    if (pair_weights() && !w_short_cleared_)
+        check(cudaMemsetAsync(&sc_->w_short, 0, sizeof(uint32_t), st_), "memset");
+    w_short_cleared_ = false;
     prof_begin(kDensity);
     if (f32_) launch_density_f32((uint32_t)n_, shape_.density, lanes_.density, kf_, cur_, fb_, lists_, st_);
     else launch_density((uint32_t)n_, shape_.density, lanes_.density, kc_, cur_, lists_, st_);
@@ -870,13 +875,13 @@ void World::step(double dt) {
     // of the current positions, rebuilding them reproduces the same bits, so
     // they are reused.
     if (!(grid_current_ && rho_current_)) {
-        build_grid(nullptr, nullptr);
+        build_grid(nullptr, nullptr, true);
         refresh_f32();
         run_density();
     }
     run_pressure();               // wcsph.rs:329
     run_forces(true, dt);         // wcsph.rs:330-342 (kick + drift fused)
-    build_grid(pos_nx_, vel_nx_); // wcsph.rs:343
+    build_grid(pos_nx_, vel_nx_, true); // wcsph.rs:343
     refresh_f32();
     run_density();                // wcsph.rs:344
     run_xsph();                   // wcsph.rs:345

@@ -188,7 +188,9 @@ class World {
     double ck_t_ = 0.0;
     float* judge_err_ = nullptr;
     void check(cudaError_t e, const char* what);
-    void build_grid(const double4* pos_next, const double4* vel_next);
+    // lists_follow: the caller builds the lists, and then the densities, next
+    void build_grid(const double4* pos_next, const double4* vel_next, bool lists_follow = false);
+    void clear_list_used();
     void ensure_lists(bool visit_only = false);
     // Visit lists of the candidates (cells of the last grid) within the
     // support radius at the present positions. The pool must have been sized (lists_checked_).
@@ -249,10 +251,12 @@ class World {
     double4* pos_nx_ = nullptr;
     double4* vel_nx_ = nullptr;
     uint32_t* slot_of_orig_ = nullptr;
-    uint32_t *cellid_ = nullptr, *tmp_old_ = nullptr, *tmp_orig_ = nullptr, *perm_ = nullptr;
+    uint32_t *cellid_ = nullptr, *rank_ = nullptr;
+    uint2* placed_ = nullptr;
     int4* key_tmp_ = nullptr;
-    uint32_t *count_ = nullptr, *fill_ = nullptr, *cell_start_ = nullptr, *occ_ = nullptr;
-    void* scan_tmp_ = nullptr;
+    uint32_t *count_ = nullptr, *cell_start_ = nullptr, *occ_ = nullptr;
+    unsigned long long* tiles_ = nullptr;
+    bool list_used_cleared_ = false, w_short_cleared_ = false;
     ListBufs lists_{};
     uint32_t* insup_ = nullptr;
     DeviceScalars* sc_ = nullptr;
