@@ -10,18 +10,24 @@
 // which the unfused path computes as three GEMM launches writing E x 128
 // activations to memory (~60 GB of traffic per hop at 3.3e7 edges) and a
 // segment sum. Here one persistent CTA per SM keeps Wc, W2 and W3 in shared
-// memory; its two warpgroups walk their own tiles of 128 edges, each with its
+// memory; its four warpgroups walk their own tiles of 128 edges, each with its
 // own 128 tensor-memory columns, buffers and barriers, so one group's MMA
-// waits and gathers overlap the other's epilogues. Per tile, x_e Wc is one
+// waits and gathers overlap the others' epilogues. Per tile, x_e Wc is one
 // K=16 tcgen05 MMA into the group's accumulator; the epilogue (thread r =
 // edge r = TMEM lane r) adds b1, P[i] and Q[j] in the unfused epilogue's
-// order (the next tile's endpoints and features, and the next 32-column block
+// order (the next tile's endpoints and features, and the next 16-column block
 // of P[i] and Q[j], are already loading), applies ReLU and
 // writes bf16 into a swizzled shared-memory tile that is the A operand of
 // the next 8 MMAs (K = 128), and so on; the last epilogue stages the
 // messages in shared memory and sums each run of equal destinations before
 // one atomic add per run and column. Activations are rounded to bf16 at the
 // same points as in the unfused path; only the message sum's order differs.
+//
+// A tile is one long chain (copy, MMA, epilogue, MMA, ...), so what counts is how
+// many run on an SM: with two groups, a third buffer and 32-column blocks in
+// flight (16 KB more a group, twice the registers) 2.56M edges took 1.72 ms, with
+// four 0.74. The shared-memory and L1 data path is 78% busy then, half of it the
+// gathers of Q[j] and the messages' staging.
 //
 // Every mbarrier wait is bounded; a wait that runs out sets bit 0 of *err and
 // ends the tile loop of the whole CTA (at the tile's end, by a block-wide
@@ -39,19 +45,23 @@ namespace {
 
 using namespace umma;
 
-constexpr int kGroups = 2;             // warpgroups per CTA, each on its own tiles
+constexpr int kGroups = 4;             // warpgroups per CTA, each on its own tiles
 constexpr int kGroupThreads = 128;     // one thread per edge of a tile (TMEM lane)
 constexpr int kEdgeThreads = kGroups * kGroupThreads;
 constexpr uint32_t kSlice = 128u * 128u;  // bytes of a 128-row x 64-column bf16 slice
-constexpr uint32_t kOffWc = 0;                    // Wc^T [128 x 16]: chunks 0-1 of one slice
-constexpr uint32_t kOffW2 = kOffWc + kSlice;      // W2^T [128 x 128]: two slices
+constexpr uint32_t kOffW2 = 0;                    // W2^T [128 x 128]: two slices
 constexpr uint32_t kOffW3 = kOffW2 + 2 * kSlice;  // W3^T: two slices
-constexpr uint32_t kOffGroup = kOffW3 + 2 * kSlice;
-// per warpgroup: the edge-feature slice [128 x 16] (chunks 0-1), which the
-// last epilogue reuses for the fp32 messages (128 rows x 32 columns, column
-// j of row r at j ^ (r & 31)), then the activation tile [128 x 128]
-constexpr uint32_t kGroupBytes = 3 * kSlice;
+// Matrices of 16 columns (two 16-byte chunks a row) share slices, four to one:
+// matrix m in chunks 2 (m % 4) and 2 (m % 4) + 1 of slice m / 4. Matrix 0 is
+// Wc^T [128 x 16], matrix 1 + g group g's edge features [128 x 16].
+constexpr uint32_t kOffNarrow = kOffW3 + 2 * kSlice;
+constexpr uint32_t kNarrowSlices = (1 + kGroups + 3) / 4;
+// per group the activation tile [128 x 128]; the last epilogue reuses it for
+// fp32 messages, a warp's 32 rows x 32 columns in its own rows of a slice
+constexpr uint32_t kOffGroup = kOffNarrow + kNarrowSlices * kSlice;
+constexpr uint32_t kGroupBytes = 2 * kSlice;
 constexpr uint32_t kSmemBytes = kOffGroup + kGroups * kGroupBytes + 1024u;  // + alignment slack
+static_assert(kSmemBytes + 2048u <= 232448u, "one CTA's shared memory, with its biases and barriers");
 
 __device__ __forceinline__ uint32_t sw_off(int row, int chunk) {
     return (uint32_t)row * 128u + ((uint32_t)(chunk ^ (row & 7)) << 4);
@@ -85,19 +95,33 @@ __device__ void stage_rows(uint8_t* dst, const __nv_bfloat16* __restrict__ src, 
     }
 }
 
-// 32 fp32 values (columns 32 cb .. 32 cb + 31 of row r) into the bf16 activation tile
-__device__ __forceinline__ void put_bf16_row(uint8_t* sA, int r, int cb, const float (&x)[32]) {
+// N fp32 values (columns c0 .. c0 + N - 1 of row r) into the bf16 activation tile
+template <int N>
+__device__ __forceinline__ void put_bf16_row(uint8_t* sA, int r, int c0, const float (&x)[N]) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < N / 8; ++q) {
         uint32_t w[4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             __nv_bfloat162 b = __floats2bfloat162_rn(x[q * 8 + 2 * h], x[q * 8 + 2 * h + 1]);
             w[h] = *reinterpret_cast<uint32_t*>(&b);
         }
-        const int cidx = cb * 4 + q;  // 16-byte chunk of the 128-column row
+        const int cidx = c0 / 8 + q;  // 16-byte chunk of the 128-column row
         *reinterpret_cast<uint4*>(sA + (uint32_t)(cidx >> 3) * kSlice + sw_off(r, cidx & 7)) =
             make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// N biases from c0 on (a multiple of 4) of a layer in shared memory
+template <int N>
+__device__ __forceinline__ void get_bias(const float* b, float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+        const float4 f = *reinterpret_cast<const float4*>(b + 4 * i);
+        v[4 * i] = f.x;
+        v[4 * i + 1] = f.y;
+        v[4 * i + 2] = f.z;
+        v[4 * i + 3] = f.w;
     }
 }
 
@@ -111,21 +135,20 @@ __device__ __forceinline__ void issue_k128(uint32_t tmem, const uint8_t* sA, con
                       sw128_desc(b0 + (uint32_t)s * kSlice + kk * 32), (s | kk) ? 1u : 0u);
 }
 
-__global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
+__global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar[kGroups];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_dst[kGroups][kGroupThreads];
+    __shared__ __align__(16) float s_bias[3][128];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = tid / kGroupThreads, gt = tid % kGroupThreads, gw = gt >> 5;
-    uint8_t* sWc = smem + kOffWc;
+    uint8_t* sWc = smem + kOffNarrow;
     uint8_t* sW2 = smem + kOffW2;
     uint8_t* sW3 = smem + kOffW3;
-    uint8_t* sX = smem + kOffGroup + (uint32_t)g * kGroupBytes;
-    float* sStage = reinterpret_cast<float*>(sX);  // free once the tile's first MMA completed
-    uint8_t* sA = sX + kSlice;
-    int* dstv = s_dst[g];
+    uint8_t* sX = smem + kOffNarrow + (uint32_t)((g + 1) / 4) * kSlice;
+    const int xc = 2 * ((g + 1) % 4);  // first chunk of the group's edge features in it
+    uint8_t* sA = smem + kOffGroup + (uint32_t)g * kGroupBytes;
 
     if (tid == 0) {
         for (int i = 0; i < kGroups; ++i) mbar_init(smem_addr(&mbar[i]), 1);
@@ -141,6 +164,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
     stage_rows(sWc, a.Wc, 16, 2);
     stage_rows(sW2, a.W2, 128, 16);
     stage_rows(sW3, a.W3, 128, 16);
+    if (tid < 3 * 128) s_bias[tid >> 7][tid & 127] = __ldg((tid < 128 ? a.b1 : tid < 256 ? a.b2 : a.b3) + (tid & 127));
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -178,12 +202,12 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
             x1 = __ldg(reinterpret_cast<const uint4*>(a.xe + (size_t)e * 16 + 8));
         }
     };
-    // 32 columns (block cb) of this edge's P[dst] and Q[src] rows
-    auto fetch_pq = [&](int d, int sj, int cb, float4 (&p)[8], float4 (&q)[8]) {
-        const float4* P4 = reinterpret_cast<const float4*>(a.P + (size_t)(d < 0 ? 0 : d) * 128 + cb * 32);
-        const float4* Q4 = reinterpret_cast<const float4*>(a.Q + (size_t)(sj < 0 ? 0 : sj) * 128 + cb * 32);
+    // 16 columns (block cb) of this edge's P[dst] and Q[src] rows
+    auto fetch_pq = [&](int d, int sj, int cb, float4 (&p)[4], float4 (&q)[4]) {
+        const float4* P4 = reinterpret_cast<const float4*>(a.P + (size_t)(d < 0 ? 0 : d) * 128 + cb * 16);
+        const float4* Q4 = reinterpret_cast<const float4*>(a.Q + (size_t)(sj < 0 ? 0 : sj) * 128 + cb * 16);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
             p[i] = __ldg(P4 + i);
             q[i] = __ldg(Q4 + i);
         }
@@ -194,50 +218,43 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
     fetch_edge(first, d, sj, x0, x1);
     for (int tile = first; tile < ntiles; tile += stride) {
         // ---- edge features and endpoints of the tile (fetched a tile ahead)
-        dstv[gt] = d;
-        *reinterpret_cast<uint4*>(sX + sw_off(gt, 0)) = x0;
-        *reinterpret_cast<uint4*>(sX + sw_off(gt, 1)) = x1;
+        *reinterpret_cast<uint4*>(sX + sw_off(gt, xc)) = x0;
+        *reinterpret_cast<uint4*>(sX + sw_off(gt, xc + 1)) = x1;
         const int dc = d, sc = sj;
         to_tensor();
         // ---- layer 1: x_e Wc (one K = 16 MMA), then + b1 + P[dst] + Q[src], ReLU
         if (gt == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            umma_bf16(tmem, sw128_desc(smem_addr(sX)), sw128_desc(smem_addr(sWc)), 0u);
+            umma_bf16(tmem, sw128_desc(smem_addr(sX) + 16u * (uint32_t)xc), sw128_desc(smem_addr(sWc)), 0u);
             umma_commit(bar);
         }
         // the next tile's edge and this edge's first P/Q block load while the MMA runs
         fetch_edge(tile + stride, d, sj, x0, x1);
-        float4 pa[8], qa[8];
-        fetch_pq(dc, sc, 0, pa, qa);
+        float4 pq[2][2][4];
+        fetch_pq(dc, sc, 0, pq[0][0], pq[0][1]);
         ok = mma_wait() && ok;
 #pragma unroll
-        for (int cb = 0; cb < 4; ++cb) {
-            float4 pb[8], qb[8];
-            if (cb < 3) fetch_pq(dc, sc, cb + 1, pb, qb);  // one block ahead
-            uint32_t v[32];
-            tmem_ld32(trow + (uint32_t)(cb * 32), v);
-            float x[32];
+        for (int cb = 0; cb < 8; ++cb) {
+            const int now = cb & 1;
+            if (cb < 7) fetch_pq(dc, sc, cb + 1, pq[now ^ 1][0], pq[now ^ 1][1]);  // one block ahead
+            uint32_t v[16];
+            tmem_ld16(trow + (uint32_t)(cb * 16), v);
+            float x[16], bias[16];
+            get_bias(s_bias[0] + cb * 16, bias);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float pv[4] = {pa[i].x, pa[i].y, pa[i].z, pa[i].w};
-                const float qv[4] = {qa[i].x, qa[i].y, qa[i].z, qa[i].w};
+            for (int i = 0; i < 4; ++i) {
+                const float4 p4 = pq[now][0][i], q4 = pq[now][1][i];
+                const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
                     const int j = i * 4 + h;
-                    float t = __uint_as_float(v[j]) + a.b1[cb * 32 + j];  // the unfused epilogue's order
+                    float t = __uint_as_float(v[j]) + bias[j];  // the unfused epilogue's order
                     t += pv[h];
                     t += qv[h];
                     x[j] = fmaxf(t, 0.f);
                 }
             }
-            put_bf16_row(sA, gt, cb, x);
-            if (cb < 3) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    pa[i] = pb[i];
-                    qa[i] = qb[i];
-                }
-            }
+            put_bf16_row(sA, gt, cb * 16, x);
         }
         to_tensor();
         // ---- layer 2: relu(z1 W2 + b2)
@@ -251,10 +268,11 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
         for (int cb = 0; cb < 4; ++cb) {
             uint32_t v[32];
             tmem_ld32(trow + (uint32_t)(cb * 32), v);
-            float x[32];
+            float x[32], bias[32];
+            get_bias(s_bias[1] + cb * 32, bias);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = fmaxf(__uint_as_float(v[j]) + a.b2[cb * 32 + j], 0.f);
-            put_bf16_row(sA, gt, cb, x);  // the MMAs that read sA have completed
+            for (int j = 0; j < 32; ++j) x[j] = fmaxf(__uint_as_float(v[j]) + bias[j], 0.f);
+            put_bf16_row(sA, gt, cb * 32, x);  // the MMAs that read sA have completed
         }
         to_tensor();
         // ---- layer 3: m_e = z2 W3 + b3, summed per destination
@@ -264,30 +282,33 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_hop(EdgeHopArgs a) {
             umma_commit(bar);
         }
         ok = mma_wait() && ok;
+        // A warp sums its own 32 rows (rows past the last edge close the tile):
+        // lane j column j, row by row, one atomic per run of a destination.
+        const int rows = __popc(__ballot_sync(0xffffffffu, dc >= 0));
+        const int above = __shfl_up_sync(0xffffffffu, dc, 1);
+        const uint32_t heads = __ballot_sync(0xffffffffu, dc >= 0 && (lane == 0 || above != dc));
 #pragma unroll 1
         for (int cb = 0; cb < 4; ++cb) {
             uint32_t v[32];
             tmem_ld32(trow + (uint32_t)(cb * 32), v);
+            float bias[32];
+            get_bias(s_bias[2] + cb * 32, bias);
+            // column j of row r at j ^ r; blocks alternate between the slices, so
+            // that one is read while the next is written
+            float* const st = reinterpret_cast<float*>(sA + (uint32_t)(cb & 1) * kSlice + (uint32_t)gw * 4096u);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) sStage[gt * 32 + (j ^ (gt & 31))] = __uint_as_float(v[j]) + a.b3[cb * 32 + j];
-            group_sync(g);
-            // thread (warp gw, column j): rows 32 gw .. 32 gw + 31, one atomic per run of a destination
-            const int j = lane;
-            int cur = -1;
-            float acc = 0.f;
-            for (int rr = 0; rr < 32; ++rr) {
-                const int row = gw * 32 + rr, dd = dstv[row];
-                if (dd < 0) break;  // rows past the last edge close the tile
-                if (dd != cur) {
-                    if (cur >= 0) atomicAdd(a.out + (size_t)cur * 128 + cb * 32 + j, acc);
-                    cur = dd;
-                    acc = 0.f;
-                }
-                acc += sStage[row * 32 + (j ^ (row & 31))];
+            for (int j = 0; j < 32; ++j) st[lane * 32 + (j ^ lane)] = __uint_as_float(v[j]) + bias[j];
+            __syncwarp();
+            for (uint32_t left = heads; left; left &= left - 1u) {
+                const int r0 = __ffs(left) - 1, r1 = (left & (left - 1u)) ? __ffs(left & (left - 1u)) - 1 : rows;
+                const int to = __shfl_sync(0xffffffffu, dc, r0);
+                float acc = 0.f;
+#pragma unroll 8
+                for (int r = r0; r < r1; ++r) acc += st[r * 32 + (lane ^ r)];
+                atomicAdd(a.out + (size_t)to * 128 + cb * 32 + lane, acc);
             }
-            if (cur >= 0) atomicAdd(a.out + (size_t)cur * 128 + cb * 32 + j, acc);
-            group_sync(g);  // the staging buffer is reused by the next column block
         }
+        __syncwarp();  // the next tile's activations go where the messages were
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         // the tile's TMEM reads and shared-memory use end before the group's
         // next tile; a run-out wait on any thread of the group stops the whole
