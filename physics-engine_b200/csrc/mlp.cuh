@@ -56,6 +56,31 @@ struct EdgeHopArgs {
 bool edge_hop_prepare();
 void launch_edge_hop(const EdgeHopArgs& a, int sms, cudaStream_t st);
 
+// A node MLP fused into one persistent kernel (node_fused.cu), for inference. x is
+// bf16 [n x min(k1, 128)] with k1 = 8, 128 or 256; with 256 the other 128 inputs
+// are bf16(scale * msg), msg fp32 [n x 128]. Weights bf16 K-major ([128 x k1],
+// [128 x 128], [n3 x 128]). n3 = 8: y fp32 [n x 8]. n3 = 128: h fp32 and hb bf16
+// [n x 128] = the output, or with fluid h += the output on fluid nodes, hb = bf16(h).
+struct NodeMlpArgs {
+    int n, k1, n3;
+    const __nv_bfloat16* x;
+    const float* msg;
+    float scale;
+    const __nv_bfloat16* W1;
+    const float* b1;
+    const __nv_bfloat16* W2;
+    const float* b2;
+    const __nv_bfloat16* W3;
+    const float* b3;
+    float* y;
+    float* h;
+    __nv_bfloat16* hb;
+    const uint8_t* fluid;
+    uint32_t* err;  // bit 0: a bounded wait ran out
+};
+bool node_mlp_prepare();
+void launch_node_mlp(const NodeMlpArgs& a, int sms, cudaStream_t st);
+
 bool gemm_prepare();
 void launch_gemm(const GemmArgs& g, int splits, cudaStream_t st);
 void launch_gemm_reduce(int M, int N, int ldc, int splits, const float* part, const float* bias, int relu,

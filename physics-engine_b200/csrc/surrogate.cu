@@ -363,7 +363,8 @@ Surrogate::Surrogate(uint64_t seed, double r_msg_over_h) : r_msg_over_h_(r_msg_o
     cu(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking), "stream");
     own_stream_ = true;
     if (!gemm_prepare()) throw std::runtime_error("surrogate: GEMM shared-memory limit");
-    if (!edge_hop_prepare()) throw std::runtime_error("surrogate: fused edge kernel shared-memory limit");
+    if (!edge_hop_prepare() || !node_mlp_prepare())
+        throw std::runtime_error("surrogate: fused kernels' shared-memory limit");
     {
         int dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess)
@@ -616,13 +617,26 @@ void Surrogate::forward(bool keep_for_backward) {
     ensure_acts(keep_for_backward);
     const int n = g_.n, E = g_.E;
     const size_t nW = (size_t)n * kWidth;
-    mlp_fwd(0, g_.f, n, enc_a1_, enc_a2_, h_);
-    k_to_bf16<<<blocks(nW, 256), 256, 0, st_>>>(nW, h_, hb_[0]);
+    const bool fused = fused_edges_ && !keep_for_backward;
+    // one fused node MLP: layers first .. first + 2 on x (and the messages)
+    auto node_mlp = [&](int first, const __nv_bfloat16* x, const float* msg, const uint8_t* fluid,
+                        __nv_bfloat16* hb) {
+        const Linear &L0 = layers_[first], &L1 = layers_[first + 1], &L2 = layers_[first + 2];
+        NodeMlpArgs na{n, L0.K, L2.Np, x, msg, kAggScale, L0.Wt16, L0.b, L1.Wt16, L1.b, L2.Wt16, L2.b, Y_, h_, hb,
+                       fluid, err_};
+        launch_node_mlp(na, sms_, st_);
+    };
+    if (fused) {
+        node_mlp(0, g_.f, nullptr, nullptr, hb_[0]);
+    } else {
+        mlp_fwd(0, g_.f, n, enc_a1_, enc_a2_, h_);
+        k_to_bf16<<<blocks(nW, 256), 256, 0, st_>>>(nW, h_, hb_[0]);
+    }
     for (int l = 0; l < 2; ++l) {
         const int base = 3 + 8 * l;
         linear_fwd(layers_[base + 0], hb_[l], n, P_, nullptr, false);
         linear_fwd(layers_[base + 1], hb_[l], n, Q_, nullptr, false);
-        if (E > 0 && fused_edges_ && !keep_for_backward) {
+        if (E > 0 && fused) {
             // the whole edge MLP and the sum per destination in one kernel
             const Linear &L0 = layers_[base + 2], &L1 = layers_[base + 3], &L2 = layers_[base + 4];
             cu(cudaMemsetAsync(A_, 0, sizeof(float) * nW, st_), "memset");
@@ -641,13 +655,17 @@ void Surrogate::forward(bool keep_for_backward) {
             linear_fwd(layers_[base + 3], eh1_[l], E, nullptr, eh2_[l], true);
             linear_fwd(layers_[base + 4], eh2_[l], E, M_, nullptr, false);
         }
-        if (!(E > 0 && fused_edges_ && !keep_for_backward))
-            k_segsum<<<blocks((size_t)n * 32, 256), 256, 0, st_>>>(n, g_.row, M_, 1.f, A_);
+        if (!(E > 0 && fused)) k_segsum<<<blocks((size_t)n * 32, 256), 256, 0, st_>>>(n, g_.row, M_, 1.f, A_);
+        if (fused) {
+            node_mlp(base + 5, hb_[l], A_, g_.fluid, hb_[l + 1]);
+            continue;
+        }
         k_concat<<<blocks(2 * nW, 256), 256, 0, st_>>>(n, hb_[l], A_, kAggScale, xn_[l]);
         mlp_fwd(base + 5, xn_[l], n, na1_[l], na2_[l], U_);
         k_residual<<<blocks(nW, 256), 256, 0, st_>>>(n, U_, g_.fluid, h_, hb_[l + 1]);
     }
-    mlp_fwd(19, hb_[2], n, da1_, da2_, Y_);
+    if (fused) node_mlp(19, hb_[2], nullptr, nullptr, nullptr);
+    else mlp_fwd(19, hb_[2], n, da1_, da2_, Y_);
     cu(cudaGetLastError(), "forward");
 }
 
