@@ -69,6 +69,15 @@ __global__ void k_residual(int n, const float* __restrict__ u, const uint8_t* __
     hb_next[i] = __float2bfloat16_rn(v);
 }
 
+// The outputs without the padding columns: what crosses to the host is what the
+// caller asked for (101,376 nodes: 0.1 ms of copy, where 3.2 MB and a loop over
+// them on the host took 0.7).
+__global__ void k_pack_outputs(int n, const float* __restrict__ Y, float4* __restrict__ out) {
+    static_assert(kOut == 4 && kOutPad == 8, "a row is the first of two float4");
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = reinterpret_cast<const float4*>(Y)[2 * (size_t)i];
+}
+
 // loss = sum over fluid nodes of |y - t|^2 / nf; dY = 2 (y - t) / nf (padding columns 0)
 __global__ void k_loss(int n, const float* __restrict__ Y, const float* __restrict__ T,
                        const uint8_t* __restrict__ fluid, float inv_nf, float* __restrict__ dY,
@@ -671,11 +680,11 @@ void Surrogate::forward(bool keep_for_backward) {
 
 void Surrogate::get_outputs(float* y) {
     const int n = g_.n;
-    std::vector<float> buf((size_t)n * kOutPad);
-    cu(cudaMemcpyAsync(buf.data(), Y_, buf.size() * 4, cudaMemcpyDeviceToHost, st_), "outputs");
+    if (n <= 0) return;
+    // dY_ is the backward pass's, which writes it before it reads it
+    k_pack_outputs<<<blocks(n, 256), 256, 0, st_>>>(n, Y_, reinterpret_cast<float4*>(dY_));
+    cu(cudaMemcpyAsync(y, dY_, sizeof(float) * kOut * (size_t)n, cudaMemcpyDeviceToHost, st_), "outputs");
     cu(cudaStreamSynchronize(st_), "outputs");
-    for (int i = 0; i < n; ++i)
-        for (int c = 0; c < kOut; ++c) y[(size_t)i * kOut + c] = buf[(size_t)i * kOutPad + c];
 }
 
 void Surrogate::linear_bwd(Linear& L, const __nv_bfloat16* X, int R, float* dZ, const __nv_bfloat16* mask,
