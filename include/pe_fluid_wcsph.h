@@ -283,6 +283,10 @@ int pe_fluid_dfsph_compute_alpha(PeDfsph* w);
  * reference counterpart): 0 (the default) picks them from the fluid count; 1, 8
  * or 32 sets them, other values return PE_ERR_ARG. No choice changes a bit. */
 int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes);
+/* Let the alpha pass keep what the solvers' passes need of each pair (on by
+ * default, while the device has room for the buffer); off, they recompute it.
+ * The results are identical. */
+int pe_fluid_dfsph_set_pair_weights(PeDfsph* w, int32_t on);
 int pe_fluid_dfsph_len(const PeDfsph* w, uint64_t* out_len);
 int pe_fluid_dfsph_get_time(const PeDfsph* w, double* t);
 int pe_fluid_dfsph_get_last_dt(const PeDfsph* w, double* out);

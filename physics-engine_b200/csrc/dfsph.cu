@@ -82,6 +82,42 @@ __device__ __forceinline__ double nmass(const DfsphConst& k, const StateBufs& s,
     return sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi) ? k.rho0 * xj.w : 0.0;
 }
 
+// What a pair contributes to a solver's passes besides velocities and pressures
+// depends on the positions alone, which stay as they are through a solver's
+// iterations (twelve error and twelve pressure passes a step at 46,620 particles).
+// So the alpha pass keeps it beside the lists, at an entry's index into the pool:
+// of a fluid slot's entry the scale of grad W, of a boundary slot's the
+// reaction's weight; kSkip where the pair adds nothing (grad W's scale and the
+// weight are never negative). Lists beyond the buffer are computed as they go.
+constexpr double kSkip = -1.0;
+
+// The reaction's weight of a fluid particle and a boundary sample (dfsph.rs:497)
+__device__ __forceinline__ double reaction_weight(double r2) {
+    return fmin(quot_any(1.0, fmax(sqrt(r2), 1e-9)), 1e6);
+}
+
+// Entry p's place in the buffer (a list that does not fit: any)
+__device__ __forceinline__ double kept_value(const ListBufs& l, bool fits, const uint32_t* p) {
+    return __ldg(l.wpair + (fits ? p - l.pool : 0));
+}
+
+// Scale of grad W and mass of entry e; false if the pair adds nothing.
+template <bool KEPT>
+__device__ __forceinline__ bool pair_scale(const DfsphConst& k, const StateBufs& s, uint32_t e, const double4& xi,
+                                           const double4& xj, const Offset& o, bool fits, double kept, double* mj,
+                                           double* sc) {
+    if (KEPT && fits) {
+        *mj = (e & kEntryBoundary) ? k.rho0 * xj.w : k.mass;
+        *sc = kept;
+        return !(kept < 0.0);
+    }
+    if (o.far(k)) return false;
+    *mj = nmass(k, s, e, xj, xi);
+    if (*mj == 0.0) return false;
+    *sc = kfn_grad_scale(k.kf, o.r2);
+    return true;
+}
+
 // dfsph.rs:718-735: boundary forces cleared, v* = v + g dt (2-D: z = 0)
 __global__ void k_df_begin(uint32_t n, DfsphConst k, double dt, StateBufs s) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -188,7 +224,7 @@ __global__ void k_df_warm_zero(uint32_t n, int which, StateBufs s) {
 
 // dfsph.rs:326-351 density_derivative of slot i with v* (every lane of the
 // group gets it; fluid: the group has a slot to do)
-template <int G>
+template <int G, bool KEPT>
 __device__ __forceinline__ double density_rate(const DfsphConst& k, const StateBufs& s, const ListBufs& l,
                                                const LaneGroup<G>& g, bool fluid, double* words) {
     const uint32_t i = g.slot;
@@ -199,24 +235,26 @@ __device__ __forceinline__ double density_rate(const DfsphConst& k, const StateB
         xi = s.pos[i];
         vi = s.acc[i];
     }
+    struct Neighbour {
+        double4 x, v;
+        double kept;
+    };
+    const bool fits = KEPT && w_fits(l, lr);
     OrderedSum<G, 1> drho(words, g, 0.0);
     group_for_each<G>(
         lr, g,
-        [&](uint32_t e, const uint32_t*) {
+        [&](uint32_t e, const uint32_t* p) {
             const uint32_t j = e & kEntrySlotMask;
-            return TwoStates{gather4(s.pos + j), gather4(((e & kEntryBoundary) ? s.vel : s.acc) + j)};
+            return Neighbour{gather4(s.pos + j), gather4(((e & kEntryBoundary) ? s.vel : s.acc) + j),
+                             KEPT ? kept_value(l, fits, p) : 0.0};
         },
-        [&](bool has, uint32_t e, const TwoStates& d, const uint32_t*) {
-            double t[1] = {0.0};
+        [&](bool has, uint32_t e, const Neighbour& d, const uint32_t*) {
+            double t[1] = {0.0}, mj, sc;
             const Offset o(xi, d.x);
-            if (has && !o.far(k)) {
-                const double mj = nmass(k, s, e, d.x, xi);
-                if (mj != 0.0) {
-                    const double sc = kfn_grad_scale(k.kf, o.r2);
-                    const double gx = o.x * sc, gy = o.y * sc, gz = o.z * sc;
-                    const double wx = vi.x - d.v.x, wy = vi.y - d.v.y, wz = vi.z - d.v.z;
-                    t[0] = mj * (wx * gx + wy * gy + wz * gz);
-                }
+            if (has && pair_scale<KEPT>(k, s, e, xi, d.x, o, fits, d.kept, &mj, &sc)) {
+                const double gx = o.x * sc, gy = o.y * sc, gz = o.z * sc;
+                const double wx = vi.x - d.v.x, wy = vi.y - d.v.y, wz = vi.z - d.v.z;
+                t[0] = mj * (wx * gx + wy * gy + wz * gz);
             }
             drho.add(t);
         });
@@ -228,7 +266,7 @@ __device__ __forceinline__ double density_rate(const DfsphConst& k, const StateB
 // One error pass of a solver (dfsph.rs:552-569 density, 604-616 divergence):
 // kappa, the warm-start accumulation, the pressure diagnostic and the error
 // term of each particle in original order.
-template <int G>
+template <int G, bool KEPT>
 __global__ void __launch_bounds__(kDfThreads) k_df_error(uint32_t n, DfsphConst k, int divergence, double dt,
                                                         double dt2, StateBufs s, ListBufs l,
                                                         const double* __restrict__ alpha, double* __restrict__ kappa,
@@ -243,7 +281,7 @@ __global__ void __launch_bounds__(kDfThreads) k_df_error(uint32_t n, DfsphConst 
         err_orig[s.orig[i]] = 0.0;
     }
     if (!__any_sync(kFullWarp, fluid)) return;
-    const double drho = density_rate<G>(k, s, l, g, fluid, s_words + g.warp * OrderedSum<G, 1>::kDoubles);
+    const double drho = density_rate<G, KEPT>(k, s, l, g, fluid, s_words + g.warp * OrderedSum<G, 1>::kDoubles);
     if (!fluid || g.sub != 0) return;
     const uint32_t o = s.orig[i];
     double kap, e;
@@ -306,10 +344,11 @@ __global__ void k_df_serial_sum(uint32_t n, const double* __restrict__ v, double
 
 // dfsph.rs:422-530, fluid side: dv from kappa, the cap, the reaction total and
 // weight sum, v* += dv.
-template <int G>
+template <int G, bool KEPT>
 __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, DfsphConst k, double dt,
                                                                  double inv_dt, StateBufs s, ListBufs l,
                                                                  const double* __restrict__ kr,
+                                                                 const double* __restrict__ wsum,
                                                                  double4* __restrict__ react) {
     extern __shared__ __align__(16) double s_words[];
     const LaneGroup<G> g;
@@ -330,32 +369,29 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, Df
     OrderedSum<G, 3> all(words, g, 0.0), bnd(words + OrderedSum<G, 3>::kDoubles, g, 0.0);
     struct Neighbour {
         double4 x;
-        double kr;
+        double kr, kept;
     };
+    const bool fits = KEPT && w_fits(l, lr);
     group_for_each<G>(
         lr, g,
-        [&](uint32_t e, const uint32_t*) {
+        [&](uint32_t e, const uint32_t* p) {
             const uint32_t j = e & kEntrySlotMask;
-            return Neighbour{gather4(s.pos + j), __ldg(kr + j)};
+            return Neighbour{gather4(s.pos + j), __ldg(kr + j), KEPT ? kept_value(l, fits, p) : 0.0};
         },
         [&](bool has, uint32_t e, const Neighbour& d, const uint32_t*) {
-            double t[3] = {0.0, 0.0, 0.0}, tb[3] = {0.0, 0.0, 0.0};
+            double t[3] = {0.0, 0.0, 0.0}, tb[3] = {0.0, 0.0, 0.0}, mj, sc;
             bool b = false;
             const Offset o(xi, d.x);
-            if (has && !o.far(k)) {
-                const double mj = nmass(k, s, e, d.x, xi);
-                if (mj != 0.0) {
-                    const double sc = kfn_grad_scale(k.kf, o.r2);
-                    const double coeff = mj * (kri + d.kr);  // mj (ki / rho_i + kj / rho_j)
-                    t[0] = (o.x * sc) * coeff;
-                    t[1] = (o.y * sc) * coeff;
-                    t[2] = (o.z * sc) * coeff;
-                    b = e & kEntryBoundary;
-                    if (b) {
-                        tb[0] = t[0];
-                        tb[1] = t[1];
-                        tb[2] = t[2];
-                    }
+            if (has && pair_scale<KEPT>(k, s, e, xi, d.x, o, fits, d.kept, &mj, &sc)) {
+                const double coeff = mj * (kri + d.kr);  // mj (ki / rho_i + kj / rho_j)
+                t[0] = (o.x * sc) * coeff;
+                t[1] = (o.y * sc) * coeff;
+                t[2] = (o.z * sc) * coeff;
+                b = e & kEntryBoundary;
+                if (b) {
+                    tb[0] = t[0];
+                    tb[1] = t[1];
+                    tb[2] = t[2];
                 }
             }
             all.add(t);
@@ -384,33 +420,15 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, Df
     bx = bx * scale;
     by = by * scale;
     bz = bz * scale;
+    if (!fluid || g.sub != 0) return;
     double4 rec = make_double4(0.0, 0.0, 0.0, 0.0);
-    const bool reacts = fluid && bx * bx + by * by + bz * bz > 0.0;
-    if (__any_sync(kFullWarp, reacts)) {
-        if (!reacts) lr.n = 0u;
-        OrderedSum<G, 1> wsum(words, g, 0.0);
-        __syncwarp();  // the words change hands
-        group_for_each<G>(
-            lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
-            [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
-                double t[1] = {0.0};
-                const bool b = has && (e & kEntryBoundary);
-                if (b) {
-                    const bool oriented = e & kEntryOriented;
-                    const uint32_t j = e & kEntrySlotMask;
-                    if (sees(k, xj, oriented ? s.nout[j] : make_double4(0, 0, 0, 0), oriented, xi))
-                        t[0] = fmin(quot_any(1.0, fmax(sqrt(Offset(xi, xj).r2), 1e-9)), 1e6);
-                }
-                if (__any_sync(kFullWarp, b)) wsum.add(t);
-            });
-        double r[1];
-        wsum.totals(r);
-        if (reacts && r[0] > 0.0) {
+    if (bx * bx + by * by + bz * bz > 0.0) {
+        const double ws = wsum[i];  // the weights of its visible samples
+        if (ws > 0.0) {
             const double m = -k.mass * inv_dt;
-            rec = make_double4(bx * m, by * m, bz * m, r[0]);
+            rec = make_double4(bx * m, by * m, bz * m, ws);
         }
     }
-    if (!fluid || g.sub != 0) return;
     react[i] = rec;
     double4 a = s.acc[i];
     a.x = a.x + dx;
@@ -419,9 +437,33 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_fluid(uint32_t n, Df
     s.acc[i] = a;
 }
 
+// The boundary slots' half of what is kept: the reaction's weight of each fluid candidate.
+template <int G>
+__global__ void __launch_bounds__(kDfThreads) k_df_boundary_weights(uint32_t n, DfsphConst k, StateBufs s, ListBufs l) {
+    const LaneGroup<G> g;
+    const uint32_t j = g.slot;
+    ListRef lr{l.pool, 0u, 0u};
+    double4 xj = make_double4(0.0, 0.0, 0.0, 0.0), nj = xj;
+    bool oriented = false;
+    if (j < n && is_boundary(s, j)) {
+        lr = list_ref(l, j, kListLower);
+        xj = s.pos[j];
+        oriented = s.flags[j] & kFlagOriented;
+        if (oriented) nj = s.nout[j];
+    }
+    const bool fits = w_fits(l, lr);
+    if (!fits && g.sub == 0) atomicOr(l.w_short, 1u);
+    group_for_each<G>(
+        lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
+        [&](bool has, uint32_t, const double4& xi, const uint32_t* p) {
+            if (has && fits)
+                l.wpair[p - l.pool] = sees(k, xj, nj, oriented, xi) ? reaction_weight(Offset(xi, xj).r2) : kSkip;
+        });
+}
+
 // dfsph.rs:508-517, boundary side: the reaction shares of the fluid
 // candidates, in ascending original index.
-template <int G>
+template <int G, bool KEPT>
 __global__ void __launch_bounds__(kDfThreads) k_df_pressure_boundary(uint32_t n, DfsphConst k, StateBufs s,
                                                                     ListBufs l, const double4* __restrict__ react) {
     extern __shared__ __align__(16) double s_words[];
@@ -439,20 +481,29 @@ __global__ void __launch_bounds__(kDfThreads) k_df_pressure_boundary(uint32_t n,
         oriented = s.flags[j] & kFlagOriented;
         if (oriented) nj = s.nout[j];
     }
+    struct Neighbour {
+        double4 rec;
+        double kept;
+    };
+    const bool fits = KEPT && w_fits(l, lr);
     const double start[3] = {f.x, f.y, f.z};
     OrderedSum<G, 3> sum(s_words + g.warp * OrderedSum<G, 3>::kDoubles, g, start);
     group_for_each<G>(
         lr, g,
-        [&](uint32_t e, const uint32_t*) {
-            const uint32_t i = e & kEntrySlotMask;
-            return TwoStates{gather4(s.pos + i), gather4(react + i)};
+        [&](uint32_t e, const uint32_t* p) {
+            return Neighbour{gather4(react + (e & kEntrySlotMask)), KEPT ? kept_value(l, fits, p) : 0.0};
         },
-        [&](bool has, uint32_t, const TwoStates& d, const uint32_t*) {
-            const double4 &xi = d.x, &rec = d.v;
+        [&](bool has, uint32_t e, const Neighbour& d, const uint32_t*) {
+            const double4& rec = d.rec;
             double t[3] = {0.0, 0.0, 0.0};
-            const bool adds = has && rec.w > 0.0 && sees(k, xj, nj, oriented, xi);
+            bool adds = has && rec.w > 0.0;
+            double wt = d.kept;
+            if (adds && !fits) {
+                const double4 xi = s.pos[e & kEntrySlotMask];
+                wt = sees(k, xj, nj, oriented, xi) ? reaction_weight(Offset(xi, xj).r2) : kSkip;
+            }
+            adds = adds && !(wt < 0.0);
             if (adds) {
-                const double wt = fmin(quot_any(1.0, fmax(sqrt(Offset(xi, xj).r2), 1e-9)), 1e6);
                 const double sh = quot_any(wt, rec.w);
                 t[0] = rec.x * sh;
                 t[1] = rec.y * sh;
@@ -542,48 +593,69 @@ __global__ void __launch_bounds__(kDfThreads) k_df_density(uint32_t n, DfsphCons
 }
 
 // dfsph.rs:252-307 alpha = rho / max(|sum m grad W|^2 + sum |m grad W|^2, floor)
+// (alpha null: left as it is). Also fills wsum, the sum of a fluid particle's
+// reaction weights, and what is kept of its pairs (l.wpair not null).
 template <int G>
 __global__ void __launch_bounds__(kDfThreads) k_df_alpha(uint32_t n, DfsphConst k, StateBufs s, ListBufs l,
-                                                        double* __restrict__ alpha) {
+                                                        double* __restrict__ alpha, double* __restrict__ wsum) {
     extern __shared__ __align__(16) double s_words[];
     const LaneGroup<G> g;
     const uint32_t i = g.slot;
     const bool fluid = i < n && !is_boundary(s, i);
-    if (i < n && !fluid && g.sub == 0) alpha[i] = 0.0;
+    if (alpha && i < n && !fluid && g.sub == 0) alpha[i] = 0.0;
     if (!__any_sync(kFullWarp, fluid)) return;
     ListRef lr{l.pool, 0u, 0u};
     double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
+    bool keep = false;
     if (fluid) {
         lr = list_ref(l, i, kListVisit);
         xi = s.pos[i];
+        if (l.wpair) {
+            keep = w_fits(l, lr);
+            if (!keep && g.sub == 0) atomicOr(l.w_short, 1u);
+        }
     }
-    OrderedSum<G, 4> sum(s_words + g.warp * OrderedSum<G, 4>::kDoubles, g, 0.0);  // m grad W, |m grad W|^2
+    double* const words = s_words + g.warp * (OrderedSum<G, 4>::kDoubles + OrderedSum<G, 1>::kDoubles);
+    OrderedSum<G, 4> sum(words, g, 0.0);  // m grad W, |m grad W|^2
+    OrderedSum<G, 1> weights(words + OrderedSum<G, 4>::kDoubles, g, 0.0);
     uint32_t nb_all = 0, nb_kept = 0;
     group_for_each<G>(
         lr, g, [&](uint32_t e, const uint32_t*) { return gather4(s.pos + (e & kEntrySlotMask)); },
-        [&](bool has, uint32_t e, const double4& xj, const uint32_t*) {
-            double t[4] = {0.0, 0.0, 0.0, 0.0};
+        [&](bool has, uint32_t e, const double4& xj, const uint32_t* p) {
+            double t[4] = {0.0, 0.0, 0.0, 0.0}, w[1] = {0.0};
+            const bool bnd = has && (e & kEntryBoundary);
             if (has) {
-                const double mj = nmass(k, s, e, xj, xi);
-                const bool bnd = e & kEntryBoundary;
-                nb_all += bnd ? 1u : 0u;
-                nb_kept += bnd && mj != 0.0 ? 1u : 0u;
                 const Offset o(xi, xj);
+                double mj = k.mass, sc = kSkip;
+                if (bnd) {
+                    const bool oriented = e & kEntryOriented;
+                    const bool seen = sees(k, xj, oriented ? s.nout[e & kEntrySlotMask] : make_double4(0, 0, 0, 0),
+                                           oriented, xi);
+                    mj = seen ? k.rho0 * xj.w : 0.0;
+                    if (seen) w[0] = reaction_weight(o.r2);
+                    nb_all += 1u;
+                    nb_kept += mj != 0.0 ? 1u : 0u;
+                }
                 if (!(bnd && mj == 0.0) && !o.far(k)) {
-                    const double sc = kfn_grad_scale(k.kf, o.r2);
+                    sc = kfn_grad_scale(k.kf, o.r2);
                     t[0] = (o.x * sc) * mj;
                     t[1] = (o.y * sc) * mj;
                     t[2] = (o.z * sc) * mj;
                     t[3] = t[0] * t[0] + t[1] * t[1] + t[2] * t[2];
                 }
+                if (keep) l.wpair[p - l.pool] = mj == 0.0 ? kSkip : sc;
             }
             sum.add(t);
+            if (__any_sync(kFullWarp, bnd)) weights.add(w);
         });
     nb_all = g.sum(nb_all);
     nb_kept = g.sum(nb_kept);
-    double r[4];
+    double r[4], ws[1];
     sum.totals(r);
+    weights.totals(ws);
     if (!fluid || g.sub != 0) return;
+    wsum[i] = ws[0];
+    if (!alpha) return;
     // every fluid candidate but i itself, and the boundary ones of non-zero mass
     const uint32_t nn = (l.ncand[i] - 1u - nb_all) + nb_kept;
     if (nn < 2) {
@@ -658,12 +730,14 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
     WorldConfig wc = cfg;
     wc.precision = 0;
     wc.use_graph = 0;
+    wc.pair_weights = 1;  // the buffer of the kept pairs, while the device has room for it
     w_.reset(new World(wp, wc, dim, rest_density, mass, h, n, xs.data(), vs.data(), kind, psi, n_out, nullptr, 1,
                        kernel_support(prm.kernel, h)));
     w_->list_keep_boundary_ = true;
     w_->refresh_step_const();
     const size_t N = std::max<uint64_t>(n, 1);
     alpha_ = w_->alloc<double>(N);
+    wsum_ = w_->alloc<double>(N);
     kappa_ = w_->alloc<double>(N);
     kr_ = w_->alloc<double>(N);
     dv_ = w_->alloc<double4>(N);
@@ -683,13 +757,18 @@ DfsphSolver::~DfsphSolver() {
     if (sum_host_) cudaFreeHost(sum_host_);
 }
 
-// ms for two steps with 1 / 8 / 32 lanes (16^3 fluid particles 15.0 / 4.2 / 2.7,
-// 36^3 24.1 / 13.0 / 14.1, 64^3 50.9 / 52.1 / 65.9, 90^3 102 / 130 / 172): many
-// lanes while the slots do not fill the chip, one where they do.
+// ms for two steps with 1 / 8 / 32 lanes a fluid slot (16^3 fluid particles 15.0 /
+// 4.2 / 2.7, 36^3 24.1 / 13.0 / 14.1, 64^3 50.9 / 52.1 / 65.9, 90^3 102 / 130 /
+// 172): many lanes while the slots do not fill the chip, one where they do. The
+// boundary slots' lists are few and long (all candidates of the cells), so these
+// take more: 36^3 20.6 / 12.4 / 11.5, 64^3 49.9 / 42.0 / 42.6.
 void DfsphSolver::set_lanes(uint32_t lanes) {
-    if (lanes == 0) lanes = n_fluid_ <= 30000 ? 32u : n_fluid_ <= 230000 ? 8u : 1u;
-    if (lanes != 1 && lanes != 8 && lanes != 32) throw std::invalid_argument("lanes per slot");
-    df_lanes_ = lanes;
+    if (lanes != 0 && lanes != 1 && lanes != 8 && lanes != 32) throw std::invalid_argument("lanes per slot");
+    df_lanes_ = df_lanes_boundary_ = lanes;
+    if (lanes == 0) {
+        df_lanes_ = n_fluid_ <= 30000 ? 32u : n_fluid_ <= 230000 ? 8u : 1u;
+        df_lanes_boundary_ = n_fluid_ <= 150000 ? 32u : 8u;
+    }
 }
 
 void DfsphSolver::rebuild_neighbours() { rebuild(); }
@@ -705,16 +784,45 @@ void DfsphSolver::compute_density() {
     w.launches_ += 1;
 }
 
-void DfsphSolver::compute_alpha() {
+void DfsphSolver::compute_alpha() { alpha_pass(alpha_); }
+
+// alpha (unless null) and what the solvers' passes read of the pairs
+void DfsphSolver::alpha_pass(double* alpha) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     if (!n) return;
+    if (w.lists_.wpair && !w.w_short_cleared_)
+        w.check(cudaMemsetAsync(&w.sc_->w_short, 0, sizeof(uint32_t), w.st_), "memset");
+    w.w_short_cleared_ = false;
     with_df_lanes(df_lanes_, [&](auto gc) {
         constexpr int G = decltype(gc)::value;
-        k_df_alpha<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, (G < 4 ? 1 : 4)>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
-                                                                                            alpha_);
+        constexpr int K = G < 4 ? 1 : 4;
+        k_df_alpha<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, K>() + df_smem<G, 1>(), w.st_>>>(
+            n, kc_, w.cur_, w.lists_, alpha, wsum_);
     });
     w.launches_ += 1;
+    if (w.lists_.wpair) {
+        with_df_lanes(df_lanes_boundary_, [&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            k_df_boundary_weights<G><<<df_blocks<G>(n), kDfThreads, 0, w.st_>>>(n, kc_, w.cur_, w.lists_);
+        });
+        w.launches_ += 1;
+    }
+    w.w_valid_ = true;
+}
+
+// Before a solver: the positions may have been set, or moved by the slip planes, since alpha's pass.
+void DfsphSolver::keep_pairs() {
+    if (!w_->w_valid_) alpha_pass(nullptr);
+}
+
+// Calls f(integral_constant<int, G>, bool_constant<KEPT>)
+template <class F>
+void DfsphSolver::with_pairs(uint32_t lanes, F&& f) {
+    with_df_lanes(lanes, [&](auto gc) {
+        if (w_->lists_.wpair) f(gc, std::true_type{});
+        else f(gc, std::false_type{});
+    });
 }
 
 double DfsphSolver::mean_density_error() {
@@ -762,6 +870,7 @@ void DfsphSolver::set_params(const DfsphParams& p) {
 void DfsphSolver::refresh_const() {
     DfsphConst& k = kc_;
     const World& w = *w_;
+    w_->w_valid_ = false;  // what is kept of the pairs is the parameters' too
     k.dim = w.dim_;
     k.kf = make_kernel_fn(prm_.kernel, w.h_, w.dim_);
     k.mass = w.mass_;
@@ -821,13 +930,18 @@ void DfsphSolver::pressure_update(double dt, bool /*divergence*/) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     const double inv_dt = 1.0 / std::fmax(dt, 1e-12);
-    with_df_lanes(df_lanes_, [&](auto gc) {
+    with_pairs(df_lanes_, [&](auto gc, auto kept) {
         constexpr int G = decltype(gc)::value;
         constexpr int K = G < 3 ? 1 : 3;
-        k_df_pressure_fluid<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(2), w.st_>>>(n, kc_, dt, inv_dt, w.cur_,
-                                                                                         w.lists_, kr_, react_);
-        k_df_pressure_boundary<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(), w.st_>>>(n, kc_, w.cur_, w.lists_,
-                                                                                           react_);
+        k_df_pressure_fluid<G, decltype(kept)::value>
+            <<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(2), w.st_>>>(n, kc_, dt, inv_dt, w.cur_, w.lists_, kr_, wsum_,
+                                                                      react_);
+    });
+    with_pairs(df_lanes_boundary_, [&](auto gc, auto kept) {
+        constexpr int G = decltype(gc)::value;
+        constexpr int K = G < 3 ? 1 : 3;
+        k_df_pressure_boundary<G, decltype(kept)::value>
+            <<<df_blocks<G>(n), kDfThreads, df_smem<G, K>(), w.st_>>>(n, kc_, w.cur_, w.lists_, react_);
     });
     w.launches_ += 2;
 }
@@ -835,9 +949,9 @@ void DfsphSolver::pressure_update(double dt, bool /*divergence*/) {
 double DfsphSolver::solve_error(double dt, bool divergence) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
-    with_df_lanes(df_lanes_, [&](auto gc) {
+    with_pairs(df_lanes_, [&](auto gc, auto kept) {
         constexpr int G = decltype(gc)::value;
-        k_df_error<G><<<df_blocks<G>(n), kDfThreads, df_smem<G, 1>(), w.st_>>>(
+        k_df_error<G, decltype(kept)::value><<<df_blocks<G>(n), kDfThreads, df_smem<G, 1>(), w.st_>>>(
             n, kc_, divergence ? 1 : 0, dt, dt * dt, w.cur_, w.lists_, alpha_, kappa_, kr_, err_orig_);
     });
     k_df_partial_sums<<<kSumBlocks, kSumThreads, 0, w.st_>>>(n, err_orig_, part_);
@@ -874,6 +988,7 @@ uint64_t DfsphSolver::correct_density_error(double dt) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     const uint32_t nb = blocks_for(n, kDfThreads);
+    keep_pairs();
     if (prm_.warm_start) {
         k_df_warm_load<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, 0, w.cur_, kappa_, kr_);
         w.launches_ += 1;
@@ -895,6 +1010,7 @@ uint64_t DfsphSolver::correct_divergence_error(double dt) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     const uint32_t nb = blocks_for(n, kDfThreads);
+    keep_pairs();
     if (prm_.warm_start) {
         k_df_warm_load<<<nb, kDfThreads, 0, w.st_>>>(n, kc_, 1, w.cur_, kappa_, kr_);
         w.launches_ += 1;
@@ -918,6 +1034,7 @@ void DfsphSolver::free_slip() {
     const uint32_t n = (uint32_t)w.n_;
     k_df_free_slip<<<blocks_for(n, kDfThreads), kDfThreads, 0, w.st_>>>(n, kc_, w.cur_);
     w.launches_ += 1;
+    w.w_valid_ = false;  // positions on the planes have moved
 }
 
 void DfsphSolver::step(double dt_in) {

@@ -80,6 +80,10 @@ class DfsphSolver {
     void refresh_const();
     void rebuild();                       // grid + lists (dfsph.rs:201-211)
     void density_and_alpha();             // dfsph.rs:214-307
+    void alpha_pass(double* alpha);
+    void keep_pairs();
+    template <class F>
+    void with_pairs(uint32_t lanes, F&& f);
     void pressure_update(double dt, bool divergence);  // dfsph.rs:422-530
     double solve_error(double dt, bool divergence);    // one error pass + its average
     uint64_t correct_density_error(double dt);         // dfsph.rs:533-584
@@ -90,13 +94,14 @@ class DfsphSolver {
     DfsphParams prm_;
     DfsphConst kc_{};
     uint64_t n_fluid_ = 0;
-    uint32_t df_lanes_ = 1;  // lanes a slot of the pair passes: 1, 8 or 32
+    uint32_t df_lanes_ = 1, df_lanes_boundary_ = 1;  // lanes a slot of the pair passes: 1, 8 or 32
     double last_dt_ = 0.0;
     bool a_adv_set_ = false;  // the non-pressure accelerations (gravity) have been computed
     uint64_t it_density_ = 0, it_divergence_ = 0;
     double err_density_ = 0.0, err_divergence_ = 0.0;
     // per slot (valid until the next re-sort)
     double* alpha_ = nullptr;
+    double* wsum_ = nullptr;         // sum of a fluid particle's reaction weights (valid with the kept pairs)
     double* kappa_ = nullptr;
     double* kr_ = nullptr;           // kappa / max(rho, 1e-12) (boundary: 0 / rho0)
     double4* dv_ = nullptr;          // xsph scratch

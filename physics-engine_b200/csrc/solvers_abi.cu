@@ -397,6 +397,14 @@ int pe_fluid_dfsph_step_adaptive(PeDfsph* w, double* dt_out) {
     });
 }
 
+int pe_fluid_dfsph_set_pair_weights(PeDfsph* w, int32_t on) {
+    if (!w) return PE_ERR_NULL;
+    return guard([&] {
+        w->s->world().set_pair_weights(on != 0);
+        return PE_OK;
+    });
+}
+
 int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes) {
     if (!w) return PE_ERR_NULL;
     return guard([&] {

@@ -1199,6 +1199,7 @@ bool World::set_vec(int which, const double* in) {
         rho_current_ = false;
         lists_valid_ = false;
         lists_checked_ = false;
+        w_valid_ = false;
     }
     return true;
 }

@@ -262,6 +262,7 @@ def load_library():
         "pe_fluid_dfsph_rebuild_neighbours": (C.c_int, [vp]),
         "pe_fluid_dfsph_compute_density": (C.c_int, [vp]),
         "pe_fluid_dfsph_set_lanes": (C.c_int, [vp, C.c_uint32]),
+        "pe_fluid_dfsph_set_pair_weights": (C.c_int, [vp, C.c_int32]),
         "pe_fluid_pbf_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_dfsph_compute_alpha": (C.c_int, [vp]),
         "pe_fluid_dfsph_len": (C.c_int, [vp, C.POINTER(u64)]),
@@ -1107,6 +1108,12 @@ class DfsphWorld:
         """Lanes of a warp on each particle's list: 0 (the default) picks them
         from the fluid count; 1, 8 or 32 sets them. The results are identical."""
         _ok(_lib.pe_fluid_dfsph_set_lanes(self._w, int(lanes)), "dfsph_set_lanes")
+
+    def set_pair_weights(self, on: bool = True):
+        """Let the alpha pass keep what the solvers' passes need of each pair
+        (on by default, while the device has room for the buffer); off, they
+        recompute it. The results are identical."""
+        _ok(_lib.pe_fluid_dfsph_set_pair_weights(self._w, 1 if on else 0), "dfsph_set_pair_weights")
 
     @property
     def t(self) -> float:
