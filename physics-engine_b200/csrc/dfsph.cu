@@ -734,6 +734,7 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
     w_.reset(new World(wp, wc, dim, rest_density, mass, h, n, xs.data(), vs.data(), kind, psi, n_out, nullptr, 1,
                        kernel_support(prm.kernel, h)));
     w_->list_keep_boundary_ = true;
+    w_->lists_outlive_poll_ = true;  // a step begins with the lists the last one ended with
     w_->refresh_step_const();
     const size_t N = std::max<uint64_t>(n, 1);
     alpha_ = w_->alloc<double>(N);

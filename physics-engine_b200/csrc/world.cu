@@ -1118,6 +1118,7 @@ uint32_t World::status() {
     if (hs.list_used * 4 > lists_.pool_groups * 3 && lists_.pool_groups < kMaxListGroups) {
         alloc_lists(2 * hs.list_used);
         lists_checked_ = false;
+        if (lists_outlive_poll_) ensure_lists();
     }
     // Pair weights that a density pass found too short cover the whole pool
     // from now on (XSPH recomputed W meanwhile).

@@ -276,6 +276,7 @@ class World {
     bool grid_current_ = false;  // grid built from the current positions
     bool rho_current_ = false;   // densities computed from the current grid and positions
     bool lists_valid_ = false;   // neighbour lists match the grid and positions
+    bool lists_outlive_poll_ = false;  // the next step reads the present lists: a poll that moves the pool rebuilds them
     bool pair_w_on_ = false;     // keep lists_.wpair (set_pair_weights)
     bool w_valid_ = false;       // lists_.wpair holds W of the current lists and positions
     void alloc_pair_weights(unsigned long long groups);

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 DX = 0.05
 
 
-def _world(dim, lanes, spread=1.0, at=0.1, wall=0.7, **kw):
+def _world(dim, lanes, spread=1.0, at=0.1, wall=0.7, neighbours=4, **kw):
     mass = pe.mass_calibrated_to_rest(1000.0, DX, 2 * DX, dim)
     p = pe.Particles(dim, 1000.0, mass, 2 * DX)
     p.fill_box((at, at, at if dim == 3 else 0.0), 10, 8, 9 if dim == 3 else 1, DX * spread)
@@ -23,7 +23,7 @@ def _world(dim, lanes, spread=1.0, at=0.1, wall=0.7, **kw):
     p.recomputed_akinci_psi()
     w = pe.DfsphWorld(p, pe.DfsphParams(adaptive_dt=False, particle_diameter=DX, max_density_iters=5,
                                         max_divergence_iters=5, xsph_epsilon=0.05, **kw),
-                      pe.WcsphConfig(max_neighbours=4))  # the first build sizes the pool
+                      pe.WcsphConfig(max_neighbours=neighbours))  # few: the first build sizes the pool
     w.set_lanes(lanes)
     return w
 
@@ -84,3 +84,22 @@ def test_lists_beyond_the_buffer(lanes, spread):
     _same(wide, direct, f"{spread} wide")
     wide.close()
     direct.close()
+
+
+def test_lists_survive_a_pool_that_grows():
+    """Particles that rush together outgrow the pool between two steps: the poll
+    after the first step moves it, and the next step begins with its lists."""
+    worlds = [_world(3, 0, 1.7, 0.45, 1.9, neighbours) for neighbours in (4, 2048)]
+    dt = 1.0 / 240.0
+    x = worlds[0].positions()
+    n = 10 * 8 * 9
+    v = np.zeros_like(x)
+    v[:n] = (x[:n].mean(0) - x[:n]) * (0.17 / dt)
+    for w in worlds:
+        w.set_velocities(v)
+        w.run(dt, 1)
+        w.set_velocities(0.0 * v)
+        w.run(dt, 2)
+    _same(*worlds, "grown")
+    for w in worlds:
+        w.close()
