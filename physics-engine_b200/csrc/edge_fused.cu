@@ -12,22 +12,26 @@
 // segment sum. Here one persistent CTA per SM keeps Wc, W2 and W3 in shared
 // memory; its four warpgroups walk their own tiles of 128 edges, each with its
 // own 128 tensor-memory columns, buffers and barriers, so one group's MMA
-// waits and gathers overlap the others' epilogues. Per tile, x_e Wc is one
-// K=16 tcgen05 MMA into the group's accumulator; the epilogue (thread r =
-// edge r = TMEM lane r) adds b1, P[i] and Q[j] in the unfused epilogue's
-// order (the next tile's endpoints and features, and the next 16-column block
-// of P[i] and Q[j], are already loading), applies ReLU and
-// writes bf16 into a swizzled shared-memory tile that is the A operand of
-// the next 8 MMAs (K = 128), and so on; the last epilogue stages the
-// messages in shared memory and sums each run of equal destinations before
-// one atomic add per run and column. Activations are rounded to bf16 at the
+// waits and gathers overlap the others' epilogues.
+//
+// The layers are computed transposed: the weights are the MMAs' A operand (128
+// features), the tile's edges the N dimension, so that a thread holds one
+// feature of all its edges. Then a warp reads 128 contiguous bytes of Q[j] for
+// each edge, P[i] once a run of equal destinations, biases stay in registers,
+// and the messages of a run are summed in registers, one atomic add per run,
+// block of 32 edges and column. Per tile, Wc^T x_e^T is one K = 16 MMA; the
+// epilogue adds b1, P[i] and Q[j] in the unfused epilogue's order (the next
+// sixteen edges' Q, the next four runs' P and the next tile's endpoints and
+// features are already loading), applies ReLU and writes bf16 into a swizzled
+// tile, a row of edges for each feature, that is the N-major B operand of the
+// next 8 MMAs (K = 128), and so on. Activations are rounded to bf16 at the
 // same points as in the unfused path; only the message sum's order differs.
 //
 // A tile is one long chain (copy, MMA, epilogue, MMA, ...), so what counts is how
-// many run on an SM: with two groups, a third buffer and 32-column blocks in
-// flight (16 KB more a group, twice the registers) 2.56M edges took 1.72 ms, with
-// four 0.74. The shared-memory and L1 data path is 78% busy then, half of it the
-// gathers of Q[j] and the messages' staging.
+// many run on an SM. 2.56M edges, a hop: 1.72 ms with two groups and a thread an
+// edge (each reading its own rows of P and Q); 0.74 with four, the shared-memory
+// and L1 path 78% busy; 0.49 with a thread a feature, that path 35%, the ALU 47%
+// (loops over the blocks unrolled, the instruction cache missed: 0.65).
 //
 // Every mbarrier wait is bounded; a wait that runs out sets bit 0 of *err and
 // ends the tile loop of the whole CTA (at the tile's end, by a block-wide
@@ -54,19 +58,43 @@ constexpr uint32_t kOffW3 = kOffW2 + 2 * kSlice;  // W3^T: two slices
 // Wc^T [128 x 16], matrix 1 + g group g's edge features [128 x 16].
 constexpr uint32_t kOffNarrow = kOffW3 + 2 * kSlice;
 constexpr uint32_t kNarrowSlices = (1 + kGroups + 3) / 4;
-// per group the activation tile [128 x 128]; the last epilogue reuses it for
-// fp32 messages, a warp's 32 rows x 32 columns in its own rows of a slice
+// per group the activation tile: a slice for 64 edges, 128 bytes of them for each feature
 constexpr uint32_t kOffGroup = kOffNarrow + kNarrowSlices * kSlice;
 constexpr uint32_t kGroupBytes = 2 * kSlice;
 constexpr uint32_t kSmemBytes = kOffGroup + kGroups * kGroupBytes + 1024u;  // + alignment slack
-static_assert(kSmemBytes + 2048u <= 232448u, "one CTA's shared memory, with its biases and barriers");
+static_assert(kSmemBytes + 2048u <= 232448u, "one CTA's shared memory, with its barriers");
+
+// 128 edges' activations (MN-major: a row of 128 edges for each feature) times W
+__device__ __forceinline__ void issue_edges(uint32_t tmem, const uint8_t* sW, const uint8_t* sZ) {
+    const uint32_t a0 = smem_addr(sW), b0 = smem_addr(sZ);
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk)
+        umma_bf16<kTileN, true>(tmem, sw128_desc(a0 + (uint32_t)(kk >> 2) * kSlice + (kk & 3) * 32),
+                                sw128_mn_desc(b0 + kk * 2048u, kSlice), kk ? 1u : 0u);
+}
+
+// N values of feature `row` for the edges from e0 on, as bf16
+template <int N>
+__device__ __forceinline__ void put_edges(uint8_t* sZ, int row, int e0, const float (&x)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 8; ++q) {
+        uint32_t w[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(x[q * 8 + 2 * h], x[q * 8 + 2 * h + 1]);
+            w[h] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        const int c = e0 / 8 + q;  // 16-byte chunk of the feature's edges
+        *reinterpret_cast<uint4*>(sZ + (uint32_t)(c >> 3) * kSlice + sw_off(row, c & 7)) =
+            make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
 
 __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar[kGroups];
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(16) float s_bias[3][128];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = tid / kGroupThreads, gt = tid % kGroupThreads, gw = gt >> 5;
     uint8_t* sWc = smem + kOffNarrow;
@@ -74,7 +102,11 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
     uint8_t* sW3 = smem + kOffW3;
     uint8_t* sX = smem + kOffNarrow + (uint32_t)((g + 1) / 4) * kSlice;
     const int xc = 2 * ((g + 1) % 4);  // first chunk of the group's edge features in it
-    uint8_t* sA = smem + kOffGroup + (uint32_t)g * kGroupBytes;
+    uint8_t* sZ = smem + kOffGroup + (uint32_t)g * kGroupBytes;
+    // endpoints of the tile's edges: sources 4 q .. 4 q + 3 in chunk 2 of row
+    // 32 g + q of the second narrow slice, destinations in chunk 3
+    uint8_t* const sEnd = smem + kOffNarrow + kSlice;
+    auto ends = [&](int q, int which) { return sEnd + sw_off(32 * g + q, 2 + which); };
 
     if (tid == 0) {
         for (int i = 0; i < kGroups; ++i) mbar_init(smem_addr(&mbar[i]), 1);
@@ -90,13 +122,13 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
     stage_rows(sWc, a.Wc, 16, 2);
     stage_rows(sW2, a.W2, 128, 16);
     stage_rows(sW3, a.W3, 128, 16);
-    if (tid < 3 * 128) s_bias[tid >> 7][tid & 127] = __ldg((tid < 128 ? a.b1 : tid < 256 ? a.b2 : a.b3) + (tid & 127));
+    const float b1 = __ldg(a.b1 + gt), b2 = __ldg(a.b2 + gt), b3 = __ldg(a.b3 + gt);  // this thread's feature
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem + 128u * (uint32_t)g;            // this group's 128 columns
-    const uint32_t trow = tmem + ((uint32_t)(gw * 32) << 16);      // this warp's lanes (warp % 4)
+    const uint32_t tmem = s_tmem + 128u * (uint32_t)g;         // this group's 128 columns
+    const uint32_t trow = tmem + ((uint32_t)(gw * 32) << 16);  // this warp's lanes (features)
     const uint32_t bar = smem_addr(&mbar[g]);
 
     bool ok = true;
@@ -111,15 +143,15 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         group_sync(g);
+        if (gt == 0) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     };
     const int ntiles = (a.E + kGroupThreads - 1) / kGroupThreads;
     const int stride = (int)gridDim.x * kGroups;
-    // This thread's edge (row gt) of a tile: endpoints and its two 16-byte
-    // chunks of edge features, loaded one tile ahead.
+    // Edge gt of a tile: endpoints and its two 16-byte chunks of edge features, loaded one tile ahead.
     auto fetch_edge = [&](int tile, int& d, int& sj, uint4& x0, uint4& x1) {
         const int e = tile * kGroupThreads + gt;
         d = -1;
-        sj = -1;
+        sj = 0;
         x0 = x1 = make_uint4(0u, 0u, 0u, 0u);
         if (tile < ntiles && e < a.E) {
             d = __ldg(a.dst + e);
@@ -128,15 +160,24 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
             x1 = __ldg(reinterpret_cast<const uint4*>(a.xe + (size_t)e * 16 + 8));
         }
     };
-    // 16 columns (block cb) of this edge's P[dst] and Q[src] rows
-    auto fetch_pq = [&](int d, int sj, int cb, float4 (&p)[4], float4 (&q)[4]) {
-        const float4* P4 = reinterpret_cast<const float4*>(a.P + (size_t)(d < 0 ? 0 : d) * 128 + cb * 16);
-        const float4* Q4 = reinterpret_cast<const float4*>(a.Q + (size_t)(sj < 0 ? 0 : sj) * 128 + cb * 16);
+    // this feature of the Q rows of the sixteen edges from e0 on
+    const float* const Qc = a.Q + gt;
+    const float* const Pc = a.P + gt;
+    auto fetch_q = [&](int e0, float (&q)[16]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            p[i] = __ldg(P4 + i);
-            q[i] = __ldg(Q4 + i);
+            const int4 j = *reinterpret_cast<const int4*>(ends(e0 / 4 + i, 0));
+            q[4 * i] = __ldg(Qc + (size_t)j.x * 128);
+            q[4 * i + 1] = __ldg(Qc + (size_t)j.y * 128);
+            q[4 * i + 2] = __ldg(Qc + (size_t)j.z * 128);
+            q[4 * i + 3] = __ldg(Qc + (size_t)j.w * 128);
         }
+    };
+    // Destinations of a block of 32 edges, a lane an edge, and where a new one begins
+    auto block_runs = [&](int b, int& dest) {
+        dest = *reinterpret_cast<const int*>(ends(8 * b + (lane >> 2), 1) + 4 * (lane & 3));
+        const int above = __shfl_up_sync(0xffffffffu, dest, 1);
+        return __ballot_sync(0xffffffffu, lane == 0 || above != dest);
     };
     int d, sj;
     uint4 x0, x1;
@@ -146,95 +187,110 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_hop(EdgeHopArgs a) {
         // ---- edge features and endpoints of the tile (fetched a tile ahead)
         *reinterpret_cast<uint4*>(sX + sw_off(gt, xc)) = x0;
         *reinterpret_cast<uint4*>(sX + sw_off(gt, xc + 1)) = x1;
-        const int dc = d, sc = sj;
+        *reinterpret_cast<int*>(ends(gt >> 2, 0) + 4 * (gt & 3)) = sj;
+        *reinterpret_cast<int*>(ends(gt >> 2, 1) + 4 * (gt & 3)) = d;
         to_tensor();
         // ---- layer 1: x_e Wc (one K = 16 MMA), then + b1 + P[dst] + Q[src], ReLU
         if (gt == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            umma_bf16(tmem, sw128_desc(smem_addr(sX) + 16u * (uint32_t)xc), sw128_desc(smem_addr(sWc)), 0u);
+            umma_bf16(tmem, sw128_desc(smem_addr(sWc)), sw128_desc(smem_addr(sX) + 16u * (uint32_t)xc), 0u);
             umma_commit(bar);
         }
-        // the next tile's edge and this edge's first P/Q block load while the MMA runs
+        // the next tile's edge and the first edges' Q load while the MMA runs
         fetch_edge(tile + stride, d, sj, x0, x1);
-        float4 pq[2][2][4];
-        fetch_pq(dc, sc, 0, pq[0][0], pq[0][1]);
+        float qa[16], qb[16];
+        fetch_q(0, qa);
         ok = mma_wait() && ok;
+        float p = 0.f;  // P of the edge's destination
+#pragma unroll 1
+        for (int b = 0; b < 4; ++b) {
+            int dest;
+            uint32_t ahead = block_runs(b, dest);
+            uint32_t heads = ahead;
+            // P of the block's runs, the next four ahead
+            auto next_p = [&]() {
+                float v = 0.f;
+                if (ahead) {
+                    const int to = __shfl_sync(0xffffffffu, dest, __ffs(ahead) - 1);
+                    ahead &= ahead - 1u;
+                    v = __ldg(Pc + (size_t)max(to, 0) * 128);
+                }
+                return v;
+            };
+            float p0 = next_p(), p1 = next_p(), p2 = next_p(), p3 = next_p();
 #pragma unroll
-        for (int cb = 0; cb < 8; ++cb) {
-            const int now = cb & 1;
-            if (cb < 7) fetch_pq(dc, sc, cb + 1, pq[now ^ 1][0], pq[now ^ 1][1]);  // one block ahead
-            uint32_t v[16];
-            tmem_ld16(trow + (uint32_t)(cb * 16), v);
-            float x[16], bias[16];
-            get_bias(s_bias[0] + cb * 16, bias);
+            for (int half = 0; half < 2; ++half) {
+                const int e0 = 32 * b + 16 * half;
+                if (half == 0) fetch_q(e0 + 16, qb);
+                else if (b < 3) fetch_q(e0 + 16, qa);
+                float pv[16];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 p4 = pq[now][0][i], q4 = pq[now][1][i];
-                const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+                for (int j = 0; j < 16; ++j) pv[j] = p;
+                for (uint32_t left = (heads >> (16 * half)) & 0xffffu; left; left &= left - 1u) {
+                    const int k = __ffs(left) - 1;  // a run begins: its P from there on
+                    p = p0;
+                    p0 = p1;
+                    p1 = p2;
+                    p2 = p3;
+                    p3 = next_p();
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int j = i * 4 + h;
-                    float t = __uint_as_float(v[j]) + bias[j];  // the unfused epilogue's order
-                    t += pv[h];
-                    t += qv[h];
+                    for (int j = 0; j < 16; ++j)
+                        if (j >= k) pv[j] = p;
+                }
+                uint32_t v[16];
+                tmem_ld16(trow + (uint32_t)e0, v);
+                float x[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float t = __uint_as_float(v[j]) + b1;  // the unfused epilogue's order
+                    t += pv[j];
+                    t += half ? qb[j] : qa[j];
                     x[j] = fmaxf(t, 0.f);
                 }
+                put_edges(sZ, gt, e0, x);
             }
-            put_bf16_row(sA, gt, cb * 16, x);
         }
         to_tensor();
         // ---- layer 2: relu(z1 W2 + b2)
         if (gt == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_k128(tmem, sA, sW2);
+            issue_edges(tmem, sW2, sZ);
             umma_commit(bar);
         }
         ok = mma_wait() && ok;
 #pragma unroll 1
-        for (int cb = 0; cb < 4; ++cb) {
+        for (int b = 0; b < 4; ++b) {
             uint32_t v[32];
-            tmem_ld32(trow + (uint32_t)(cb * 32), v);
-            float x[32], bias[32];
-            get_bias(s_bias[1] + cb * 32, bias);
+            tmem_ld32(trow + (uint32_t)(b * 32), v);
+            float x[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = fmaxf(__uint_as_float(v[j]) + bias[j], 0.f);
-            put_bf16_row(sA, gt, cb * 32, x);  // the MMAs that read sA have completed
+            for (int j = 0; j < 32; ++j) x[j] = fmaxf(__uint_as_float(v[j]) + b2, 0.f);
+            put_edges(sZ, gt, 32 * b, x);  // the MMAs that read sZ have completed
         }
         to_tensor();
         // ---- layer 3: m_e = z2 W3 + b3, summed per destination
         if (gt == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_k128(tmem, sA, sW3);
+            issue_edges(tmem, sW3, sZ);
             umma_commit(bar);
         }
         ok = mma_wait() && ok;
-        // A warp sums its own 32 rows (rows past the last edge close the tile):
-        // lane j column j, row by row, one atomic per run of a destination.
-        const int rows = __popc(__ballot_sync(0xffffffffu, dc >= 0));
-        const int above = __shfl_up_sync(0xffffffffu, dc, 1);
-        const uint32_t heads = __ballot_sync(0xffffffffu, dc >= 0 && (lane == 0 || above != dc));
 #pragma unroll 1
-        for (int cb = 0; cb < 4; ++cb) {
+        for (int b = 0; b < 4; ++b) {
+            int dest;
+            const uint32_t heads = block_runs(b, dest);
             uint32_t v[32];
-            tmem_ld32(trow + (uint32_t)(cb * 32), v);
-            float bias[32];
-            get_bias(s_bias[2] + cb * 32, bias);
-            // column j of row r at j ^ r; blocks alternate between the slices, so
-            // that one is read while the next is written
-            float* const st = reinterpret_cast<float*>(sA + (uint32_t)(cb & 1) * kSlice + (uint32_t)gw * 4096u);
+            tmem_ld32(trow + (uint32_t)(b * 32), v);
+            int to = -1;
+            float acc = 0.f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) st[lane * 32 + (j ^ lane)] = __uint_as_float(v[j]) + bias[j];
-            __syncwarp();
-            for (uint32_t left = heads; left; left &= left - 1u) {
-                const int r0 = __ffs(left) - 1, r1 = (left & (left - 1u)) ? __ffs(left & (left - 1u)) - 1 : rows;
-                const int to = __shfl_sync(0xffffffffu, dc, r0);
-                float acc = 0.f;
-#pragma unroll 8
-                for (int r = r0; r < r1; ++r) acc += st[r * 32 + (lane ^ r)];
-                atomicAdd(a.out + (size_t)to * 128 + cb * 32 + lane, acc);
+            for (int j = 0; j < 32; ++j) {
+                if ((heads >> j) & 1u) {
+                    if (j && to >= 0) atomicAdd(a.out + (size_t)to * 128 + gt, acc);
+                    to = __shfl_sync(0xffffffffu, dest, j);  // -1 past the last edge
+                    acc = 0.f;
+                }
+                acc += __uint_as_float(v[j]) + b3;
             }
+            if (to >= 0) atomicAdd(a.out + (size_t)to * 128 + gt, acc);
         }
-        __syncwarp();  // the next tile's activations go where the messages were
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         // the tile's TMEM reads and shared-memory use end before the group's
         // next tile; a run-out wait on any thread of the group stops the whole

@@ -34,6 +34,19 @@ constexpr uint32_t idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
 
+// MN-major operand in 128-byte-swizzled shared memory: rows of 64 elements (128
+// bytes) along M or N, one for each k; eight rows are 1024 bytes, the next eight k
+// follow, and the next 64 elements are `next` bytes on.
+__device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t saddr, uint32_t next) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((next >> 4) & 0x3FFFu) << 16;  // leading byte offset: along M or N
+    d |= (uint64_t)(1024u >> 4) << 32;             // stride byte offset: along k
+    d |= (uint64_t)1u << 46;
+    d |= (uint64_t)2u << 61;
+    return d;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t addr, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(addr), "r"(count) : "memory");
 }
@@ -53,13 +66,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase) {
     return false;
 }
 
-template <int N = kTileN>
+// B_MN: B is MN-major
+template <int N = kTileN, bool B_MN = false>
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc_bf16(N)), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+        "l"(adesc), "l"(bdesc), "r"(idesc_bf16(N) | (B_MN ? 1u << 16 : 0u)), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
