@@ -217,6 +217,18 @@ FeatScale scales_of(const World& w, double r_over_h) {
 
 // ------------------------------------------------------------ surrogate side
 
+void Surrogate::scan_counts(int n, int* row) {
+    size_t need = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, need, cnt_, row, n + 1, st_);
+    if (need > scan_bytes_) {
+        cu(cudaStreamSynchronize(st_), "scan");
+        if (scan_tmp_) cudaFree(scan_tmp_);
+        cu(cudaMalloc(&scan_tmp_, need), "cudaMalloc scan");
+        scan_bytes_ = need;
+    }
+    cu(cub::DeviceScan::ExclusiveSum(scan_tmp_, scan_bytes_, cnt_, row, n + 1, st_), "scan");
+}
+
 void Surrogate::graph_from_world(World& w, uint32_t s0, uint32_t s1) {
     if (s1 <= s0 || s1 > w.n_) throw std::invalid_argument("graph range");
     if (!(w.grid_current_ && w.rho_current_)) {  // as the step starts (wcsph.rs:327-328)
@@ -234,15 +246,7 @@ void Surrogate::graph_from_world(World& w, uint32_t s0, uint32_t s1) {
     for (int pass = 0; pass < 2; ++pass) {
         ensure_graph((int)n, std::max(g_.cap_e, E));
         k_msg_count<<<blocks(n + 1, 256), 256, 0, st_>>>(s0, n, w.cur_, w.lists_, fs, cnt_);
-        size_t need = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, need, cnt_, g_.row, (int)n + 1, st_);
-        if (need > scan_bytes_) {
-            cu(cudaStreamSynchronize(st_), "scan");
-            if (scan_tmp_) cudaFree(scan_tmp_);
-            cu(cudaMalloc(&scan_tmp_, need), "cudaMalloc scan");
-            scan_bytes_ = need;
-        }
-        cu(cub::DeviceScan::ExclusiveSum(scan_tmp_, scan_bytes_, cnt_, g_.row, (int)n + 1, st_), "scan");
+        scan_counts((int)n, g_.row);
         cu(cudaMemcpyAsync(&E, g_.row + n, sizeof(int), cudaMemcpyDeviceToHost, st_), "edges");
         cu(cudaStreamSynchronize(st_), "edges");
         if (E <= g_.cap_e) break;  // else grow (which drops the offsets) and count again

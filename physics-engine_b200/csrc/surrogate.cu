@@ -98,15 +98,33 @@ __global__ void k_loss(int n, const float* __restrict__ Y, const float* __restri
     if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l * inv_nf);
 }
 
+// Whether this block is the last of `blocks` to arrive here, whose writes before
+// are then visible to it (ticket is zero before the first arrives and after the last).
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned blocks) {
+    __shared__ bool s_last;
+    const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+    __threadfence();
+    __syncthreads();
+    if (first) {
+        s_last = atomicAdd(ticket, 1u) == blocks - 1u;
+        if (s_last) *ticket = 0u;
+    }
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last;
+}
+
 // dZ (fp32 [R x N]) masked in place by mask > 0; bf16 copies dZ [R8 x N] and
 // dZ^T [N x R8] (zero-padded rows / columns); column sums into gbias. A block
-// takes `tiles` tiles of 32 rows, so that a column's sum costs one atomic a
-// block: one a tile and row group put 306,000 edges' sums on 128 addresses
-// 9,556 x 8 times over (802 us of a pass that moves 470 MB). Unmasked, dZ stays
-// as it is and is not written back.
+// takes `tiles` tiles of 32 rows and leaves their sums in part [blocks x N]; the
+// last block adds these up in block order, so that a gradient's bits do not
+// depend on which block came first. (One atomic a tile and row group put 306,000
+// edges' sums on 128 addresses 9,556 x 8 times over: 802 us of a pass that moves
+// 470 MB.) Unmasked, dZ stays as it is and is not written back.
 __global__ void k_grad_prep(int R, int R8, int N, int tiles, float* __restrict__ dZ,
                             const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ g16,
-                            __nv_bfloat16* __restrict__ gT, float* __restrict__ gbias) {
+                            __nv_bfloat16* __restrict__ gT, float* __restrict__ gbias, float* __restrict__ part,
+                            unsigned* ticket) {
     __shared__ float tile[32][33];
     __shared__ float sums[8][32];
     const int c0 = blockIdx.y * 32;
@@ -137,14 +155,23 @@ __global__ void k_grad_prep(int R, int R8, int N, int tiles, float* __restrict__
         __syncthreads();
     }
     if (!gbias) return;
-    sums[ty][tx] = csum;
-    __syncthreads();
-    if (ty == 0 && c0 + tx < N) {
+    auto block_sum = [&]() {  // over the eight rows of threads, in order
+        sums[ty][tx] = csum;
+        __syncthreads();
         float v = sums[0][tx];
 #pragma unroll
         for (int k = 1; k < 8; ++k) v += sums[k][tx];
-        if (v != 0.f) atomicAdd(&gbias[c0 + tx], v);
-    }
+        return v;
+    };
+    const float mine = block_sum();
+    if (ty == 0 && c0 + tx < N) part[(size_t)blockIdx.x * N + c0 + tx] = mine;
+    if (!last_block(ticket + blockIdx.y, gridDim.x)) return;
+    csum = 0.f;
+    if (c0 + tx < N)
+#pragma unroll 8
+        for (unsigned b = ty; b < gridDim.x; b += 8) csum += __ldcg(part + (size_t)b * N + c0 + tx);
+    const float all = block_sum();
+    if (ty == 0 && c0 + tx < N) gbias[c0 + tx] = all;
 }
 
 // k_grad_prep for 128 columns, and with idx (rows gathered: dZ's row r is in's
@@ -158,7 +185,8 @@ __global__ void __launch_bounds__(256) k_grad_prep128(int R, int R8, int tiles, 
                                                       const int* __restrict__ idx,
                                                       const __nv_bfloat16* __restrict__ mask,
                                                       __nv_bfloat16* __restrict__ g16, __nv_bfloat16* __restrict__ gT,
-                                                      float* __restrict__ gbias) {
+                                                      float* __restrict__ gbias, float* __restrict__ part,
+                                                      unsigned* ticket) {
     // element (c, r) of the transposed tile; 16-byte piece p of column c at p ^ ((c / 4) & 7)
     __shared__ __align__(16) __nv_bfloat16 tile[kWidth][kPrepRows];
     __shared__ float4 sums[8][32];
@@ -210,9 +238,10 @@ __global__ void __launch_bounds__(256) k_grad_prep128(int R, int R8, int tiles, 
         __syncthreads();
     }
     if (!gbias) return;
-    sums[warp][lane] = csum;
-    __syncthreads();
-    if (warp == 0) {
+    auto block_sum = [&](float4* out) {  // over the warps, in order
+        sums[warp][lane] = csum;
+        __syncthreads();
+        if (warp != 0) return;
 #pragma unroll
         for (int k = 1; k < 8; ++k) {
             const float4 v = sums[k][lane];
@@ -221,11 +250,21 @@ __global__ void __launch_bounds__(256) k_grad_prep128(int R, int R8, int tiles, 
             csum.z += v.z;
             csum.w += v.w;
         }
-        atomicAdd(&gbias[c0], csum.x);
-        atomicAdd(&gbias[c0 + 1], csum.y);
-        atomicAdd(&gbias[c0 + 2], csum.z);
-        atomicAdd(&gbias[c0 + 3], csum.w);
+        out[lane] = csum;
+    };
+    float4* const rows = reinterpret_cast<float4*>(part);
+    block_sum(rows + (size_t)blockIdx.x * 32);
+    if (!last_block(ticket, gridDim.x)) return;
+    csum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (unsigned b = warp; b < gridDim.x; b += 8) {
+        const float4 v = __ldcg(rows + (size_t)b * 32 + lane);
+        csum.x += v.x;
+        csum.y += v.y;
+        csum.z += v.z;
+        csum.w += v.w;
     }
+    block_sum(reinterpret_cast<float4*>(gbias));
 }
 
 // k_transpose for K a multiple of 16: a tile of 64 rows x 16 columns a warp,
@@ -294,12 +333,53 @@ __global__ void k_split_dxn(int n, const float* __restrict__ dH, const float* __
     da[i] = scale * dXN[node * 2 * kWidth + kWidth + c];
 }
 
-__global__ void k_scatter_add(int E, const int* __restrict__ idx, const float* __restrict__ in,
-                              float* __restrict__ out) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)E * kWidth) return;
-    const float v = in[i];
-    if (v != 0.f) atomicAdd(&out[(size_t)idx[i / kWidth] * kWidth + i % kWidth], v);
+// The edges by source, each source's in ascending order: a count that keeps every
+// edge's arrival number, then (after the scan of the counts) the edges in their
+// source's run in order of arrival, then each edge at its rank within the run.
+__global__ void k_source_count(int E, const int* __restrict__ src, int* __restrict__ cnt, int* __restrict__ arrival) {
+    const int e = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (e < E) arrival[e] = atomicAdd(&cnt[src[e]], 1);
+}
+
+__global__ void k_source_place(int E, const int* __restrict__ src, const int* __restrict__ srow,
+                               const int* __restrict__ arrival, int* __restrict__ placed) {
+    const int e = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (e < E) placed[srow[src[e]] + arrival[e]] = e;
+}
+
+__global__ void k_source_order(int E, const int* __restrict__ src, const int* __restrict__ srow,
+                               const int* __restrict__ placed, int* __restrict__ by_src) {
+    const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k >= E) return;
+    const int e = placed[k], s = src[e], b = srow[s], end = srow[s + 1];
+    int at = b;
+#pragma unroll 4
+    for (int j = b; j < end; ++j) at += placed[j] < e;
+    by_src[at] = e;
+}
+
+// out_j = sum of the rows of in that node j sends, in edge order (a warp per node).
+// The sums are rounded to bf16 next, where one that lies at a boundary costs every
+// gradient behind it 2^-9 of that element: fp32 atomics in order of arrival left two
+// runs on the same inputs up to 5e-5 apart. Edge order is also about the order they
+// arrived in, so the gradients stay where most of those runs had them (sums in
+// fp64 do not: 2.5e-5 off on a graph whose runs agreed to 4e-6).
+__global__ void k_source_sum(int n, const int* __restrict__ srow, const int* __restrict__ by_src,
+                             const float* __restrict__ in, float* __restrict__ out) {
+    const int node = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (node >= n) return;
+    float x = 0.f, y = 0.f, z = 0.f, w = 0.f;
+    const int end = srow[node + 1];
+#pragma unroll 4
+    for (int k = srow[node]; k < end; ++k) {
+        const float4 v = reinterpret_cast<const float4*>(in + (size_t)by_src[k] * kWidth)[lane];
+        x += v.x;
+        y += v.y;
+        z += v.z;
+        w += v.w;
+    }
+    reinterpret_cast<float4*>(out + (size_t)node * kWidth)[lane] = make_float4(x, y, z, w);
 }
 
 __global__ void k_add(size_t n, float* __restrict__ a, const float* __restrict__ b) {
@@ -383,6 +463,8 @@ Surrogate::Surrogate(uint64_t seed, double r_msg_over_h) : r_msg_over_h_(r_msg_o
     allocs_.push_back(err_);
     loss_ = dalloc<float>(1);
     allocs_.push_back(loss_);
+    tickets_ = dalloc<unsigned>(kTickets);
+    allocs_.push_back(tickets_);
     for (int c = 0; c < kOut; ++c) {
         stats_.mean[c] = 0.f;
         stats_.std[c] = 1.f;
@@ -489,6 +571,7 @@ void Surrogate::set_param(int i, const float* W, const float* b) {
 }
 
 void Surrogate::ensure_graph(int n, int E) {
+    g_.by_source = false;
     if (n <= g_.cap_n && E <= g_.cap_e) {
         g_.n = n;
         g_.E = E;
@@ -510,6 +593,8 @@ void Surrogate::ensure_graph(int n, int E) {
     g_.row = static_cast<int*>(ga((size_t)(cn + 1) * 4));
     g_.src = static_cast<int*>(ga((size_t)ce * 4));
     g_.dst = static_cast<int*>(ga((size_t)ce * 4));
+    g_.srow = static_cast<int*>(ga((size_t)(cn + 1) * 4));
+    g_.by_src = static_cast<int*>(ga((size_t)ce * 4));
     g_.xe = static_cast<__nv_bfloat16*>(ga((size_t)ce * kEdgeFeat * 2));
     g_.f = static_cast<__nv_bfloat16*>(ga((size_t)cn * kNodeFeat * 2));
     g_.fluid = static_cast<uint8_t*>(ga((size_t)cn));
@@ -590,17 +675,24 @@ void Surrogate::ensure_acts(bool train) {
     act_train_ = train;
 }
 
+// Room for `need` partial sums of the launch that follows.
+float* Surrogate::partials(size_t need) {
+    if (need > part_floats_) {
+        cu(cudaStreamSynchronize(st_), "part");
+        if (part_) cudaFree(part_);
+        part_ = nullptr;
+        part_floats_ = 0;
+        cu(cudaMalloc(&part_, need * 4), "cudaMalloc part");
+        part_floats_ = need;
+    }
+    return part_;
+}
+
 void Surrogate::gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* Bt, int ldb, int M, int N, int K,
                      float* Cf, __nv_bfloat16* Cb, int ldc, const float* bias, bool relu, int splits) {
     if (M <= 0 || N <= 0) return;
     if (splits > 1) {
-        const size_t need = (size_t)splits * M * ldc;
-        if (need > part_floats_) {
-            cu(cudaStreamSynchronize(st_), "part");
-            if (part_) cudaFree(part_);
-            cu(cudaMalloc(&part_, need * 4), "cudaMalloc part");
-            part_floats_ = need;
-        }
+        partials((size_t)splits * M * ldc);
         GemmArgs g{A, Bt, part_, nullptr, nullptr, M, N, K, lda, ldb, ldc, 0, err_};
         launch_gemm(g, splits, st_);
         launch_gemm_reduce(M, N, ldc, splits, part_, bias, relu ? 1 : 0, Cf, Cb, st_);
@@ -697,12 +789,16 @@ void Surrogate::linear_bwd(Linear& L, const __nv_bfloat16* X, int R, float* dZ, 
     if (L.Np == kWidth) {
         const int row_tiles = (int)blocks(R8, kPrepRows);
         const int tiles = std::max(1, std::min(32, row_tiles / (8 * sms_)));
-        k_grad_prep128<<<blocks(row_tiles, tiles), 256, 0, st_>>>(R, R8, tiles, dZ, rows, mask, gb16_, gbT_, gb);
+        const unsigned nb = blocks(row_tiles, tiles);
+        k_grad_prep128<<<nb, 256, 0, st_>>>(R, R8, tiles, dZ, rows, mask, gb16_, gbT_, gb,
+                                            partials((size_t)nb * kWidth), tickets_);
     } else {
         const int row_tiles = (int)blocks(R8, 32), col_tiles = (int)blocks(L.Np, 32);
         const int tiles = std::max(1, std::min(32, row_tiles * col_tiles / (8 * sms_)));
         dim3 gz(blocks(row_tiles, tiles), col_tiles);
-        k_grad_prep<<<gz, tb, 0, st_>>>(R, R8, L.Np, tiles, dZ, mask, gb16_, gbT_, gb);
+        if (col_tiles > kTickets) throw std::length_error("surrogate: layer width");
+        k_grad_prep<<<gz, tb, 0, st_>>>(R, R8, L.Np, tiles, dZ, mask, gb16_, gbT_, gb,
+                                        partials((size_t)gz.x * L.Np), tickets_);
     }
     if (L.K % 16 == 0) {
         k_transpose16<<<dim3(blocks(R8, kPrepRows), blocks(L.K, 128)), 256, 0, st_>>>(R, R8, L.K, X, xT_);
@@ -736,8 +832,24 @@ void Surrogate::adam(Linear& L, float lr) {
     refresh_bf16(L);
 }
 
+// The graph's edges by source, for the backward pass: laid out once a graph.
+void Surrogate::order_by_source() {
+    const int n = g_.n, E = g_.E;
+    if (g_.by_source || E <= 0) return;
+    int* const placed = reinterpret_cast<int*>(M_);  // free between the forward pass and the next: 128 words an edge
+    int* const arrival = placed + E;
+    cu(cudaMemsetAsync(cnt_, 0, (size_t)(n + 1) * 4, st_), "memset");
+    k_source_count<<<blocks(E, 256), 256, 0, st_>>>(E, g_.src, cnt_, arrival);
+    scan_counts(n, g_.srow);
+    k_source_place<<<blocks(E, 256), 256, 0, st_>>>(E, g_.src, g_.srow, arrival, placed);
+    k_source_order<<<blocks(E, 256), 256, 0, st_>>>(E, g_.src, g_.srow, placed, g_.by_src);
+    cu(cudaGetLastError(), "edges by source");
+    g_.by_source = true;
+}
+
 float Surrogate::train_step(float lr) {
     forward(true);
+    order_by_source();
     const int n = g_.n, E = g_.E;
     const size_t nW = (size_t)n * kWidth;
     std::vector<uint8_t> fl(n);
@@ -755,13 +867,11 @@ float Surrogate::train_step(float lr) {
         mlp_bwd(base + 5, xn_[l], n, na1_[l], na2_[l], U_, dXN_);
         k_split_dxn<<<blocks(nW, 256), 256, 0, st_>>>(n, dH_, dXN_, kAggScale, dHp_, A_);
         if (E > 0) {
-            const size_t eW = (size_t)E * kWidth;
             linear_bwd(layers_[base + 4], eh2_[l], E, A_, nullptr, dE2_, g_.dst);  // the messages' rows of A_
             linear_bwd(layers_[base + 3], eh1_[l], E, dE2_, eh2_[l], dE_);
             linear_bwd(layers_[base + 2], g_.xe, E, dE_, eh1_[l], nullptr);  // masks dE_ to dZ1
             k_segsum<<<blocks((size_t)n * 32, 256), 256, 0, st_>>>(n, g_.row, dE_, 1.f, dP_);
-            cu(cudaMemsetAsync(dQ_, 0, nW * 4, st_), "memset");
-            k_scatter_add<<<blocks(eW, 256), 256, 0, st_>>>(E, g_.src, dE_, dQ_);
+            k_source_sum<<<blocks((size_t)n * 32, 256), 256, 0, st_>>>(n, g_.srow, g_.by_src, dE_, dQ_);
             linear_bwd(layers_[base + 0], hb_[l], n, dP_, nullptr, dT1_);
             k_add<<<blocks(nW, 256), 256, 0, st_>>>(nW, dHp_, dT1_);
             linear_bwd(layers_[base + 1], hb_[l], n, dQ_, nullptr, dT1_);

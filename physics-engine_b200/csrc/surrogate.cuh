@@ -48,6 +48,9 @@ struct MsgGraph {
     int* row = nullptr;              // [n + 1]
     int* src = nullptr;              // [E]
     int* dst = nullptr;              // [E]
+    int* srow = nullptr;             // [n + 1], by_src [E]: each source's edges in ascending order (training)
+    int* by_src = nullptr;
+    bool by_source = false;          // they are those of the present edges
     __nv_bfloat16* xe = nullptr;     // [E x 16]
     __nv_bfloat16* f = nullptr;      // [n x 8]
     uint8_t* fluid = nullptr;        // [n]
@@ -110,7 +113,10 @@ class Surrogate {
     void alloc_params(uint64_t seed);
     void ensure_graph(int n, int E);
     void ensure_acts(bool train);
+    void order_by_source();
+    void scan_counts(int n, int* row);  // exclusive sums of cnt_[0 .. n]
     void refresh_bf16(Linear& L);
+    float* partials(size_t need);
     void gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* Bt, int ldb, int M, int N, int K, float* Cf,
               __nv_bfloat16* Cb, int ldc, const float* bias, bool relu, int splits = 1);
     void linear_fwd(const Linear& L, const __nv_bfloat16* X, int R, float* Yf, __nv_bfloat16* Yb, bool relu);
@@ -142,6 +148,8 @@ class Surrogate {
     float* loss_ = nullptr;
     float* part_ = nullptr;
     size_t part_floats_ = 0;
+    static constexpr int kTickets = 8;
+    unsigned* tickets_ = nullptr;
 
     MsgGraph g_;
     uint32_t* node_orig_ = nullptr;   // original index of each graph node
