@@ -26,13 +26,15 @@
 // (or four) threads per particle; the fused kernel is compiled for three
 // resident CTAs per SM (80 registers), which the 32-centre tile's shared
 // memory allows. Each warp computes the in-support bit masks of 32 centres
-// over its share of the union words on the tensor cores (word_bytes); the
+// over its share of the union words on the tensor cores (word_masks); the
 // chunk's longest list sizes one block of the list pool, reserved with one
 // atomic add; then the entries are written, each thread an equal share of its
 // particle's list (a share of the words would leave most of the kept
 // candidates, which lie in the middle words, to two threads). While a thread
 // walks its kept candidates it sets the bits of the lower ones in a second
 // mask over the sorted positions, from which the lower list is written.
+//
+// A union with positions far from its cell is staged as f32 offsets there too.
 //
 // k_nlist_visit stages f32 offsets and tests them in packed f32 arithmetic: its
 // lists feed the single-precision form, whose compensated sums notice a
@@ -286,23 +288,42 @@ __device__ __forceinline__ uint32_t word_mask(const Stage& st, uint32_t base, co
 // ---- the fused kernel's stage and test ----
 
 // Features of a staged candidate: eight halves (x, y, z, nh, nl, 1, 1, 0) with
-// (x, y, z) its offset from the middle of the centre cell in units of the cell
-// (within +-1.5), rounded to half, and nh + nl the squared length of the
-// rounded offset. With a centre's row (-2x, -2y, -2z, 1, 1, ah, al, 0),
+// (x, y, z) its offset from the middle of the centre cell in units of the cell,
+// rounded to half, and nh + nl the squared length of the rounded offset. With a
+// centre's row (-2x, -2y, -2z, 1, 1, ah, al, 0),
 // ah + al = its own squared length minus the bound, the product of the two is
 // |xi - xj|^2 - bound, exact but for the splits (2^-20) and the f32 sum: the
 // sign bit is the test, and one m16n8k8 tensor instruction makes 128 of them.
 //
-// The bound: an offset's rounding error is at most 2^-11 a component, so a
-// pair's distance is off by at most 2 sqrt(3) 2^-11 = 0.0017 cells, and a pair
-// within the support (one cell) has a rounded squared distance of at most
-// 1.0034. The filter keeps ~0.5 % more candidates than the support holds.
+// The bound: the rounding error of an offset below kFeatureReach cells is at most
+// 2^-11 a component, so a pair's distance is off by at most 2 sqrt(3) 2^-11 =
+// 0.0017 cells, and a pair within the support (one cell) has a rounded squared
+// distance of at most 1.0034. The filter keeps ~0.5 % more candidates than the
+// support holds. Positions of the grid the cells were built from are within 1.5
+// cells; those the host has set since, or of a particle outside the domain, may be
+// any number away, and a union that holds one is staged as f32 offsets instead
+// (wide_masks).
 constexpr float kBound2 = 1.0036f;
+constexpr float kFeatureReach = 2.0f;
+constexpr float kLargestFloat = 3.402823466e38f;
 
 struct Features {
     __half2 xy, zn, m1, one;
 };
 static_assert(sizeof(Features) == 16, "one 16-byte store a candidate");
+
+// The largest magnitudes of the rounded offsets seen: (x, y) and (z, unused).
+struct Reach {
+    __half2 xy, z;
+    __device__ __forceinline__ Reach() : xy(__float2half2_rn(0.0f)), z(__float2half2_rn(0.0f)) {}
+    __device__ __forceinline__ void add(const Features& f) {
+        xy = __hmax2(xy, __habs2(f.xy));
+        z = __hmax2(z, __habs2(f.zn));
+    }
+    __device__ __forceinline__ bool beyond() const {
+        return !(fmaxf(fmaxf(__low2float(xy), __high2float(xy)), __low2float(z)) < kFeatureReach);
+    }
+};
 
 template <int DIM>
 __device__ __forceinline__ Features features(double px, double py, double pz, const CellUnion& cu, float inv_cell) {
@@ -1065,12 +1086,15 @@ __global__ void __launch_bounds__(32 * kNearWarps, 8) k_nlist_near(GridDesc g, T
 // Stages candidate u of a union: features, list entry and staged word.
 template <int DIM>
 __device__ __forceinline__ uint32_t stage_candidate(const StateBufs& s, const CellUnion& cu, float inv_cell,
-                                                    uint32_t slot, uint32_t u, Features* st, uint32_t* s_ent) {
+                                                    uint32_t slot, uint32_t u, Features* st, uint32_t* s_ent,
+                                                    Reach& reach) {
     const double4 p = s.pos[slot];
     const uint8_t fl = s.flags[slot];
     const uint32_t w = s.orig[slot] | ((fl & kFlagBoundary) ? kStageBoundary : 0u) |
                        ((fl & kFlagOriented) ? kStageOriented : 0u);
-    st[feature_pos(u)] = features<DIM>(p.x, p.y, p.z, cu, inv_cell);
+    const Features f = features<DIM>(p.x, p.y, p.z, cu, inv_cell);
+    st[feature_pos(u)] = f;
+    reach.add(f);
     s_ent[u] = slot | entry_flags(w);
     return w;
 }
@@ -1088,6 +1112,43 @@ __device__ __forceinline__ void centre_masks(const Features* st, uint32_t* masks
     } else {
         const uint32_t a1[2] = {at(row + 16u), at(row + 24u)};
         word_masks<kChunk, false>(st, masks, a0, a1, wb, we);
+    }
+}
+
+// The union staged anew as f32 offsets, in place of the features; raises *far to the
+// bits of the largest one (a position that is no number has no neighbours).
+template <int DIM>
+__device__ __forceinline__ void stage_wide(const double4* __restrict__ pos, double ox, double oy, double oz, uint32_t U,
+                                           const uint32_t* s_ent, Features* st, uint32_t* far) {
+    float4* const at = reinterpret_cast<float4*>(st);
+    for (uint32_t u = threadIdx.x; u < U; u += blockDim.x) {
+        const double4 p = pos[s_ent[u] & kEntrySlotMask];
+        const float4 o = make_float4((float)(p.x - ox), (float)(p.y - oy), DIM == 3 ? (float)(p.z - oz) : 0.0f, 0.0f);
+        at[u] = o;
+        const float m = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
+        if (m <= kLargestFloat) atomicMax(far, __float_as_uint(m));
+    }
+}
+
+// centre_masks from f32 offsets, for the thread's own centre (union position me).
+// In line: as calls, these two cost the unions that never come here 4 % (list build
+// at 1M 2.73 ms; 2.65 so, 2.63 without them).
+// The margin follows the union's largest offset `far`: an offset is rounded by at
+// most far / 2^24 a component and a difference of two by far / 2^23, below far /
+// 2^21 in distance. (A difference that overflows is no neighbour's.) A candidate
+// more adds +-0 to the sums.
+template <uint32_t kChunk>
+__device__ __forceinline__ void wide_masks(const Features* st, uint32_t* mask, uint32_t me, float far, float r2f,
+                                           uint32_t wb, uint32_t we) {
+    const float4* const at = reinterpret_cast<const float4*>(st);
+    const float4 a = at[me];
+    const float r = sqrtf(r2f) + far * 0x1p-21f;
+    const float limit = fminf(r * r * (1.f + 0x1p-20f), kLargestFloat);
+    for (uint32_t w = wb; w < we; ++w) {
+        uint32_t m = 0;
+#pragma unroll 4
+        for (uint32_t b = 0; b < 32u; ++b) m |= within(at[32u * w + b], a, limit) ? 1u << b : 0u;
+        mask[w * kChunk] = m;
     }
 }
 
@@ -1138,7 +1199,8 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
     uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_lmask);
     __shared__ uint32_t s_cstart[NC];
     __shared__ uint32_t s_off[NC + 1];
-    __shared__ uint32_t s_nf, s_omin, s_omax;
+    __shared__ uint32_t s_nf, s_omin, s_omax, s_far;
+    __shared__ bool s_wide;
     __shared__ uint32_t s_cv[kWays][kChunk], s_cl[kWays][kChunk];
     __shared__ uint32_t s_red[kWarps];
     __shared__ ChunkBlock s_blk;
@@ -1161,6 +1223,8 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
             s_nf = 0;
             s_omin = 0xffffffffu;
             s_omax = 0u;
+            s_far = 0u;
+            s_wide = false;
         }
         const CellUnion cu = cell_union<DIM>(g, tk, occ[it], cell_start, s_cstart, s_off);
         const uint32_t U = cu.U;
@@ -1169,12 +1233,13 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
             // Stage the union; fluid entries are appended to s_sorted with one
             // shared atomic per warp, their index range reduced per warp.
             uint32_t tmin = 0xffffffffu, tmax = 0u;
+            Reach reach;
             for (uint32_t u0 = 0; u0 < U; u0 += blockDim.x) {
                 const uint32_t u = u0 + tid;
                 bool fluid = false;
                 if (u < U) {
                     const uint32_t w = stage_candidate<DIM>(s, cu, inv_cell, slot_of_union<NC>(s_off, s_cstart, u), u,
-                                                            st, s_ent);
+                                                            st, s_ent, reach);
                     s_w[u] = w;
                     fluid = !(w & kStageBoundary);
                     if (fluid) {
@@ -1197,8 +1262,11 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
                 atomicMin(&s_omin, tmin);
                 atomicMax(&s_omax, tmax);
             }
+            if (reach.beyond()) s_wide = true;
             __syncthreads();
             const uint32_t nf = s_nf;
+            const bool wide = s_wide && !all;
+            if (wide) stage_wide<DIM>(s.pos, cu.ox, cu.oy, cu.oz, U, s_ent, st, &s_far);
             radix_sort_by_orig(s_w, s_sorted, s_tmp, s_cnt, nf, s_omin, s_omax);
             for (uint32_t u = 2u * tid; u < U; u += 2u * blockDim.x)
                 *reinterpret_cast<uint32_t*>(s_rank + u) = kNoRank | kNoRank << 16;
@@ -1213,8 +1281,13 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
                 const uint32_t myu = cu.center_off + c0 + lane;
                 // ---- pass 1: in-support masks of this share of the union words
                 // (no fluid in reach: no list to build)
-                if (cb < nc && !all && nf)
-                    centre_masks<kChunk>(st, s_vmask + cb, cu.center_off + c0 + cb, min(nc - cb, 32u), wb, we);
+                if (!all && nf) {
+                    if (wide) {
+                        if (active) wide_masks<kChunk>(st, s_vmask + lane, myu, __uint_as_float(s_far), r2f, wb, we);
+                    } else if (cb < nc) {
+                        centre_masks<kChunk>(st, s_vmask + cb, cu.center_off + c0 + cb, min(nc - cb, 32u), wb, we);
+                    }
+                }
                 __syncwarp();
                 // R: the centre's lower list holds the kept fluid candidates of
                 // rank below R (all of them for a boundary centre)
