@@ -720,6 +720,7 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
             vs[3 * i + 2] = 0.0;
         }
     for (uint64_t i = 0; i < n; ++i) n_fluid_ += kind[i] == 0;
+    n_ = n;
     set_lanes(0);
     WorldParams wp{};
     wp.kernel = 0;
@@ -758,17 +759,12 @@ DfsphSolver::~DfsphSolver() {
     if (sum_host_) cudaFreeHost(sum_host_);
 }
 
-// ms for two steps with 1 / 8 / 32 lanes a fluid slot (16^3 fluid particles 15.0 /
-// 4.2 / 2.7, 36^3 24.1 / 13.0 / 14.1, 64^3 50.9 / 52.1 / 65.9, 90^3 102 / 130 /
-// 172): many lanes while the slots do not fill the chip, one where they do. The
-// boundary slots' lists are few and long (all candidates of the cells), so these
-// take more: 36^3 20.6 / 12.4 / 11.5, 64^3 49.9 / 42.0 / 42.6.
 void DfsphSolver::set_lanes(uint32_t lanes) {
     if (lanes != 0 && lanes != 1 && lanes != 8 && lanes != 32) throw std::invalid_argument("lanes per slot");
     df_lanes_ = df_lanes_boundary_ = lanes;
     if (lanes == 0) {
-        df_lanes_ = n_fluid_ <= 30000 ? 32u : n_fluid_ <= 230000 ? 8u : 1u;
-        df_lanes_boundary_ = n_fluid_ <= 150000 ? 32u : 8u;
+        df_lanes_ = dfsph_lanes(n_fluid_, n_);
+        df_lanes_boundary_ = dfsph_boundary_lanes(n_fluid_, n_);
     }
 }
 

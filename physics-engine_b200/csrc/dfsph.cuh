@@ -93,7 +93,7 @@ class DfsphSolver {
     std::unique_ptr<World> w_;
     DfsphParams prm_;
     DfsphConst kc_{};
-    uint64_t n_fluid_ = 0;
+    uint64_t n_fluid_ = 0, n_ = 0;
     uint32_t df_lanes_ = 1, df_lanes_boundary_ = 1;  // lanes a slot of the pair passes: 1, 8 or 32
     double last_dt_ = 0.0;
     bool a_adv_set_ = false;  // the non-pressure accelerations (gravity) have been computed

@@ -16,6 +16,7 @@
 // so a round needs one warp barrier.
 #pragma once
 
+#include "lane_rules.cuh"
 #include "wcsph_device.cuh"
 
 namespace pe {
@@ -28,7 +29,7 @@ struct LaneGroup {
     uint32_t sub, grp, warp, slot;  // lane in group, group in warp, warp in CTA, the group's slot
     __device__ __forceinline__ LaneGroup()
         : sub(threadIdx.x % G), grp((threadIdx.x & 31u) / G), warp(threadIdx.x >> 5),
-          slot((blockIdx.x * blockDim.x + threadIdx.x) / G) {}
+          slot(lane_slot<G>(blockIdx.x, blockDim.x, threadIdx.x)) {}
     // this group's bits of a warp ballot
     __device__ __forceinline__ uint32_t bits(uint32_t ballot) const {
         return G == 32 ? ballot : (ballot >> (grp * G)) & ((1u << (G % 32)) - 1u);

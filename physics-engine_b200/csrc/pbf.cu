@@ -388,6 +388,7 @@ PbfSolver::PbfSolver(const PbfParams& prm, const WorldConfig& cfg, int dim, doub
                      const double* psi, const double* n_out)
     : prm_(prm) {
     for (uint64_t i = 0; i < n; ++i) n_fluid_ += kind[i] == 0;
+    n_ = n;
     set_lanes(0);
     WorldParams wp{};
     wp.kernel = 0;
@@ -522,11 +523,8 @@ void PbfSolver::lists(bool reused) {
     w.build_near_lists();
 }
 
-// ms for ten steps with 1 / 8 lanes: 6^3 fluid particles 3.7 / 2.4, 20^3 5.4 / 4.1,
-// 30^3 6.0 / 5.3, 40^3 7.4 / 7.5, 50^3 11.4 / 11.7, 70^3 25.4 / 29.2: a list of ~33
-// entries shared out while the slots do not fill the chip.
 void PbfSolver::set_lanes(uint32_t lanes) {
-    if (lanes == 0) lanes = n_fluid_ <= 48000 ? 8u : 1u;
+    if (lanes == 0) lanes = pbf_lanes(n_fluid_, n_);
     if (lanes != 1 && lanes != 8) throw std::invalid_argument("lanes per slot");
     lanes_ = lanes;
 }

@@ -68,7 +68,7 @@ class PbfSolver {
     std::unique_ptr<World> w_;
     PbfParams prm_;
     PbfConst kc_{};
-    uint64_t n_fluid_ = 0;
+    uint64_t n_fluid_ = 0, n_ = 0;
     uint32_t lanes_ = 8;         // lanes a slot of the constraint passes
     double* lambda_ = nullptr;   // per slot
     double* lambda_orig_ = nullptr;  // the same values in original order

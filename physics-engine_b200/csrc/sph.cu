@@ -818,33 +818,6 @@ void forces_prepare() {
     allow_forces_smem<32>();
 }
 
-// Lanes per slot of each pass, from the slots that have work and the pairs
-// each has (~250 in 3-D, ~50 in 2-D). More lanes shorten a slot's serial chain;
-// fewer waste less on the exchange of terms once the slots alone fill the SMs.
-// us a pass, 1 / 4 / 8 / 16 / 32 lanes, dam-break tanks of side^3 fluid:
-//            13^3                  32^3                    64^3                     80^3
-//   density  83/31/19/15/14.5      98/72/59/63/75          331/389/386/442/548      579/732/736/858/1065
-//   forces   187/53/35/24/19       228/129/118/121/141     767/707/773/849/1033     1344/1319/1468/1642/1998
-//   XSPH     70/32/25/19/20        96/92/71/82/110         301/430/446/519/782      507/793/841/1003/1507
-//   boundary 46/23/15/12/11        51/28/20/17/21          64/46/44/58/95           74/63/67/97/165
-// and of side^2: 40,000 particles density 24/20/20/25/37, forces 41/31/33/40/64;
-// 160,000 density 49/52/60/82/135, forces 86/94/113/148/256.
-PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t boundary) {
-    struct Limits {
-        uint64_t l32, l16, l8, l4;  // the most slots each lane count is taken for
-    };
-    auto pick = [](uint64_t n, const Limits& m) -> uint32_t {
-        return n <= m.l32 ? 32u : n <= m.l16 ? 16u : n <= m.l8 ? 8u : n <= m.l4 ? 4u : 1u;
-    };
-    PassLanes r;
-    const bool d3 = dim == 3;
-    r.density = pick(fluid, d3 ? Limits{3000, 10000, 190000, 190000} : Limits{600, 10000, 40000, 100000});
-    r.forces = pick(fluid, d3 ? Limits{8000, 20000, 40000, 700000} : Limits{1000, 3000, 12000, 80000});
-    r.xsph = pick(fluid, d3 ? Limits{1500, 10000, 45000, 45000} : Limits{1000, 3000, 12000, 25000});
-    r.boundary = pick(boundary, d3 ? Limits{10000, 25000, 100000, 1000000} : Limits{10000, 10000, 100000, 1000000});
-    return r;
-}
-
 // Calls f(integral_constant<int, G>) for the lanes per slot.
 template <class F>
 static void with_lanes(uint32_t lanes, F&& f) {

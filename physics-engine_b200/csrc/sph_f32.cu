@@ -662,31 +662,6 @@ __global__ void k_bf_to_f64(uint32_t n, const float* __restrict__ bf, StateBufs 
 
 }  // namespace
 
-// Lanes of a particle's list in the three pair passes. One lane a particle
-// streams its rows best once the particles alone fill the chip; below that the
-// walk of one list is the pass's length, and 8 lanes (32 for the smallest
-// scenes) shorten it. Cubes of the dam break, us a pass, 1 / 8 / 32 lanes:
-//   particles   density          forces           XSPH
-//         216   56 / 21 / 13     101 / 31 / 20    51 / 21 / 16
-//       2,197   62 / 22 / 18     112 / 32 / 27    61 / 22 / 20
-//       6,859   64 / 28 / 30     112 / 40 / 40    64 / 26 / 31
-//      32,768   73 / 62 / 100    132 / 83 / 119   74 / 56 / 94
-//      68,921   91 / 110 / 198   171 / 144 / 228  100 / 98 / 181
-//     125,000   134 / 186 / 351  250 / 242 / 401  111 / 161 / 320
-//   2-D   900   17 / 10 / 9      33 / 18 / 14     18 / 12 / 13
-//       6,400   18 / 11 / 13     34 / 18 / 22     21 / 13 / 17
-//      40,000   19 / 20 / 39     38 / 31 / 53     23 / 22 / 43
-// (Four lanes were slower than one or eight at every size.)
-PassLanes pass_lanes_f32(int dim, uint64_t fluid) {
-    const uint64_t few = dim == 2 ? 2048 : 4096;
-    const auto rule = [&](uint64_t eight) { return fluid <= few ? 32u : fluid <= eight ? 8u : 1u; };
-    PassLanes r;
-    r.density = rule(dim == 2 ? 32768 : 49152);
-    r.forces = rule(98304);
-    r.xsph = rule(dim == 2 ? 40960 : 65536);
-    return r;
-}
-
 template <class F>
 static void with_f32_lanes(uint32_t lanes, F&& f) {
     if (lanes == 8) f(std::integral_constant<int, 8>{});

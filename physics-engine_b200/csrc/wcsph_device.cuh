@@ -194,15 +194,7 @@ struct PassShape {
     uint32_t density = 128, forces = 128, xsph = 128;
 };
 
-// Lanes of a warp that share one slot's list in each f64 pass (lane_group.cuh):
-// 1, 4, 8, 16 or 32.
-struct PassLanes {
-    uint32_t density = 1, forces = 1, boundary = 1, xsph = 1;
-};
-PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t boundary);
-
-// Single-precision form (sph_f32.cu): 1, 8 or 32 lanes.
-PassLanes pass_lanes_f32(int dim, uint64_t fluid);
+// Single-precision form (sph_f32.cu).
 struct F32Const {
     int dim;
     float h, inv_h, alpha, mass, rho0, rho_self, cell;

@@ -984,7 +984,7 @@ bool World::capture_graph(double dt) {
 }
 
 void World::set_lanes(uint32_t lanes) {
-    if (lanes == 0) lanes_ = f32_ ? pass_lanes_f32(dim_, n_fluid_) : pass_lanes(dim_, n_fluid_, n_ - n_fluid_);
+    if (lanes == 0) lanes_ = f32_ ? pass_lanes_f32(dim_, n_fluid_, n_) : pass_lanes(dim_, n_fluid_, n_);
     else if (lanes == 1 || lanes == 8 || lanes == 32 || (!f32_ && (lanes == 4 || lanes == 16)))
         lanes_.density = lanes_.forces = lanes_.boundary = lanes_.xsph = lanes;
     else throw std::invalid_argument("lanes per slot");

@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+#include "lane_rules.cuh"
 #include "transfer.cuh"
 #include "wcsph_device.cuh"
 
