@@ -15,8 +15,9 @@
 // 16,000 in 2-D 146 and 127; 57,570 487 and 457).
 // The counting pass keeps each slot's rank in its cell, so that placing needs no
 // second round of atomics, and adds up the scan's tiles, so that the scan is one
-// pass; the scan clears the counts and the placing pass the tiles for the next
-// build; a slot's thread finds its place in its cell and moves the state there.
+// pass (two beyond kFlatTiles tiles); the scan clears the counts and the placing
+// pass the tiles for the next build; a slot's thread finds its place in its cell
+// and moves the state there.
 #include "pe_math.cuh"
 #include "wcsph_device.cuh"
 
@@ -27,6 +28,12 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+// Up to this many tiles each adds up the ones before it; beyond, where that sum
+// would be quadratic in the cells, one block scans the tiles' sums first. us a
+// build of 8,000 particles, flat / scanned first: 2.0M cells 32 / 35, 3.9M 40 / 41,
+// 8.2M 58 / 56, 33M 160 / 145, 130M 628 / 462, 267M 1534 / 900 (a batch of tanks
+// may have 2^31).
+constexpr uint32_t kFlatTiles = 1536;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
@@ -124,20 +131,55 @@ __device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t* ea
     __syncthreads();
 }
 
-// cell_start (exclusive) and the list of occupied cells in linear order; each
-// tile adds up the ones before it. Clears count. clear_lists: a list build and
-// its density pass follow, their counters are cleared too.
-__global__ void k_scan(uint32_t ncell, uint32_t* __restrict__ count, const unsigned long long* __restrict__ tiles,
-                       uint32_t* __restrict__ cell_start, uint32_t* __restrict__ occ, DeviceScalars* sc,
-                       int clear_lists) {
-    uint32_t pa = 0, pb = 0;
-    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) {
-        const unsigned long long v = tiles[t];
-        pa += (uint32_t)v;
-        pb += (uint32_t)(v >> 32);
+// Each tile's sum becomes that of the tiles before it (one block).
+__global__ void k_scan_tiles(uint32_t ntiles, unsigned long long* __restrict__ tiles) {
+    uint32_t carry_a = 0, carry_b = 0;
+    for (uint32_t off = 0; off < ntiles; off += kScanTile) {
+        const uint32_t first = off + threadIdx.x * kScanItems;
+        unsigned long long v[kScanItems];
+        uint32_t a = 0, b = 0;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = first + i < ntiles ? tiles[first + i] : 0ull;
+            a += (uint32_t)v[i];
+            b += (uint32_t)(v[i] >> 32);
+        }
+        uint32_t ea, eb, ta, tb;
+        block_scan2(a, b, &ea, &eb, &ta, &tb);
+        ea += carry_a;
+        eb += carry_b;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            if (first + i < ntiles) tiles[first + i] = (unsigned long long)ea | ((unsigned long long)eb << 32);
+            ea += (uint32_t)v[i];
+            eb += (uint32_t)(v[i] >> 32);
+        }
+        carry_a += ta;
+        carry_b += tb;
     }
-    uint32_t ea, eb, before_a, before_b;
-    block_scan2(pa, pb, &ea, &eb, &before_a, &before_b);
+}
+
+// cell_start (exclusive) and the list of occupied cells in linear order; each
+// tile adds up the ones before it, or with `summed` reads their sum. Clears count.
+// clear_lists: a list build and its density pass follow, their counters are
+// cleared too.
+__global__ void k_scan(uint32_t ncell, uint32_t* __restrict__ count, const unsigned long long* __restrict__ tiles,
+                       bool summed, uint32_t* __restrict__ cell_start, uint32_t* __restrict__ occ, DeviceScalars* sc,
+                       int clear_lists) {
+    uint32_t before_a, before_b;
+    if (summed) {
+        const unsigned long long v = tiles[blockIdx.x];
+        before_a = (uint32_t)v;
+        before_b = (uint32_t)(v >> 32);
+    } else {
+        uint32_t pa = 0, pb = 0, ea, eb;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) {
+            const unsigned long long v = tiles[t];
+            pa += (uint32_t)v;
+            pb += (uint32_t)(v >> 32);
+        }
+        block_scan2(pa, pb, &ea, &eb, &before_a, &before_b);
+    }
     uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t a = 0, b = 0;
@@ -149,7 +191,7 @@ __global__ void k_scan(uint32_t ncell, uint32_t* __restrict__ count, const unsig
         a += v[i];
         b += v[i] != 0u;
     }
-    uint32_t ta, tb;
+    uint32_t ea, eb, ta, tb;
     block_scan2(a, b, &ea, &eb, &ta, &tb);
     uint32_t ra = before_a + ea, rb = before_b + eb;
 #pragma unroll
@@ -254,15 +296,19 @@ size_t scan_tiles_bytes(uint32_t ncell) {
     return sizeof(unsigned long long) * (size_t)((ncell + kScanTile - 1) / kScanTile + 1);
 }
 
-void launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur, const double4* pos_next,
-                      const uint8_t* flags, const uint32_t* orig, const GridBufs& b, DeviceScalars* sc,
-                      bool clear_lists, cudaStream_t st) {
+uint32_t launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur,
+                          const double4* pos_next, const uint8_t* flags, const uint32_t* orig, const GridBufs& b,
+                          DeviceScalars* sc, bool clear_lists, cudaStream_t st) {
     const uint32_t ntiles = (g.ncell + kScanTile - 1) / kScanTile, nb = blocks_for(n, 256);
     if (n)
         k_cell_ids<<<nb, 256, 0, st>>>(g, tk, n, pos_cur, pos_next, flags, b.cellid, b.key_tmp, b.count, b.rank,
                                        b.tiles, sc);
-    k_scan<<<ntiles, kScanThreads, 0, st>>>(g.ncell, b.count, b.tiles, b.cell_start, b.occ, sc, clear_lists ? 1 : 0);
+    const bool summed = ntiles > kFlatTiles;
+    if (summed) k_scan_tiles<<<1, kScanThreads, 0, st>>>(ntiles, b.tiles);
+    k_scan<<<ntiles, kScanThreads, 0, st>>>(g.ncell, b.count, b.tiles, summed, b.cell_start, b.occ, sc,
+                                            clear_lists ? 1 : 0);
     if (n) k_place<<<nb, 256, 0, st>>>(n, b.cellid, b.rank, b.cell_start, orig, b.placed, b.tiles, ntiles);
+    return summed ? 4u : 3u;
 }
 
 void launch_order(uint32_t n, const GridBufs& b, uint32_t* perm, cudaStream_t st) {

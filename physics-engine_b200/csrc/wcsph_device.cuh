@@ -242,10 +242,10 @@ struct GridBufs {
 size_t scan_tiles_bytes(uint32_t ncell);
 // Cell ranges, occupied cells and the slots of each cell (in any order).
 // clear_lists: clears sc->list_used and sc->w_short for the list build and
-// density pass that follow.
-void launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur, const double4* pos_next,
-                      const uint8_t* flags, const uint32_t* orig, const GridBufs& b, DeviceScalars* sc,
-                      bool clear_lists, cudaStream_t st);
+// density pass that follow. Returns the kernels launched.
+uint32_t launch_cell_sort(const GridDesc& g, const Tanks& tk, uint32_t n, const double4* pos_cur,
+                          const double4* pos_next, const uint8_t* flags, const uint32_t* orig, const GridBufs& b,
+                          DeviceScalars* sc, bool clear_lists, cudaStream_t st);
 // Then either perm (new slot -> old slot) or the state moved to its new slots.
 void launch_order(uint32_t n, const GridBufs& b, uint32_t* perm, cudaStream_t st);
 void launch_move(uint32_t n, const GridBufs& b, const StateBufs& src, const double4* pos_next,

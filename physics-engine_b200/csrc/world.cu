@@ -629,9 +629,9 @@ void World::build_grid(const double4* pos_next, const double4* vel_next, bool li
     const uint32_t n = (uint32_t)n_;
     const GridBufs b{cellid_, key_tmp_, rank_, placed_, count_, tiles_, cell_start_, occ_};
     prof_begin(kGrid);
-    launch_cell_sort(g_, tanks_, n, cur_.pos, pos_next, cur_.flags, cur_.orig, b, sc_, lists_follow, st_);
+    launches_ += 1 + launch_cell_sort(g_, tanks_, n, cur_.pos, pos_next, cur_.flags, cur_.orig, b, sc_, lists_follow,
+                                      st_);
     launch_move(n, b, cur_, pos_next, vel_next, alt_, slot_of_orig_, st_);
-    launches_ += 4;
     list_used_cleared_ = w_short_cleared_ = lists_follow;
     prof_end();
     std::swap(cur_, alt_);
