@@ -287,6 +287,9 @@ int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes);
  * default, while the device has room for the buffer); off, they recompute it.
  * The results are identical. */
 int pe_fluid_dfsph_set_pair_weights(PeDfsph* w, int32_t on);
+/* out as pe_fluid_wcsph_pair_weight_info's, of the buffer the alpha pass fills (made
+ * by the first pass that does). Synchronous. */
+int pe_fluid_dfsph_pair_weight_info(PeDfsph* w, uint64_t out[3]);
 int pe_fluid_dfsph_len(const PeDfsph* w, uint64_t* out_len);
 int pe_fluid_dfsph_get_time(const PeDfsph* w, double* t);
 int pe_fluid_dfsph_get_last_dt(const PeDfsph* w, double* out);

@@ -731,7 +731,7 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
     WorldConfig wc = cfg;
     wc.precision = 0;
     wc.use_graph = 0;
-    wc.pair_weights = 1;  // the buffer of the kept pairs, while the device has room for it
+    wc.pair_weights = 0;
     w_.reset(new World(wp, wc, dim, rest_density, mass, h, n, xs.data(), vs.data(), kind, psi, n_out, nullptr, 1,
                        kernel_support(prm.kernel, h)));
     w_->list_keep_boundary_ = true;
@@ -752,6 +752,10 @@ DfsphSolver::DfsphSolver(const DfsphParams& prm, const WorldConfig& cfg, int dim
     // dfsph.rs:177-179
     rebuild();
     density_and_alpha();
+    // The buffer of the kept pairs is made by the first pass that fills it (as the
+    // first guess of the list pool's and again as the sized pool's it made up a
+    // tenth of the creation of a world of 46,620 particles).
+    w_->pair_w_on_ = true;
     w_->check(cudaStreamSynchronize(w_->st_), "dfsph init");
 }
 
@@ -788,6 +792,7 @@ void DfsphSolver::alpha_pass(double* alpha) {
     World& w = *w_;
     const uint32_t n = (uint32_t)w.n_;
     if (!n) return;
+    w.make_pair_weights();
     if (w.lists_.wpair && !w.w_short_cleared_)
         w.check(cudaMemsetAsync(&w.sc_->w_short, 0, sizeof(uint32_t), w.st_), "memset");
     w.w_short_cleared_ = false;
@@ -810,6 +815,7 @@ void DfsphSolver::alpha_pass(double* alpha) {
 
 // Before a solver: the positions may have been set, or moved by the slip planes, since alpha's pass.
 void DfsphSolver::keep_pairs() {
+    w_->make_pair_weights();
     if (!w_->w_valid_) alpha_pass(nullptr);
 }
 

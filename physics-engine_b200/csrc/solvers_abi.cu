@@ -405,6 +405,14 @@ int pe_fluid_dfsph_set_pair_weights(PeDfsph* w, int32_t on) {
     });
 }
 
+int pe_fluid_dfsph_pair_weight_info(PeDfsph* w, uint64_t out[3]) {
+    if (!w || !out) return PE_ERR_NULL;
+    return guard([&] {
+        w->s->world().pair_weight_info(out);
+        return PE_OK;
+    });
+}
+
 int pe_fluid_dfsph_set_lanes(PeDfsph* w, uint32_t lanes) {
     if (!w) return PE_ERR_NULL;
     return guard([&] {

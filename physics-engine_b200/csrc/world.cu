@@ -383,6 +383,7 @@ void World::alloc_lists(unsigned long long groups) {
     lists_.wpair32 = nullptr;
     lists_.w_cap = 0;
     w_valid_ = false;
+    pair_w_tried_ = false;
     if (pair_w_on_) alloc_pair_weights(pair_weight_groups());
     lists_valid_ = false;
     invalidate_graph();
@@ -399,6 +400,7 @@ unsigned long long World::pair_weight_groups() const {
 
 void World::alloc_pair_weights(unsigned long long groups) {
     if (pair_weights() || !groups) return;
+    pair_w_tried_ = true;
     // Kept only with room to spare: the buffer is an optimisation, so it
     // gives way to the list pool (a 512-tank batch's pool alone is ~55 GB).
     const size_t bytes = (size_t)groups * 4u * (f32_ ? sizeof(float) : sizeof(double));
@@ -443,6 +445,10 @@ void World::pair_weight_info(uint64_t out[3]) {
     out[0] = pair_weights() ? 1u : 0u;
     out[1] = lists_.w_cap;
     out[2] = pair_weights() && hs.w_short ? 1u : 0u;
+}
+
+void World::make_pair_weights() {
+    if (pair_w_on_ && !pair_weights() && !pair_w_tried_) alloc_pair_weights(pair_weight_groups());
 }
 
 void World::set_pair_weights(bool on) {

@@ -279,8 +279,10 @@ class World {
     bool lists_valid_ = false;   // neighbour lists match the grid and positions
     bool lists_outlive_poll_ = false;  // the next step reads the present lists: a poll that moves the pool rebuilds them
     bool pair_w_on_ = false;     // keep lists_.wpair (set_pair_weights)
+    bool pair_w_tried_ = false;  // its allocation for the present pool has been tried
     bool w_valid_ = false;       // lists_.wpair holds W of the current lists and positions
     void alloc_pair_weights(unsigned long long groups);
+    void make_pair_weights();  // the present pool's buffer, if it is wanted and none has been tried
     void free_pair_weights();
     unsigned long long pair_weight_groups() const;
     bool lists_checked_ = false; // list capacity verified for the current positions

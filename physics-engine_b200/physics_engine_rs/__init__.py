@@ -263,6 +263,7 @@ def load_library():
         "pe_fluid_dfsph_compute_density": (C.c_int, [vp]),
         "pe_fluid_dfsph_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_dfsph_set_pair_weights": (C.c_int, [vp, C.c_int32]),
+        "pe_fluid_dfsph_pair_weight_info": (C.c_int, [vp, vp]),
         "pe_fluid_pbf_set_lanes": (C.c_int, [vp, C.c_uint32]),
         "pe_fluid_dfsph_compute_alpha": (C.c_int, [vp]),
         "pe_fluid_dfsph_len": (C.c_int, [vp, C.POINTER(u64)]),
@@ -1114,6 +1115,13 @@ class DfsphWorld:
         (on by default, while the device has room for the buffer); off, they
         recompute it. The results are identical."""
         _ok(_lib.pe_fluid_dfsph_set_pair_weights(self._w, 1 if on else 0), "dfsph_set_pair_weights")
+
+    def pair_weight_info(self) -> dict:
+        """{in_use, entries (list entries the buffer covers), short (the last
+        alpha pass met a list beyond them, whose pairs are recomputed)}."""
+        out = np.zeros(3, np.uint64)
+        _ok(_lib.pe_fluid_dfsph_pair_weight_info(self._w, _ptr(out)), "dfsph_pair_weight_info")
+        return {"in_use": bool(out[0]), "entries": int(out[1]), "short": bool(out[2])}
 
     @property
     def t(self) -> float:
