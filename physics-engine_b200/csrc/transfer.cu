@@ -13,8 +13,9 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
 #include <thread>
+
+#include "parts.cuh"
 
 namespace pe {
 
@@ -74,29 +75,17 @@ bool HostTransfer::prepare(const void* host, size_t bytes, int device, int* thre
     return true;
 }
 
-// Calls part(t, begin, end) for `threads` parts of the bytes, each by its own
-// thread (the first by the caller, as are those no thread could be had for).
+// Calls part(t, begin, end) for `threads` parts of the bytes, each by its own thread.
 template <class F>
 cudaError_t HostTransfer::share_out(size_t bytes, int threads, int device, F&& part) {
     cudaError_t err[kThreads] = {};
-    std::thread pool[kThreads];
     const size_t step = (bytes / (size_t)threads + 4095u) & ~(size_t)4095u;
     auto run = [&](int t) noexcept {
         DeviceScope scope(device);
         const size_t b = std::min(bytes, step * (size_t)t), e = t == threads - 1 ? bytes : std::min(bytes, b + step);
         err[t] = b < e ? part(t, b, e) : cudaSuccess;
     };
-    for (int t = 1; t < threads; ++t) {
-        try {
-            pool[t] = std::thread(run, t);
-        } catch (const std::system_error&) {
-        }
-    }
-    run(0);
-    for (int t = 1; t < threads; ++t) {
-        if (pool[t].joinable()) pool[t].join();
-        else run(t);
-    }
+    run_parts<kThreads>(threads, run);
     for (int t = 0; t < threads; ++t)
         if (err[t] != cudaSuccess) return err[t];
     return cudaSuccess;

@@ -19,8 +19,8 @@ class HostTransfer {
     HostTransfer(const HostTransfer&) = delete;
     HostTransfer& operator=(const HostTransfer&) = delete;
     ~HostTransfer();
-    // The source may be written to again when the call returns; the device
-    // copy is ordered on st.
+    // The device copy is ordered on st. A pageable source may be written to again
+    // when the call returns, a pinned one when the copy has been done.
     cudaError_t to_device(void* dst, const void* src, size_t bytes, int device, cudaStream_t st);
     // The bytes are in dst when the call returns without an error.
     cudaError_t to_host(void* dst, const void* src, size_t bytes, int device, cudaStream_t st);
