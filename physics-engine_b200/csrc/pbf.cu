@@ -411,11 +411,15 @@ PbfSolver::PbfSolver(const PbfParams& prm, const WorldConfig& cfg, int dim, doub
 
 PbfSolver::~PbfSolver() = default;
 
+// Whether a step's constraint iterations look for neighbours in cells built before the first.
+static bool cells_reused(const PbfParams& p) { return p.reuse_neighbours && p.iterations > 1; }
+
 void PbfSolver::set_params(const PbfParams& p) {
     const double h = w_->h_;
     const double s_old = std::fmax(kernel_support(prm_.density_kernel, h), kernel_support(prm_.grad_kernel, h));
     const double s_new = std::fmax(kernel_support(p.density_kernel, h), kernel_support(p.grad_kernel, h));
     if (s_old != s_new) throw std::invalid_argument("the support radius is fixed at creation");
+    if (cells_reused(p) && !cells_reused(prm_)) w_->lists_checked_ = false;  // the pool holds candidates in support
     prm_ = p;
     refresh_const();
 }
@@ -507,9 +511,9 @@ void PbfSolver::refresh_const() {
     k.gz = prm_.gravity[2];
 }
 
-// Lists at the present positions. A new state's pool is first sized by its
-// candidates where the cells outlive the positions (reused): no later iteration's
-// lists can be longer.
+// Lists at the present positions. A new state's pool, or that of a world whose cells
+// now outlive the positions (reused), is first sized by all its candidates there: no
+// later iteration's lists can be longer.
 void PbfSolver::lists(bool reused) {
     World& w = *w_;
     if (!w.lists_checked_) {
@@ -570,7 +574,7 @@ void PbfSolver::step(double dt) {
     // pbf.rs:146-156: candidates of the neighbour cells, kept while the
     // predictions move (reuse_neighbours). The others add +-0, so each
     // iteration's lists hold the candidates then in support.
-    const bool reused = prm_.reuse_neighbours && prm_.iterations > 1;
+    const bool reused = cells_reused(prm_);
     // pbf.rs:403-411: constraint iterations
     for (uint64_t it = 0; it < prm_.iterations; ++it) {
         if (it > 0 && !prm_.reuse_neighbours) w.build_grid(nullptr, nullptr, true);
