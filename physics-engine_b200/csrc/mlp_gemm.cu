@@ -15,11 +15,11 @@
 // the tile). With gridDim.z > 1 the K range is split and each split writes its
 // own fp32 partial (summed by launch_gemm_reduce).
 //
-// Two shapes. Layers (K of 2 to 4 slices, thousands of rows): BN = 128, two
-// stages, three CTAs an SM; the whole K range is in flight at once. Weight
-// gradients (K = the rows, one or two 128 x 128 outputs): BN = 32 and eight
-// stages, so that four CTAs share an output and each keeps six slices in
-// flight. The 13,800 rows of a node layer's gradient: 979 us on one CTA with two
+// Two shapes. Layers (K of 2 to 4 slices, thousands of rows), and whatever has
+// outputs for the whole chip: BN = 128, two stages, three CTAs an SM; a layer's
+// whole K range is in flight at once. Weight gradients (K = the rows, one or two
+// 128 x 128 outputs): BN = 32 and eight stages, so that four CTAs share an output
+// and each keeps six slices in flight. The 13,800 rows of a node layer's gradient: 979 us on one CTA with two
 // stages loaded by the compute threads, 135 now (0.62 us a slice, which is the
 // latency of a copy: the proxy fence before a slice's MMAs waits for the copies
 // behind it too); 306,000 edge rows in 37 splits 629 -> 85 us; a 128-wide layer
@@ -43,7 +43,13 @@ using namespace umma;
 
 constexpr int kBM = kTileM, kBK = 64;
 constexpr int kGemmThreads = 128;
-constexpr int kLongK = 8;  // slices from which the weight-gradient shape is taken
+// The weight-gradient shape is taken from kLongK slices on where all its CTAs are
+// resident at once, one an SM; beyond, each reads its rows of A again for 32 columns
+// where the other shape does for 128. us, weight-gradient / layer shape: 4,736 x 128
+// x 2,048 (148 CTAs) 47 / 60, 6,400 x 128 x 2,048 (200) 71 / 59, 128 x 128 x 306,000
+// in 37 splits (148) 110 / 125, in 64 (256) 125 / 89, 4,096 x 4,096 x 4,096 1194 / 245.
+constexpr int kLongK = 8;
+constexpr long long kLongCtas = 148;
 
 template <int BN, int STAGES>
 struct GemmShape {
@@ -238,7 +244,7 @@ void launch_gemm(const GemmArgs& g, int splits, cudaStream_t st) {
     if (splits < 1) splits = 1;
     const int slices = ((g.K + kBK - 1) / kBK + splits - 1) / splits;
     const unsigned mt = (unsigned)((g.M + kBM - 1) / kBM);
-    if (slices >= kLongK)
+    if (slices >= kLongK && (long long)mt * ((g.N + 31) / 32) * splits <= kLongCtas)
         k_gemm_bf16<32, 8><<<dim3(mt, (g.N + 31) / 32, splits), kGemmThreads, GemmShape<32, 8>::kBytes, st>>>(g);
     else
         k_gemm_bf16<128, 2><<<dim3(mt, (g.N + 127) / 128, splits), kGemmThreads, GemmShape<128, 2>::kBytes, st>>>(g);
