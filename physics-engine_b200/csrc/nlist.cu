@@ -727,9 +727,15 @@ struct EntryOut {
 };
 
 // CTAs a cell: its chunks are shared out over several (each stages the union
-// again) while the occupied cells leave most of the grid idle.
+// again) while the occupied cells leave most of the grid's 2,368 CTAs idle. us a
+// build with 1 / 2 / 4 / 8 of them, f64 and f32: 48 cells -/28/22/23, 22/17/15/15;
+// 118 cells 50/35/33/35, 31/21/21/22; 237 56/41/39/46, 37/27/24/25; 406 63/48/48/65,
+// 41/31/29/34; 663 67/55/66/112, 45/35/35/53; 1,050 75/77/108/186, 51/42/54/79. A 2-D
+// cell is one chunk: 113 cells 15/17/18/17, 10/11/12/13.
+template <int DIM>
 __device__ __forceinline__ uint32_t cell_parts(uint32_t nocc) {
-    return min(max(gridDim.x / (8u * max(nocc, 1u)), 1u), 4u);
+    if (DIM == 2) return 1u;
+    return 16u * nocc <= gridDim.x ? 4u : 3u * nocc <= gridDim.x ? 2u : 1u;
 }
 
 // ----------------------------------------------------------------- visit
@@ -762,7 +768,7 @@ __global__ void __launch_bounds__(kNlThreads, 4) k_nlist_visit(GridDesc g, Tanks
     uint32_t max_union = 0;
     if (tid == 0) s_overflow = false;
 
-    const uint32_t parts = cell_parts(nocc);
+    const uint32_t parts = cell_parts<DIM>(nocc);
     for (uint32_t item = blockIdx.x; item < nocc * parts; item += gridDim.x) {
         const uint32_t it = item / parts, part = item - it * parts;
         const CellUnion cu = cell_union<DIM>(g, tk, occ[it], cell_start, s_cstart, s_off);
@@ -989,7 +995,8 @@ __global__ void __launch_bounds__(32 * kNearWarps, 8) k_nlist_near(GridDesc g, T
                         const float4 p = sm.at[32u * w + lane];
                         const float ax = p.x - a.x, ay = p.y - a.y, az = p.z - a.z;
                         const float bx = p.x - b.x, by = p.y - b.y, bz = p.z - b.z;
-                        // a position that is no number stays in, as in every pass
+                        // (unlike the other builds' tests, this one keeps a position that is no
+                        // number: PBF's passes then carry it on as those of all candidates did)
                         const uint32_t ma = __ballot_sync(kAll, !(ax * ax + ay * ay + az * az > limit));
                         const uint32_t mb = __ballot_sync(kAll, !(bx * bx + by * by + bz * bz > limit));
                         if (lane == w) {
@@ -1216,7 +1223,7 @@ __global__ void __launch_bounds__(kNlThreads, 3) k_nlist_both(GridDesc g, Tanks 
     uint32_t max_union = 0;
     if (tid == 0) s_overflow = false;
 
-    const uint32_t parts = cell_parts(nocc);
+    const uint32_t parts = cell_parts<DIM>(nocc);
     for (uint32_t item = blockIdx.x; item < nocc * parts; item += gridDim.x) {
         const uint32_t it = item / parts, part = item - it * parts;
         if (tid == 0) {
@@ -1447,12 +1454,6 @@ uint32_t nlist_union_capacity(uint32_t max_union) {
     if (want < kStageStep) want = kStageStep;
     if (want > kMaxUnionStage) want = kMaxUnionStage;
     return (uint32_t)want;
-}
-
-size_t nlist_smem_bytes(uint32_t ucap, uint32_t chunk) {
-    chunk = valid_chunk(ucap, chunk);
-    const size_t a = visit_smem_bytes(ucap, chunk), b = both_smem_bytes(ucap, chunk);
-    return a > b ? a : b;
 }
 
 namespace {

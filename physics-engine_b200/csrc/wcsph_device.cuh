@@ -253,7 +253,6 @@ void launch_move(uint32_t n, const GridBufs& b, const StateBufs& src, const doub
 
 // ----- neighbour lists -----
 uint32_t nlist_union_capacity(uint32_t max_union);
-size_t nlist_smem_bytes(uint32_t ucap, uint32_t chunk = 64);
 void launch_surface_tension(uint32_t n, const StepConst& k, const SurfConst& c, const StateBufs& s,
                             const ListBufs& l, double4* normals, double4* out, cudaStream_t st);
 // Sets the dynamic shared-memory limit of the list kernel for this stage size
