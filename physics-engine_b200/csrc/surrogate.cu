@@ -611,68 +611,70 @@ void Surrogate::ensure_graph(int n, int E) {
     g_.E = E;
 }
 
-void Surrogate::ensure_acts(bool train) {
-    // Inference keeps one hop's edge activations and no backward buffers: at a
-    // million particles (~3e7 edges) that is ~1.5 KB per edge instead of ~4.6.
+// Buffers of a forward pass: what the fused kernels of inference touch (kActsFused:
+// nodes only), the layers' activations beside them (kActsLayers: ~1.5 KB an edge,
+// one hop's), or those of both hops and the backward pass's (kActsTrain: ~4.6 KB).
+// At 101,376 nodes and 2.56M edges a new network's first forward pass allocated
+// 4.6 GB for the 0.36 it uses: 12.5 ms, 5.6 now.
+void Surrogate::ensure_acts(int level) {
     const int n = g_.n, E = g_.E;
-    if (n <= act_n_ && E <= act_e_ && (act_train_ || !train)) return;
+    if (act_level_ >= level && n <= act_n_ && (level == kActsFused || E <= act_e_)) return;
     cu(cudaStreamSynchronize(st_), "acts");
     for (void* p : act_allocs_) cudaFree(p);
     act_allocs_.clear();
     // grow with a quarter of headroom; a switch to training sizes for the
     // current graph only (training buffers cost ~3x per edge)
-    const bool keep = act_train_ || !train;
+    const bool keep = act_level_ >= level, layers = level >= kActsLayers, train = level >= kActsTrain;
     const int cn = round8(std::max(n + n / 4, keep ? act_n_ : 0));
-    const int ce = round8(std::max(E + E / 4, keep ? act_e_ : 0));
-    auto fa = [&](size_t count) {
+    const int ce = layers ? round8(std::max(E + E / 4, keep ? act_e_ : 0)) : 0;
+    act_n_ = act_e_ = 0;  // until all of them are there
+    act_level_ = -1;
+    auto take = [&](bool wanted, size_t bytes) -> void* {
+        if (!wanted) return nullptr;
         void* p = nullptr;
-        cu(cudaMalloc(&p, std::max<size_t>(count * 4, 256)), "cudaMalloc acts");
+        cu(cudaMalloc(&p, std::max<size_t>(bytes, 256)), "cudaMalloc acts");
         act_allocs_.push_back(p);
-        return static_cast<float*>(p);
+        return p;
     };
-    auto ba = [&](size_t count) {
-        void* p = nullptr;
-        cu(cudaMalloc(&p, std::max<size_t>(count * 2, 256)), "cudaMalloc acts");
-        act_allocs_.push_back(p);
-        return static_cast<__nv_bfloat16*>(p);
-    };
-    const size_t W = kWidth;
-    enc_a1_ = ba(cn * W);
-    enc_a2_ = ba(cn * W);
-    h_ = fa(cn * W);
-    for (auto& p : hb_) p = ba(cn * W);
-    P_ = fa(cn * W);
-    Q_ = fa(cn * W);
+    auto fa = [&](size_t count, bool wanted) { return static_cast<float*>(take(wanted, count * 4)); };
+    auto ba = [&](size_t count, bool wanted) { return static_cast<__nv_bfloat16*>(take(wanted, count * 2)); };
+    const size_t W = kWidth, N = (size_t)cn * W, NE = (size_t)ce * W;
+    h_ = fa(N, true);
+    for (auto& p : hb_) p = ba(N, true);
+    P_ = fa(N, true);
+    Q_ = fa(N, true);
+    A_ = fa(N, true);
+    Y_ = fa((size_t)cn * kOutPad, true);
+    dY_ = fa((size_t)cn * kOutPad, true);  // inference packs its outputs there
+    enc_a1_ = ba(N, layers);
+    enc_a2_ = ba(N, layers);
     for (int l = 0; l < 2; ++l) {
-        eh1_[l] = (l == 0 || train) ? ba(ce * W) : eh1_[0];
-        eh2_[l] = (l == 0 || train) ? ba(ce * W) : eh2_[0];
-        xn_[l] = ba(cn * 2 * W);
-        na1_[l] = ba(cn * W);
-        na2_[l] = ba(cn * W);
+        eh1_[l] = (l == 0 || train) ? ba(NE, layers) : eh1_[0];
+        eh2_[l] = (l == 0 || train) ? ba(NE, layers) : eh2_[0];
+        xn_[l] = ba(2 * N, layers);
+        na1_[l] = ba(N, layers);
+        na2_[l] = ba(N, layers);
     }
-    M_ = fa(ce * W);
-    A_ = fa(cn * W);
-    U_ = fa(cn * W);
-    da1_ = ba(cn * W);
-    da2_ = ba(cn * W);
-    Y_ = fa(cn * kOutPad);
-    dY_ = fa(cn * kOutPad);
-    dH_ = fa(cn * W);
-    dHp_ = fa(cn * W);
-    dXN_ = fa(cn * 2 * W);
-    dE_ = train ? fa(ce * W) : nullptr;
-    dE2_ = train ? fa(ce * W) : nullptr;
-    dP_ = fa(cn * W);
-    dQ_ = fa(cn * W);
-    dT1_ = fa(cn * W);
-    dT2_ = fa(cn * W);
-    const size_t rows = train ? (size_t)std::max(cn, ce) : 0;
-    gb16_ = train ? ba(rows * 2 * W) : nullptr;
-    gbT_ = train ? ba(rows * 2 * W) : nullptr;
-    xT_ = train ? ba(rows * 2 * W) : nullptr;
+    M_ = fa(NE, layers);
+    U_ = fa(N, layers);
+    da1_ = ba(N, layers);
+    da2_ = ba(N, layers);
+    dH_ = fa(N, train);
+    dHp_ = fa(N, train);
+    dXN_ = fa(2 * N, train);
+    dE_ = fa(NE, train);
+    dE2_ = fa(NE, train);
+    dP_ = fa(N, train);
+    dQ_ = fa(N, train);
+    dT1_ = fa(N, train);
+    dT2_ = fa(N, train);
+    const size_t rows = (size_t)std::max(cn, ce);
+    gb16_ = ba(rows * 2 * W, train);
+    gbT_ = ba(rows * 2 * W, train);
+    xT_ = ba(rows * 2 * W, train);
     act_n_ = cn;
     act_e_ = ce;
-    act_train_ = train;
+    act_level_ = level;
 }
 
 // Room for `need` partial sums of the launch that follows.
@@ -715,10 +717,10 @@ void Surrogate::mlp_fwd(int first, const __nv_bfloat16* X, int R, __nv_bfloat16*
 }
 
 void Surrogate::forward(bool keep_for_backward) {
-    ensure_acts(keep_for_backward);
+    const bool fused = fused_edges_ && !keep_for_backward;
+    ensure_acts(keep_for_backward ? kActsTrain : fused ? kActsFused : kActsLayers);
     const int n = g_.n, E = g_.E;
     const size_t nW = (size_t)n * kWidth;
-    const bool fused = fused_edges_ && !keep_for_backward;
     // one fused node MLP: layers first .. first + 2 on x (and the messages)
     auto node_mlp = [&](int first, const __nv_bfloat16* x, const float* msg, const uint8_t* fluid,
                         __nv_bfloat16* hb) {

@@ -112,7 +112,8 @@ class Surrogate {
    private:
     void alloc_params(uint64_t seed);
     void ensure_graph(int n, int E);
-    void ensure_acts(bool train);
+    enum { kActsFused, kActsLayers, kActsTrain };
+    void ensure_acts(int level);
     void order_by_source();
     void scan_counts(int n, int* row);  // exclusive sums of cnt_[0 .. n]
     void refresh_bf16(Linear& L);
@@ -161,7 +162,7 @@ class Surrogate {
     float* target_ = nullptr;         // [n x 4] normalised targets
     // activations (rows: nodes or edges)
     int act_n_ = 0, act_e_ = 0;
-    bool act_train_ = false;
+    int act_level_ = -1;
     __nv_bfloat16 *enc_a1_ = nullptr, *enc_a2_ = nullptr;
     float* h_ = nullptr;                   // latent fp32 [n x 128]
     __nv_bfloat16* hb_[3] = {};            // latent bf16 per level
