@@ -104,8 +104,9 @@ class Surrogate {
     void set_stream(cudaStream_t s) { st_ = s; }
     uint32_t device_error();
     // inference (forward without backward) runs each hop's edge MLP as one
-    // fused kernel (edge_fused.cu) when on; off: the three GEMMs and the
-    // segment sum that training uses
+    // fused kernel (edge_fused.cu), and the encoder, the node MLPs and the decoder
+    // as one each (node_fused.cu), when on; off: the GEMMs, the segment sum and the
+    // elementwise kernels that training uses
     void set_fused_edges(bool on) { fused_edges_ = on; }
     bool fused_edges() const { return fused_edges_; }
 

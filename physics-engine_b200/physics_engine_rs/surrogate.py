@@ -116,8 +116,9 @@ class Surrogate:
         return y
 
     def set_fused_edges(self, on: bool):
-        """Inference's edge MLP as one fused kernel (True, the default) or as
-        the GEMMs and segment sum that training uses (False)."""
+        """Inference's edge MLPs, encoder, node MLPs and decoder as one fused
+        kernel each (True, the default), or as the GEMMs, segment sum and
+        elementwise kernels that training uses (False)."""
         _ok(self._L.pe_surrogate_set_fused_edges(self._s, 1 if on else 0), "set_fused_edges")
 
     def train_step(self, lr: float = 0.0) -> float:
