@@ -581,9 +581,12 @@ void Surrogate::ensure_graph(int n, int E) {
     for (void* p : graph_allocs_) cudaFree(p);
     graph_allocs_.clear();
     if (scan_tmp_) cudaFree(scan_tmp_);
+    scan_tmp_ = nullptr;
+    scan_bytes_ = 0;
     // grow with a quarter of headroom: the edge count creeps up step by step as
     // the fluid compresses, and every growth reallocates
     const int cn = std::max(n + n / 4, g_.cap_n), ce = std::max(E + E / 4, g_.cap_e);
+    g_.cap_n = g_.cap_e = 0;  // until all of them are there
     auto ga = [&](size_t bytes) {
         void* p = nullptr;
         cu(cudaMalloc(&p, std::max<size_t>(bytes, 256)), "cudaMalloc graph");
@@ -603,8 +606,6 @@ void Surrogate::ensure_graph(int n, int E) {
     target_ = static_cast<float*>(ga((size_t)cn * kOut * 4));
     raw_t_ = static_cast<float*>(ga((size_t)cn * kOut * 4));
     cnt_ = static_cast<int*>(ga((size_t)(cn + 1) * 4));
-    scan_tmp_ = nullptr;
-    scan_bytes_ = 0;
     g_.cap_n = cn;
     g_.cap_e = ce;
     g_.n = n;
