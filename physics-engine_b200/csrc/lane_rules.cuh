@@ -53,6 +53,8 @@ inline uint32_t fit_lanes(uint32_t lanes, uint64_t slots, uint64_t most, bool fe
 //   46,656     101/85/79/86/102   248/168/161/165/192 96/109/103/108/153  53/29/21/21/26 (74,766)
 //   125,000    219/203/190        445/357/382         197/229/222         58/33/31 (176,472)
 //   151,686    228/-/230          488/-/459           205/-/267           61/-/33 (210,648)
+//     (Wendland) 255/233/236      627/515/549         208/258/272
+//   166,375    230/-/254          512/-/504           210/-/296           61/-/35 (229,377)
 //   185,193    236/269/272        578/507/549         212/297/317         61/37/36 (252,227)
 //   512,000    579/732/736        1344/1319/1468      507/793/841         74/63/67
 //   681,472    768/954/968        1658/1732/1948      670/1026/1099       79/74/81 (840,094)
@@ -71,7 +73,7 @@ inline PassLanes pass_lanes(int dim, uint64_t fluid, uint64_t slots) {
     const bool d3 = dim == 3;
     const uint64_t most = 48000000;
     PassLanes r;
-    r.density = fit_lanes(pick(fluid, d3 ? Limits{3000, 10000, 150000, 150000} : Limits{600, 10000, 40000, 100000}), slots, most);
+    r.density = fit_lanes(pick(fluid, d3 ? Limits{3000, 10000, 158000, 158000} : Limits{600, 10000, 40000, 100000}), slots, most);
     r.forces = fit_lanes(pick(fluid, d3 ? Limits{8000, 20000, 64000, 600000} : Limits{1000, 3000, 12000, 80000}), slots, most);
     r.xsph = fit_lanes(pick(fluid, d3 ? Limits{1500, 10000, 45000, 45000} : Limits{1000, 3000, 12000, 25000}), slots, most);
     r.boundary = fluid == slots ? 1u : fit_lanes(32u, slots, d3 ? 16000000 : 4000000);
